@@ -95,7 +95,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     DenseSmemTail *tail = reinterpret_cast<DenseSmemTail *>(smem_aligned + kDStages * kDStageBytes);
     volatile uint32_t *abort_flag = &tail->abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_id_uniform();
     const int lane = threadIdx.x & 31;
     const int tiles_m = static_cast<int>((p.M + kDM - 1) / kDM);
     const int tiles_n = static_cast<int>((p.N + kDN - 1) / kDN);
@@ -123,7 +123,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tail->tmem_base;
+    const uint32_t tmem_base = warp_uniform(tail->tmem_base);
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------

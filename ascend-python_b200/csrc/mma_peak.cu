@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(128, 1) int8_mma_peak_kernel(int batches, long
     __shared__ uint64_t bar;
     __shared__ uint32_t tbase, abort_flag;
     const uint32_t sb = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_id_uniform(), lane = threadIdx.x & 31;
     // any bit pattern is a valid int8 operand; fill with a fixed non-trivial one (data toggling costs power)
     uint32_t *w = reinterpret_cast<uint32_t *>(smem_raw + (sb - smem_u32(smem_raw)));
     for (uint32_t i = threadIdx.x; i < (16384 + 32768) / 4; i += blockDim.x) w[i] = 0x9e3779b9u * (i + 1u);

@@ -14,7 +14,7 @@ w4a16_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     GSmemTail *tail = reinterpret_cast<GSmemTail *>(smem_aligned + nstages * kGStageBytes);
     volatile uint32_t *abort_flag = &tail->abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_id_uniform();
     const int lane = threadIdx.x & 31;
     const int64_t total = static_cast<int64_t>(p.units_n) * p.ngroups;
     const int64_t G = gridDim.x;

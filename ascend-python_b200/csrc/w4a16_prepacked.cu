@@ -157,7 +157,7 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
     PSmemTail *tail = reinterpret_cast<PSmemTail *>(smem_aligned + w_off + nstages * kPStageWBytes);
     volatile uint32_t *abort_flag = &tail->abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_id_uniform();
     const int lane = threadIdx.x & 31;
     const int64_t total = static_cast<int64_t>(p.tiles_n) * p.nchunks;
     const int64_t G = gridDim.x;
@@ -194,7 +194,7 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tail->tmem_base;
+    const uint32_t tmem_base = warp_uniform(tail->tmem_base);
 
     if (warp == 0) {
         // ---------------- weight producer: one bulk copy of 17408 contiguous bytes per stage ----------------

@@ -18,7 +18,7 @@ w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     float *xs_smem = reinterpret_cast<float *>(tail + 1);  // [ngroups][mpad] when p.xs_in_smem
     volatile uint32_t *abort_flag = &tail->abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_id_uniform();
     const int lane = threadIdx.x & 31;
     const int64_t total = static_cast<int64_t>(p.units_n) * p.ngroups;
     const int64_t G = gridDim.x;
@@ -60,7 +60,7 @@ w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tail->tmem_base;
+    const uint32_t tmem_base = warp_uniform(tail->tmem_base);
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------

@@ -91,7 +91,7 @@ w8a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     TileSmemTail *tail = reinterpret_cast<TileSmemTail *>(epi_cols + kEpiWarps * kEpiColFloats);
     volatile uint32_t *abort_flag = &tail->abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_id_uniform();
     const int lane = threadIdx.x & 31;
     const int tiles_m = static_cast<int>((ep.M + kBM - 1) / kBM);
     const int tiles_n = static_cast<int>((ep.N + kBN - 1) / kBN);
@@ -123,7 +123,7 @@ w8a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tail->tmem_base;
+    const uint32_t tmem_base = warp_uniform(tail->tmem_base);
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------

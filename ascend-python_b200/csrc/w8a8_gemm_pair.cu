@@ -155,7 +155,7 @@ w8a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         return;
     }
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_id_uniform();
     const int lane = threadIdx.x & 31;
     const int tiles_m = static_cast<int>((ep.M + 2 * kPM - 1) / (2 * kPM));
     const int tiles_n = static_cast<int>((ep.N + kPN - 1) / kPN);
@@ -205,7 +205,7 @@ w8a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     __syncthreads();
     cluster_sync_all();  // the peer's barriers are initialised before anything signals them
     tc_fence_after();
-    const uint32_t tmem_base = tail->tmem_base;
+    const uint32_t tmem_base = warp_uniform(tail->tmem_base);
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------

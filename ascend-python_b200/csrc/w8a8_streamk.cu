@@ -70,7 +70,7 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     SkSmemTail *tail = reinterpret_cast<SkSmemTail *>(smem_aligned + p.stages * p.stage_bytes);
     volatile uint32_t *abort_flag = &tail->abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_id_uniform();
     const int lane = threadIdx.x & 31;
 
     // this CTA's contiguous range of (tile, k-block) units
@@ -103,7 +103,7 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tail->tmem_base;
+    const uint32_t tmem_base = warp_uniform(tail->tmem_base);
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
