@@ -35,6 +35,8 @@ template <typename T, int VPT>
 __global__ void __launch_bounds__(512)
 dynamic_quant_vec_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_x, int8_t *__restrict__ q,
                          int64_t ld_q, float *__restrict__ scale, int tpr) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float s_part[16];
     const int tpr_shift = __ffs(tpr) - 1;  // tpr is a power of two
     const int rows_per_cta = blockDim.x >> tpr_shift;
@@ -90,6 +92,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 dynamic_quant_generic_kernel(const T *__restrict__ x, int64_t rows, int64_t cols, int64_t ld_x,
                              int8_t *__restrict__ q, int64_t ld_q, float *__restrict__ scale) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float s_part[8];
     const int64_t row = blockIdx.x;
     if (row >= rows) return;
@@ -126,24 +130,16 @@ int launch_dynamic_quant(const T *x, int64_t rows, int64_t cols, int64_t ld_x, i
         const int rows_per_cta = threads / tpr;
         const int64_t grid = (rows + rows_per_cta - 1) / rows_per_cta;
         const int icols = static_cast<int>(cols);
-        switch (vpt) {
-            case 1:
-                dynamic_quant_vec_kernel<T, 1><<<grid, threads, 0, stream>>>(x, rows, icols, ld_x, q, ld_q, scale, tpr);
-                break;
-            case 2:
-                dynamic_quant_vec_kernel<T, 2><<<grid, threads, 0, stream>>>(x, rows, icols, ld_x, q, ld_q, scale, tpr);
-                break;
-            case 4:
-                dynamic_quant_vec_kernel<T, 4><<<grid, threads, 0, stream>>>(x, rows, icols, ld_x, q, ld_q, scale, tpr);
-                break;
-            default:
-                dynamic_quant_vec_kernel<T, 8><<<grid, threads, 0, stream>>>(x, rows, icols, ld_x, q, ld_q, scale, tpr);
-                break;
-        }
+        auto kern = vpt == 1   ? dynamic_quant_vec_kernel<T, 1>
+                    : vpt == 2 ? dynamic_quant_vec_kernel<T, 2>
+                    : vpt == 4 ? dynamic_quant_vec_kernel<T, 4>
+                               : dynamic_quant_vec_kernel<T, 8>;
+        QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(static_cast<unsigned>(threads)), 0, stream, x, rows,
+                               icols, ld_x, q, ld_q, scale, tpr));
     } else {
-        dynamic_quant_generic_kernel<T><<<rows, 256, 0, stream>>>(x, rows, cols, ld_x, q, ld_q, scale);
+        QMM_CUDA_OK(launch_pdl(dynamic_quant_generic_kernel<T>, dim3(static_cast<unsigned>(rows)), dim3(256), 0, stream, x, rows,
+                               cols, ld_x, q, ld_q, scale));
     }
-    QMM_CUDA_OK(cudaGetLastError());
     return QMM_OK;
 }
 

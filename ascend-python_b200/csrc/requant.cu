@@ -36,6 +36,8 @@ __global__ void __launch_bounds__(256)
 requant_vec16_kernel(const int32_t *__restrict__ acc, int64_t M, int64_t N, const float *__restrict__ scale,
                      int scale_scalar, const float *__restrict__ pertoken, const float *__restrict__ offset,
                      int offset_scalar, int8_t *__restrict__ out, int64_t ld_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int64_t n = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 16;
     if (n >= N) return;
     const bool has_pt = pertoken != nullptr, has_off = offset != nullptr;
@@ -77,6 +79,8 @@ __global__ void __launch_bounds__(256)
 requant_kernel(const int32_t *__restrict__ acc, int64_t M, int64_t N, const float *__restrict__ scale, int scale_scalar,
                const float *__restrict__ pertoken, const float *__restrict__ offset, int offset_scalar,
                int8_t *__restrict__ out, int64_t ld_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     const bool vec = (N & 3) == 0 && (ld_out & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0;
     const bool has_pt = pertoken != nullptr, has_off = offset != nullptr;
     if (vec) {
@@ -161,18 +165,16 @@ extern "C" int qmm_quant_matmul_int8(const int8_t *x1, int64_t ld_x1, const int8
         if (gy > M) gy = M;
         if (gy > 65535) gy = 65535;
         if (gy < 1) gy = 1;
-        requant_vec16_kernel<<<dim3(gx, static_cast<unsigned>(gy)), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-            acc, M, N, scale, scale_scalar, pertoken_scale, offset, offset_scalar, out, ld_out);
-        QMM_CUDA_OK(cudaGetLastError());
+        QMM_CUDA_OK(launch_pdl(requant_vec16_kernel, dim3(gx, static_cast<unsigned>(gy)), dim3(256), 0,
+                               static_cast<cudaStream_t>(stream), acc, M, N, scale, scale_scalar, pertoken_scale, offset,
+                               offset_scalar, out, ld_out));
         return QMM_OK;
     }
     const int64_t items = ((N & 3) == 0) ? M * (N >> 2) : M * N;
     int64_t grid = (items + 255) / 256;
     const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
     if (grid > cap) grid = cap;
-    requant_kernel<<<static_cast<unsigned>(grid), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        acc, M, N, scale, (scale_len == 1 && N != 1) ? 1 : 0, pertoken_scale, offset, (offset_len == 1 && N != 1) ? 1 : 0,
-        out, ld_out);
-    QMM_CUDA_OK(cudaGetLastError());
+    QMM_CUDA_OK(launch_pdl(requant_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, static_cast<cudaStream_t>(stream), acc,
+                           M, N, scale, scale_scalar, pertoken_scale, offset, offset_scalar, out, ld_out));
     return QMM_OK;
 }

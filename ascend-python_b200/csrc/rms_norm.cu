@@ -85,6 +85,8 @@ __global__ void __launch_bounds__(512)
 rms_norm_vec_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_x, const T *__restrict__ gamma,
                     float eps, T *__restrict__ y, int64_t ld_y, int8_t *__restrict__ q, int64_t ld_q,
                     float *__restrict__ scale, float *__restrict__ rstd_out, int tpr) {
+    pdl_launch_dependents();
+    pdl_wait();
     constexpr int E = VecOf<T>::kElems;
     __shared__ float s_part[2][16];
     const int tpr_shift = __ffs(tpr) - 1;  // tpr is a power of two
@@ -182,6 +184,8 @@ __global__ void __launch_bounds__(256)
 rms_norm_generic_kernel(const T *__restrict__ x, int64_t rows, int64_t cols, int64_t ld_x, const T *__restrict__ gamma,
                         float eps, T *__restrict__ y, int64_t ld_y, int8_t *__restrict__ q, int64_t ld_q,
                         float *__restrict__ scale, float *__restrict__ rstd_out) {
+    pdl_launch_dependents();
+    pdl_wait();
     __shared__ float s_part[8];
     __shared__ float s_bcast;
     const int64_t row = blockIdx.x;
@@ -245,21 +249,16 @@ int launch_rms_norm(const T *x, int64_t rows, int64_t cols, int64_t ld_x, const 
         const int rows_per_cta = threads / tpr;
         const int64_t grid = (rows + rows_per_cta - 1) / rows_per_cta;
         const int icols = static_cast<int>(cols);
-#define QMM_RMS_LAUNCH(V)                                                                                        \
-    rms_norm_vec_kernel<T, V, QUANT><<<grid, threads, 0, stream>>>(x, rows, icols, ld_x, gamma, eps, y, ld_y, q, ld_q, \
-                                                                   scale, rstd, tpr)
-        switch (vpt) {
-            case 1: QMM_RMS_LAUNCH(1); break;
-            case 2: QMM_RMS_LAUNCH(2); break;
-            case 4: QMM_RMS_LAUNCH(4); break;
-            default: QMM_RMS_LAUNCH(8); break;
-        }
-#undef QMM_RMS_LAUNCH
+        auto kern = vpt == 1   ? rms_norm_vec_kernel<T, 1, QUANT>
+                    : vpt == 2 ? rms_norm_vec_kernel<T, 2, QUANT>
+                    : vpt == 4 ? rms_norm_vec_kernel<T, 4, QUANT>
+                               : rms_norm_vec_kernel<T, 8, QUANT>;
+        QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(static_cast<unsigned>(threads)), 0, stream, x, rows,
+                               icols, ld_x, gamma, eps, y, ld_y, q, ld_q, scale, rstd, tpr));
     } else {
-        rms_norm_generic_kernel<T, QUANT><<<rows, 256, 0, stream>>>(x, rows, cols, ld_x, gamma, eps, y, ld_y, q, ld_q,
-                                                                    scale, rstd);
+        QMM_CUDA_OK(launch_pdl(rms_norm_generic_kernel<T, QUANT>, dim3(static_cast<unsigned>(rows)), dim3(256), 0, stream, x,
+                               rows, cols, ld_x, gamma, eps, y, ld_y, q, ld_q, scale, rstd));
     }
-    QMM_CUDA_OK(cudaGetLastError());
     return QMM_OK;
 }
 

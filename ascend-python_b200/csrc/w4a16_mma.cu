@@ -236,8 +236,7 @@ int launch_w4a16_mma_t(const W4Params &w, void *workspace, cudaStream_t stream) 
             kern = w4a16_mma_kernel<T, 2, 2, false>;
     }
     QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    kern<<<pl.grid, (1 + pl.sets * kGColWarps) * 32, smem, stream>>>(tw, tx, p);
-    QMM_CUDA_OK(cudaGetLastError());
+    QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(pl.grid)), dim3((1 + pl.sets * kGColWarps) * 32), smem, stream, tw, tx, p));
     return QMM_OK;
 }
 

@@ -34,6 +34,8 @@ w4a16_mma_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         tma_prefetch_desc(&tmap_w);
         tma_prefetch_desc(&tmap_x);
     }
+    pdl_launch_dependents();
+    pdl_wait();
     __syncthreads();
 
     if (warp == 0) {

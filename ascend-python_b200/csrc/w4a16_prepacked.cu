@@ -191,6 +191,8 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
         tmem_alloc(smem_u32(&tail->tmem_base), kPTmemCols);
         tmem_relinquish();
     }
+    pdl_launch_dependents();
+    pdl_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -603,6 +605,7 @@ __device__ __forceinline__ uint4 ldg_stream(const uint8_t *p) {
 template <typename T, int M>
 __global__ void __launch_bounds__(kGvThreads, kGvCtasPerSm)
 w4a16_gemv_kernel(GvParams p) {
+    pdl_launch_dependents();
     extern __shared__ uint4 gv_smem[];  // digits of a run of blocks [nb][M][2][8], then esc [nb][M], xs [nb][M]
     __shared__ uint32_t s_is_last;
     const int r = threadIdx.x;
@@ -636,7 +639,7 @@ w4a16_gemv_kernel(GvParams p) {
         // the digits come from the kernel launched just before this one (programmatic dependent launch: this
         // kernel may start while that one still runs)
         if (!waited) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");
+            pdl_wait();
             waited = true;
         }
         __syncthreads();  // the previous segment's digits are no longer read
@@ -758,7 +761,8 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 w4a16_gemv_digits_kernel(const T *__restrict__ x, int64_t ld_x, int M, int64_t K, int nblocks, int8_t *__restrict__ xd,
                          float *__restrict__ esc, float *__restrict__ xs) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the matmul may start its weight loads
+    pdl_wait();
+    pdl_launch_dependents();  // not before the wait: the matmul reads its first weights without waiting for this kernel
     const int lane = threadIdx.x & 31;
     const int blk = blockIdx.x * 4 + (threadIdx.x >> 5), m = blockIdx.y;
     if (blk >= nblocks) return;
@@ -863,9 +867,8 @@ int launch_gemv_t(const uint8_t *packed, const void *x, int64_t ld_x, const void
     int8_t *xd = reinterpret_cast<int8_t *>(ws + kPCounterBytes + pl.slots_bytes);
     float *esc = reinterpret_cast<float *>(ws + kPCounterBytes + pl.slots_bytes + pl.xd_bytes);
     float *xs = reinterpret_cast<float *>(ws + kPCounterBytes + pl.slots_bytes + pl.xd_bytes + pl.tab_bytes);
-    w4a16_gemv_digits_kernel<T><<<dim3(static_cast<unsigned>((pl.nblocks + 3) / 4), static_cast<unsigned>(M)), 128, 0,
-                                  stream>>>(static_cast<const T *>(x), ld_x, static_cast<int>(M), K, pl.nblocks, xd, esc, xs);
-    QMM_CUDA_OK(cudaGetLastError());
+    QMM_CUDA_OK(launch_pdl(w4a16_gemv_digits_kernel<T>, dim3(static_cast<unsigned>((pl.nblocks + 3) / 4), static_cast<unsigned>(M)),
+                           dim3(128), 0, stream, static_cast<const T *>(x), ld_x, static_cast<int>(M), K, pl.nblocks, xd, esc, xs));
     GvParams p;
     p.packed = packed;
     p.bias = bias;
@@ -884,20 +887,10 @@ int launch_gemv_t(const uint8_t *packed, const void *x, int64_t ld_x, const void
     // programmatic dependent launch: the kernel starts (and requests its first weights) while the digits
     // kernel still runs, and waits for it (griddepcontrol.wait) before it reads the digits
     const size_t smem = static_cast<size_t>(pl.max_run) * M * (256 + 8);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(pl.grid));
-    cfg.blockDim = dim3(kGvThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     auto launch = [&](auto kern) -> int {
         if (smem > 48 * 1024)
             QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        QMM_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, p));
+        QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(pl.grid)), dim3(kGvThreads), smem, stream, p));
         return QMM_OK;
     };
     switch (M) {
@@ -940,8 +933,7 @@ int launch_prepacked_t(const uint8_t *packed, const void *x, int64_t ld_x, const
                         static_cast<size_t>(pl.nstages) * kPStageWBytes + 1024;
     auto kern = w4a16_prepacked_kernel<T>;
     QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    kern<<<pl.grid, kPThreads, smem, stream>>>(tx, p);
-    QMM_CUDA_OK(cudaGetLastError());
+    QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(pl.grid)), dim3(kPThreads), smem, stream, tx, p));
     return QMM_OK;
 }
 

@@ -201,6 +201,8 @@ w8a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         tmem_alloc_pair(smem_u32(&tail->tmem_base), kPTmemCols);
         tmem_relinquish_pair();
     }
+    if constexpr (!FUSED) pdl_launch_dependents();
+    pdl_wait();
     tc_fence_before();
     __syncthreads();
     cluster_sync_all();  // the peer's barriers are initialised before anything signals them
@@ -406,13 +408,15 @@ int launch_pair_t(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_
     cfg.blockDim = dim3(kPThreads);
     cfg.dynamicSmemBytes = kPairSmemBytes;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = opts == nullptr ? 2 : 1;  // a matmul that talks to other GPUs starts on an idle GPU, as before
     int raster = pair_choose_raster(ep.M, ep.N, K, static_cast<int64_t>(sizeof(OutT)), pairs);
     PushMaps push;
     memset(&push, 0, sizeof(push));

@@ -100,6 +100,8 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         tmem_alloc(smem_u32(&tail->tmem_base), kSkTmemCols);
         tmem_relinquish();
     }
+    pdl_launch_dependents();
+    pdl_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -383,8 +385,7 @@ static int launch_streamk_t(const int8_t *x1, int64_t ld_x1, const int8_t *x2, i
     auto kern = mn_major ? w8a8_streamk_kernel<OutT, true> : w8a8_streamk_kernel<OutT, false>;
     QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(kSkSmemBudget)));
-    kern<<<grid, kSkThreads, smem, stream>>>(tw, tx, p);
-    QMM_CUDA_OK(cudaGetLastError());
+    QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(kSkThreads), smem, stream, tw, tx, p));
     return QMM_OK;
 }
 
