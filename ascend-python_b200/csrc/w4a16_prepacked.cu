@@ -58,7 +58,8 @@ constexpr int kPSubs = kPChunkK / kPSubK;             // 4
 constexpr int kPWBytes = kPTileN * kPChunkK / 2;      // 8192
 constexpr int kPSOBytes = 2 * kPTileN * 2;            // 512: scale, offset * scale
 constexpr int kPBlockBytes = kPWBytes + kPSOBytes;    // 8704
-constexpr int kPMaxM = 64;                            // token rows per launch
+constexpr int kPMaxM = 64;                            // token rows of the narrow form
+constexpr int kPMaxWide = 256;                        // token rows of a tile of the wide form
 constexpr int kPPair = 2;                             // blocks per stage
 constexpr int kPStageK = kPPair * kPChunkK;           // 256 k rows per stage
 constexpr int kPStageWBytes = kPPair * kPBlockBytes;  // 17408 bytes of packed weights per stage
@@ -69,25 +70,38 @@ constexpr int kPMmaWarp = 2;
 constexpr int kPFirstUnpackWarp = 3;
 constexpr int kPFirstEpiWarp = kPFirstUnpackWarp + kPUnpackWarps;
 constexpr int kPThreads = (kPFirstEpiWarp + kPEpiWarps) * 32;  // 736
-constexpr int kPRing = 3;                             // stages of the operand ring in tensor memory
+constexpr int kPMaxRing = 3;
 constexpr int kPMaxXStages = 8;                       // activation tiles in shared memory
 constexpr uint32_t kPRingCols = kPStageK / 2;         // 128 columns per stage: two 16-bit k per column
-constexpr uint32_t kPDBufs = 2;
-constexpr uint32_t kPACol0 = kPDBufs * kPMaxM;        // accumulators in columns [0, 128), the ring behind: [128, 512)
+constexpr uint32_t kPMaxDBufs = 2;
+// Two forms of the kernel.  Narrow (up to 64 token rows, weight-bandwidth bound): two accumulators in columns
+// [0, 128), three stages of the operand ring behind, activation stages of 256 k.  Wide (more rows, bound by the MMAs,
+// 8 * rows clocks per 256-k stage, from about 140 rows on; by the unpack warps below that): one accumulator of up to
+// 256 columns, two ring stages, activation stages of 64 k, since a tile of 256 rows x 256 k alone is 128 KiB.
+template <bool WIDE>
+struct PForm {
+    static constexpr int kTok = WIDE ? kPMaxWide : kPMaxM;
+    static constexpr uint32_t kDBufs = WIDE ? 1 : 2;
+    static constexpr uint32_t kACol0 = kDBufs * kTok;
+    static constexpr int kRing = WIDE ? 2 : 3;
+    static constexpr int kXBoxes = WIDE ? 1 : 4;      // boxes of 64 k per activation stage
+    static_assert(kACol0 + kRing * kPRingCols <= 512, "tensor memory");
+};
 constexpr uint32_t kPTmemCols = 512;
 constexpr int kPMaxStages = 8;
 constexpr size_t kPCounterBytes = 64 * 1024;          // tile counters: a fixed area at the start of the scratch
-constexpr size_t kPSmemBudget = 200 * 1024;
+constexpr size_t kPSmemBudget = 200 * 1024, kPSmemBudgetWide = 220 * 1024;
+constexpr int kPWideStages = 4;                       // packed-weight stages of the wide form
 
 struct PSmemTail {
     uint64_t w_full[kPMaxStages];   // packed weights of a stage have landed
     uint64_t w_empty[kPMaxStages];  // ... and have been read into registers by all unpack warps
     uint64_t x_full[kPMaxXStages];  // activation tile of a stage has landed
     uint64_t x_empty[kPMaxXStages]; // ... and the MMAs that read it are complete
-    uint64_t a_full[kPRing];        // operand columns of a ring slot are written (16 unpack warps)
-    uint64_t mma_done[kPRing];      // the MMAs of a ring slot are complete: its columns are free
-    uint64_t tmem_full[kPDBufs];
-    uint64_t tmem_empty[kPDBufs];
+    uint64_t a_full[kPMaxRing];        // operand columns of a ring slot are written (16 unpack warps)
+    uint64_t mma_done[kPMaxRing];      // the MMAs of a ring slot are complete: its columns are free
+    uint64_t tmem_full[kPMaxDBufs];
+    uint64_t tmem_empty[kPMaxDBufs];
     uint32_t tmem_base;
     uint32_t abort_flag;
     uint32_t is_last;
@@ -100,21 +114,55 @@ struct PParams {
     void *out;
     int64_t ld_out;
     int M, N;
-    int mpad;         // M rounded up to 16
+    int mpad;         // token rows of a tile, a multiple of 16
+    int nblk;         // tiles of token rows; an output tile is q = column tile * nblk + row tile
+    int share, extra, grain;  // see p_first_item; grain = nchunks: whole output tiles, 1: equal shares of the block pairs
+    int out_vec;      // rows of out meet the alignment of 8-byte stores
     int x_box_bytes;  // mpad * 128: one [mpad][64 k] activation box
     int nstages;      // packed-weight stages in shared memory
     int nxstages;     // activation tiles in shared memory
     int tiles_n;
     int nchunks;      // block PAIRS along K
     int max_slots;
-    float *slots;        // [tiles_n][max_slots][mpad][128]
-    uint32_t *counters;  // [tiles_n], zero between calls
+    float *slots;        // [output tiles][max_slots][mpad][128]
+    uint32_t *counters;  // [output tiles], zero between calls
     uint32_t *status;
 };
 
 __device__ __forceinline__ int p_cta_of_item(int64_t u, int64_t total, int64_t G) {
     return static_cast<int>((u * G + G - 1) / total);
 }
+
+// Four K=16 MMAs (64 k, one activation box) under one election; see mma_f16_ts_warp_x8.
+__device__ __forceinline__ void p_mma_x4(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
+                                         uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, e, t;\n\t"
+        ".reg .b64 bd;\n\t"
+        ".reg .b32 a, bl;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "setp.eq.b32 t, 0, 0;\n\t"
+        "mov.b64 bd, {%2, %3};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t"
+        "add.u32 a, %1, 8;\n\t"
+        "add.u32 bl, %2, 2;\n\t"
+        "mov.b64 bd, {bl, %3};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %4, t;\n\t"
+        "add.u32 a, %1, 16;\n\t"
+        "add.u32 bl, %2, 4;\n\t"
+        "mov.b64 bd, {bl, %3};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %4, t;\n\t"
+        "add.u32 a, %1, 24;\n\t"
+        "add.u32 bl, %2, 6;\n\t"
+        "mov.b64 bd, {bl, %3};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a], bd, %4, t;\n\t"
+        "}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 __device__ __forceinline__ void pepi_bar_sync() { asm volatile("bar.sync 3, 128;" ::: "memory"); }
 
 // (a & b) ^ c in one logic instruction
@@ -142,16 +190,110 @@ struct PMagic<__half> {
     static __device__ __forceinline__ T2 bias2() { return __floats2half2_rn(1032.0f, 1032.0f); }
 };
 
+// Items are dealt out in contiguous ranges of p.share, or one more for the first p.extra CTAs, times p.grain.
+__device__ __forceinline__ int p_first_item(const PParams &p, int cta) { return (cta * p.share + min(cta, p.extra)) * p.grain; }
+__device__ __forceinline__ int p_cta_of(const PParams &p, int item) {
+    const int i = item / p.grain, edge = p.extra * (p.share + 1);
+    return i < edge ? i / (p.share + 1) : p.extra + (i - edge) / p.share;
+}
+// CTAs whose ranges overlap output tile q
+__device__ __forceinline__ int p_slot_count(const PParams &p, int q) {
+    return p_cta_of(p, q * p.nchunks + p.nchunks - 1) - p_cta_of(p, q * p.nchunks) + 1;
+}
+
+// Adds the slots of tile q in slot order and stores the tile; thread `tid` of `threads`.
 template <typename T>
+__device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots, int tid, int threads) {
+    const T *bias = static_cast<const T *>(p.bias);
+    const int m0 = (q % p.nblk) * p.mpad, ncol0 = (q / p.nblk) * kPTileN;
+    const int vecs = min(p.mpad, p.M - m0) * (kPTileN / 4);
+    const int64_t slot_vecs = static_cast<int64_t>(p.mpad) * (kPTileN / 4);
+    const float4 *src = reinterpret_cast<const float4 *>(p.slots) + static_cast<int64_t>(q) * p.max_slots * slot_vecs;
+    constexpr int kElems = 2;
+    for (int e0 = tid; e0 < vecs; e0 += kElems * threads) {
+        float4 v[kElems];
+#pragma unroll
+        for (int e = 0; e < kElems; ++e) v[e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int s0 = 0; s0 < nslots; s0 += 4) {
+            float4 part[4][kElems];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int e = 0; e < kElems; ++e) {
+                    part[k][e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (s0 + k < nslots && e0 + e * threads < vecs) part[k][e] = __ldcg(src + (s0 + k) * slot_vecs + e0 + e * threads);
+                }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int e = 0; e < kElems; ++e) {
+                    v[e].x += part[k][e].x;
+                    v[e].y += part[k][e].y;
+                    v[e].z += part[k][e].z;
+                    v[e].w += part[k][e].w;
+                }
+        }
+#pragma unroll
+        for (int e = 0; e < kElems; ++e) {
+            const int idx = e0 + e * threads;
+            const int n = ncol0 + (idx % (kPTileN / 4)) * 4;
+            if (idx >= vecs || n >= p.N) continue;  // N is a multiple of eight
+            float f[4] = {v[e].x, v[e].y, v[e].z, v[e].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) f[k] += bias != nullptr ? to_float(bias[n + k]) : 0.0f;
+            T *o = static_cast<T *>(p.out) + static_cast<int64_t>(m0 + idx / (kPTileN / 4)) * p.ld_out + n;
+            if (p.out_vec) {
+                *reinterpret_cast<uint2 *>(o) = make_uint2(pack2<T>(f[0], f[1]), pack2<T>(f[2], f[3]));
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) o[k] = from_float<T>(f[k]);
+            }
+        }
+    }
+}
+
+// The calling threads have stored this CTA's sums of tile q: reports that, and if it completes the tile adds the slots
+// and stores the tile.  EPILOGUE: the four epilogue warps call, otherwise the whole CTA.  Inlined, and the parameters by
+// value: a call with their address costs the whole kernel its uniform registers (34 -> 43 us for 16 tokens).
+template <typename T, bool EPILOGUE>
+__device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatile uint32_t *abort_flag, uint32_t *flag) {
+    auto barrier = [] {
+        if (EPILOGUE)
+            pepi_bar_sync();
+        else
+            __syncthreads();
+    };
+    const int nslots = p_slot_count(p, q);
+    if (nslots <= 1) return;
+    const int tid = static_cast<int>(threadIdx.x) - (EPILOGUE ? kPFirstEpiWarp * 32 : 0);
+    barrier();
+    if (tid == 0) {
+        uint32_t last = 0;
+        if (*abort_flag == 0) {  // a CTA that was cut short never completes a tile
+            uint32_t old;
+            // release: cumulative over the CTA's slot stores, which the barrier has ordered; acquire: the others'
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(p.counters + q) : "memory");
+            last = old + 1 == static_cast<uint32_t>(nslots) ? 1u : 0u;
+            if (last) p.counters[q] = 0;
+        }
+        *flag = last;
+    }
+    barrier();
+    if (*reinterpret_cast<volatile uint32_t *>(flag) != 0) p_add_slots<T>(p, q, nslots, tid, EPILOGUE ? kPEpiWarps * 32 : kPThreads);
+    barrier();  // the flag is written again for the next tile
+}
+
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(kPThreads, 1)
 w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
     using T2 = typename PMagic<T>::T2;
+    using F = PForm<WIDE>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
     const uint32_t nstages = static_cast<uint32_t>(p.nstages);
     const uint32_t x_box = static_cast<uint32_t>(p.x_box_bytes);
-    const uint32_t x_slot = 4u * x_box;           // [mpad][256 k] as four boxes
+    const uint32_t x_slot = F::kXBoxes * x_box;   // an activation stage: boxes of [mpad][64 k]
     const uint32_t nxstages = static_cast<uint32_t>(p.nxstages);
     const uint32_t w_off = nxstages * x_slot;     // the packed-weight stages sit behind the activation tiles
     PSmemTail *tail = reinterpret_cast<PSmemTail *>(smem_aligned + w_off + nstages * kPStageWBytes);
@@ -159,10 +301,9 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
 
     const int warp = warp_id_uniform();
     const int lane = threadIdx.x & 31;
-    const int64_t total = static_cast<int64_t>(p.tiles_n) * p.nchunks;
-    const int64_t G = gridDim.x;
-    const int64_t u_begin = total * blockIdx.x / G;
-    const int64_t u_end = total * (blockIdx.x + 1) / G;
+    // this CTA's contiguous range of (output tile, block pair) items
+    const int cta = static_cast<int>(blockIdx.x);
+    const int u_begin = p_first_item(p, cta), u_end = p_first_item(p, cta + 1);
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < nstages; ++s) {
@@ -173,16 +314,15 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
             mbar_init(smem_u32(&tail->x_full[a]), 1);
             mbar_init(smem_u32(&tail->x_empty[a]), 1);
         }
-        for (int a = 0; a < kPRing; ++a) {
+        for (int a = 0; a < F::kRing; ++a) {
             mbar_init(smem_u32(&tail->a_full[a]), kPUnpackWarps);
             mbar_init(smem_u32(&tail->mma_done[a]), 1);
         }
-        for (uint32_t b = 0; b < kPDBufs; ++b) {
+        for (uint32_t b = 0; b < F::kDBufs; ++b) {
             mbar_init(smem_u32(&tail->tmem_full[b]), 1);
             mbar_init(smem_u32(&tail->tmem_empty[b]), kPEpiWarps);
         }
         tail->abort_flag = 0;
-        tail->is_last = 0;
         tail->epi_abort = 0;
         mbar_fence_init();
         tma_prefetch_desc(&tmap_x);
@@ -200,87 +340,102 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
 
     if (warp == 0) {
         // ---------------- weight producer: one bulk copy of 17408 contiguous bytes per stage ----------------
-        const uint8_t *src = p.packed + u_begin * kPStageWBytes;  // items are consecutive in [tile][pair] order
+        int q = u_begin / p.nchunks, c = u_begin - q * p.nchunks;
         uint32_t st = 0, ph = 0;
         const uint32_t full0 = smem_u32(&tail->w_full[0]), empty0 = smem_u32(&tail->w_empty[0]);
-        for (int64_t it = u_begin; it < u_end; ++it, src += kPStageWBytes) {
+        for (int it = u_begin; it < u_end; ++it) {
             if (!mbar_wait(empty0 + st * 8, ph ^ 1, abort_flag, 0x50)) break;
             if (lane == 0) {
                 mbar_expect_tx(full0 + st * 8, kPStageWBytes);
-                bulk_load_1d(smem_base + w_off + st * kPStageWBytes, src, kPStageWBytes, full0 + st * 8);
+                bulk_load_1d(smem_base + w_off + st * kPStageWBytes,
+                             p.packed + (static_cast<int64_t>(q / p.nblk) * p.nchunks + c) * kPStageWBytes, kPStageWBytes,
+                             full0 + st * 8);
             }
             __syncwarp();
             if (++st == nstages) {
                 st = 0;
                 ph ^= 1;
             }
+            if (++c == p.nchunks) {
+                c = 0;
+                ++q;
+            }
         }
     } else if (warp == 1) {
-        // ---------------- activation producer: one [mpad][256 k] tile per stage ----------------
-        int c = static_cast<int>(u_begin % p.nchunks);
+        // ---------------- activation producer: steps of kXBoxes boxes, 4 / kXBoxes steps an item ----------------
+        constexpr int kSteps = 4 / F::kXBoxes;
+        int q = u_begin / p.nchunks, k0 = (u_begin - q * p.nchunks) * kPStageK, row0 = (q % p.nblk) * p.mpad;
+        const int k_end = p.nchunks * kPStageK;
         uint32_t rs = 0, rph = 0;
-        for (int64_t it = u_begin; it < u_end; ++it) {
+        for (int i = (u_end - u_begin) * kSteps; i > 0; --i) {
             if (!mbar_wait(smem_u32(&tail->x_empty[rs]), rph ^ 1, abort_flag, 0x57)) break;
             if (lane == 0) {
                 const uint32_t bar = smem_u32(&tail->x_full[rs]);
                 const uint32_t dst = smem_base + rs * x_slot;
                 mbar_expect_tx(bar, x_slot);
 #pragma unroll
-                for (int b = 0; b < 4; ++b)  // rows beyond M and k beyond K arrive as zeros
-                    tma_load_2d(dst + b * x_box, &tmap_x, c * kPStageK + b * 64, 0, bar);
+                for (int b = 0; b < F::kXBoxes; ++b)  // rows beyond M and k beyond K arrive as zeros
+                    tma_load_2d(dst + b * x_box, &tmap_x, k0 + b * 64, row0, bar);
             }
             __syncwarp();
             if (++rs == nxstages) {
                 rs = 0;
                 rph ^= 1;
             }
-            if (++c == p.nchunks) c = 0;
+            k0 += F::kXBoxes * 64;
+            if (k0 == k_end) {
+                k0 = 0;
+                ++q;
+                row0 = (q % p.nblk) * p.mpad;
+            }
         }
     } else if (warp == kPMmaWarp) {
         // ---------------- MMA issuer (whole warp, one elected lane issues) ----------------
         const uint32_t idesc = make_idesc(/*c=f32*/ 1, PMagic<T>::kFmt, PMagic<T>::kFmt, /*a*/ 0, /*b K-major*/ 0,
                                           kPTileN, static_cast<uint32_t>(p.mpad));
         constexpr uint32_t kDescHi = smem_desc_hi_sw128(1024);
-        int c = static_cast<int>(u_begin % p.nchunks);
-        uint32_t rs = 0, rph = 0, xs = 0, xph = 0, pb = 0, pb_phase = 0, accumulate = 0;
-        bool ok = true;
-        for (int64_t it = u_begin; it < u_end && ok; ++it) {
-            const bool first = (it == u_begin) || (c == 0);
-            const bool last = (it + 1 == u_end) || (c + 1 == p.nchunks);
-            if (first) {
-                ok = mbar_wait(smem_u32(&tail->tmem_empty[pb]), pb_phase ^ 1, abort_flag, 0x51);
-                if (!ok) break;
-                accumulate = 0;
+        constexpr int kSteps = 4 / F::kXBoxes;
+        const uint32_t box = x_box >> 4;
+        int left = p.nchunks - u_begin % p.nchunks;  // items until the end of the output tile
+        uint32_t rs = 0, rph = 0, xs = 0, xph = 0, pb = 0, pb_phase = 0, accumulate = 0, step = 0;
+        for (int i = (u_end - u_begin) * kSteps; i > 0; --i) {
+            if (step == 0) {
+                if (accumulate == 0 && !mbar_wait(smem_u32(&tail->tmem_empty[pb]), pb_phase ^ 1, abort_flag, 0x51)) break;
+                if (!mbar_wait(smem_u32(&tail->a_full[rs]), rph, abort_flag, 0x53)) break;
             }
-            ok = mbar_wait(smem_u32(&tail->x_full[xs]), xph, abort_flag, 0x52) &&
-                 mbar_wait(smem_u32(&tail->a_full[rs]), rph, abort_flag, 0x53);
-            if (!ok) break;
+            if (!mbar_wait(smem_u32(&tail->x_full[xs]), xph, abort_flag, 0x52)) break;
             tc_fence_after();
-            const uint32_t d = tmem_base + pb * kPMaxM;
-            const uint32_t a = tmem_base + kPACol0 + rs * kPRingCols;
+            const uint32_t d = tmem_base + pb * F::kTok;
+            const uint32_t a = tmem_base + F::kACol0 + rs * kPRingCols;
             const uint32_t x_lo = smem_desc_lo(smem_base + xs * x_slot, 16);
-            const uint32_t box = x_box >> 4;
-            mma_f16_ts_warp_x8(d, a, x_lo, x_lo + box, kDescHi, idesc, accumulate);
-            mma_f16_ts_warp_x8(d, a + 64, x_lo + 2 * box, x_lo + 3 * box, kDescHi, idesc, 1);
+            if constexpr (WIDE) {
+                p_mma_x4(d, a + step * 32, x_lo, kDescHi, idesc, accumulate);
+            } else {
+                mma_f16_ts_warp_x8(d, a, x_lo, x_lo + box, kDescHi, idesc, accumulate);
+                mma_f16_ts_warp_x8(d, a + 64, x_lo + 2 * box, x_lo + 3 * box, kDescHi, idesc, 1);
+            }
             accumulate = 1;
-            tc_commit_warp(smem_u32(&tail->mma_done[rs]));
             tc_commit_warp(smem_u32(&tail->x_empty[xs]));
             if (++xs == nxstages) {
                 xs = 0;
                 xph ^= 1;
             }
-            if (last) {
+            if (++step < kSteps) continue;
+            step = 0;
+            tc_commit_warp(smem_u32(&tail->mma_done[rs]));
+            if (++rs == F::kRing) {
+                rs = 0;
+                rph ^= 1;
+            }
+            if (--left == 0 || i == 1) {  // the tile's or the range's last item
+                left = p.nchunks;
                 tc_commit_warp(smem_u32(&tail->tmem_full[pb]));
-                if (++pb == kPDBufs) {
+                accumulate = 0;
+                if (++pb == F::kDBufs) {
                     pb = 0;
                     pb_phase ^= 1;
                 }
             }
-            if (++rs == kPRing) {
-                rs = 0;
-                rph ^= 1;
-            }
-            if (++c == p.nchunks) c = 0;
         }
     } else if (warp < kPFirstEpiWarp) {
         // ---------------- unpack warps ----------------
@@ -291,10 +446,10 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
         const uint32_t flip = PMagic<T>::kFlip;
         const T2 bias2 = PMagic<T>::bias2();
         // this warp's 16 columns of sub-step `team` of block 0; block 1 is 64 columns further
-        const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kPACol0 + team * 16;
+        const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + F::kACol0 + team * 16;
         uint32_t st = 0, ph = 0, rs = 0, rph = 0;
         int pending = -1;  // ring slot whose stores are in flight
-        for (int64_t it = u_begin; it < u_end; ++it) {
+        for (int it = u_begin; it < u_end; ++it) {
             if (!mbar_wait(smem_u32(&tail->w_full[st]), ph, abort_flag, 0x54)) break;
             const uint8_t *blk = smem_aligned + w_off + st * kPStageWBytes;
             uint4 wv[kPPair];
@@ -338,7 +493,7 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
             tmem_st_32x16(lane_taddr + rs * kPRingCols, v[0]);
             tmem_st_32x16(lane_taddr + rs * kPRingCols + 64, v[1]);
             pending = static_cast<int>(rs);
-            if (++rs == kPRing) {
+            if (++rs == F::kRing) {
                 rs = 0;
                 rph ^= 1;
             }
@@ -357,19 +512,19 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
         // ---------------- epilogue warps: thread = tensor-memory lane = one output column ----------------
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
-        const bool leader_thread = (threadIdx.x == kPFirstEpiWarp * 32);
         const T *bias = static_cast<const T *>(p.bias);
         T *out = static_cast<T *>(p.out);
         const int M = p.M;
-        int64_t u = u_begin;
+        int u = u_begin;
         uint32_t pb = 0, pb_phase = 0;
         while (u < u_end) {
-            const int tile = static_cast<int>(u / p.nchunks);
-            const int64_t tile_begin = static_cast<int64_t>(tile) * p.nchunks;
-            const int64_t tile_end = tile_begin + p.nchunks;
-            const int64_t seg_end = tile_end < u_end ? tile_end : u_end;
+            const int q = u / p.nchunks;
+            const int tile_begin = q * p.nchunks, tile_end = tile_begin + p.nchunks;
+            const int seg_end = min(tile_end, u_end);
             const bool whole = (u == tile_begin && seg_end == tile_end);
-            const int64_t n = static_cast<int64_t>(tile) * kPTileN + row;
+            const int64_t n = static_cast<int64_t>(q / p.nblk) * kPTileN + row;
+            const int m0 = (q % p.nblk) * p.mpad;
+            const int rows = min(p.mpad, M - m0);  // token rows of this tile
             const bool n_ok = n < p.N;
             const float b = (n_ok && bias != nullptr) ? to_float(bias[n]) : 0.0f;
 
@@ -379,14 +534,10 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
             pepi_bar_sync();
             if (*reinterpret_cast<volatile uint32_t *>(&tail->epi_abort) != 0) break;
             tc_fence_after();
-            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + pb * kPMaxM;
-
-            const int first_cta = p_cta_of_item(tile_begin, total, G);
-            const int last_cta = p_cta_of_item(tile_end - 1, total, G);
-            const int nslots = last_cta - first_cta + 1;
+            const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + pb * F::kTok;
             const int64_t slot_elems = static_cast<int64_t>(p.mpad) * kPTileN;
-            float *tile_slots = p.slots + static_cast<int64_t>(tile) * p.max_slots * slot_elems;
-            float *mine = tile_slots + (static_cast<int>(blockIdx.x) - first_cta) * slot_elems + row;
+            float *mine = p.slots + (static_cast<int64_t>(q) * p.max_slots + cta - p_cta_of(p, tile_begin)) * slot_elems + row;
+            T *o = out + static_cast<int64_t>(m0) * p.ld_out + n;
             for (int c0 = 0; c0 < p.mpad; c0 += 16) {
                 uint32_t v[16];
                 tmem_ld_32x16(taddr + c0, v);
@@ -395,50 +546,24 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
                     if (n_ok) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j)
-                            if (c0 + j < M)
-                                out[static_cast<int64_t>(c0 + j) * p.ld_out + n] = from_float<T>(__uint_as_float(v[j]) + b);
+                            if (c0 + j < rows) o[static_cast<int64_t>(c0 + j) * p.ld_out] = from_float<T>(__uint_as_float(v[j]) + b);
                     }
                 } else {
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        if (c0 + j < M) __stcg(mine + (c0 + j) * kPTileN, __uint_as_float(v[j]));
+                        if (c0 + j < rows) __stcg(mine + (c0 + j) * kPTileN, __uint_as_float(v[j]));
                 }
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&tail->tmem_empty[pb]));
-            if (++pb == kPDBufs) {
+            if (++pb == F::kDBufs) {
                 pb = 0;
                 pb_phase ^= 1;
             }
-            if (!whole) {
-                __threadfence();
-                pepi_bar_sync();
-                if (leader_thread) {
-                    const uint32_t old = atomicAdd(p.counters + tile, 1u);
-                    const bool is_last = (old + 1 == static_cast<uint32_t>(nslots));
-                    if (is_last) p.counters[tile] = 0;
-                    tail->is_last = is_last ? 1u : 0u;
-                    __threadfence();
-                }
-                pepi_bar_sync();
-                if (*reinterpret_cast<volatile uint32_t *>(&tail->is_last) != 0 && n_ok) {
-                    for (int m0 = 0; m0 < M; m0 += 16) {
-                        float v[16];
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] = 0.0f;
-                        for (int sl = 0; sl < nslots; ++sl) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j)
-                                if (m0 + j < M) v[j] += __ldcg(tile_slots + sl * slot_elems + row + (m0 + j) * kPTileN);
-                        }
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (m0 + j < M) out[static_cast<int64_t>(m0 + j) * p.ld_out + n] = from_float<T>(v[j] + b);
-                    }
-                }
-                pepi_bar_sync();  // is_last is rewritten by the next shared tile
-            }
+            // a tile that this CTA shares and leaves before the end of its range: these four warps report it, while
+            // the others go on
+            if (!whole && seg_end < u_end) p_finish_shared<T, true>(p, q, abort_flag, &tail->is_last);
             u = seg_end;
         }
     }
@@ -451,6 +576,10 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kPTmemCols);
     }
+    // Output tiles shared with other CTAs: only the first and the last of a contiguous range can be.  The CTA that
+    // arrives last adds the slots.  Most tiles are completed at the end of a range, by then with all threads, so that
+    // the slots' loads of many elements are in flight together.
+    if (p.grain == 1 && u_begin < u_end) p_finish_shared<T, false>(p, (u_end - 1) / p.nchunks, abort_flag, &tail->is_last);
 }
 
 // ---- layout pass and its inverse ----------------------------------------------------------------------
@@ -515,25 +644,59 @@ w4a16_unpack_kernel(const uint8_t *__restrict__ packed, int64_t N, int64_t K, in
 }
 
 struct PPlan {
-    int mpad, tiles_n, nchunks, grid, max_slots, nstages, nxstages;
-    size_t slots_bytes;
+    int mpad, nblk, tiles_n, nchunks, grid, share, extra, grain, max_slots, nstages, nxstages;
+    size_t slots_bytes, smem;
 };
 
 PPlan p_make_plan(int64_t M, int64_t N, int64_t K) {
     PPlan pl;
-    const int64_t m = M < kPMaxM ? M : kPMaxM;
-    pl.mpad = static_cast<int>((m + 15) / 16 * 16);
+    const int64_t sms = sm_count();
     pl.tiles_n = static_cast<int>((N + kPTileN - 1) / kPTileN);
     pl.nchunks = static_cast<int>((K + kPStageK - 1) / kPStageK);  // block pairs
-    const int64_t total = static_cast<int64_t>(pl.tiles_n) * pl.nchunks;
-    pl.grid = static_cast<int>(total < sm_count() ? total : sm_count());
-    const int64_t ipc = total / pl.grid;  // items per CTA, rounded down (>= 1)
-    pl.max_slots = static_cast<int>((pl.nchunks + ipc - 1) / ipc + 1);
-    // activation tiles: enough to cover the L2 latency of their loads; the rest of the budget holds weights
-    pl.nxstages = pl.mpad <= 16 ? 8 : (pl.mpad <= 32 ? 6 : 4);
-    pl.nstages = static_cast<int>((kPSmemBudget - static_cast<size_t>(pl.nxstages) * pl.mpad * 512) / kPStageWBytes);
-    if (pl.nstages > kPMaxStages) pl.nstages = kPMaxStages;
-    pl.slots_bytes = static_cast<size_t>(pl.tiles_n) * pl.max_slots * pl.mpad * kPTileN * sizeof(float);
+    if (M <= kPMaxM) {
+        pl.mpad = static_cast<int>((M + 15) / 16 * 16);
+        pl.nblk = 1;
+        pl.grain = 1;
+        // activation tiles: enough to cover the L2 latency of their loads; the rest of the budget holds weights
+        pl.nxstages = pl.mpad <= 16 ? 8 : (pl.mpad <= 32 ? 6 : 4);
+        pl.nstages = static_cast<int>((kPSmemBudget - static_cast<size_t>(pl.nxstages) * pl.mpad * 512) / kPStageWBytes);
+        if (pl.nstages > kPMaxStages) pl.nstages = kPMaxStages;
+        pl.smem = 2048 + static_cast<size_t>(pl.nxstages) * pl.mpad * 512 + static_cast<size_t>(pl.nstages) * kPStageWBytes;
+    } else {
+        // Rows per tile and the way of sharing tiles out that take least time by this model (clocks): a stage costs
+        // what its sixteen MMAs take (8 a row) or what unpacking it takes (about 1150), a tile some 12 a row more to
+        // leave tensor memory.  Whole tiles per CTA leave the last wave uneven; equal shares of the stages do not, but
+        // every CTA then writes up to two tiles' sums and someone adds them (16 clocks a row each).
+        int64_t best = -1;
+        const int64_t min_blk = (M + kPMaxWide - 1) / kPMaxWide;
+        for (int64_t nblk = min_blk; nblk <= min_blk + 8 && nblk <= (M + 63) / 64; ++nblk) {
+            const int64_t mpad = ((M + nblk - 1) / nblk + 15) / 16 * 16;
+            if (mpad > kPMaxWide) continue;
+            const int64_t tiles = static_cast<int64_t>(pl.tiles_n) * ((M + mpad - 1) / mpad);
+            const int64_t stage = mpad * 8 > 1150 ? mpad * 8 : 1150, tile = pl.nchunks * stage + 12 * mpad;
+            const int64_t whole = (tiles + sms - 1) / sms * tile;
+            const int64_t shared = tiles > static_cast<int64_t>(kPCounterBytes / 4) ? whole + 1  // a counter a tile
+                                                                                     : tiles * tile / sms + stage + 2 * 16 * mpad + 4000;
+            const int64_t cost = whole < shared ? whole : shared;
+            if (best < 0 || cost < best) {
+                best = cost;
+                pl.mpad = static_cast<int>(mpad);
+                pl.nblk = static_cast<int>((M + mpad - 1) / mpad);
+                pl.grain = whole <= shared ? pl.nchunks : 1;
+            }
+        }
+        pl.nstages = kPWideStages;
+        pl.nxstages = static_cast<int>((kPSmemBudgetWide - 2048 - kPWideStages * kPStageWBytes) / (static_cast<size_t>(pl.mpad) * 128));
+        if (pl.nxstages > kPMaxXStages) pl.nxstages = kPMaxXStages;
+        pl.smem = 2048 + static_cast<size_t>(pl.nxstages) * pl.mpad * 128 + static_cast<size_t>(pl.nstages) * kPStageWBytes;
+    }
+    const int64_t out_tiles = static_cast<int64_t>(pl.tiles_n) * pl.nblk;
+    const int64_t grains = out_tiles * (pl.nchunks / pl.grain);
+    pl.grid = static_cast<int>(grains < sms ? grains : sms);
+    pl.share = static_cast<int>(grains / pl.grid);  // >= 1
+    pl.extra = static_cast<int>(grains % pl.grid);
+    pl.max_slots = pl.grain > 1 ? 0 : (pl.nchunks + pl.share - 1) / pl.share + 1;
+    pl.slots_bytes = static_cast<size_t>(out_tiles) * pl.max_slots * pl.mpad * kPTileN * sizeof(float);
     return pl;
 }
 
@@ -913,6 +1076,11 @@ int launch_prepacked_t(const uint8_t *packed, const void *x, int64_t ld_x, const
     p.M = static_cast<int>(M);
     p.N = static_cast<int>(N);
     p.mpad = pl.mpad;
+    p.nblk = pl.nblk;
+    p.share = pl.share;
+    p.extra = pl.extra;
+    p.grain = pl.grain;
+    p.out_vec = (reinterpret_cast<uintptr_t>(out) & 7) == 0 && (ld_out & 3) == 0;
     p.x_box_bytes = pl.mpad * 128;
     p.nstages = pl.nstages;
     p.nxstages = pl.nxstages;
@@ -929,11 +1097,9 @@ int launch_prepacked_t(const uint8_t *packed, const void *x, int64_t ld_x, const
                           static_cast<uint32_t>(pl.mpad), true);
     if (rc != QMM_OK) return rc;
     static_assert(sizeof(PSmemTail) <= 1024, "the tail has 1 KiB");
-    const size_t smem = 1024 + static_cast<size_t>(pl.nxstages) * pl.mpad * 512 +
-                        static_cast<size_t>(pl.nstages) * kPStageWBytes + 1024;
-    auto kern = w4a16_prepacked_kernel<T>;
-    QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(pl.grid)), dim3(kPThreads), smem, stream, tx, p));
+    auto kern = M <= kPMaxM ? w4a16_prepacked_kernel<T, false> : w4a16_prepacked_kernel<T, true>;
+    QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pl.smem)));
+    QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(pl.grid)), dim3(kPThreads), pl.smem, stream, tx, p));
     return QMM_OK;
 }
 
@@ -1033,17 +1199,9 @@ extern "C" int qmm_weight_quant_batchmatmul_prepacked(const void *x, int x_dtype
                                                   workspace, s)
                    : launch_gemv_t<__half>(static_cast<const uint8_t *>(packed), x, ld_x, bias, out, ld_out, M, N, K,
                                            workspace, s);
-    const size_t elt = 2;
-    for (int64_t m0 = 0; m0 < M; m0 += kPMaxM) {  // 64 token rows per launch (the accumulator's columns)
-        const int64_t mc = (M - m0) < kPMaxM ? (M - m0) : kPMaxM;
-        const void *xc = static_cast<const uint8_t *>(x) + static_cast<size_t>(m0) * ld_x * elt;
-        void *oc = static_cast<uint8_t *>(out) + static_cast<size_t>(m0) * ld_out * elt;
-        const int rc = (x_dtype == QMM_DTYPE_BF16)
-                           ? launch_prepacked_t<__nv_bfloat16>(static_cast<const uint8_t *>(packed), xc, ld_x, bias, oc,
-                                                               ld_out, mc, N, K, workspace, s)
-                           : launch_prepacked_t<__half>(static_cast<const uint8_t *>(packed), xc, ld_x, bias, oc, ld_out,
-                                                        mc, N, K, workspace, s);
-        if (rc != QMM_OK) return rc;
-    }
-    return QMM_OK;
+    return (x_dtype == QMM_DTYPE_BF16)
+               ? launch_prepacked_t<__nv_bfloat16>(static_cast<const uint8_t *>(packed), x, ld_x, bias, out, ld_out, M, N, K,
+                                                   workspace, s)
+               : launch_prepacked_t<__half>(static_cast<const uint8_t *>(packed), x, ld_x, bias, out, ld_out, M, N, K,
+                                            workspace, s);
 }
