@@ -663,28 +663,19 @@ PPlan p_make_plan(int64_t M, int64_t N, int64_t K) {
         if (pl.nstages > kPMaxStages) pl.nstages = kPMaxStages;
         pl.smem = 2048 + static_cast<size_t>(pl.nxstages) * pl.mpad * 512 + static_cast<size_t>(pl.nstages) * kPStageWBytes;
     } else {
-        // Rows per tile and the way of sharing tiles out that take least time by this model (clocks): a stage costs
-        // what its sixteen MMAs take (8 a row) or what unpacking it takes (about 1150), a tile some 12 a row more to
-        // leave tensor memory.  Whole tiles per CTA leave the last wave uneven; equal shares of the stages do not, but
-        // every CTA then writes up to two tiles' sums and someone adds them (16 clocks a row each).
-        int64_t best = -1;
-        const int64_t min_blk = (M + kPMaxWide - 1) / kPMaxWide;
-        for (int64_t nblk = min_blk; nblk <= min_blk + 8 && nblk <= (M + 63) / 64; ++nblk) {
-            const int64_t mpad = ((M + nblk - 1) / nblk + 15) / 16 * 16;
-            if (mpad > kPMaxWide) continue;
-            const int64_t tiles = static_cast<int64_t>(pl.tiles_n) * ((M + mpad - 1) / mpad);
-            const int64_t stage = mpad * 8 > 1150 ? mpad * 8 : 1150, tile = pl.nchunks * stage + 12 * mpad;
-            const int64_t whole = (tiles + sms - 1) / sms * tile;
-            const int64_t shared = tiles > static_cast<int64_t>(kPCounterBytes / 4) ? whole + 1  // a counter a tile
-                                                                                     : tiles * tile / sms + stage + 2 * 16 * mpad + 4000;
-            const int64_t cost = whole < shared ? whole : shared;
-            if (best < 0 || cost < best) {
-                best = cost;
-                pl.mpad = static_cast<int>(mpad);
-                pl.nblk = static_cast<int>((M + mpad - 1) / mpad);
-                pl.grain = whole <= shared ? pl.nchunks : 1;
-            }
-        }
+        // As few row tiles as 256 columns of accumulator allow: every further one unpacks the weight again (1000 rows,
+        // K=4096, N=28672: 201 us with four row tiles, 205, 209, 214, 226 us with five to eight, although seven fill the
+        // last wave best).  Then the cheaper way of sharing tiles out by this model (clocks): a stage costs what its MMAs
+        // take (8 a row) or what unpacking it takes (about 1150), a tile some 12 a row more to leave tensor memory.
+        // Whole tiles leave the last wave uneven; equal shares of the stages do not, but every CTA then writes up to two
+        // tiles' sums and someone adds them (16 a row each).
+        const int64_t nblk = (M + kPMaxWide - 1) / kPMaxWide;
+        pl.mpad = static_cast<int>(((M + nblk - 1) / nblk + 15) / 16 * 16);
+        pl.nblk = static_cast<int>((M + pl.mpad - 1) / pl.mpad);
+        const int64_t tiles = static_cast<int64_t>(pl.tiles_n) * pl.nblk;
+        const int64_t stage = pl.mpad * 8 > 1150 ? pl.mpad * 8 : 1150, tile = pl.nchunks * stage + 12 * pl.mpad;
+        const int64_t whole = (tiles + sms - 1) / sms * tile, shared = tiles * tile / sms + stage + 2 * 16 * pl.mpad + 4000;
+        pl.grain = whole <= shared || tiles > static_cast<int64_t>(kPCounterBytes / 4) ? pl.nchunks : 1;  // (a counter a tile)
         pl.nstages = kPWideStages;
         pl.nxstages = static_cast<int>((kPSmemBudgetWide - 2048 - kPWideStages * kPStageWBytes) / (static_cast<size_t>(pl.mpad) * 128));
         if (pl.nxstages > kPMaxXStages) pl.nxstages = kPMaxXStages;
