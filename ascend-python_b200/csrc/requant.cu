@@ -6,117 +6,24 @@
 //     acc[m,n] = sum_k x1[m,k] * x2[k,n] + bias[n]                      int32, exact (bias int32)
 //     v        = float(acc) * scale[n] (* pertoken_scale[m]) (+ offset[n])   fp32, one rounding per operation
 //     out      = clamp(rint(v), -128, 127)                              round half to even
-// It runs as two launches: the W8A8 kernels produce the exact int32 accumulator (their int32 output
-// mode) into scratch, and requant_kernel below makes one pass over it.  That costs 5 bytes of HBM
-// traffic per output element more than an epilogue fused into every matmul kernel would; no
-// configuration of the benchmark uses an int8 output.
+// The requantization is one more output type of the matmul kernels' epilogue.  (As a pass of its own over an int32
+// accumulator it cost 5 bytes of traffic per output element and a launch: 2048 x 14336 x 4096 took 114 us.)
 #include "qmm_common.cuh"
-
-extern "C" int qmm_quant_matmul(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_stride_k,
-                                int64_t x2_stride_n, const float *scale, int64_t scale_len,
-                                const float *pertoken_scale, const void *bias, int bias_dtype, void *out,
-                                int out_dtype, int64_t ld_out, int64_t M, int64_t N, int64_t K, int algo,
-                                void *workspace, size_t workspace_bytes, void *stream);
-extern "C" int qmm_quant_matmul_workspace_size(int64_t M, int64_t N, int64_t K, int algo, size_t *bytes);
+#include "w8a8_epilogue.cuh"
 
 namespace qmm {
+int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
+                          const EpilogueParams &ep, int out_dtype, int64_t K, int algo, void *workspace,
+                          size_t workspace_bytes, cudaStream_t stream, LaunchOptions *opts);
+int validate_quant_matmul(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
+                          const float *scale, int64_t scale_len, const void *bias, int bias_dtype, void *out,
+                          int out_dtype, int64_t ld_out, int64_t M, int64_t N, int64_t K);
 namespace {
-
-__device__ __forceinline__ int requant_one(int32_t acc, float sc, float pt, bool has_pt, float off, bool has_off) {
-    float v = __fmul_rn(static_cast<float>(acc), sc);
-    if (has_pt) v = __fmul_rn(v, pt);
-    if (has_off) v = __fadd_rn(v, off);
-    return max(-128, min(127, __float2int_rn(v)));
-}
-
-// Sixteen columns per thread (64 bytes of accumulators in flight per thread, one 16-byte store), one row per
-// blockIdx.y step: no index division, per-column constants as 16-byte loads.  Needs N % 16 == 0 and 16-byte
-// aligned rows of `out`; other shapes take requant_kernel below.
-__global__ void __launch_bounds__(256)
-requant_vec16_kernel(const int32_t *__restrict__ acc, int64_t M, int64_t N, const float *__restrict__ scale,
-                     int scale_scalar, const float *__restrict__ pertoken, const float *__restrict__ offset,
-                     int offset_scalar, int8_t *__restrict__ out, int64_t ld_out) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int64_t n = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 16;
-    if (n >= N) return;
-    const bool has_pt = pertoken != nullptr, has_off = offset != nullptr;
-    float sc[16], off[16];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const float4 s4 = scale_scalar ? make_float4(__ldg(scale), __ldg(scale), __ldg(scale), __ldg(scale))
-                                       : __ldg(reinterpret_cast<const float4 *>(scale + n) + q);
-        float4 o4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (has_off)
-            o4 = offset_scalar ? make_float4(__ldg(offset), __ldg(offset), __ldg(offset), __ldg(offset))
-                               : __ldg(reinterpret_cast<const float4 *>(offset + n) + q);
-        sc[4 * q] = s4.x, sc[4 * q + 1] = s4.y, sc[4 * q + 2] = s4.z, sc[4 * q + 3] = s4.w;
-        off[4 * q] = o4.x, off[4 * q + 1] = o4.y, off[4 * q + 2] = o4.z, off[4 * q + 3] = o4.w;
-    }
-    for (int64_t m = blockIdx.y; m < M; m += gridDim.y) {
-        const int4 *src = reinterpret_cast<const int4 *>(acc + m * N + n);
-        int4 a[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) a[q] = __ldcs(src + q);
-        const float pt = has_pt ? __ldg(pertoken + m) : 1.0f;
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int32_t av[4] = {a[q].x, a[q].y, a[q].z, a[q].w};
-            uint32_t packed = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                packed |= (static_cast<uint32_t>(requant_one(av[j], sc[4 * q + j], pt, has_pt, off[4 * q + j], has_off)) & 0xffu)
-                          << (8 * j);
-            w[q] = packed;
-        }
-        *reinterpret_cast<uint4 *>(out + m * ld_out + n) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-}
-
-// four columns per thread where N allows
-__global__ void __launch_bounds__(256)
-requant_kernel(const int32_t *__restrict__ acc, int64_t M, int64_t N, const float *__restrict__ scale, int scale_scalar,
-               const float *__restrict__ pertoken, const float *__restrict__ offset, int offset_scalar,
-               int8_t *__restrict__ out, int64_t ld_out) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const bool vec = (N & 3) == 0 && (ld_out & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0;
-    const bool has_pt = pertoken != nullptr, has_off = offset != nullptr;
-    if (vec) {
-        const int64_t per_row = N >> 2;
-        const int64_t total = M * per_row;
-        for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-             i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-            const int64_t m = i / per_row, n = (i - m * per_row) << 2;
-            const int4 a = __ldcs(reinterpret_cast<const int4 *>(acc + m * N + n));
-            const float pt = has_pt ? __ldg(pertoken + m) : 1.0f;
-            const int32_t av[4] = {a.x, a.y, a.z, a.w};
-            uint32_t packed = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float sc = scale_scalar ? __ldg(scale) : __ldg(scale + n + j);
-                const float off = has_off ? (offset_scalar ? __ldg(offset) : __ldg(offset + n + j)) : 0.0f;
-                packed |= (static_cast<uint32_t>(requant_one(av[j], sc, pt, has_pt, off, has_off)) & 0xffu) << (8 * j);
-            }
-            *reinterpret_cast<uint32_t *>(out + m * ld_out + n) = packed;
-        }
-    } else {
-        const int64_t total = M * N;
-        for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-             i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-            const int64_t m = i / N, n = i - m * N;
-            const float sc = scale_scalar ? __ldg(scale) : __ldg(scale + n);
-            const float off = has_off ? (offset_scalar ? __ldg(offset) : __ldg(offset + n)) : 0.0f;
-            out[m * ld_out + n] = static_cast<int8_t>(requant_one(acc[i], sc, has_pt ? __ldg(pertoken + m) : 1.0f, has_pt, off, has_off));
-        }
-    }
-}
-
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
-
 }  // namespace
 }  // namespace qmm
+
+extern "C" int qmm_quant_matmul_workspace_size(int64_t M, int64_t N, int64_t K, int algo, size_t *bytes);
 
 extern "C" int qmm_quant_matmul_int8_workspace_size(int64_t M, int64_t N, int64_t K, size_t *bytes) {
     using namespace qmm;
@@ -125,8 +32,8 @@ extern "C" int qmm_quant_matmul_int8_workspace_size(int64_t M, int64_t N, int64_
     size_t inner = 0;
     int rc = qmm_quant_matmul_workspace_size(M, N, K, QMM_ALGO_AUTO, &inner);
     if (rc != QMM_OK) return rc;
-    // [the matmul's own scratch (zero before first use)][int32 accumulator M x N]
-    *bytes = align256(inner) + align256(static_cast<size_t>(M) * N * 4);
+    // the matmul's own scratch; never empty, so that a workspace is always asked for
+    *bytes = inner > 0 ? align256(inner) : 256;
     return QMM_OK;
 }
 
@@ -148,33 +55,26 @@ extern "C" int qmm_quant_matmul_int8(const int8_t *x1, int64_t ld_x1, const int8
     if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0)
         return fail(QMM_ERR_WORKSPACE, "qmm_quant_matmul_int8: workspace missing, not 256-byte aligned or smaller than "
                                        "qmm_quant_matmul_int8_workspace_size reports");
-    int32_t *acc = reinterpret_cast<int32_t *>(static_cast<uint8_t *>(workspace) + align256(inner));
-    // the matmul kernels want their scratch zeroed; where it sits depends on the shape, and a call of another
-    // shape may have left accumulators there, so it is cleared per call (decode shapes only: inner is 0 for M > 128)
-    if (inner > 0) QMM_CUDA_OK(cudaMemsetAsync(workspace, 0, inner, static_cast<cudaStream_t>(stream)));
-    int rc = qmm_quant_matmul(x1, ld_x1, x2, x2_stride_k, x2_stride_n, nullptr, 0, nullptr, bias,
-                              bias ? QMM_DTYPE_I32 : QMM_DTYPE_NONE, acc, QMM_DTYPE_I32, N, M, N, K, QMM_ALGO_AUTO,
-                              inner ? workspace : nullptr, inner, stream);
+    // validated as the accumulator pass that the operator's definition names (int32 bias); K == 0 included
+    int rc = validate_quant_matmul(x1, ld_x1, x2, x2_stride_k, x2_stride_n, nullptr, 0, bias, bias ? QMM_DTYPE_I32 : QMM_DTYPE_NONE,
+                                   out, QMM_DTYPE_I32, ld_out, M, N, K);
     if (rc != QMM_OK) return rc;
-    const int scale_scalar = (scale_len == 1 && N != 1) ? 1 : 0, offset_scalar = (offset_len == 1 && N != 1) ? 1 : 0;
-    if ((N & 15) == 0 && (ld_out & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 &&
-        (scale_scalar || (reinterpret_cast<uintptr_t>(scale) & 15) == 0) &&
-        (offset == nullptr || offset_scalar || (reinterpret_cast<uintptr_t>(offset) & 15) == 0)) {
-        const unsigned gx = static_cast<unsigned>((N / 16 + 255) / 256);
-        int64_t gy = static_cast<int64_t>(sm_count()) * 16 / gx;
-        if (gy > M) gy = M;
-        if (gy > 65535) gy = 65535;
-        if (gy < 1) gy = 1;
-        QMM_CUDA_OK(launch_pdl(requant_vec16_kernel, dim3(gx, static_cast<unsigned>(gy)), dim3(256), 0,
-                               static_cast<cudaStream_t>(stream), acc, M, N, scale, scale_scalar, pertoken_scale, offset,
-                               offset_scalar, out, ld_out));
-        return QMM_OK;
-    }
-    const int64_t items = ((N & 3) == 0) ? M * (N >> 2) : M * N;
-    int64_t grid = (items + 255) / 256;
-    const int64_t cap = static_cast<int64_t>(sm_count()) * 16;
-    if (grid > cap) grid = cap;
-    QMM_CUDA_OK(launch_pdl(requant_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, static_cast<cudaStream_t>(stream), acc,
-                           M, N, scale, scale_scalar, pertoken_scale, offset, offset_scalar, out, ld_out));
-    return QMM_OK;
+    // the matmul kernels want their scratch zeroed; callers need not prepare it (decode shapes only: 0 for M > 128)
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (inner > 0) QMM_CUDA_OK(cudaMemsetAsync(workspace, 0, inner, s));
+    EpilogueParams ep;
+    ep.scale = scale;
+    ep.pertoken_scale = pertoken_scale;
+    ep.bias = bias;
+    ep.bias_dtype = bias ? QMM_DTYPE_I32 : QMM_DTYPE_NONE;
+    ep.scale_is_scalar = (scale_len == 1 && N != 1) ? 1 : 0;
+    ep.out = out;
+    ep.ld_out = ld_out;
+    ep.M = M;
+    ep.N = N;
+    ep.offset = offset;
+    ep.offset_is_scalar = (offset_len == 1 && N != 1) ? 1 : 0;
+    // K == 0: an empty reduction, the epilogue of zeros
+    return quant_matmul_dispatch(x1, ld_x1, x2, x2_stride_k, x2_stride_n, ep, kOutI8, K, K == 0 ? QMM_ALGO_SIMT : QMM_ALGO_AUTO,
+                                 inner ? workspace : nullptr, inner, s, nullptr);
 }

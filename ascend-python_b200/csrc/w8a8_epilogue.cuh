@@ -1,7 +1,8 @@
 // Fused dequantization epilogue shared by every W8A8 kernel.
 //
 //   out_dtype int32 : out = acc (+ int32 bias)
-//   otherwise       : out = cast(float(acc) * scale[n] * pertoken_scale[m] + float(bias[n]))
+//   bf16, f16       : out = cast(float(acc) * scale[n] * pertoken_scale[m] + float(bias[n]))
+//   int8            : out = clamp(rint(float(acc + int32 bias) * scale[n] * pertoken_scale[m] + offset[n]), -128, 127)
 // evaluated in fp32 with one rounding per operation in exactly this order, so
 // that the result equals the CPU oracle's fp32 epilogue bit for bit before the
 // final round-to-nearest-even conversion to bf16/f16.
@@ -21,7 +22,12 @@ struct EpilogueParams {
     int64_t ld_out;
     int64_t M;
     int64_t N;
+    const float *offset = nullptr;  // [N] or [1] or nullptr; int8 output only
+    int offset_is_scalar = 0;
 };
+
+// out_dtype of quant_matmul_dispatch for the int8 output (the C ABI has an entry point of its own for it)
+constexpr int kOutI8 = 100;
 
 // Row-parallel matmul whose output tiles go straight to the rank that will reduce them: rank o owns the
 // rows [o * rows_per, (o+1) * rows_per) and receives them from rank s at
@@ -69,80 +75,23 @@ __device__ __forceinline__ float dequant_one(int32_t acc, float scale_n, float p
     return v;
 }
 
-// One thread finishes `COUNT` consecutive columns [n0, n0+COUNT) of row m
-// (COUNT a multiple of 8).  OutT is __nv_bfloat16, __half or int32_t.
-template <typename OutT, int COUNT>
-__device__ __forceinline__ void epilogue_row_segment(const EpilogueParams &p, int64_t m, int64_t n0,
-                                                     const uint32_t (&acc)[COUNT]) {
-    if (m >= p.M || n0 >= p.N) return;
-    OutT *orow = static_cast<OutT *>(p.out) + m * p.ld_out + n0;
-    const bool full = (n0 + COUNT <= p.N);
-    if constexpr (sizeof(OutT) == 4) {
-        const bool has_bias = (p.bias != nullptr && p.bias_dtype == QMM_DTYPE_I32);
-        const int32_t *b = static_cast<const int32_t *>(p.bias);
-        const bool vec = full && ((reinterpret_cast<uintptr_t>(orow) & 15) == 0);
-        if (vec) {
-#pragma unroll
-            for (int j = 0; j < COUNT; j += 4) {
-                int32_t v[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    v[t] = static_cast<int32_t>(acc[j + t]) + (has_bias ? __ldg(b + n0 + j + t) : 0);
-                *reinterpret_cast<int4 *>(orow + j) = make_int4(v[0], v[1], v[2], v[3]);
-            }
-        } else {
-            for (int j = 0; j < COUNT; ++j) {
-                if (n0 + j < p.N)
-                    reinterpret_cast<int32_t *>(orow)[j] =
-                        static_cast<int32_t>(acc[j]) + (has_bias ? __ldg(b + n0 + j) : 0);
-            }
-        }
-    } else {
-        const bool has_bias = (p.bias != nullptr && p.bias_dtype != QMM_DTYPE_NONE && p.bias_dtype != QMM_DTYPE_I32);
-        const bool has_pt = (p.pertoken_scale != nullptr);
-        const float pt = has_pt ? __ldg(p.pertoken_scale + m) : 1.0f;
-        const float s0 = __ldg(p.scale);
-        const bool vec = full && ((reinterpret_cast<uintptr_t>(orow) & 15) == 0);
-        if (vec) {
-#pragma unroll
-            for (int j = 0; j < COUNT; j += 8) {
-                float f[8];
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    const int64_t n = n0 + j + t;
-                    const float sc = p.scale_is_scalar ? s0 : __ldg(p.scale + n);
-                    const float bi = has_bias ? load_bias_f32(p, n) : 0.0f;
-                    f[t] = dequant_one(static_cast<int32_t>(acc[j + t]), sc, pt, has_pt, bi, has_bias);
-                }
-                uint4 w;
-                w.x = pack2<OutT>(f[0], f[1]);
-                w.y = pack2<OutT>(f[2], f[3]);
-                w.z = pack2<OutT>(f[4], f[5]);
-                w.w = pack2<OutT>(f[6], f[7]);
-                *reinterpret_cast<uint4 *>(orow + j) = w;
-            }
-        } else {
-            for (int j = 0; j < COUNT; ++j) {
-                const int64_t n = n0 + j;
-                if (n < p.N) {
-                    const float sc = p.scale_is_scalar ? s0 : __ldg(p.scale + n);
-                    const float bi = has_bias ? load_bias_f32(p, n) : 0.0f;
-                    orow[j] = from_float<OutT>(dequant_one(static_cast<int32_t>(acc[j]), sc, pt, has_pt, bi, has_bias));
-                }
-            }
-        }
-    }
+__device__ __forceinline__ int requant_one(int32_t acc, float scale_n, float pertoken_m, bool has_pertoken, float offset_n,
+                                           bool has_offset) {
+    return max(-128, min(127, __float2int_rn(dequant_one(acc, scale_n, pertoken_m, has_pertoken, offset_n, has_offset))));
 }
 
 // ---------------------------------------------------------------------------
-// Epilogue of one warp through shared memory and TMA stores.
+// Epilogue of one warp through shared memory.
 //
 // The warp owns 32 accumulator rows (TMEM lanes) of a tile that is TILE_N
 // columns wide.  It walks the tile in chunks whose rows are 128 bytes of
-// output (64 columns of bf16/f16, 32 of int32): TMEM -> registers -> fp32
-// dequantization -> a 4 KiB staging buffer laid out with the 128-byte swizzle
+// output (128 columns of int8, 64 of bf16/f16, 32 of int32): TMEM -> registers ->
+// fp32 dequantization -> a 4 KiB staging buffer laid out with the 128-byte swizzle
 // (bank-conflict free 16-byte stores) -> one TMA store per chunk.  Two staging
 // buffers alternate so that the store of chunk c overlaps the math of c+1.
+// Outputs that break TMA's 16-byte rules (USE_TMA false at run time) leave the same
+// staging row by row, a warp's lanes on consecutive columns: with every lane on a
+// row of its own they took 2.9 ms at 8170 x 1952 x 23465.
 // Per-column scale and bias of a chunk are fetched once per warp (coalesced)
 // into a small shared array and read back as broadcasts.
 //
@@ -155,21 +104,39 @@ struct EpiChunk {
     static constexpr int kCols = 128 / static_cast<int>(sizeof(OutT));  // columns per 128-byte row
 };
 
+// rows of a staged chunk -> global memory, element by element
+template <typename OutT>
+__device__ __forceinline__ void epilogue_store_rows(const EpilogueParams &p, const uint8_t *staged, int64_t m_warp0, int64_t n0) {
+    constexpr int S = static_cast<int>(sizeof(OutT)), CC = EpiChunk<OutT>::kCols;
+    const int lane = threadIdx.x & 31;
+    const int rows = static_cast<int>(p.M - m_warp0 < 32 ? p.M - m_warp0 : 32);
+    OutT *out = static_cast<OutT *>(p.out) + m_warp0 * p.ld_out + n0;
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r) {
+#pragma unroll
+        for (int i = 0; i < CC; i += 32) {
+            const int byte = (i + lane) * S;
+            const OutT v = *reinterpret_cast<const OutT *>(staged + r * 128 + ((((byte >> 4) ^ (r & 7))) << 4) + (byte & 15));
+            if (n0 + i + lane < p.N) out[r * p.ld_out + i + lane] = v;
+        }
+    }
+}
+
 template <typename OutT, int TILE_N>
-__device__ __forceinline__ void epilogue_warp_tile_tma(const EpilogueParams &p, const CUtensorMap *tmap_out,
-                                                       uint32_t taddr_warp, int64_t m_warp0, int64_t n_tile0,
-                                                       uint8_t *stage, float *colbuf, uint32_t &chunk_counter,
-                                                       int64_t store_row0 = -1) {
+__device__ __forceinline__ void epilogue_warp_tile(const EpilogueParams &p, const CUtensorMap *tmap_out, bool use_tma,
+                                                   uint32_t taddr_warp, int64_t m_warp0, int64_t n_tile0,
+                                                   uint8_t *stage, float *colbuf, uint32_t &chunk_counter,
+                                                   int64_t store_row0 = -1) {
     // store_row0: row coordinate of the warp's first row in tmap_out when that map does not start at
     // row 0 of the output (tiles pushed into another rank's receive area); -1: same as m_warp0
     constexpr int CC = EpiChunk<OutT>::kCols;
     const int lane = threadIdx.x & 31;
     const int64_t m = m_warp0 + lane;
-    const bool is_int = (sizeof(OutT) == 4);
+    constexpr bool is_int = (sizeof(OutT) == 4), is_i8 = (sizeof(OutT) == 1);
     const bool has_pt = !is_int && (p.pertoken_scale != nullptr);
-    const bool has_bias = (p.bias != nullptr) && (is_int ? p.bias_dtype == QMM_DTYPE_I32
-                                                         : (p.bias_dtype != QMM_DTYPE_NONE &&
-                                                            p.bias_dtype != QMM_DTYPE_I32));
+    const bool has_bias = (p.bias != nullptr) && (is_int || is_i8 ? p.bias_dtype == QMM_DTYPE_I32
+                                                                  : (p.bias_dtype != QMM_DTYPE_NONE &&
+                                                                     p.bias_dtype != QMM_DTYPE_I32));
     const float pt = (has_pt && m < p.M) ? __ldg(p.pertoken_scale + m) : 1.0f;
     const uint32_t stage_u32 = smem_u32(stage);
     if (m_warp0 >= p.M) return;  // the warp's rows are all padding
@@ -183,31 +150,68 @@ __device__ __forceinline__ void epilogue_warp_tile_tma(const EpilogueParams &p, 
         if (lane == 0) tma_store_wait_read<1>();
         __syncwarp();
 
-        // per-column constants of this chunk -> shared (coalesced), as fp32 bit patterns
+        if constexpr (!is_i8) {
+            // per-column constants of this chunk -> shared (coalesced), as fp32 bit patterns
 #pragma unroll
-        for (int i = lane; i < CC; i += 32) {
-            const int64_t n = n0 + i;
-            float sc = 1.0f, bi = 0.0f;
-            if (n < p.N) {
-                if (is_int) {
-                    if (has_bias) bi = __int_as_float(__ldg(static_cast<const int32_t *>(p.bias) + n));
-                } else {
-                    sc = p.scale_is_scalar ? __ldg(p.scale) : __ldg(p.scale + n);
-                    if (has_bias) bi = load_bias_f32(p, n);
+            for (int i = lane; i < CC; i += 32) {
+                const int64_t n = n0 + i;
+                float sc = 1.0f, bi = 0.0f;
+                if (n < p.N) {
+                    if (is_int) {
+                        if (has_bias) bi = __int_as_float(__ldg(static_cast<const int32_t *>(p.bias) + n));
+                    } else {
+                        sc = p.scale_is_scalar ? __ldg(p.scale) : __ldg(p.scale + n);
+                        if (has_bias) bi = load_bias_f32(p, n);
+                    }
                 }
+                colbuf[i] = sc;
+                colbuf[64 + i] = bi;
             }
-            colbuf[i] = sc;
-            colbuf[64 + i] = bi;
+            __syncwarp();
         }
-        __syncwarp();
 
         uint8_t *dst_row = stage + buf * 4096 + lane * 128;
 #pragma unroll
         for (int h = 0; h < CC / 32; ++h) {
+            if constexpr (is_i8) {  // scale, offset and int32 bias of 32 columns at a time
+                const int64_t n = n0 + h * 32 + lane;
+                float sc = 0.0f, off = 0.0f;
+                int32_t bi = 0;
+                if (n < p.N) {
+                    sc = p.scale_is_scalar ? __ldg(p.scale) : __ldg(p.scale + n);
+                    if (p.offset != nullptr) off = p.offset_is_scalar ? __ldg(p.offset) : __ldg(p.offset + n);
+                    if (has_bias) bi = __ldg(static_cast<const int32_t *>(p.bias) + n);
+                }
+                __syncwarp();  // the previous columns' constants have been read
+                colbuf[lane] = sc;
+                colbuf[32 + lane] = off;
+                colbuf[64 + lane] = __int_as_float(bi);
+                __syncwarp();
+            }
             uint32_t acc[32];
             tmem_ld_32x32(taddr_warp + c * CC + h * 32, acc);
             tmem_ld_wait();
-            if constexpr (sizeof(OutT) == 4) {
+            if constexpr (is_i8) {
+                const bool has_off = p.offset != nullptr;
+#pragma unroll
+                for (int j = 0; j < 32; j += 16) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float4 s4 = *reinterpret_cast<const float4 *>(colbuf + j + q * 4);
+                        const float4 o4 = *reinterpret_cast<const float4 *>(colbuf + 32 + j + q * 4);
+                        const float4 b4 = *reinterpret_cast<const float4 *>(colbuf + 64 + j + q * 4);
+                        const float sv[4] = {s4.x, s4.y, s4.z, s4.w}, ov[4] = {o4.x, o4.y, o4.z, o4.w}, bv[4] = {b4.x, b4.y, b4.z, b4.w};
+                        w[q] = 0;
+#pragma unroll
+                        for (int t = 0; t < 4; ++t)
+                            w[q] |= (static_cast<uint32_t>(requant_one(static_cast<int32_t>(acc[j + q * 4 + t]) + __float_as_int(bv[t]), sv[t],
+                                                                       pt, has_pt, ov[t], has_off)) & 0xffu) << (8 * t);
+                    }
+                    const int chunk16 = (h * 32 + j) / 16;
+                    *reinterpret_cast<uint4 *>(dst_row + ((chunk16 ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+            } else if constexpr (sizeof(OutT) == 4) {
 #pragma unroll
                 for (int j = 0; j < 32; j += 4) {
                     const float4 b4 = *reinterpret_cast<const float4 *>(colbuf + 64 + h * 32 + j);
@@ -242,6 +246,12 @@ __device__ __forceinline__ void epilogue_warp_tile_tma(const EpilogueParams &p, 
                 }
             }
         }
+        if (!use_tma) {
+            __syncwarp();
+            epilogue_store_rows<OutT>(p, stage + buf * 4096, m_warp0, n0);
+            ++chunk_counter;
+            continue;
+        }
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
@@ -258,7 +268,13 @@ template <typename OutT>
 __device__ __forceinline__ void epilogue_one(const EpilogueParams &p, int64_t m, int64_t n, int32_t acc) {
     if (m >= p.M || n >= p.N) return;
     OutT *o = static_cast<OutT *>(p.out) + m * p.ld_out + n;
-    if constexpr (sizeof(OutT) == 4) {
+    if constexpr (sizeof(OutT) == 1) {
+        const bool has_pt = (p.pertoken_scale != nullptr), has_off = (p.offset != nullptr);
+        const float sc = p.scale_is_scalar ? __ldg(p.scale) : __ldg(p.scale + n);
+        const float off = has_off ? (p.offset_is_scalar ? __ldg(p.offset) : __ldg(p.offset + n)) : 0.0f;
+        const int32_t bi = p.bias != nullptr ? __ldg(static_cast<const int32_t *>(p.bias) + n) : 0;
+        *o = static_cast<OutT>(requant_one(acc + bi, sc, has_pt ? __ldg(p.pertoken_scale + m) : 1.0f, has_pt, off, has_off));
+    } else if constexpr (sizeof(OutT) == 4) {
         const bool has_bias = (p.bias != nullptr && p.bias_dtype == QMM_DTYPE_I32);
         *reinterpret_cast<int32_t *>(o) = acc + (has_bias ? __ldg(static_cast<const int32_t *>(p.bias) + n) : 0);
     } else {

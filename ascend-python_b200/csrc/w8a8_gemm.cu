@@ -230,19 +230,9 @@ w8a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             tc_fence_after();
             const int64_t m_warp0 = static_cast<int64_t>(m_blk) * kBM + quarter * 32;
             const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kBN;
-            if (use_tma_store) {
-                epilogue_warp_tile_tma<OutT, kBN>(ep, &tmap_out, taddr, m_warp0, static_cast<int64_t>(n_blk) * kBN,
-                                                  my_stage, my_cols, chunk_counter,
-                                                  slices > 1 ? static_cast<int64_t>(slice) * slice_rows + m_warp0 : -1);
-            } else {
-#pragma unroll 1
-                for (int c = 0; c < kBN / 32; ++c) {
-                    uint32_t acc[32];
-                    tmem_ld_32x32(taddr + c * 32, acc);
-                    tmem_ld_wait();
-                    epilogue_row_segment<OutT, 32>(ep, m_warp0 + lane, static_cast<int64_t>(n_blk) * kBN + c * 32, acc);
-                }
-            }
+            epilogue_warp_tile<OutT, kBN>(ep, &tmap_out, use_tma_store != 0, taddr, m_warp0, static_cast<int64_t>(n_blk) * kBN,
+                                          my_stage, my_cols, chunk_counter,
+                                          slices > 1 ? static_cast<int64_t>(slice) * slice_rows + m_warp0 : -1);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&tail->tmem_empty[buf]));
@@ -602,6 +592,8 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
                     return launch_tile<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, stream);
                 case QMM_DTYPE_F16:
                     return launch_tile<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, stream);
+                case kOutI8:
+                    return launch_tile<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, stream);
                 default:
                     return launch_tile<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, stream);
             }
@@ -619,6 +611,8 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
                     return launch_tile_splitk<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, stream);
                 case QMM_DTYPE_F16:
                     return launch_tile_splitk<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, stream);
+                case kOutI8:
+                    return launch_tile_splitk<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, stream);
                 default:
                     return launch_tile_splitk<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, stream);
             }
@@ -630,6 +624,8 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
                     return launch_simt<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, stream);
                 case QMM_DTYPE_F16:
                     return launch_simt<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, stream);
+                case kOutI8:
+                    return launch_simt<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, stream);
                 default:
                     return launch_simt<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, stream);
             }

@@ -329,26 +329,16 @@ w8a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             tc_fence_after();
             const int64_t m_warp0 = static_cast<int64_t>(m_blk) * 2 * kPM + cta_rank * kPM + quarter * 32;
             const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * kPN;
-            if (use_tma_store) {
-                // with push targets the tile goes to the receive area of the rank that owns its rows
-                const CUtensorMap *omap = &tmap_out;
-                int64_t store_row0 = -1;
-                if (push.enabled) {
-                    const int owner = static_cast<int>(m_warp0 / push.rows_per);
-                    omap = &push.m[owner];
-                    store_row0 = m_warp0 - owner * push.rows_per;
-                }
-                epilogue_warp_tile_tma<OutT, kPN>(ep, omap, taddr, m_warp0, static_cast<int64_t>(n_blk) * kPN,
-                                                  my_stage, my_cols, chunk_counter, store_row0);
-            } else {
-#pragma unroll 1
-                for (int c = 0; c < kPN / 32; ++c) {
-                    uint32_t acc[32];
-                    tmem_ld_32x32(taddr + c * 32, acc);
-                    tmem_ld_wait();
-                    epilogue_row_segment<OutT, 32>(ep, m_warp0 + lane, static_cast<int64_t>(n_blk) * kPN + c * 32, acc);
-                }
+            // with push targets the tile goes to the receive area of the rank that owns its rows
+            const CUtensorMap *omap = &tmap_out;
+            int64_t store_row0 = -1;
+            if (push.enabled) {
+                const int owner = static_cast<int>(m_warp0 / push.rows_per);
+                omap = &push.m[owner];
+                store_row0 = m_warp0 - owner * push.rows_per;
             }
+            epilogue_warp_tile<OutT, kPN>(ep, omap, use_tma_store != 0, taddr, m_warp0, static_cast<int64_t>(n_blk) * kPN, my_stage,
+                                          my_cols, chunk_counter, store_row0);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tail->tmem_empty[buf]), 0));
@@ -496,6 +486,8 @@ int launch_pair(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk
             return launch_pair_t<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, opts, stream);
         case QMM_DTYPE_F16:
             return launch_pair_t<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, opts, stream);
+        case kOutI8:
+            return launch_pair_t<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, opts, stream);
         default:
             return launch_pair_t<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, opts, stream);
     }

@@ -237,7 +237,9 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const bool has_pt = (ep.pertoken_scale != nullptr);
             bool has_bias = false;
             if (n_ok) {
-                if constexpr (sizeof(OutT) == 4) {
+                if constexpr (sizeof(OutT) == 1) {
+                    // fetched where it is used
+                } else if constexpr (sizeof(OutT) == 4) {
                     has_bias = (ep.bias != nullptr && ep.bias_dtype == QMM_DTYPE_I32);
                     if (has_bias) bi32 = __ldg(static_cast<const int32_t *>(ep.bias) + n);
                 } else {
@@ -249,7 +251,9 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             }
             auto finish = [&](int m, int32_t acc) {
                 OutT *o = static_cast<OutT *>(ep.out) + static_cast<int64_t>(m) * ep.ld_out + n;
-                if constexpr (sizeof(OutT) == 4) {
+                if constexpr (sizeof(OutT) == 1) {
+                    epilogue_one<OutT>(ep, m, n, acc);
+                } else if constexpr (sizeof(OutT) == 4) {
                     *reinterpret_cast<int32_t *>(o) = acc + bi32;
                 } else {
                     const float pt = has_pt ? tail->pertoken[m] : 1.0f;
@@ -404,6 +408,8 @@ int launch_streamk(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2
             return launch_streamk_t<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), stream);
         case QMM_DTYPE_F16:
             return launch_streamk_t<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), stream);
+        case kOutI8:
+            return launch_streamk_t<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), stream);
         default:
             return launch_streamk_t<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), stream);
     }

@@ -1,0 +1,34 @@
+"""Outputs of the W8A8 kernels at the edges of their epilogue: rows that break TMA's 16-byte rules (odd widths with the
+transposed weight view), partial tiles in both directions, every output type, scalar and per-column constants.  All
+results are exact: integer sums, then fp32 operations with one rounding each in a fixed order."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float16, torch.int32, torch.int8])
+@pytest.mark.parametrize("shape", [(1, 32, 17), (13, 256, 129), (31, 2064, 257), (128, 1040, 385), (129, 160, 255),
+                                   (300, 144, 513), (300, 144, 512), (515, 272, 100), (40, 4096, 264)])
+def test_edges(capi, oracle, dev, shape, out):
+    M, K, N = shape
+    g = torch.Generator().manual_seed(M * 31 + N)
+    a = torch.randint(-127, 128, (M, K), generator=g, dtype=torch.int8)
+    wt = torch.randint(-127, 128, (N, K), generator=g, dtype=torch.int8)  # stored [N, K], used as its transposed view
+    pt = torch.rand(M, generator=g) * 1e-2 + 1e-3
+    whole = not out.is_floating_point
+    bias = torch.randint(-4096, 4096, (N,), generator=g, dtype=torch.int32) if whole else torch.randn(N, generator=g).to(out)
+    for scalar in (False, True):
+        n = 1 if scalar else N
+        scale = torch.rand(n, generator=g) * (0.02 if out == torch.int8 else 1e-2) + 1e-4
+        offset = torch.empty(n).uniform_(-9, 9, generator=g) if out == torch.int8 else None
+        d = [t.to(dev) for t in (a, wt, scale, pt, bias)]
+        if out == torch.int8:
+            y = capi.quant_matmul_int8(d[0], d[1].t(), d[2], offset=offset.to(dev), pertoken_scale=d[3], bias=d[4])
+        elif out == torch.int32:
+            y = capi.quant_matmul(d[0], d[1].t(), None, bias=d[4], output_dtype=out)
+        else:
+            y = capi.quant_matmul(d[0], d[1].t(), d[2], pertoken_scale=d[3], bias=d[4], output_dtype=out)
+        want = oracle.quant_matmul(a, wt.t(), scale, offset=offset, pertoken_scale=pt if out != torch.int32 else None,
+                                   bias=bias, output_dtype=out)
+        assert torch.equal(y.cpu(), want)
