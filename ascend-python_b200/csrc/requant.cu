@@ -1,8 +1,7 @@
 // int8 output of npu_quant_matmul (`output_dtype = int8`, with the optional `offset`).
 //
-// The operator and its arithmetic are not in the reference snapshot; the form below is this build's
-// stated choice (the argument list is the one the task gives: x1, x2, scale, offset, pertoken_scale,
-// bias, output_dtype):
+// The reference does not define this operator's arithmetic; the stated choice here (x1, x2, scale, offset,
+// pertoken_scale, bias, output_dtype) is:
 //     acc[m,n] = sum_k x1[m,k] * x2[k,n] + bias[n]                      int32, exact (bias int32)
 //     v        = float(acc) * scale[n] (* pertoken_scale[m]) (+ offset[n])   fp32, one rounding per operation
 //     out      = clamp(rint(v), -128, 127)                              round half to even

@@ -30,20 +30,23 @@
 // tensor memory over the whole K range: no per-group pass over the accumulator, whatever M is.
 //
 // Warp roles (736 threads): warp 0 streams the packed weights (a stage is a pair of blocks = 17408
-// contiguous bytes, one bulk copy); warp 1 streams the matching [Mpad][256 k] activation tiles by TMA
-// into a ring of their own; warp 2 issues the MMAs (eight per block under one election: the issue
-// rate of these small MMAs, about 45 clocks each, is one of the kernel's limits); warps 3-18 unpack
+// contiguous bytes, one bulk copy); warp 1 streams the matching activation tiles by TMA into a ring
+// of their own; warp 2 issues the MMAs (several under one election); warps 3-18 unpack
 // (four teams of four warps; team s converts sub-step s of both blocks of a stage; a warp touches the
-// 32 tensor-memory lanes 32 * (warp % 4)); warps 19-22 are the epilogue.  The operand ring in tensor
-// memory holds three stages.  An unpack warp announces the operand columns of stage i only after it
-// has converted stage i+1, so the latency of its tensor-memory stores hides behind the next stage's
-// arithmetic.  Work is cut stream-K style into equal contiguous ranges of (column tile, block pair);
-// a tile shared by several CTAs is summed from per-CTA slots in slot order by the CTA that arrives
-// last, so results do not depend on arrival order.
+// 32 tensor-memory lanes 32 * (warp % 4)); warps 19-22 are the epilogue.  An unpack warp announces the
+// operand columns of stage i only after it has converted stage i+1, so the latency of its
+// tensor-memory stores hides behind the next stage's arithmetic.  A narrow form serves up to 64 token
+// rows, a wide form row tiles of up to 256 (PForm).  Work is cut into contiguous ranges of (output
+// tile, block pair), equal shares or whole tiles; a tile shared by several CTAs is summed from per-CTA
+// slots in slot order by the CTA that arrives last, so results do not depend on arrival order.
 //
-// Measured bounds (B200, M = 16, K = 8192, N = 28672, per 256-k stage and SM): the conversion costs
-// about 670 clocks per unpack warp - the packed 16-bit subtract and multiply-add issue at half rate on
-// this part (64 lanes per clock and SM) - and the issue of the stage's 16 MMAs about 730 clocks.
+// Measured bounds (B200, K = 8192, N = 28672).  Narrow: instruction issue.  The conversion is 15
+// instructions per word (the packed 16-bit ones and the logic ones issue at half rate, 64 lanes per
+// clock and SM), about 1100 clocks per 256-k stage and SM where the memory needs 760: 16 tokens 37 us,
+// 64 tokens 38-41 us.  An MMA of these sizes takes about 17 clocks when eight are issued under one
+// election with uniform operands; with the role index not known to be warp-uniform the MMA warp spent
+// 75 clocks on each (45 / 51 us).  Wide: the tensor pipe and the power cap: 256 tokens 100 us, 2048
+// tokens 733 us = 1.31 PFLOP/s of a measured 1.41 sustained.
 #include "qmm_common.cuh"
 #include "w4a16_simt.cuh"
 
@@ -724,10 +727,10 @@ size_t p_packed_bytes(int64_t N, int64_t K) {
 // measured slower still (37 us against 33 us at two tokens): the loads are not the limit.  Making the digits inside this kernel (every
 // CTA for its own blocks) instead of in a kernel in front was measured slower: 30 us against 26 us for one token;
 // so was pulling lines of later blocks into L2 with prefetch instructions (29.6 us).
-// Two mma.sync forms of the same idea (the split words as register operands of m16n8k32.s8 on these digits, or
-// pairs (k, k+1) as 16-bit operands of m16n8k16) were built and measured for 3..16 tokens: correct, but the legacy
-// MMA instructions cost 10-19 clocks each per SM on this part (41 / 63 us at 8 tokens, 63 / 116 us at 16), slower
-// than the kernels those sizes already have.  Work is cut into equal contiguous
+// mma.sync forms of the same idea (the split words as register operands of m16n8k32 on these digits, pairs (k, k+1)
+// as 16-bit operands of m16n8k16, the nibbles as e4m3) were built and measured: correct, and the 16-bit and int8 MMAs
+// take 2.0 clocks an SM, but issue bounds them: 28 us at one token, 30 at eight, 42 at sixteen for the int8 form with
+// its digits made in the kernel, 35 / 45 us with 16-bit operands; the e4m3 MMA is emulated (43 / 71 us).  Work is cut into equal contiguous
 // runs of blocks, many CTAs per SM; a tile's partial sums go to per-CTA slots that the last arriver adds in
 // slot order, as in the tensor-core kernel.
 constexpr int kGvMaxM = 2;            // measured (K=8192, N=28672): 26 / 33 us for 1 / 2 tokens, 41 / 51 us for 3 / 4

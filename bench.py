@@ -807,7 +807,7 @@ def run_case(args):
         gamma = torch.randn(K, device=dev, dtype=torch.bfloat16)
         fn = lambda i: capi.rms_norm(xs[i % nb], gamma, 1e-6)  # noqa: E731
     elif args.case == "quant_matmul_int8":
-        # the requantized int8 output: int32 accumulator pass + requantize kernel
+        # the requantized int8 output (in the matmul kernels' epilogue)
         a = torch.randint(-127, 128, (M, K), dtype=torch.int8, device=dev)
         ws = [torch.randint(-127, 128, (K, N), dtype=torch.int8, device=dev) for _ in range(nb)]
         scale = torch.empty(N, device=dev).uniform_(1e-5, 1e-4)

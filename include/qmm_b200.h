@@ -155,8 +155,8 @@ QMM_API int qmm_quant_matmul(const int8_t *x1, int64_t ld_x1, const int8_t *x2, 
  *   acc = x1 @ x2 + bias (int32, exact);  v = float(acc) * scale[n] (* pertoken_scale[m]) (+ offset[n])  in fp32,
  *   one rounding per operation;  out = clamp(rint(v), -128, 127), ties to even.
  * scale / offset: fp32 with N elements or one; offset, pertoken_scale and bias (int32 [N]) may be NULL.
- * workspace: 256-byte aligned, qmm_quant_matmul_int8_workspace_size bytes; it holds the matmul kernels' own
- * scratch (cleared by the call) and the int32 accumulator, and needs no preparation by the caller.
+ * workspace: 256-byte aligned, qmm_quant_matmul_int8_workspace_size bytes (never 0); it holds the matmul kernels'
+ * own scratch (cleared by the call) and needs no preparation by the caller.
  */
 QMM_API int qmm_quant_matmul_int8_workspace_size(int64_t M, int64_t N, int64_t K, size_t *bytes);
 QMM_API int qmm_quant_matmul_int8(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_stride_k,
