@@ -96,6 +96,12 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// the int8 results are the low bytes of the biased floats: gather (b0..b3) and (b4..b7)
+__device__ __forceinline__ uint2 gather_low_bytes(const uint32_t (&b)[8]) {
+    return make_uint2(__byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410),
+                      __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410));
+}
+
 // int8 values of eight row elements, packed (elements 0..3 in .x, 4..7 in .y).  `fast`: the row's scale
 // meets the preconditions of the FMA-pipe division (uniform over the row).
 __device__ __forceinline__ uint2 quantize8(const float (&f)[8], const RowQuant &rq, bool fast) {
@@ -111,9 +117,7 @@ __device__ __forceinline__ uint2 quantize8(const float (&f)[8], const RowQuant &
             const float q1 = fmaf(rem, rq.inv, q0);  // the IEEE quotient f / scale
             b[j] = __float_as_uint(q1 + kMagic);
         }
-        // the int8 results are the low bytes of the biased floats: gather (b0..b3) and (b4..b7)
-        lo = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
-        hi = __byte_perm(__byte_perm(b[4], b[5], 0x0040), __byte_perm(b[6], b[7], 0x0040), 0x5410);
+        return gather_low_bytes(b);
     } else {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {

@@ -15,6 +15,8 @@
 // amax / 127, q = rint(y / scale), exactly the arithmetic of qmm_dynamic_quant applied to the y that
 // qmm_rms_norm would have stored, so fused and unfused results are identical bit for bit while y
 // never travels to HBM and back (2 * cols bytes written + 2 * cols bytes read per row saved).
+#include <type_traits>
+
 #include "dynamic_quant.cuh"
 
 namespace qmm {
@@ -178,6 +180,175 @@ rms_norm_vec_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_
     }
 }
 
+// two fp32 operations an instruction, each rounded as the scalar one
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("{.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "mul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+        "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "add.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+
+// The fused kernel for rows of up to 256 threads: a CTA walks rows.  FULL: the row fills all vectors (cols == tpr * VPT *
+// 8), no guards.  What bounds it is instruction issue: with one row per CTA and scalar arithmetic (the kernel above) it
+// took 20 instructions an element, 29.3 us at 8192 x 4096 where the memory needs 15.  So the fp32 arithmetic is two
+// elements an instruction where its order allows, guards and the choice of quantizer are outside the loops over
+// elements, there is a variant for every number of vectors, and the next row's loads are under way while a row is
+// worked on (its registers are free as soon as the row is unpacked).  8192 x 4096: 25.4 us; 8192 x 8192: 50.6 -> 45.8;
+// 4096 x 16384: 52.1 -> 47.8; 4096 x 5128: 20.4 -> 18.9.  Rows of 512 threads leave one CTA an SM and nothing to overlap
+// its barriers with (1000 x 30000: 30.1 us against 28.0): they stay with the kernel above, and so does the plain
+// operator, which is close to the memory's rate.  The sum of squares is taken in that kernel's order.
+template <typename T, int VPT, bool FULL>
+__global__ void __launch_bounds__(256, 2)
+rms_norm_quant_walk_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_x, const T *__restrict__ gamma,
+                    float eps, int8_t *__restrict__ q, int64_t ld_q,
+                    float *__restrict__ scale, float *__restrict__ rstd_out, int tpr) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int E = VecOf<T>::kElems, H = E / 2;
+    static_assert(E == 8, "16-bit types");
+    constexpr bool kKeepGamma = VPT * E <= 32;
+    __shared__ float s_part[2][2][8];  // [row parity][sum, absmax][warp]
+    const int tpr_shift = __ffs(tpr) - 1;
+    const int rows_per_cta = blockDim.x >> tpr_shift;
+    const int row_in_cta = threadIdx.x >> tpr_shift;
+    const int t = threadIdx.x & (tpr - 1);
+    const int nvec = cols / E;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warps_per_row = tpr >> 5;
+    const int w0 = row_in_cta * warps_per_row;
+    auto has = [&](int i) { return FULL || t + i * tpr < nvec; };
+
+    float2 g[kKeepGamma ? VPT : 1][H];
+    auto load_gamma = [&](int i, float2 (&out)[H]) {
+        float f[E];
+        unpack_vec<T>(has(i) ? __ldg(reinterpret_cast<const uint4 *>(gamma) + t + i * tpr) : make_uint4(0, 0, 0, 0), f);
+#pragma unroll
+        for (int j = 0; j < H; ++j) out[j] = make_float2(f[2 * j], f[2 * j + 1]);
+    };
+    if constexpr (kKeepGamma) {
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) load_gamma(i, g[i]);
+    }
+    uint4 v[VPT];
+    auto load_row = [&](int64_t row) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(x + row * ld_x);
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) v[i] = row < rows && has(i) ? __ldg(src + t + i * tpr) : make_uint4(0, 0, 0, 0);
+    };
+    const int64_t step = static_cast<int64_t>(gridDim.x) * rows_per_cta;
+    int64_t row = static_cast<int64_t>(blockIdx.x) * rows_per_cta + row_in_cta;
+    load_row(row);
+    int parity = 0;
+    // all rows of a CTA advance together (the barriers below); rows beyond the last one are zeros and write nothing
+    for (int64_t base = static_cast<int64_t>(blockIdx.x) * rows_per_cta; base < rows; base += step, row += step, parity ^= 1) {
+        float2 f[VPT][H];
+        float sumsq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            float e[E];
+            unpack_vec<T>(v[i], e);
+#pragma unroll
+            for (int j = 0; j < H; ++j) {
+                f[i][j] = make_float2(e[2 * j], e[2 * j + 1]);
+                sumsq = fmaf(e[2 * j], e[2 * j], sumsq);
+                sumsq = fmaf(e[2 * j + 1], e[2 * j + 1], sumsq);
+            }
+        }
+        load_row(row + step);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sumsq += __shfl_xor_sync(0xffffffffu, sumsq, o);
+        if (tpr > 32) {
+            if (lane == 0) s_part[parity][0][warp] = sumsq;
+            __syncthreads();
+            float s = 0.0f;
+            for (int w = 0; w < warps_per_row; ++w) s += s_part[parity][0][w0 + w];
+            sumsq = s;
+        }
+        const float rstd = rstd_of(sumsq, cols, eps);
+        const bool row_ok = row < rows;
+        if (row_ok && t == 0) rstd_out[row] = rstd;
+
+        // y = (x * rstd) * gamma, rounded once to T
+        const float2 rstd2 = make_float2(rstd, rstd);
+        float amax = 0.0f;
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            float2 gi[H];
+            if constexpr (!kKeepGamma) load_gamma(i, gi);
+            float e[E];
+#pragma unroll
+            for (int j = 0; j < H; ++j) {
+                const float2 n = mul2(mul2(f[i][j], rstd2), kKeepGamma ? g[kKeepGamma ? i : 0][j] : gi[j]);
+                e[2 * j] = n.x;
+                e[2 * j + 1] = n.y;
+            }
+            const uint4 w = pack_vec<T>(e);
+            // guarded vectors hold zeros unless rstd is infinite or NaN: those rows are not finite anyway
+            if (FULL || has(i)) amax = max_nan(amax, dq::absmax8<T>(w));  // of the rounded values
+            unpack_vec<T>(w, e);
+#pragma unroll
+            for (int j = 0; j < H; ++j) f[i][j] = make_float2(e[2 * j], e[2 * j + 1]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if (tpr > 32) {
+            if (lane == 0) s_part[parity][1][warp] = amax;
+            __syncthreads();
+            float m = 0.0f;
+            for (int w = 0; w < warps_per_row; ++w) m = max_nan(m, s_part[parity][1][w0 + w]);
+            amax = m;
+        }
+        const dq::RowQuant rq = dq::make_row_quant(amax);
+        if (row_ok && t == 0) scale[row] = rq.scale;
+        uint2 *dst = reinterpret_cast<uint2 *>(q + row * ld_q);
+        if (!rq.exact_only && rq.scale != 0.0f) {  // as dq::quantize8, two elements an instruction
+            const float2 inv2 = make_float2(rq.inv, rq.inv), neg2 = make_float2(-rq.scale, -rq.scale);
+            const float2 magic2 = make_float2(12582912.0f, 12582912.0f);
+#pragma unroll
+            for (int i = 0; i < VPT; ++i) {
+                uint32_t b[E];
+#pragma unroll
+                for (int j = 0; j < H; ++j) {
+                    const float2 q0 = mul2(f[i][j], inv2);
+                    const float2 r = add2(fma2(fma2(q0, neg2, f[i][j]), inv2, q0), magic2);
+                    b[2 * j] = __float_as_uint(r.x);
+                    b[2 * j + 1] = __float_as_uint(r.y);
+                }
+                if (row_ok && has(i)) dst[t + i * tpr] = dq::gather_low_bytes(b);
+            }
+        } else if (row_ok) {
+#pragma unroll
+            for (int i = 0; i < VPT; ++i) {
+                float e[E];
+#pragma unroll
+                for (int j = 0; j < H; ++j) {
+                    e[2 * j] = f[i][j].x;
+                    e[2 * j + 1] = f[i][j].y;
+                }
+                if (has(i)) dst[t + i * tpr] = dq::quantize8(e, rq, false);
+            }
+        }
+    }
+}
+
 // Any column count, stride or alignment: one CTA per row, the row is read again from L2 for each pass.
 template <typename T, bool QUANT>
 __global__ void __launch_bounds__(256)
@@ -244,15 +415,35 @@ int launch_rms_norm(const T *x, int64_t rows, int64_t cols, int64_t ld_x, const 
         // the per-thread fixed cost (row scale, reductions, index arithmetic) is then spread over more elements
         while (tpr < 512 && tpr * 8 < nvec) tpr <<= 1;
         const int need = (nvec + tpr - 1) / tpr;
-        const int vpt = need <= 1 ? 1 : need <= 2 ? 2 : need <= 4 ? 4 : 8;
         const int threads = tpr > 128 ? tpr : 128;  // small CTAs: the tail of the grid is one CTA long
         const int rows_per_cta = threads / tpr;
         const int64_t grid = (rows + rows_per_cta - 1) / rows_per_cta;
         const int icols = static_cast<int>(cols);
-        auto kern = vpt == 1   ? rms_norm_vec_kernel<T, 1, QUANT>
-                    : vpt == 2 ? rms_norm_vec_kernel<T, 2, QUANT>
-                    : vpt == 4 ? rms_norm_vec_kernel<T, 4, QUANT>
-                               : rms_norm_vec_kernel<T, 8, QUANT>;
+        if constexpr (QUANT) {
+            if (tpr <= 256) {
+                const bool full = nvec == tpr * need;
+                auto pick = [&](auto v) {
+                    constexpr int V = decltype(v)::value;
+                    return full ? rms_norm_quant_walk_kernel<T, V, true> : rms_norm_quant_walk_kernel<T, V, false>;
+                };
+                using Kernel = decltype(&rms_norm_quant_walk_kernel<T, 1, true>);
+                const Kernel kernels[8] = {pick(std::integral_constant<int, 1>()), pick(std::integral_constant<int, 2>()),
+                                           pick(std::integral_constant<int, 3>()), pick(std::integral_constant<int, 4>()),
+                                           pick(std::integral_constant<int, 5>()), pick(std::integral_constant<int, 6>()),
+                                           pick(std::integral_constant<int, 7>()), pick(std::integral_constant<int, 8>())};
+                const int64_t resident = static_cast<int64_t>(sm_count()) * (512 / threads);
+                QMM_CUDA_OK(launch_pdl(kernels[need - 1], dim3(static_cast<unsigned>(grid < resident ? grid : resident)),
+                                       dim3(static_cast<unsigned>(threads)), 0, stream, x, rows, icols, ld_x, gamma, eps, q, ld_q,
+                                       scale, rstd, tpr));
+                return QMM_OK;
+            }
+        }
+        auto kern = rms_norm_vec_kernel<T, 8, QUANT>;  // fused: rows of more than 256 x 8 vectors only
+        if constexpr (!QUANT) {
+            if (need <= 1) kern = rms_norm_vec_kernel<T, 1, QUANT>;
+            else if (need <= 2) kern = rms_norm_vec_kernel<T, 2, QUANT>;
+            else if (need <= 4) kern = rms_norm_vec_kernel<T, 4, QUANT>;
+        }
         QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(static_cast<unsigned>(threads)), 0, stream, x, rows,
                                icols, ld_x, gamma, eps, y, ld_y, q, ld_q, scale, rstd, tpr));
     } else {

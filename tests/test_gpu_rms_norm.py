@@ -75,6 +75,29 @@ def test_fused_equals_composition(capi, oracle, dev, shape, dtype):
     np.testing.assert_allclose(scale.cpu().numpy(), scale_ref.numpy(), rtol=2.0 ** -7)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [8, 256, 504, 1032, 2048, 2056, 5128, 8192, 14344, 16384, 16392])
+def test_fused_equals_composition_many_rows(capi, dev, cols, dtype):
+    """Each row length class of the fused kernel (8 to 512 vectors of a row, full and partly filled, one length past
+    its range) with fewer and more rows than fit on the chip at once, rows of zeros, infinities, NaNs and extremes."""
+    g = torch.Generator(device=dev).manual_seed(cols)
+    for rows in (1, 7, 5003):
+        x = (torch.randn((rows, cols), generator=g, device=dev) * 3).to(dtype)
+        if rows > 1:
+            x[0] = 0
+            x[1, cols // 2] = float("inf")
+            x[2, 0] = float("nan")
+            x[3] *= 1e-6
+            x[rows - 1] = torch.finfo(dtype).max
+        gamma = (torch.rand(cols, generator=g, device=dev) - 0.3).to(dtype)
+        q, scale, rstd = capi.rms_norm_dynamic_quant(x, gamma, 1e-6)
+        y, rstd_u = capi.rms_norm(x, gamma, 1e-6)
+        q_u, scale_u = capi.dynamic_quant(y)
+        torch.testing.assert_close(rstd, rstd_u, rtol=0, atol=0, equal_nan=True)
+        torch.testing.assert_close(scale, scale_u, rtol=0, atol=0, equal_nan=True)
+        assert torch.equal(q, q_u)
+
+
 def test_full_size(capi, oracle, dev):
     """8192 x 4096 bf16 (the prefill activation): properties over the whole output, oracle on a row sample."""
     g = torch.Generator(device=dev).manual_seed(5)
