@@ -211,7 +211,7 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 // took 20 instructions an element, 29.3 us at 8192 x 4096 where the memory needs 15.  So the fp32 arithmetic is two
 // elements an instruction where its order allows, guards and the choice of quantizer are outside the loops over
 // elements, there is a variant for every number of vectors, and the next row's loads are under way while a row is
-// worked on (its registers are free as soon as the row is unpacked).  8192 x 4096: 25.4 us; 8192 x 8192: 50.6 -> 45.8;
+// worked on (its registers are free as soon as the row is unpacked).  8192 x 4096: 25.7 us; 8192 x 8192: 50.6 -> 45.8;
 // 4096 x 16384: 52.1 -> 47.8; 4096 x 5128: 20.4 -> 18.9.  Rows of 512 threads leave one CTA an SM and nothing to overlap
 // its barriers with (1000 x 30000: 30.1 us against 28.0): they stay with the kernel above, and so does the plain
 // operator, which is close to the memory's rate.  The sum of squares is taken in that kernel's order.
