@@ -119,7 +119,7 @@ struct PParams {
     int M, N;
     int mpad;         // token rows of a tile, a multiple of 16
     int nblk;         // tiles of token rows; an output tile is q = column tile * nblk + row tile
-    int share, extra, grain;  // see p_first_item; grain = nchunks: whole output tiles, 1: equal shares of the block pairs
+    int share, extra, grain;  // wide form, see p_first_item; grain = nchunks: whole output tiles, 1: equal shares of the block pairs
     int out_vec;      // rows of out meet the alignment of 8-byte stores
     int x_box_bytes;  // mpad * 128: one [mpad][64 k] activation box
     int nstages;      // packed-weight stages in shared memory
@@ -193,15 +193,26 @@ struct PMagic<__half> {
     static __device__ __forceinline__ T2 bias2() { return __floats2half2_rn(1032.0f, 1032.0f); }
 };
 
-// Items are dealt out in contiguous ranges of p.share, or one more for the first p.extra CTAs, times p.grain.
-__device__ __forceinline__ int p_first_item(const PParams &p, int cta) { return (cta * p.share + min(cta, p.extra)) * p.grain; }
+// Items are dealt out in contiguous ranges, as even as they go.  The narrow form cuts at total * cta / CTAs: where an fp32
+// sum is cut decides its last bits, so results of up to 64 tokens depend on this rule.  The wide form deals out p.share
+// items, or one more for the first p.extra CTAs, times p.grain.
+template <bool WIDE>
+__device__ __forceinline__ int p_first_item(const PParams &p, int cta) {
+    if constexpr (WIDE) return (cta * p.share + min(cta, p.extra)) * p.grain;
+    return static_cast<int>(static_cast<int64_t>(p.tiles_n) * p.nchunks * cta / gridDim.x);
+}
+template <bool WIDE>
 __device__ __forceinline__ int p_cta_of(const PParams &p, int item) {
-    const int i = item / p.grain, edge = p.extra * (p.share + 1);
-    return i < edge ? i / (p.share + 1) : p.extra + (i - edge) / p.share;
+    if constexpr (WIDE) {
+        const int i = item / p.grain, edge = p.extra * (p.share + 1);
+        return i < edge ? i / (p.share + 1) : p.extra + (i - edge) / p.share;
+    }
+    return p_cta_of_item(item, static_cast<int64_t>(p.tiles_n) * p.nchunks, gridDim.x);
 }
 // CTAs whose ranges overlap output tile q
+template <bool WIDE>
 __device__ __forceinline__ int p_slot_count(const PParams &p, int q) {
-    return p_cta_of(p, q * p.nchunks + p.nchunks - 1) - p_cta_of(p, q * p.nchunks) + 1;
+    return p_cta_of<WIDE>(p, q * p.nchunks + p.nchunks - 1) - p_cta_of<WIDE>(p, q * p.nchunks) + 1;
 }
 
 // Adds the slots of tile q in slot order and stores the tile; thread `tid` of `threads`.
@@ -258,7 +269,7 @@ __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots,
 // The calling threads have stored this CTA's sums of tile q: reports that, and if it completes the tile adds the slots
 // and stores the tile.  EPILOGUE: the four epilogue warps call, otherwise the whole CTA.  Inlined, and the parameters by
 // value: a call with their address costs the whole kernel its uniform registers (34 -> 43 us for 16 tokens).
-template <typename T, bool EPILOGUE>
+template <typename T, bool WIDE, bool EPILOGUE>
 __device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatile uint32_t *abort_flag, uint32_t *flag) {
     auto barrier = [] {
         if (EPILOGUE)
@@ -266,7 +277,7 @@ __device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatil
         else
             __syncthreads();
     };
-    const int nslots = p_slot_count(p, q);
+    const int nslots = p_slot_count<WIDE>(p, q);
     if (nslots <= 1) return;
     const int tid = static_cast<int>(threadIdx.x) - (EPILOGUE ? kPFirstEpiWarp * 32 : 0);
     barrier();
@@ -306,7 +317,7 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
     const int lane = threadIdx.x & 31;
     // this CTA's contiguous range of (output tile, block pair) items
     const int cta = static_cast<int>(blockIdx.x);
-    const int u_begin = p_first_item(p, cta), u_end = p_first_item(p, cta + 1);
+    const int u_begin = p_first_item<WIDE>(p, cta), u_end = p_first_item<WIDE>(p, cta + 1);
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < nstages; ++s) {
@@ -539,7 +550,7 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
             tc_fence_after();
             const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + pb * F::kTok;
             const int64_t slot_elems = static_cast<int64_t>(p.mpad) * kPTileN;
-            float *mine = p.slots + (static_cast<int64_t>(q) * p.max_slots + cta - p_cta_of(p, tile_begin)) * slot_elems + row;
+            float *mine = p.slots + (static_cast<int64_t>(q) * p.max_slots + cta - p_cta_of<WIDE>(p, tile_begin)) * slot_elems + row;
             T *o = out + static_cast<int64_t>(m0) * p.ld_out + n;
             for (int c0 = 0; c0 < p.mpad; c0 += 16) {
                 uint32_t v[16];
@@ -566,7 +577,7 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
             }
             // a tile that this CTA shares and leaves before the end of its range: these four warps report it, while
             // the others go on
-            if (!whole && seg_end < u_end) p_finish_shared<T, true>(p, q, abort_flag, &tail->is_last);
+            if (!whole && seg_end < u_end) p_finish_shared<T, WIDE, true>(p, q, abort_flag, &tail->is_last);
             u = seg_end;
         }
     }
@@ -582,7 +593,7 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
     // Output tiles shared with other CTAs: only the first and the last of a contiguous range can be.  The CTA that
     // arrives last adds the slots.  Most tiles are completed at the end of a range, by then with all threads, so that
     // the slots' loads of many elements are in flight together.
-    if (p.grain == 1 && u_begin < u_end) p_finish_shared<T, false>(p, (u_end - 1) / p.nchunks, abort_flag, &tail->is_last);
+    if (p.grain == 1 && u_begin < u_end) p_finish_shared<T, WIDE, false>(p, (u_end - 1) / p.nchunks, abort_flag, &tail->is_last);
 }
 
 // ---- layout pass and its inverse ----------------------------------------------------------------------

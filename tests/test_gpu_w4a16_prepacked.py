@@ -146,3 +146,32 @@ def test_more_than_64_rows(capi, oracle, dev, shape, dtype):
     y = capi.weight_quant_batchmatmul_prepacked(x.to(dev), buf, N)
     _assert_close(y, y_ref, _rss(oracle, x, packed_w, scale, offset, group), dtype)
     assert torch.equal(y, capi.weight_quant_batchmatmul_prepacked(x.to(dev), buf, N))
+
+
+@pytest.mark.parametrize("shape", [(3, 8192, 1024), (16, 8192, 1024), (64, 2304, 7168), (33, 28672, 1024)])
+def test_cut_points_up_to_64_rows(capi, dev, shape):
+    """Where the K sum of a tile is cut into partial sums decides its last bits: CTA c of G takes the block pairs
+    [total * c / G, total * (c + 1) / G).  One nonzero k per block pair (256 k), values 2^25, 2, 2, ..., 2, -2^25: a 2 is
+    lost in a sum that holds 2^25 (half of its unit, to even or cut off) and kept in one that starts after a cut, so the
+    output counts the pairs behind the cuts.  The sums below are exact or round as said; the output is a small integer."""
+    M, K, N = shape
+    pairs, tiles = K // 256, N // 128
+    total = pairs * tiles
+    G = min(total, torch.cuda.get_device_properties(dev).multi_processor_count)
+    assert total % G != 0
+    v = np.full(pairs, 2.0, dtype=np.float32)
+    v[0], v[-1] = 2.0 ** 25, -2.0 ** 25
+    x = torch.zeros((M, K), dtype=torch.bfloat16)
+    x[:, 5::256] = torch.from_numpy(v).to(torch.bfloat16)
+    w = torch.full((K, N // 8), 0x11111111, dtype=torch.int32)
+    buf = capi.w4a16_prepack(w.to(dev), torch.ones((1, N), dtype=torch.bfloat16, device=dev), None, group_size=0)
+    y = capi.weight_quant_batchmatmul_prepacked(x.to(dev), buf, N).float().cpu().numpy()
+    cuts = sorted({total * c // G for c in range(G + 1)} | {t * pairs for t in range(tiles + 1)})
+    expect = np.zeros(tiles, dtype=np.float32)
+    for a, b in zip(cuts, cuts[1:]):
+        part = np.float32(0)
+        for i in range(a, b):
+            part = np.float32(part + v[i % pairs])
+        expect[a // pairs] = np.float32(expect[a // pairs] + part)
+    assert len(np.unique(expect)) > 1
+    np.testing.assert_array_equal(y, np.broadcast_to(np.repeat(expect, 128), (M, N)))
