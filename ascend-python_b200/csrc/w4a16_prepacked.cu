@@ -126,8 +126,7 @@ struct PParams {
     int nxstages;     // activation tiles in shared memory
     int tiles_n;
     int nchunks;      // block PAIRS along K
-    int max_slots;
-    float *slots;        // [output tiles][max_slots][mpad][128]
+    float *slots;        // [slots][mpad][128], see p_slot
     uint32_t *counters;  // [output tiles], zero between calls
     uint32_t *status;
 };
@@ -215,14 +214,25 @@ __device__ __forceinline__ int p_slot_count(const PParams &p, int q) {
     return p_cta_of<WIDE>(p, q * p.nchunks + p.nchunks - 1) - p_cta_of<WIDE>(p, q * p.nchunks) + 1;
 }
 
-// Adds the slots of tile q in slot order and stores the tile; thread `tid` of `threads`.
-template <typename T>
+// Slot of CTA `cta`'s sums of output tile q.  A contiguous range shares at most its first and its last tile, so slots
+// belong to CTAs and not to tiles: a slot for every tile took 235 MB for 1000 x 4096 x 28672 and 1.88 GB for 8192 rows.
+// With T tiles for G CTAs, G + min(T, G) slots are enough.  T >= G: a range begins at or behind tile `cta`, the minimum
+// is cta + 0 or 1, two slots for every CTA.  T < G: it begins at or before tile `cta`, the minimum is q, and cta + q
+// grows from one (CTA, tile) pair to the next.
+template <bool WIDE>
+__device__ __forceinline__ int p_slot(const PParams &p, int cta, int q) {
+    return cta + min(q, cta + (p_first_item<WIDE>(p, cta) < q * p.nchunks ? 1 : 0));
+}
+
+// Adds the sums of tile q by its `nslots` CTAs in their order and stores the tile; thread `tid` of `threads`.
+template <typename T, bool WIDE>
 __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots, int tid, int threads) {
     const T *bias = static_cast<const T *>(p.bias);
     const int m0 = (q % p.nblk) * p.mpad, ncol0 = (q / p.nblk) * kPTileN;
     const int vecs = min(p.mpad, p.M - m0) * (kPTileN / 4);
     const int64_t slot_vecs = static_cast<int64_t>(p.mpad) * (kPTileN / 4);
-    const float4 *src = reinterpret_cast<const float4 *>(p.slots) + static_cast<int64_t>(q) * p.max_slots * slot_vecs;
+    const float4 *slots = reinterpret_cast<const float4 *>(p.slots);
+    const int cta0 = p_cta_of<WIDE>(p, q * p.nchunks), slot0 = p_slot<WIDE>(p, cta0, q);
     constexpr int kElems = 2;
     for (int e0 = tid; e0 < vecs; e0 += kElems * threads) {
         float4 v[kElems];
@@ -231,12 +241,15 @@ __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots,
         for (int s0 = 0; s0 < nslots; s0 += 4) {
             float4 part[4][kElems];
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
+            for (int k = 0; k < 4; ++k) {
+                const int cta = cta0 + s0 + k;  // only the first one's range can begin before the tile
+                const float4 *src = slots + (cta == cta0 ? slot0 : cta + min(q, cta)) * slot_vecs;
 #pragma unroll
                 for (int e = 0; e < kElems; ++e) {
                     part[k][e] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (s0 + k < nslots && e0 + e * threads < vecs) part[k][e] = __ldcg(src + (s0 + k) * slot_vecs + e0 + e * threads);
+                    if (s0 + k < nslots && e0 + e * threads < vecs) part[k][e] = __ldcg(src + e0 + e * threads);
                 }
+            }
 #pragma unroll
             for (int k = 0; k < 4; ++k)
 #pragma unroll
@@ -293,7 +306,7 @@ __device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatil
         *flag = last;
     }
     barrier();
-    if (*reinterpret_cast<volatile uint32_t *>(flag) != 0) p_add_slots<T>(p, q, nslots, tid, EPILOGUE ? kPEpiWarps * 32 : kPThreads);
+    if (*reinterpret_cast<volatile uint32_t *>(flag) != 0) p_add_slots<T, WIDE>(p, q, nslots, tid, EPILOGUE ? kPEpiWarps * 32 : kPThreads);
     barrier();  // the flag is written again for the next tile
 }
 
@@ -550,7 +563,7 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
             tc_fence_after();
             const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + pb * F::kTok;
             const int64_t slot_elems = static_cast<int64_t>(p.mpad) * kPTileN;
-            float *mine = p.slots + (static_cast<int64_t>(q) * p.max_slots + cta - p_cta_of<WIDE>(p, tile_begin)) * slot_elems + row;
+            float *mine = p.slots + p_slot<WIDE>(p, cta, q) * slot_elems + row;
             T *o = out + static_cast<int64_t>(m0) * p.ld_out + n;
             for (int c0 = 0; c0 < p.mpad; c0 += 16) {
                 uint32_t v[16];
@@ -658,7 +671,7 @@ w4a16_unpack_kernel(const uint8_t *__restrict__ packed, int64_t N, int64_t K, in
 }
 
 struct PPlan {
-    int mpad, nblk, tiles_n, nchunks, grid, share, extra, grain, max_slots, nstages, nxstages;
+    int mpad, nblk, tiles_n, nchunks, grid, share, extra, grain, nstages, nxstages;
     size_t slots_bytes, smem;
 };
 
@@ -700,8 +713,9 @@ PPlan p_make_plan(int64_t M, int64_t N, int64_t K) {
     pl.grid = static_cast<int>(grains < sms ? grains : sms);
     pl.share = static_cast<int>(grains / pl.grid);  // >= 1
     pl.extra = static_cast<int>(grains % pl.grid);
-    pl.max_slots = pl.grain > 1 ? 0 : (pl.nchunks + pl.share - 1) / pl.share + 1;
-    pl.slots_bytes = static_cast<size_t>(out_tiles) * pl.max_slots * pl.mpad * kPTileN * sizeof(float);
+    // p_slot; none where no tile is shared: whole tiles, which a single block pair along K always is
+    const int64_t slots = pl.grain == pl.nchunks ? 0 : pl.grid + (out_tiles < pl.grid ? out_tiles : pl.grid);
+    pl.slots_bytes = static_cast<size_t>(slots) * pl.mpad * kPTileN * sizeof(float);
     return pl;
 }
 
@@ -1091,7 +1105,6 @@ int launch_prepacked_t(const uint8_t *packed, const void *x, int64_t ld_x, const
     p.nxstages = pl.nxstages;
     p.tiles_n = pl.tiles_n;
     p.nchunks = pl.nchunks;
-    p.max_slots = pl.max_slots;
     uint8_t *ws = static_cast<uint8_t *>(workspace);
     p.counters = reinterpret_cast<uint32_t *>(ws);
     p.slots = reinterpret_cast<float *>(ws + kPCounterBytes);

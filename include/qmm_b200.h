@@ -240,7 +240,8 @@ QMM_API int qmm_weight_quant_batchmatmul(const void *x, int x_dtype, int64_t ld_
  *   - sdtype (BF16/F16) is the dtype of scale and offset and must equal the x_dtype used later.
  *   - packed: 16-byte aligned, at least qmm_w4a16_prepack_size bytes.
  *   - qmm_w4a16_unpack_weight restores the stock int32 [K, N/8] words exactly.
- *   - workspace of the matmul: 256-byte aligned, zero-filled before its first use only.
+ *   - workspace of the matmul: 256-byte aligned, its first 64 KiB zero-filled before the first use only; at most two
+ *     fp32 tiles of min(M, 256) x 128 for every SM behind them (38.8 MB on 148 SMs), whatever M, N and K are.
  */
 QMM_API int qmm_w4a16_prepack_size(int64_t N, int64_t K, int64_t group, size_t *bytes);
 QMM_API int qmm_w4a16_prepack(const int32_t *weight, int64_t ld_w, const void *antiquant_scale,

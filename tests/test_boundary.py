@@ -71,6 +71,19 @@ def test_validation_needs_no_gpu(capi):
     assert lib.qmm_weight_quant_batchmatmul_prepacked_workspace_size(0, 28672, 8192, ctypes.byref(n)) == 0 and n.value == 0
 
 
+def test_prepacked_scratch_is_bounded(capi):
+    """Scratch of the prepacked matmul: 64 KiB of counters and at most two fp32 tiles of up to 256 x 128 for every SM (148
+    where no device is visible), whatever M is; no tiles where no output tile is shared (one block pair along K)."""
+    lib, n = capi.lib(), ctypes.c_size_t(0)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 148
+    for M in (3, 64, 65, 200, 257, 1000, 4096, 8192, 65536):
+        for K, N in ((256, 28672), (512, 28672), (4096, 28672), (8192, 28672), (28672, 8192), (8192, 136), (4096, 12808)):
+            assert lib.qmm_weight_quant_batchmatmul_prepacked_workspace_size(M, N, K, ctypes.byref(n)) == 0
+            rows = min((M + 15) // 16 * 16, 256)
+            assert 65536 <= n.value <= 65536 + 2 * sms * rows * 128 * 4, (M, K, N)
+            assert K > 256 or n.value == 65536
+
+
 def test_missing_library_fails_loudly(capi, monkeypatch):
     monkeypatch.setattr(capi, "_lib", None)
     monkeypatch.setattr(capi, "LIB_PATH", Path("/nonexistent/libqmm_b200.so"))

@@ -175,3 +175,29 @@ def test_cut_points_up_to_64_rows(capi, dev, shape):
         expect[a // pairs] = np.float32(expect[a // pairs] + part)
     assert len(np.unique(expect)) > 1
     np.testing.assert_array_equal(y, np.broadcast_to(np.repeat(expect, 128), (M, N)))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(65, 8192, 136, 128), (200, 4096, 264, 4096), (257, 28672, 1032, 128),
+                                   (520, 2560, 12808, 256), (600, 4096, 1152, 128)])
+def test_more_than_64_rows_shared_tiles(capi, oracle, dev, shape, dtype):
+    """The wide form with equal shares: many CTAs a tile, several row tiles with a ragged last one, and tiles of two CTAs
+    whose ranges end inside them (on 148 SMs).  Bias; the second call finds the first one's counters; a call with another
+    plan (whole tiles) on the same scratch in between."""
+    M, K, N, group = shape
+    x, packed_w, scale, offset = oracle.make_w4a16_inputs(M, K, N, seed=M + K + N, group=group, dtype=dtype)
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(N)).to(dtype)
+    buf = capi.w4a16_prepack(packed_w.to(dev), scale.to(dev), offset.to(dev), group_size=group)
+    xd, bd = x.to(dev), bias.to(dev)
+    y = capi.weight_quant_batchmatmul_prepacked(xd, buf, N, bias=bd)
+    # a sample of columns: every tile's edges and something between
+    cols = sorted({c for c in range(0, N, 128)} | {min(c + 127, N - 1) for c in range(0, N, 128)} | set(range(64, N, 509)))
+    words = sorted({c // 8 for c in cols})
+    cols = torch.tensor([8 * i + j for i in words for j in range(8)])
+    y_ref = oracle.weight_quant_batchmatmul(x, packed_w[:, words], scale[:, cols], offset[:, cols], bias=bias[cols],
+                                            antiquant_group_size=group)
+    rss = _rss(oracle, x, packed_w[:, words], scale[:, cols], offset[:, cols], group)
+    _assert_close(y[:, cols.to(dev)], y_ref, rss, dtype)
+    capi.weight_quant_batchmatmul_prepacked(torch.ones((65, 256), dtype=dtype, device=dev),
+                                            torch.zeros(capi.w4a16_prepack_size(19200, 256, 256), dtype=torch.uint8, device=dev), 19200)
+    assert torch.equal(y, capi.weight_quant_batchmatmul_prepacked(xd, buf, N, bias=bd))
