@@ -205,6 +205,43 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         // every thread needs every row's per-token scale: one coalesced fetch per CTA, broadcasts afterwards
         if (ep.pertoken_scale != nullptr && row < M) tail->pertoken[row] = __ldg(ep.pertoken_scale + row);
         epi_bar_sync();
+        // constants of an output column, fetched once and not for every token row
+        struct Column {
+            float scale = 0.0f, add = 0.0f;  // add: the bias of a 16-bit output, the offset of an int8 one
+            int32_t bias = 0;                // of an int32 or int8 output
+        };
+        const bool has_pt = (ep.pertoken_scale != nullptr);
+        const bool has_add = sizeof(OutT) == 1 ? ep.offset != nullptr
+                                               : ep.bias != nullptr && ep.bias_dtype != QMM_DTYPE_NONE && ep.bias_dtype != QMM_DTYPE_I32;
+        auto column = [&](int64_t n) {
+            Column col;
+            if (n < ep.N) {
+                if constexpr (sizeof(OutT) != 2) {
+                    if (ep.bias != nullptr && ep.bias_dtype == QMM_DTYPE_I32) col.bias = __ldg(static_cast<const int32_t *>(ep.bias) + n);
+                }
+                if constexpr (sizeof(OutT) != 4) {
+                    col.scale = ep.scale_is_scalar ? __ldg(ep.scale) : __ldg(ep.scale + n);
+                    if constexpr (sizeof(OutT) == 1) {
+                        if (has_add) col.add = ep.offset_is_scalar ? __ldg(ep.offset) : __ldg(ep.offset + n);
+                    } else {
+                        if (has_add) col.add = load_bias_f32(ep, n);
+                    }
+                }
+            }
+            return col;
+        };
+        auto finish = [&](const Column &col, int64_t n, int m, int32_t acc) {
+            OutT *o = static_cast<OutT *>(ep.out) + static_cast<int64_t>(m) * ep.ld_out + n;
+            if constexpr (sizeof(OutT) == 4) {
+                *reinterpret_cast<int32_t *>(o) = acc + col.bias;
+            } else {
+                const float pt = has_pt ? tail->pertoken[m] : 1.0f;
+                if constexpr (sizeof(OutT) == 1)
+                    *o = static_cast<OutT>(requant_one(acc + col.bias, col.scale, pt, has_pt, col.add, has_add));
+                else
+                    *o = from_float<OutT>(dequant_one(acc, col.scale, pt, has_pt, col.add, has_add));
+            }
+        };
         int seg = 0;
         bool ok = true;
         int64_t u = u_begin;
@@ -231,36 +268,7 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const bool n_ok = n < ep.N;
             const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * 256 + h * kSkTileN;
 
-            // per-column constants of the dequantization
-            float sc = 0.0f, bi = 0.0f;
-            int32_t bi32 = 0;
-            const bool has_pt = (ep.pertoken_scale != nullptr);
-            bool has_bias = false;
-            if (n_ok) {
-                if constexpr (sizeof(OutT) == 1) {
-                    // fetched where it is used
-                } else if constexpr (sizeof(OutT) == 4) {
-                    has_bias = (ep.bias != nullptr && ep.bias_dtype == QMM_DTYPE_I32);
-                    if (has_bias) bi32 = __ldg(static_cast<const int32_t *>(ep.bias) + n);
-                } else {
-                    has_bias = (ep.bias != nullptr && ep.bias_dtype != QMM_DTYPE_NONE &&
-                                ep.bias_dtype != QMM_DTYPE_I32);
-                    sc = ep.scale_is_scalar ? __ldg(ep.scale) : __ldg(ep.scale + n);
-                    if (has_bias) bi = load_bias_f32(ep, n);
-                }
-            }
-            auto finish = [&](int m, int32_t acc) {
-                OutT *o = static_cast<OutT *>(ep.out) + static_cast<int64_t>(m) * ep.ld_out + n;
-                if constexpr (sizeof(OutT) == 1) {
-                    epilogue_one<OutT>(ep, m, n, acc);
-                } else if constexpr (sizeof(OutT) == 4) {
-                    *reinterpret_cast<int32_t *>(o) = acc + bi32;
-                } else {
-                    const float pt = has_pt ? tail->pertoken[m] : 1.0f;
-                    *o = from_float<OutT>(dequant_one(acc, sc, pt, has_pt, bi, has_bias));
-                }
-            };
-
+            const Column col = column(n);
             int32_t *ws = p.ws_acc + (static_cast<int64_t>(tile * kSkHalves + h) * p.mpad) * kSkTileN + row;
             for (int c = 0; c < p.mpad; c += 16) {
                 uint32_t acc[16];
@@ -272,7 +280,7 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                         const int m = c + j;
                         if (m < M) {
                             if (whole)
-                                finish(m, static_cast<int32_t>(acc[j]));
+                                finish(col, n, m, static_cast<int32_t>(acc[j]));
                             else
                                 atomicAdd(ws + static_cast<int64_t>(m) * kSkTileN, static_cast<int32_t>(acc[j]));
                         }
@@ -299,6 +307,7 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     for (int h = 0; h < kSkHalves; ++h) {
                         const int64_t n = static_cast<int64_t>(tile) * kSkUnitN + h * kSkTileN + row;
                         if (n < ep.N) {
+                            const Column col = column(n);
                             int32_t *ws = p.ws_acc + (static_cast<int64_t>(tile * kSkHalves + h) * p.mpad) * kSkTileN + row;
                             // sixteen independent loads at a time: one L2 round trip per batch, not per row
                             for (int m0 = 0; m0 < M; m0 += 16) {
@@ -311,7 +320,7 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                                     if (m0 + j < M) __stcg(ws + static_cast<int64_t>(m0 + j) * kSkTileN, 0);
 #pragma unroll
                                 for (int j = 0; j < 16; ++j)
-                                    if (m0 + j < M) epilogue_one<OutT>(ep, m0 + j, n, v[j]);
+                                    if (m0 + j < M) finish(col, n, m0 + j, v[j]);
                             }
                         }
                     }
