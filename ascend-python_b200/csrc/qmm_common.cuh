@@ -140,6 +140,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 
 // Programmatic dependent launch (launch_pdl below): the next kernel of the stream may be set up from here on; and:
 // everything that the kernels before this one wrote is visible, everything they read may be overwritten.
+// A kernel that uses tensor memory calls the first behind its allocation, in the warp that allocates.  One call of any
+// thread releases a CTA: in front of the allocation, a CTA of the next kernel that fits on the SM could take the columns
+// and then wait for this kernel, which waits for the columns.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -357,8 +357,8 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
     if (warp == kPMmaWarp) {
         tmem_alloc(smem_u32(&tail->tmem_base), kPTmemCols);
         tmem_relinquish();
+        pdl_launch_dependents();
     }
-    pdl_launch_dependents();
     pdl_wait();
     tc_fence_before();
     __syncthreads();

@@ -119,10 +119,10 @@ w8a8_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     if (warp == 1) {
         tmem_alloc(smem_u32(&tail->tmem_base), kTmemCols);
         tmem_relinquish();
+        // not with split-K: the reduce pass's CTAs would fill the SMs while this kernel still streams (M = 32, K = 28672,
+        // N = 8192: 50.4 us with the early start, 45.0 us without)
+        if (slices == 1) pdl_launch_dependents();
     }
-    // not with split-K: the reduce pass's CTAs would fill the SMs while this kernel still streams (M = 32, K = 28672,
-    // N = 8192: 50.4 us with the early start, 45.0 us without)
-    if (slices == 1) pdl_launch_dependents();
     pdl_wait();
     tc_fence_before();
     __syncthreads();

@@ -200,8 +200,8 @@ w8a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     if (warp == 1) {
         tmem_alloc_pair(smem_u32(&tail->tmem_base), kPTmemCols);
         tmem_relinquish_pair();
+        if constexpr (!FUSED) pdl_launch_dependents();
     }
-    if constexpr (!FUSED) pdl_launch_dependents();
     pdl_wait();
     tc_fence_before();
     __syncthreads();

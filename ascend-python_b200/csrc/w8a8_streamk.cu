@@ -99,8 +99,8 @@ w8a8_streamk_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     if (warp == 1) {
         tmem_alloc(smem_u32(&tail->tmem_base), kSkTmemCols);
         tmem_relinquish();
+        pdl_launch_dependents();
     }
-    pdl_launch_dependents();
     pdl_wait();
     tc_fence_before();
     __syncthreads();

@@ -1,4 +1,5 @@
 """Kernels whose set-up overlaps the end of the kernel before them (programmatic dependent launch): what it must not cost."""
+import re
 import sys
 from pathlib import Path
 
@@ -53,3 +54,17 @@ def test_odd_columns_back_to_back(npu, dev, op):
             "matmul": lambda: npu.npu_quant_matmul(a, w, scale, output_dtype=torch.bfloat16)}[op]
     together, apart = _us([call]), _us([call, lambda: one.add_(1)])
     assert together < apart, f"{together:.1f} us back to back, {apart:.1f} us apart"
+
+
+def test_released_behind_the_tensor_memory_allocation():
+    """A kernel that allocates tensor memory releases its successor behind that, in the allocating warp: released earlier,
+    a CTA of another kernel could hold the columns and wait for this one.  Read from the sources."""
+    checked = 0
+    for f in sorted((PKG_DIR / "csrc").glob("*.[ci]*")):
+        for body in re.split(r"\b__global__\b", re.sub(r"//[^\n]*", "", f.read_text()))[1:]:
+            if "tmem_alloc" in body and "pdl_launch_dependents" in body:
+                block = re.search(r"if \(warp == \w+\) \{\s*tmem_alloc[^{}]*\}", body)
+                assert block and block.group(0).count("pdl_launch_dependents") == 1, f.name
+                assert body.count("pdl_launch_dependents") == 1, f.name
+                checked += 1
+    assert checked >= 4
