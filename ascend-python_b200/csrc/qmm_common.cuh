@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 
 #include "qmm_b200.h"
 
@@ -576,8 +577,10 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
 // Launches a kernel whose set-up may overlap the end of the kernel before it in the stream.  Every kernel launched
 // this way calls pdl_wait() before its first access to global memory, so the order of a stream is kept whatever the
 // kernels around it are; what overlaps is the launch itself, the placing of the CTAs and the prologue.
+// overlap == false: an ordinary launch of such a kernel.
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+inline cudaError_t launch_pdl_if(bool overlap, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                 A &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -587,8 +590,12 @@ inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+    return launch_pdl_if(true, kern, grid, block, smem, stream, std::forward<A>(args)...);
 }
 
 #endif  // __CUDACC__

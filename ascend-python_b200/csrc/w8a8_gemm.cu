@@ -323,7 +323,7 @@ w8a8_simt_kernel(const int8_t *__restrict__ x1, int64_t ld_x1, const int8_t *__r
 // ---------------------------------------------------------------------------
 template <typename OutT>
 int launch_tile(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
-                const EpilogueParams &ep, int64_t K, int sm_reserve, cudaStream_t stream) {
+                const EpilogueParams &ep, int64_t K, int sm_reserve, bool overlap, cudaStream_t stream) {
     CUtensorMap ta, tb;
     int rc = make_tmap_2d(&ta, x1, 1, static_cast<uint64_t>(K), static_cast<uint64_t>(ep.M),
                           static_cast<uint64_t>(ld_x1), kBK, kBM, true);
@@ -356,8 +356,8 @@ int launch_tile(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk
     auto kern = mn_major ? w8a8_tile_kernel<OutT, true> : w8a8_tile_kernel<OutT, false>;
     QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(kTileSmemBytes)));
-    QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(kTileThreads), kTileSmemBytes, stream, ta, tb, tout, ep,
-                           static_cast<int>(K), use_tma_store, 1, 0, status));
+    QMM_CUDA_OK(launch_pdl_if(overlap, kern, dim3(static_cast<unsigned>(grid)), dim3(kTileThreads), kTileSmemBytes, stream, ta,
+                              tb, tout, ep, static_cast<int>(K), use_tma_store, 1, 0, status));
     return QMM_OK;
 }
 
@@ -455,7 +455,8 @@ size_t splitk_scratch_bytes(int64_t M, int64_t N, int64_t K) {
 
 template <typename OutT>
 int launch_tile_splitk(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
-                       const EpilogueParams &ep, int64_t K, void *workspace, int sm_reserve, cudaStream_t stream) {
+                       const EpilogueParams &ep, int64_t K, void *workspace, int sm_reserve, bool overlap,
+                       cudaStream_t stream) {
     const int slices = splitk_slices(ep.M, ep.N, K);
     const int64_t slice_rows = (ep.M + kBM - 1) / kBM * kBM;
     CUtensorMap ta, tb, tout;
@@ -491,8 +492,8 @@ int launch_tile_splitk(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_
     auto kern = mn_major ? w8a8_tile_kernel<int32_t, true> : w8a8_tile_kernel<int32_t, false>;
     QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(kTileSmemBytes)));
-    QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(kTileThreads), kTileSmemBytes, stream, ta, tb, tout, raw,
-                           static_cast<int>(K), 1, slices, static_cast<int>(slice_rows), device_status_word()));
+    QMM_CUDA_OK(launch_pdl_if(overlap, kern, dim3(static_cast<unsigned>(grid)), dim3(kTileThreads), kTileSmemBytes, stream, ta,
+                              tb, tout, raw, static_cast<int>(K), 1, slices, static_cast<int>(slice_rows), device_status_word()));
     if constexpr (sizeof(OutT) == 2) {
         if ((ep.N & 7) == 0 && (ep.ld_out & 7) == 0 && (reinterpret_cast<uintptr_t>(ep.out) & 15) == 0 && slices <= 8) {
             const unsigned gx = static_cast<unsigned>((ep.N / 8 + 255) / 256);
@@ -509,14 +510,14 @@ int launch_tile_splitk(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_
                           : slices == 6 ? splitk_reduce_vec8_kernel<OutT, 6>
                           : slices == 7 ? splitk_reduce_vec8_kernel<OutT, 7>
                                         : splitk_reduce_vec8_kernel<OutT, 8>;
-            QMM_CUDA_OK(launch_pdl(reduce, rg, dim3(256), 0, stream, sp, se, ep));
+            QMM_CUDA_OK(launch_pdl_if(overlap, reduce, rg, dim3(256), 0, stream, sp, se, ep));
             return QMM_OK;
         }
     }
     const int64_t vecs = ep.M * ep.N / 4;
     const int rgrid = static_cast<int>(vecs / 256 + 1 < 4 * sm_count() ? vecs / 256 + 1 : 4 * sm_count());
-    QMM_CUDA_OK(launch_pdl(splitk_reduce_kernel<OutT>, dim3(static_cast<unsigned>(rgrid)), dim3(256), 0, stream,
-                           static_cast<int32_t *>(workspace), slices, slice_rows * ep.N, ep));
+    QMM_CUDA_OK(launch_pdl_if(overlap, splitk_reduce_kernel<OutT>, dim3(static_cast<unsigned>(rgrid)), dim3(256), 0, stream,
+                              static_cast<int32_t *>(workspace), slices, slice_rows * ep.N, ep));
     return QMM_OK;
 }
 
@@ -558,7 +559,7 @@ bool tma_compatible(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x
 // Implemented in w8a8_streamk.cu
 int launch_streamk(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
                    const EpilogueParams &ep, int out_dtype, int64_t K, void *workspace, size_t workspace_bytes,
-                   cudaStream_t stream);
+                   bool overlap, cudaStream_t stream);
 size_t streamk_workspace_bytes(int64_t M, int64_t N, int64_t K);
 bool streamk_supported(int64_t M, int64_t N, int64_t K, int64_t x2_sn);
 
@@ -566,6 +567,8 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
                           const EpilogueParams &ep, int out_dtype, int64_t K, int algo, void *workspace,
                           size_t workspace_bytes, cudaStream_t stream, LaunchOptions *opts) {
     const int sm_reserve = (opts != nullptr && opts->sm_reserve > 0) ? opts->sm_reserve : 0;
+    // beside a collective every launch waits for the kernel before it: CTAs placed early would sit on the reserved SMs
+    const bool overlap = opts == nullptr;
     const bool tma_ok = tma_compatible(x1, ld_x1, x2, x2_sk, x2_sn) && K < (1ll << 31) && ep.M < (1ll << 31) &&
                         ep.N < (1ll << 31);
     if (algo == QMM_ALGO_AUTO) {
@@ -591,13 +594,13 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
         case QMM_ALGO_TCGEN05_TILE:
             switch (out_dtype) {
                 case QMM_DTYPE_BF16:
-                    return launch_tile<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, stream);
+                    return launch_tile<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, overlap, stream);
                 case QMM_DTYPE_F16:
-                    return launch_tile<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, stream);
+                    return launch_tile<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, overlap, stream);
                 case kOutI8:
-                    return launch_tile<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, stream);
+                    return launch_tile<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, overlap, stream);
                 default:
-                    return launch_tile<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, stream);
+                    return launch_tile<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, sm_reserve, overlap, stream);
             }
         case QMM_ALGO_TCGEN05_PAIR:
             return launch_pair(x1, ld_x1, x2, x2_sk, x2_sn, ep, out_dtype, K, opts, stream);
@@ -610,16 +613,16 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
                             "4 and the scratch qmm_quant_matmul_workspace_size reports");
             switch (out_dtype) {
                 case QMM_DTYPE_BF16:
-                    return launch_tile_splitk<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, stream);
+                    return launch_tile_splitk<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, overlap, stream);
                 case QMM_DTYPE_F16:
-                    return launch_tile_splitk<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, stream);
+                    return launch_tile_splitk<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, overlap, stream);
                 case kOutI8:
-                    return launch_tile_splitk<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, stream);
+                    return launch_tile_splitk<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, overlap, stream);
                 default:
-                    return launch_tile_splitk<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, stream);
+                    return launch_tile_splitk<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, overlap, stream);
             }
         case QMM_ALGO_TCGEN05_STREAMK:
-            return launch_streamk(x1, ld_x1, x2, x2_sk, x2_sn, ep, out_dtype, K, workspace, workspace_bytes, stream);
+            return launch_streamk(x1, ld_x1, x2, x2_sk, x2_sn, ep, out_dtype, K, workspace, workspace_bytes, overlap, stream);
         case QMM_ALGO_SIMT:
             switch (out_dtype) {
                 case QMM_DTYPE_BF16:

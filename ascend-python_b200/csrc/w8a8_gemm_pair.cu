@@ -406,7 +406,7 @@ int launch_pair_t(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = opts == nullptr ? 2 : 1;  // a matmul that talks to other GPUs starts on an idle GPU, as before
+    cfg.numAttrs = opts == nullptr ? 2 : 1;  // beside a collective: an ordinary launch
     int raster = pair_choose_raster(ep.M, ep.N, K, static_cast<int64_t>(sizeof(OutT)), pairs);
     PushMaps push;
     memset(&push, 0, sizeof(push));

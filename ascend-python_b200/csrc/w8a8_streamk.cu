@@ -363,7 +363,7 @@ size_t streamk_workspace_bytes(int64_t M, int64_t N, int64_t K) {
 template <typename OutT>
 static int launch_streamk_t(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
                             const EpilogueParams &ep, int64_t K, void *workspace, uint32_t *status,
-                            cudaStream_t stream) {
+                            bool overlap, cudaStream_t stream) {
     SkParams p;
     p.ep = ep;
     p.K = static_cast<int>(K);
@@ -398,13 +398,13 @@ static int launch_streamk_t(const int8_t *x1, int64_t ld_x1, const int8_t *x2, i
     auto kern = mn_major ? w8a8_streamk_kernel<OutT, true> : w8a8_streamk_kernel<OutT, false>;
     QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(kSkSmemBudget)));
-    QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(kSkThreads), smem, stream, tw, tx, p));
+    QMM_CUDA_OK(launch_pdl_if(overlap, kern, dim3(static_cast<unsigned>(grid)), dim3(kSkThreads), smem, stream, tw, tx, p));
     return QMM_OK;
 }
 
 int launch_streamk(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
                    const EpilogueParams &ep, int out_dtype, int64_t K, void *workspace, size_t workspace_bytes,
-                   cudaStream_t stream) {
+                   bool overlap, cudaStream_t stream) {
     if (!streamk_supported(ep.M, ep.N, K, x2_sn))
         return fail(QMM_ERR_UNSUPPORTED, "qmm_quant_matmul: the stream-K kernel handles 1 <= M <= 128 only");
     if (workspace == nullptr || workspace_bytes < streamk_workspace_bytes(ep.M, ep.N, K))
@@ -414,13 +414,13 @@ int launch_streamk(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2
         return fail(QMM_ERR_WORKSPACE, "qmm_quant_matmul: workspace must be 16-byte aligned");
     switch (out_dtype) {
         case QMM_DTYPE_BF16:
-            return launch_streamk_t<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), stream);
+            return launch_streamk_t<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), overlap, stream);
         case QMM_DTYPE_F16:
-            return launch_streamk_t<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), stream);
+            return launch_streamk_t<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), overlap, stream);
         case kOutI8:
-            return launch_streamk_t<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), stream);
+            return launch_streamk_t<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), overlap, stream);
         default:
-            return launch_streamk_t<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), stream);
+            return launch_streamk_t<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, device_status_word(), overlap, stream);
     }
 }
 
@@ -558,11 +558,11 @@ extern "C" int qmm_quant_matmul_decode_noalloc(const int8_t *x1, int64_t ld_x1, 
     ep.N = N;
     switch (out_dtype) {
         case QMM_DTYPE_BF16:
-            return launch_streamk_t<__nv_bfloat16>(x1, ld_x1, x2, x2_stride_k, x2_stride_n, ep, K, scratch, status, s);
+            return launch_streamk_t<__nv_bfloat16>(x1, ld_x1, x2, x2_stride_k, x2_stride_n, ep, K, scratch, status, true, s);
         case QMM_DTYPE_F16:
-            return launch_streamk_t<__half>(x1, ld_x1, x2, x2_stride_k, x2_stride_n, ep, K, scratch, status, s);
+            return launch_streamk_t<__half>(x1, ld_x1, x2, x2_stride_k, x2_stride_n, ep, K, scratch, status, true, s);
         default:
-            return launch_streamk_t<int32_t>(x1, ld_x1, x2, x2_stride_k, x2_stride_n, ep, K, scratch, status, s);
+            return launch_streamk_t<int32_t>(x1, ld_x1, x2, x2_stride_k, x2_stride_n, ep, K, scratch, status, true, s);
     }
 }
 

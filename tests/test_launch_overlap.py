@@ -1,4 +1,5 @@
 """Kernels whose set-up overlaps the end of the kernel before them (programmatic dependent launch): what it must not cost."""
+import ctypes
 import re
 import sys
 from pathlib import Path
@@ -68,3 +69,45 @@ def test_released_behind_the_tensor_memory_allocation():
                 assert body.count("pdl_launch_dependents") == 1, f.name
                 checked += 1
     assert checked >= 4
+
+
+class _EdgeData(ctypes.Structure):
+    _fields_ = [("from_port", ctypes.c_ubyte), ("to_port", ctypes.c_ubyte), ("type", ctypes.c_ubyte), ("reserved", ctypes.c_ubyte * 5)]
+
+
+def _overlapped_edges(call):
+    """Number of programmatic edges in the graph that `call` captures to."""
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        keep = call()
+    get_edges, handle, n = ctypes.CDLL("libcuda.so.1").cuGraphGetEdges_v2, ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert get_edges(handle, None, None, None, ctypes.byref(n)) == 0
+    ends, data = [(ctypes.c_void_p * (n.value + 1))() for _ in range(2)], (_EdgeData * (n.value + 1))()
+    assert get_edges(handle, ends[0], ends[1], data, ctypes.byref(n)) == 0
+    del keep, graph
+    return sum(d.type == 1 for d in data[:n.value])  # CU_GRAPH_DEPENDENCY_TYPE_PROGRAMMATIC
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(300, 512, 768), (300, 512, 32768), (300, 8192, 256)])
+def test_no_overlap_beside_collectives(npu, capi, dev, shape):
+    """The matmul launches of the all-reduce leave SMs to a collective: none may be placed early, whichever kernel takes the
+    last, small chunk of rows (stream-K, tile, split-K); the same matmuls outside it are."""
+    M, K, N = shape
+    lib = capi.lib()
+    uid = ctypes.create_string_buffer(capi.UNIQUE_ID_BYTES)
+    capi.check(lib.qmm_comm_unique_id(uid), "qmm_comm_unique_id")
+    capi.check(lib.qmm_comm_init_rank(b"overlap", uid, 1, 0), "qmm_comm_init_rank")
+    try:
+        a = torch.ones((M, K), dtype=torch.int8, device=dev)
+        w = torch.ones((K, N), dtype=torch.int8, device=dev)
+        scale, pt = torch.rand(N, device=dev), torch.rand(M, device=dev)
+        assert _overlapped_edges(lambda: npu.npu_mm_all_reduce_base(a, w, "overlap", reduce_op="sum", dequant_scale=scale,
+                                                                    pertoken_scale=pt, comm_turn=3)) == 0
+        plain = lambda: [npu.npu_quant_matmul(a[:44], w, scale, pertoken_scale=pt[:44], output_dtype=torch.bfloat16)  # noqa: E731
+                         for _ in range(2)]
+        assert _overlapped_edges(plain) > 0
+    finally:
+        capi.check(lib.qmm_comm_destroy(b"overlap"), "qmm_comm_destroy")
