@@ -111,3 +111,130 @@ def test_no_overlap_beside_collectives(npu, capi, dev, shape):
         assert _overlapped_edges(plain) > 0
     finally:
         capi.check(lib.qmm_comm_destroy(b"overlap"), "qmm_comm_destroy")
+
+
+class _Layer:
+    """Two quantized projections and a W4A16 one behind norms, all of 1024 columns: every call reads what the call before
+    wrote, and the allocator gives the buffers freed on the way out again."""
+
+    def __init__(self, npu, dev, seed):
+        g = torch.Generator(device=dev).manual_seed(seed)
+        self.npu = npu
+        self.w8 = torch.randint(-127, 128, (1024, 1024), generator=g, device=dev, dtype=torch.int8)
+        self.scale = torch.rand(1024, generator=g, device=dev) * 1e-3 + 1e-4
+        self.gamma = (torch.rand(1024, generator=g, device=dev) + 0.5).to(torch.bfloat16)
+        self.w4 = torch.randint(-2 ** 31, 2 ** 31 - 1, (1024, 128), generator=g, device=dev, dtype=torch.int64).to(torch.int32)
+        self.s4 = (torch.rand((8, 1024), generator=g, device=dev) * 1e-2).to(torch.bfloat16)
+
+    def steps(self, x, layers=3):
+        """The calls one by one: yields after each, ends with the result."""
+        npu = self.npu
+        for _ in range(layers):
+            q, s, _r = npu.npu_rms_norm_dynamic_quant(x, self.gamma)
+            yield
+            y = npu.npu_quant_matmul(q, self.w8, self.scale, pertoken_scale=s, output_dtype=torch.bfloat16)
+            yield
+            del q, s
+            y, _r = npu.npu_rms_norm(y, self.gamma)
+            yield
+            q, s = npu.npu_dynamic_quant(y)
+            yield
+            y = npu.npu_quant_matmul(q, self.w8.t(), self.scale, pertoken_scale=s, output_dtype=torch.bfloat16)
+            yield
+            del q, s
+            x = npu.npu_weight_quant_batchmatmul(y, self.w4, self.s4, antiquant_group_size=128)
+            yield
+        self.out = x
+
+    def run(self, x, sync=False):
+        for _ in self.steps(x):
+            if sync:
+                torch.cuda.synchronize()
+        return self.out
+
+
+ROWS = [1, 2, 5, 16, 64, 100, 300]  # every kernel of the two matmuls
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", ROWS)
+def test_chain_over_reused_buffers(npu, dev, M):
+    """Calls that overlap give what calls one after the other give, also when the input is overwritten right behind them."""
+    layer = _Layer(npu, dev, M)
+    g = torch.Generator(device=dev).manual_seed(M)
+    inputs = [torch.randn((M, 1024), generator=g, device=dev).to(torch.bfloat16) for _ in range(6)]
+    want = [layer.run(x, sync=True).clone() for x in inputs]
+    x = torch.empty_like(inputs[0])
+    for _ in range(3):
+        got = []
+        for i in inputs:
+            x.copy_(i)
+            got.append(layer.run(x))
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", ROWS)
+def test_chain_captured(npu, dev, M):
+    layer = _Layer(npu, dev, M + 100)
+    x = torch.zeros((M, 1024), device=dev, dtype=torch.bfloat16)
+    layer.run(x)  # weights prepacked
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = layer.run(x)
+    g = torch.Generator(device=dev).manual_seed(M)
+    for _ in range(4):
+        value = torch.randn((M, 1024), generator=g, device=dev).to(torch.bfloat16)
+        want = layer.run(value, sync=True).clone()
+        x.copy_(value)
+        graph.replay()
+        got = y.clone()
+        x.zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 16, 300])
+def test_two_streams(npu, dev, M):
+    layers = [_Layer(npu, dev, 7), _Layer(npu, dev, 8)]
+    xs = [torch.randn((M, 1024), device=dev).to(torch.bfloat16) for _ in layers]
+    want = [layer.run(x, sync=True).clone() for layer, x in zip(layers, xs)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(4):
+        gens = [layer.steps(x) for layer, x in zip(layers, xs)]
+        live = [True, True]
+        while any(live):  # call by call in turn
+            for i, gen in enumerate(gens):
+                if live[i]:
+                    with torch.cuda.stream(streams[i]):
+                        live[i] = next(gen, "end") is None
+        torch.cuda.synchronize()
+        assert all(torch.equal(layer.out, w) for layer, w in zip(layers, want))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [1, 2])
+def test_weight_rewritten_and_used_at_once(npu, dev, M):
+    """One or two tokens read weights before they wait for the kernel in front (which has waited): a weight written again,
+    and with it packed again, right before the call is the one that is used."""
+    K = N = 2048
+    g = torch.Generator(device=dev).manual_seed(5)
+    x = torch.randn((M, K), generator=g, device=dev).to(torch.bfloat16)
+    scale = (torch.rand((K // 128, N), generator=g, device=dev) * 1e-2).to(torch.bfloat16)
+    ws = [torch.randint(-2 ** 31, 2 ** 31 - 1, (K, N // 8), generator=g, device=dev, dtype=torch.int64).to(torch.int32)
+          for _ in range(4)]
+    want = []
+    for w in ws:
+        torch.cuda.synchronize()
+        want.append(npu.npu_weight_quant_batchmatmul(x, w, scale, antiquant_group_size=128))
+    torch.cuda.synchronize()
+    w = torch.zeros_like(ws[0])
+    for _ in range(3):
+        got = []
+        for v in ws:
+            w.copy_(v)
+            got.append(npu.npu_weight_quant_batchmatmul(x, w, scale, antiquant_group_size=128))
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
