@@ -1,6 +1,7 @@
 """Outputs of the W8A8 kernels at the edges of their epilogue: rows that break TMA's 16-byte rules (odd widths with the
 transposed weight view), partial tiles in both directions, every output type, scalar and per-column constants.  All
 results are exact: integer sums, then fp32 operations with one rounding each in a fixed order."""
+import ctypes
 import sys
 from pathlib import Path
 
@@ -35,6 +36,38 @@ def test_edges(capi, oracle, dev, shape, out):
         want = oracle.quant_matmul(a, wt.t(), scale, offset=offset, pertoken_scale=pt if out != torch.int32 else None,
                                    bias=bias, output_dtype=out)
         assert torch.equal(y.cpu(), want)
+
+
+@pytest.mark.parametrize("out", [torch.bfloat16, torch.float16, torch.int32, torch.int8])
+@pytest.mark.parametrize("shape", [(1, 256, 512), (40, 4096, 272), (64, 1024, 1040), (128, 512, 128), (300, 256, 784)])
+def test_output_pitch(capi, dev, shape, out):
+    """Row-major weight, output rows at odd addresses (pitch N + 3, one element from the start of the buffer) through the C
+    ABI: the bits of the contiguous call, and nothing written beside the rows."""
+    M, K, N = shape
+    g = torch.Generator(device=dev).manual_seed(M + N)
+    a = torch.randint(-127, 128, (M, K), generator=g, device=dev, dtype=torch.int8)
+    w = torch.randint(-127, 128, (K, N), generator=g, device=dev, dtype=torch.int8)
+    scale, pt = torch.rand(N, generator=g, device=dev) * 1e-2, torch.rand(M, generator=g, device=dev) * 1e-2
+    flat = torch.full((M * (N + 3) + 1,), 7, dtype=out, device=dev)
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    at, stream, lib, n = ctypes.c_void_p(flat.data_ptr() + flat.element_size()), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), capi.lib(), ctypes.c_size_t(0)
+    if out == torch.int8:
+        want = capi.quant_matmul_int8(a, w, scale, offset=scale, pertoken_scale=pt)
+        capi.check(lib.qmm_quant_matmul_int8_workspace_size(M, N, K, ctypes.byref(n)), "size")
+        ws = torch.zeros(n.value, dtype=torch.uint8, device=dev)
+        capi.check(lib.qmm_quant_matmul_int8(ptr(a), K, ptr(w), N, 1, ptr(scale), N, ptr(scale), N, ptr(pt), None, at, N + 3, M, N, K,
+                                             ptr(ws), n.value, stream), "matmul")
+    else:
+        whole = out == torch.int32
+        want = capi.quant_matmul(a, w, None if whole else scale, pertoken_scale=None if whole else pt, output_dtype=out)
+        capi.check(lib.qmm_quant_matmul_workspace_size(M, N, K, capi.ALGO_AUTO, ctypes.byref(n)), "size")
+        ws = torch.zeros(max(n.value, 16), dtype=torch.uint8, device=dev)
+        capi.check(lib.qmm_quant_matmul(ptr(a), K, ptr(w), N, 1, None if whole else ptr(scale), 0 if whole else N, None if whole else ptr(pt),
+                                        None, capi.DTYPE_NONE, at, capi.dtype_code(out), N + 3, M, N, K, capi.ALGO_AUTO, ptr(ws), n.value,
+                                        stream), "matmul")
+    rows = flat[1:].view(M, N + 3)
+    assert torch.equal(rows[:, :N], want)
+    assert (rows[:, N:] == 7).all() and flat[0] == 7
 
 
 def test_int8_stream_k_time(dev):

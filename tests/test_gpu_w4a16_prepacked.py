@@ -11,6 +11,8 @@ The bound asserted is
     |y - y_ref| <= 2 u * |y_ref| + 8 u * rss[m,n]             (u = 2^-9 bf16, 2^-12 f16)
 i.e. the output rounding plus about 18 standard deviations of the accumulated weight rounding.
 """
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -201,3 +203,32 @@ def test_more_than_64_rows_shared_tiles(capi, oracle, dev, shape, dtype):
     capi.weight_quant_batchmatmul_prepacked(torch.ones((65, 256), dtype=dtype, device=dev),
                                             torch.zeros(capi.w4a16_prepack_size(19200, 256, 256), dtype=torch.uint8, device=dev), 19200)
     assert torch.equal(y, capi.weight_quant_batchmatmul_prepacked(xd, buf, N, bias=bd))
+
+
+@pytest.mark.parametrize("shape", [(65, 256, 136), (96, 2048, 19208), (200, 4096, 264), (600, 4096, 1152), (33, 1024, 264)])
+def test_row_pitches_and_unaligned_output(capi, dev, shape):
+    """Rows of x with a pitch, rows of the output at odd addresses (stores element by element), with bias, through the C ABI:
+    the bits of the contiguous call, and nothing written beside the rows.  Whole and shared tiles."""
+    M, K, N = shape
+    g = torch.Generator(device=dev).manual_seed(M)
+    x = torch.randn((M, K), generator=g, device=dev).to(torch.bfloat16)
+    w = torch.randint(-2 ** 31, 2 ** 31 - 1, (K, N // 8), generator=g, device=dev, dtype=torch.int64).to(torch.int32)
+    scale = (torch.rand((K // 128, N), generator=g, device=dev) * 1e-2).to(torch.bfloat16)
+    bias = torch.randn(N, generator=g, device=dev).to(torch.bfloat16)
+    buf = capi.w4a16_prepack(w, scale, None, group_size=128)
+    want = capi.weight_quant_batchmatmul_prepacked(x, buf, N, bias=bias)
+    xp = torch.full((M, K + 24), float("nan"), dtype=torch.bfloat16, device=dev)
+    xp[:, :K] = x
+    flat = torch.full((M * (N + 5) + 1,), 7.0, dtype=torch.bfloat16, device=dev)
+    n = ctypes.c_size_t(0)
+    capi.check(capi.lib().qmm_weight_quant_batchmatmul_prepacked_workspace_size(M, N, K, ctypes.byref(n)), "size")
+    ws = torch.zeros(n.value, dtype=torch.uint8, device=dev)
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    for _ in range(2):
+        capi.check(capi.lib().qmm_weight_quant_batchmatmul_prepacked(
+            ptr(xp), capi.dtype_code(torch.bfloat16), K + 24, ptr(buf), buf.numel(), ptr(bias),
+            ctypes.c_void_p(flat.data_ptr() + 2), N + 5, M, N, K, ptr(ws), n.value,
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "matmul")
+        rows = flat[1:].view(M, N + 5)
+        assert torch.equal(rows[:, :N], want)
+        assert (rows[:, N:] == 7.0).all() and flat[0] == 7.0
