@@ -67,10 +67,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// A value that is the same in all lanes, in a form the compiler recognises as such.  Without it a branch on
-// `threadIdx.x / 32` counts as divergent, uniform registers are out of reach inside the branch, and every operand of
-// a tcgen05 or bulk-copy instruction is moved there by an instruction sequence of its own: an MMA issue loop with
-// operands that change per iteration then takes about 75 clocks per MMA, against 40 with it.
+// A value that is the same in all lanes, in a form the compiler recognises as such, which a branch on `threadIdx.x / 32`
+// is not.  An MMA issue loop with operands that change per iteration takes about 75 clocks per MMA without it, 40 with it.
 __device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ int warp_id_uniform() { return static_cast<int>(warp_uniform(threadIdx.x >> 5)); }
 
@@ -576,7 +574,11 @@ __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) {
 
 // Launches a kernel whose set-up may overlap the end of the kernel before it in the stream.  Every kernel launched
 // this way calls pdl_wait() before its first access to global memory, so the order of a stream is kept whatever the
-// kernels around it are; what overlaps is the launch itself, the placing of the CTAs and the prologue.
+// kernels around it are; what overlaps is the launch itself, the placing of the CTAs and the prologue.  One exception:
+// w4a16_gemv_kernel loads weights before its wait.  The kernel directly in front of it is always w4a16_gemv_digits_kernel,
+// which releases it only behind its own wait, when everything before the two (a weight just packed) is complete.
+// Not for kernels of a few long-running CTAs for every SM: their CTAs are placed around those of the kernel before them
+// (w8a8_simt_kernel), or around those of the same kernel if that releases its successor early (dynamic_quant_generic_kernel).
 // overlap == false: an ordinary launch of such a kernel.
 template <typename... P, typename... A>
 inline cudaError_t launch_pdl_if(bool overlap, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

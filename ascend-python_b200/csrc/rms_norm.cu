@@ -207,11 +207,12 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 }
 
 // The fused kernel for rows of up to 256 threads: a CTA walks rows.  FULL: the row fills all vectors (cols == tpr * VPT *
-// 8), no guards.  What bounds it is instruction issue: with one row per CTA and scalar arithmetic (the kernel above) it
-// took 20 instructions an element, 29.3 us at 8192 x 4096 where the memory needs 15.  So the fp32 arithmetic is two
+// 8), no guards.  With one row per CTA and scalar arithmetic (the kernel above) it was bound by instruction issue: 20
+// instructions an element, 30.8 us at 8192 x 4096 where the memory needs 15.  So the fp32 arithmetic is two
 // elements an instruction where its order allows, guards and the choice of quantizer are outside the loops over
 // elements, there is a variant for every number of vectors, and the next row's loads are under way while a row is
-// worked on (its registers are free as soon as the row is unpacked).  8192 x 4096: 25.7 us; 8192 x 8192: 50.6 -> 45.8;
+// worked on (its registers are free as soon as the row is unpacked).  8192 x 4096: 25.7 us, 16 instructions an element at
+// 63 % of the issue slots: 128 registers leave 16 warps an SM, too few to fill the rest; 8192 x 8192: 50.6 -> 45.8;
 // 4096 x 16384: 52.1 -> 47.8; 4096 x 5128: 20.4 -> 18.9.  Rows of 512 threads leave one CTA an SM and nothing to overlap
 // its barriers with (1000 x 30000: 30.1 us against 28.0): they stay with the kernel above, and so does the plain
 // operator, which is close to the memory's rate.  The sum of squares is taken in that kernel's order.

@@ -40,10 +40,11 @@
 // tile, block pair), equal shares or whole tiles; a tile shared by several CTAs is summed from per-CTA
 // slots in slot order by the CTA that arrives last, so results do not depend on arrival order.
 //
-// Measured bounds (B200, K = 8192, N = 28672).  Narrow: instruction issue.  The conversion is 15
+// Measured bounds (B200, K = 8192, N = 28672).  Narrow: the unpack warps.  The conversion is 15
 // instructions per word (the packed 16-bit ones and the logic ones issue at half rate, 64 lanes per
-// clock and SM), about 1100 clocks per 256-k stage and SM where the memory needs 760: 16 tokens 37 us,
-// 64 tokens 38-41 us.  An MMA of these sizes takes about 17 clocks when eight are issued under one
+// clock and SM), about 1100 clocks per 256-k stage and SM where the memory needs 760: 27 us of the 37 us
+// that 16 tokens take (64 tokens 38-41 us) at 66 % of the issue slots; the rest is start, last sums and
+// hand-offs between the roles.  An MMA of these sizes takes about 17 clocks when eight are issued under one
 // election with uniform operands; with the role index not known to be warp-uniform the MMA warp spent
 // 75 clocks on each (45 / 51 us).  Wide: the tensor pipe and the power cap: 256 tokens 100 us, 2048
 // tokens 733 us = 1.31 PFLOP/s of a measured 1.41 sustained.
@@ -280,8 +281,8 @@ __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots,
 }
 
 // The calling threads have stored this CTA's sums of tile q: reports that, and if it completes the tile adds the slots
-// and stores the tile.  EPILOGUE: the four epilogue warps call, otherwise the whole CTA.  Inlined, and the parameters by
-// value: a call with their address costs the whole kernel its uniform registers (34 -> 43 us for 16 tokens).
+// and stores the tile.  EPILOGUE: the four epilogue warps call, otherwise the whole CTA.  Inlined: as a call with the
+// parameters' address it slows the whole kernel down (34 -> 43 us for 16 tokens).
 template <typename T, bool WIDE, bool EPILOGUE>
 __device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatile uint32_t *abort_flag, uint32_t *flag) {
     auto barrier = [] {
@@ -691,8 +692,8 @@ PPlan p_make_plan(int64_t M, int64_t N, int64_t K) {
         pl.smem = 2048 + static_cast<size_t>(pl.nxstages) * pl.mpad * 512 + static_cast<size_t>(pl.nstages) * kPStageWBytes;
     } else {
         // As few row tiles as 256 columns of accumulator allow: every further one unpacks the weight again (1000 rows,
-        // K=4096, N=28672: 201 us with four row tiles, 205, 209, 214, 226 us with five to eight, although seven fill the
-        // last wave best).  Then the cheaper way of sharing tiles out by this model (clocks): a stage costs what its MMAs
+        // K=4096, N=28672, short runs at the full clock: 201 us with four row tiles, 205, 209, 214, 226 us with five to eight,
+        // although seven fill the last wave best; under the power cap 231 us with four, 244 with seven).  Then the cheaper way of sharing tiles out by this model (clocks): a stage costs what its MMAs
         // take (8 a row) or what unpacking it takes (about 1150), a tile some 12 a row more to leave tensor memory.
         // Whole tiles leave the last wave uneven; equal shares of the stages do not, but every CTA then writes up to two
         // tiles' sums and someone adds them (16 a row each).
@@ -747,8 +748,7 @@ size_t p_packed_bytes(int64_t N, int64_t K) {
 //     y[m, n] += scale * esc[m] * (128 D1 + D2) + (offset*scale - 8 scale) * xs[m],
 // esc = 2^(e - 14), xs = esc * sum X; the weight itself is never rounded.  About 1.3 instructions per weight
 // for one token; every further token adds 64 dp4a per block and thread, which at the rate dp4a issues here costs
-// 7-8 us per token, so beyond two tokens the tensor-core kernels are faster (the kernel itself is written for up
-// to four).  A form with four columns per lane, which needs a quarter of the broadcast loads of digits, was
+// 7-8 us per token, so beyond two tokens the tensor-core kernels are faster.  A form with four columns per lane, which needs a quarter of the broadcast loads of digits, was
 // measured slower still (37 us against 33 us at two tokens): the loads are not the limit.  Making the digits inside this kernel (every
 // CTA for its own blocks) instead of in a kernel in front was measured slower: 30 us against 26 us for one token;
 // so was pulling lines of later blocks into L2 with prefetch instructions (29.6 us).
@@ -808,7 +808,8 @@ w4a16_gemv_kernel(GvParams p) {
         const int64_t n = static_cast<int64_t>(tile) * kPTileN + r;
         const bool n_ok = n < p.N;
         const int nb = static_cast<int>(seg_end - u), b_first = static_cast<int>(u - tile_begin);
-        // the first two blocks' weights are on their way before anything else happens
+        // the first two blocks' weights are on their way before anything else happens, the wait below included: see launch_pdl
+        // for why that is safe
         const uint8_t *blk = p.packed + u * kPBlockBytes;
         uint4 wv[kPSubs], n1[kPSubs], n2[kPSubs];
 #pragma unroll
@@ -1077,9 +1078,7 @@ int launch_gemv_t(const uint8_t *packed, const void *x, int64_t ld_x, const void
     };
     switch (M) {
         case 1: return launch(w4a16_gemv_kernel<T, 1>);
-        case 2: return launch(w4a16_gemv_kernel<T, 2>);
-        case 3: return launch(w4a16_gemv_kernel<T, 3>);
-        default: return launch(w4a16_gemv_kernel<T, 4>);
+        default: return launch(w4a16_gemv_kernel<T, 2>);  // kGvMaxM
     }
 }
 

@@ -337,8 +337,8 @@ int launch_tile(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk
                           static_cast<uint64_t>(x2_sn), kBK, kBN, true);
     }
     if (rc != QMM_OK) return rc;
-    // The epilogue stores through TMA when the output meets the 16-byte rules; it writes
-    // straight from registers otherwise.
+    // The epilogue stores through TMA when the output meets the 16-byte rules, row by row from its staging
+    // buffer otherwise.
     constexpr int kElt = static_cast<int>(sizeof(OutT));
     CUtensorMap tout = ta;
     int use_tma_store = 0;
@@ -533,12 +533,13 @@ int launch_simt(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk
 }
 
 // Decode shapes (M <= 128): stream-K keeps every SM streaming weights whatever N is, but its split
-// tiles pay for the int32 scratch traffic, which grows with M.  Measured on B200 (graph replay):
-// K x N = 8192 x 28672: M = 1 stream-K 46.9 us, tile kernel 54.2 us; M = 8 49.8 / 52.8 us; M = 32
-// 59 / 44 us; M = 128 110 / 46 us.  So up to 16 tokens stream-K wins everywhere; beyond that the
-// one-CTA tile kernel is ahead as soon as its 128 x 256 tiles occupy most SMs.  Shapes with few tiles
-// and a long K (28672 x 8192) go to the tile kernel over K slices before this function is asked
-// (M = 32 47 us, M = 128 61 us against 59 / 85 us for the better of the other two).
+// tiles pay for the int32 scratch traffic, which grows with M.  Measured on B200 (graph replay, bf16):
+// K x N = 8192 x 28672: M = 1 stream-K 45.8 us, tile kernel 62.8 us; M = 8 48.0 / 56.3 us; M = 16
+// 50.7 / 42.7 us; M = 32 59.6 / 43.1 us; M = 128 99.6 / 45.0 us.  Shapes with few tiles and a long K
+// (28672 x 8192) go to the tile kernel over K slices before this function is asked (M = 32 43.2 us,
+// M = 128 51.7 us against 52.3 / 82.0 us for the better of the other two).  Known to be on the wrong side of
+// these lines: M = 16, and short K, where nearly every tile is shared (M x K x N = 16 x 1024 x 8192 stream-K
+// 13.7 us, tile kernel 8.4 us; 64 x 1024 x 8192 42.2 / 8.6 us; 64 x 1024 x 1024 23.3 / 8.2 us).
 bool prefer_streamk(int64_t M, int64_t N) {
     if (M <= 16) return true;
     const int64_t tiles = (N + kBN - 1) / kBN;

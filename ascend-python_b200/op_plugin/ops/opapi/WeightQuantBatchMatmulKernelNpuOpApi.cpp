@@ -10,7 +10,7 @@
 // Weight format.  The reference keeps matmul weights in a private device format and casts between it and
 // the plain layout around the matmul (ND <-> FRACTAL_NZ, op_plugin/ops/base_ops/aclops/MmKernelNpu.cpp:80-94,
 // :301-316).  The counterpart here is the k-major int4 stream of qmm_w4a16_prepack: the first call that
-// benefits from it (more than eight token rows) rewrites the weight once, and a cache keyed by the data
+// benefits from it (one, two or more than eight token rows) rewrites the weight once, and a cache keyed by the data
 // pointers of weight, scale and offset serves every later call.  An entry stays valid while the three
 // storages are alive and their version counters are unchanged (an in-place update re-packs); the cache holds
 // a second copy of the weights, bounded by QMM_W4_PREPACK_MAX_MB (default 16384; QMM_W4_PREPACK=0 switches
@@ -185,8 +185,10 @@ at::Tensor npu_weight_quant_batchmatmul(const at::Tensor &x, const at::Tensor &w
     at::Tensor sc = antiquant_scale.contiguous();
     at::Tensor oc = offset_real.defined() ? offset_real.contiguous() : offset_real;
     at::Tensor bc = bias_real.defined() ? bias_real.contiguous() : bias_real;
-    // one or two token rows (integer dot products at the speed of the weight stream) and more than eight (operand
-    // unpacked into tensor memory): the kernels over the prepacked stream are the faster ones
+    // One or two token rows (integer dot products) and more than eight (operand unpacked into tensor memory) go to the
+    // kernels over the prepacked stream.  Three to eight stay on the stock layout, whose kernel does not round the weight
+    // to 16 bits, although it is slower by now (8 tokens, stock / prepacked: 8192 x 28672 39.3 / 34.0 us, 4096 x 4096
+    // 33.7 / 9.0 us; 9 tokens 47.8 / 34.0 and 33.0 / 9.2 us).
     if (prepack_enabled() && (M <= 2 || M > 8) && K > 0) {
         at::Tensor packed = prepacked_weight(wc, sc, oc, group, N, K);
         if (packed.defined()) {
