@@ -1,9 +1,11 @@
 #include "op_plugin/utils/qmm_api_common.h"
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
 #include <utility>
+#include <vector>
 
 namespace op_plugin_utils {
 
@@ -40,12 +42,18 @@ std::map<std::tuple<int, int, void *>, at::Tensor> &workspace_cache()
     static auto &cache = *new std::map<std::tuple<int, int, void *>, at::Tensor>();
     return cache;
 }
+std::vector<at::Tensor> &outgrown()
+{
+    static auto &buffers = *new std::vector<at::Tensor>();  // leaked like the cache
+    return buffers;
+}
 }  // namespace
 
 void qmm_workspace_reset()
 {
     std::lock_guard<std::mutex> lock(workspace_mutex());
     workspace_cache().clear();
+    outgrown().clear();
 }
 
 MatmulOperandB describe_operand_b(const at::Tensor &x2, int64_t K, int64_t N)
@@ -73,12 +81,20 @@ at::Tensor qmm_workspace(const at::Tensor &like, size_t bytes, int family)
     std::lock_guard<std::mutex> lock(mutex);
     auto key = std::make_tuple(family, static_cast<int>(like.device().index()), current_stream(like));
     auto it = cache.find(key);
-    if (it == cache.end() || static_cast<size_t>(it->second.numel()) < bytes) {
-        at::Tensor ws = at::zeros({static_cast<int64_t>(bytes)}, like.options().dtype(at::kByte));
-        cache[key] = ws;
-        return ws;
+    if (it != cache.end() && static_cast<size_t>(it->second.numel()) >= bytes) {
+        return it->second;
     }
-    return it->second;
+    // The buffer that is outgrown stays allocated: a graph captured on this stream may hold its address.  Growing at least
+    // twofold keeps all outgrown ones together smaller than the current one.
+    if (it != cache.end()) {
+        bytes = std::max(bytes, 2 * static_cast<size_t>(it->second.numel()));
+    }
+    at::Tensor ws = at::zeros({static_cast<int64_t>(bytes)}, like.options().dtype(at::kByte));
+    if (it != cache.end()) {
+        outgrown().push_back(it->second);
+    }
+    cache[key] = ws;
+    return ws;
 }
 
 }  // namespace op_plugin_utils

@@ -33,8 +33,9 @@ int qmm_dtype(at::ScalarType t);
 void *current_stream(const at::Tensor &like);
 
 // Zero-initialised scratch of at least `bytes`, cached per (device, stream) and
-// grown on demand.  The kernels that use it leave it zeroed, so one buffer is
-// reused by consecutive launches of the same stream (stream order serializes them).
+// grown on demand (an outgrown buffer is kept: captured graphs may use it).  The
+// kernels that use it leave it zeroed, so one buffer is reused by consecutive
+// launches of the same stream (stream order serializes them).
 // `family` separates kernel families: each relies on the state it left in its own buffer.
 at::Tensor qmm_workspace(const at::Tensor &like, size_t bytes, int family = 0);
 

@@ -148,3 +148,30 @@ def test_quant_matmul_int8_output_and_offset(torch_npu, oracle, dev):
     with pytest.raises(RuntimeError, match="offset only applies to an int8 output"):
         torch_npu.npu_quant_matmul(x1.to(dev), x2.to(dev), scale.to(dev), offset=offset.to(dev),
                                    output_dtype=torch.bfloat16)
+
+
+def test_scratch_of_a_captured_call_outlives_growth(torch_npu, dev):
+    """A call captured on a stream whose scratch a later, larger call outgrows: replays still own their scratch (nothing
+    allocated since is written) and give the captured call's result."""
+    K, N = 8192, 1024
+    g = torch.Generator(device=dev).manual_seed(9)
+    w = torch.randint(-2 ** 31, 2 ** 31 - 1, (K, N // 8), generator=g, device=dev, dtype=torch.int64).to(torch.int32)
+    scale = (torch.rand((K // 128, N), generator=g, device=dev) * 1e-2).to(torch.bfloat16)
+    small, large = (torch.randn((m, K), generator=g, device=dev).to(torch.bfloat16) for m in (100, 1000))
+    call = lambda x: torch_npu.npu_weight_quant_batchmatmul(x, w, scale, antiquant_group_size=128)  # noqa: E731
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        want = call(small).clone()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            y = call(small)
+        call(large)
+        torch.cuda.synchronize()
+        others = [torch.full((n << 18,), 3.0, device=dev) for n in (1, 2, 4, 8, 9, 16, 4, 2, 8) for _ in range(2)]
+        for _ in range(3):
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, want)
+            assert all((o == 3.0).all() for o in others)
