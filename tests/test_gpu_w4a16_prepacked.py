@@ -139,8 +139,8 @@ def test_decode_full_size(capi, oracle, dev, M):
 @pytest.mark.parametrize("shape", [(65, 128, 136, 128), (128, 640, 8, 640), (129, 1152, 264, 384), (255, 384, 1032, 128),
                                    (257, 256, 19200, 256), (600, 512, 1152, 512), (1030, 128, 136, 128)])
 def test_more_than_64_rows(capi, oracle, dev, shape, dtype):
-    """The wide form: one to five row tiles, ragged last ones, odd numbers of blocks, fewer output tiles than SMs (shared
-    tiles, added from slots) and more (whole tiles); and a result that two calls repeat."""
+    """The wide form: one to five row tiles, ragged last ones, odd numbers of blocks, fewer output tiles than SMs and more,
+    on 148 SMs all of them whole tiles; and a result that two calls repeat."""
     M, K, N, group = shape
     x, packed_w, scale, offset = oracle.make_w4a16_inputs(M, K, N, seed=M + K + N, group=group, dtype=dtype)
     y_ref = oracle.weight_quant_batchmatmul(x, packed_w, scale, offset, antiquant_group_size=group)
