@@ -128,6 +128,59 @@ __device__ __forceinline__ uint2 quantize8(const float (&f)[8], const RowQuant &
     return make_uint2(lo, hi);
 }
 
+// ---- rows that do not begin on a vector boundary ----
+//
+// An odd number of columns shifts every row by some elements against the 16-byte grid of its input; the int8 output
+// shifts by as many bytes against its 8-byte grid, so both stay aligned at the same elements when their addresses agree
+// modulo eight elements (two dense tensors always do).  A row is then a run of aligned vectors of which the first and the
+// last are partial: those go element by element, all others as in a row without a shift.  The generic kernels, which read two
+// bytes a load and every row two or three times, are left with rows of more than 32761 elements and unequal shifts: quantization
+// of 8192 x 4097 62.9 -> 27.8 us (15.4 at the memory's rate), 8192 x 16383 221 -> 91, 300 x 16383 14.5 -> 6.6; rms_norm of
+// 8192 x 6001 76.7 -> 44.7; the two fused 128 -> 72.  What is left is instructions: the funnel shift of gamma and the guards.
+
+// elements by which a row of 16-bit values begins behind a 16-byte boundary
+__device__ __forceinline__ int row_shift(const void *row) { return static_cast<int>(reinterpret_cast<uintptr_t>(row) >> 1) & 7; }
+inline bool same_shift(const void *x, int64_t ld_x, int x_bytes, const void *out, int64_t ld_out, int out_bytes) {
+    return ((reinterpret_cast<uintptr_t>(x) / x_bytes - reinterpret_cast<uintptr_t>(out) / out_bytes) & 7) == 0 &&
+           ((ld_x - ld_out) & 7) == 0 && reinterpret_cast<uintptr_t>(x) % x_bytes == 0 && reinterpret_cast<uintptr_t>(out) % out_bytes == 0;
+}
+
+// columns [c, c + 8) of a row of `cols` 16-bit values, zeros where there is no such column.  row + c is 16-byte aligned.
+template <typename T>
+__device__ __forceinline__ uint4 load8_edge(const T *row, int c, int cols) {
+    if (c >= 0 && c + 8 <= cols) return __ldg(reinterpret_cast<const uint4 *>(row + c));
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int e = c + 2 * j;
+        const uint32_t lo = e >= 0 && e < cols ? __ldg(reinterpret_cast<const unsigned short *>(row) + e) : 0;
+        const uint32_t hi = e + 1 >= 0 && e + 1 < cols ? __ldg(reinterpret_cast<const unsigned short *>(row) + e + 1) : 0;
+        w[j] = lo | hi << 16;
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+// the inverse: int8 and 16-bit rows
+__device__ __forceinline__ void store8_edge(int8_t *row, int c, int cols, const uint2 &v) {
+    if (c >= 0 && c + 8 <= cols) {
+        *reinterpret_cast<uint2 *>(row + c) = v;
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (c + j >= 0 && c + j < cols) row[c + j] = static_cast<int8_t>((j < 4 ? v.x : v.y) >> (8 * (j & 3)));
+}
+template <typename T>
+__device__ __forceinline__ void store8_edge(T *row, int c, int cols, const uint4 &v) {
+    if (c >= 0 && c + 8 <= cols) {
+        *reinterpret_cast<uint4 *>(row + c) = v;
+        return;
+    }
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (c + j >= 0 && c + j < cols)
+            reinterpret_cast<unsigned short *>(row)[c + j] = static_cast<unsigned short>(w[j >> 1] >> (16 * (j & 1)));
+}
 
 }  // namespace dq
 }  // namespace qmm

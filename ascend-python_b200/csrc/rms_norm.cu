@@ -81,8 +81,26 @@ __device__ __forceinline__ float rstd_of(float sumsq, int cols, float eps) {
     return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(variance, eps)));
 }
 
-// `tpr` threads per row, each holding VPT 16-byte vectors.  QUANT: write int8 + scale instead of y.
-template <typename T, int VPT, bool QUANT>
+// Columns [c, c + 8) of gamma, whose vectors are aligned where c is a multiple of eight, for a row that is shifted against
+// them by c mod 8 elements (the same for all threads of a row): two vectors and a funnel shift.
+template <typename T>
+__device__ __forceinline__ uint4 load_gamma_shifted(const T *gamma, int c, int cols) {
+    const int s = c & 7;
+    const uint4 a = dq::load8_edge(gamma, c - s, cols);
+    if (s == 0) return a;
+    const uint4 b = dq::load8_edge(gamma, c - s + 8, cols);
+    const bool far = (s & 4) != 0, odd = (s & 2) != 0;
+    uint32_t w[6] = {far ? a.z : a.x, far ? a.w : a.y, far ? b.x : a.z, far ? b.y : a.w, far ? b.z : b.x, far ? b.w : b.y};
+#pragma unroll
+    for (int j = 0; j < 5; ++j) w[j] = odd ? w[j + 1] : w[j];
+    const uint32_t bits = (s & 1) * 16;
+    return make_uint4(__funnelshift_r(w[0], w[1], bits), __funnelshift_r(w[1], w[2], bits), __funnelshift_r(w[2], w[3], bits),
+                      __funnelshift_r(w[3], w[4], bits));
+}
+
+// `tpr` threads per row, each holding VPT 16-byte vectors.  QUANT: write int8 + scale instead of y.  SHIFTED: 16-bit rows
+// that begin off the vector grid (see dynamic_quant.cuh).
+template <typename T, int VPT, bool QUANT, bool SHIFTED = false>
 __global__ void __launch_bounds__(512)
 rms_norm_vec_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_x, const T *__restrict__ gamma,
                     float eps, T *__restrict__ y, int64_t ld_y, int8_t *__restrict__ q, int64_t ld_q,
@@ -97,7 +115,8 @@ rms_norm_vec_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_
     const int t = threadIdx.x & (tpr - 1);
     const int64_t row = static_cast<int64_t>(blockIdx.x) * rows_per_cta + row_in_cta;
     const bool row_ok = row < rows;
-    const int nvec = cols / E;
+    const int shift = SHIFTED ? dq::row_shift(x + row * ld_x) : 0;
+    const int nvec = (SHIFTED ? cols + shift + E - 1 : cols) / E;
     const int warp = threadIdx.x >> 5;
     const int warps_per_row = tpr >> 5;
     const int w0 = row_in_cta * warps_per_row;
@@ -105,11 +124,17 @@ rms_norm_vec_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_
     uint4 v[VPT];
     float sumsq = 0.0f;
     if (row_ok) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(x + row * ld_x);
+        const T *src = x + row * ld_x;
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
             const int idx = t + i * tpr;
-            v[i] = idx < nvec ? __ldg(src + idx) : make_uint4(0, 0, 0, 0);
+            v[i] = make_uint4(0, 0, 0, 0);
+            if (idx < nvec) {
+                if constexpr (SHIFTED)
+                    v[i] = dq::load8_edge(src, idx * E - shift, cols);
+                else
+                    v[i] = __ldg(reinterpret_cast<const uint4 *>(src) + idx);
+            }
         }
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
@@ -141,12 +166,17 @@ rms_norm_vec_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_
             if (idx < nvec) {
                 float f[E], g[E];
                 unpack_vec<T>(v[i], f);
-                unpack_vec<T>(__ldg(gsrc + idx), g);
+                if constexpr (SHIFTED)
+                    unpack_vec<T>(load_gamma_shifted(gamma, idx * E - shift, cols), g);
+                else
+                    unpack_vec<T>(__ldg(gsrc + idx), g);
 #pragma unroll
                 for (int j = 0; j < E; ++j) f[j] = __fmul_rn(__fmul_rn(f[j], rstd), g[j]);
                 v[i] = pack_vec<T>(f);
                 if constexpr (QUANT) {
                     amax = max_nan(amax, dq::absmax8<T>(v[i]));  // of the rounded values
+                } else if constexpr (SHIFTED) {
+                    dq::store8_edge(y + row * ld_y, idx * E - shift, cols, v[i]);
                 } else {
                     reinterpret_cast<uint4 *>(y + row * ld_y)[idx] = v[i];
                 }
@@ -167,14 +197,18 @@ rms_norm_vec_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_
         const dq::RowQuant rq = dq::make_row_quant(amax);
         if (t == 0) scale[row] = rq.scale;
         const bool fast = !rq.exact_only && rq.scale != 0.0f;
-        uint2 *dst = reinterpret_cast<uint2 *>(q + row * ld_q);
+        int8_t *dst = q + row * ld_q;
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
             const int idx = t + i * tpr;
             if (idx < nvec) {
                 float f[8];
                 dq::unpack8<T>(v[i], f);
-                dst[idx] = dq::quantize8(f, rq, fast);
+                const uint2 b = dq::quantize8(f, rq, fast);
+                if constexpr (SHIFTED)
+                    dq::store8_edge(dst, idx * E - shift, cols, b);
+                else
+                    reinterpret_cast<uint2 *>(dst)[idx] = b;
             }
         }
     }
@@ -216,7 +250,8 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 // 4096 x 16384: 52.1 -> 47.8; 4096 x 5128: 20.4 -> 18.9.  Rows of 512 threads leave one CTA an SM and nothing to overlap
 // its barriers with (1000 x 30000: 30.1 us against 28.0): they stay with the kernel above, and so does the plain
 // operator, which is close to the memory's rate.  The sum of squares is taken in that kernel's order.
-template <typename T, int VPT, bool FULL>
+// SHIFTED: rows that begin off the vector grid (see dynamic_quant.cuh); gamma is then read again for every row.
+template <typename T, int VPT, bool FULL, bool SHIFTED = false>
 __global__ void __launch_bounds__(256, 2)
 rms_norm_quant_walk_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_x, const T *__restrict__ gamma,
                     float eps, int8_t *__restrict__ q, int64_t ld_q,
@@ -225,13 +260,21 @@ rms_norm_quant_walk_kernel(const T *__restrict__ x, int64_t rows, int cols, int6
     pdl_wait();
     constexpr int E = VecOf<T>::kElems, H = E / 2;
     static_assert(E == 8, "16-bit types");
-    constexpr bool kKeepGamma = VPT * E <= 32;
+    constexpr bool kKeepGamma = VPT * E <= 32 && !SHIFTED;
     __shared__ float s_part[2][2][8];  // [row parity][sum, absmax][warp]
     const int tpr_shift = __ffs(tpr) - 1;
     const int rows_per_cta = blockDim.x >> tpr_shift;
     const int row_in_cta = threadIdx.x >> tpr_shift;
     const int t = threadIdx.x & (tpr - 1);
-    const int nvec = cols / E;
+    int64_t row = static_cast<int64_t>(blockIdx.x) * rows_per_cta + row_in_cta;
+    int shift = 0, nvec = cols / E;  // of the row that is worked on
+    auto set_shift = [&](int64_t r) {
+        if constexpr (SHIFTED) {
+            shift = dq::row_shift(x + r * ld_x);
+            nvec = (cols + shift + E - 1) / E;
+        }
+    };
+    set_shift(row);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int warps_per_row = tpr >> 5;
     const int w0 = row_in_cta * warps_per_row;
@@ -240,7 +283,10 @@ rms_norm_quant_walk_kernel(const T *__restrict__ x, int64_t rows, int cols, int6
     float2 g[kKeepGamma ? VPT : 1][H];
     auto load_gamma = [&](int i, float2 (&out)[H]) {
         float f[E];
-        unpack_vec<T>(has(i) ? __ldg(reinterpret_cast<const uint4 *>(gamma) + t + i * tpr) : make_uint4(0, 0, 0, 0), f);
+        if constexpr (SHIFTED)
+            unpack_vec<T>(has(i) ? load_gamma_shifted(gamma, (t + i * tpr) * E - shift, cols) : make_uint4(0, 0, 0, 0), f);
+        else
+            unpack_vec<T>(has(i) ? __ldg(reinterpret_cast<const uint4 *>(gamma) + t + i * tpr) : make_uint4(0, 0, 0, 0), f);
 #pragma unroll
         for (int j = 0; j < H; ++j) out[j] = make_float2(f[2 * j], f[2 * j + 1]);
     };
@@ -250,16 +296,23 @@ rms_norm_quant_walk_kernel(const T *__restrict__ x, int64_t rows, int cols, int6
     }
     uint4 v[VPT];
     auto load_row = [&](int64_t row) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(x + row * ld_x);
+        if constexpr (SHIFTED) {
+            const T *src = x + row * ld_x;
+            const int s = dq::row_shift(src);
 #pragma unroll
-        for (int i = 0; i < VPT; ++i) v[i] = row < rows && has(i) ? __ldg(src + t + i * tpr) : make_uint4(0, 0, 0, 0);
+            for (int i = 0; i < VPT; ++i) v[i] = row < rows ? dq::load8_edge(src, (t + i * tpr) * E - s, cols) : make_uint4(0, 0, 0, 0);
+        } else {
+            const uint4 *src = reinterpret_cast<const uint4 *>(x + row * ld_x);
+#pragma unroll
+            for (int i = 0; i < VPT; ++i) v[i] = row < rows && has(i) ? __ldg(src + t + i * tpr) : make_uint4(0, 0, 0, 0);
+        }
     };
     const int64_t step = static_cast<int64_t>(gridDim.x) * rows_per_cta;
-    int64_t row = static_cast<int64_t>(blockIdx.x) * rows_per_cta + row_in_cta;
     load_row(row);
     int parity = 0;
     // all rows of a CTA advance together (the barriers below); rows beyond the last one are zeros and write nothing
     for (int64_t base = static_cast<int64_t>(blockIdx.x) * rows_per_cta; base < rows; base += step, row += step, parity ^= 1) {
+        set_shift(row);
         float2 f[VPT][H];
         float sumsq = 0.0f;
 #pragma unroll
@@ -319,7 +372,13 @@ rms_norm_quant_walk_kernel(const T *__restrict__ x, int64_t rows, int cols, int6
         }
         const dq::RowQuant rq = dq::make_row_quant(amax);
         if (row_ok && t == 0) scale[row] = rq.scale;
-        uint2 *dst = reinterpret_cast<uint2 *>(q + row * ld_q);
+        int8_t *dst = q + row * ld_q;
+        auto store = [&](int i, const uint2 &b) {
+            if constexpr (SHIFTED)
+                dq::store8_edge(dst, (t + i * tpr) * E - shift, cols, b);
+            else
+                reinterpret_cast<uint2 *>(dst)[t + i * tpr] = b;
+        };
         if (!rq.exact_only && rq.scale != 0.0f) {  // as dq::quantize8, two elements an instruction
             const float2 inv2 = make_float2(rq.inv, rq.inv), neg2 = make_float2(-rq.scale, -rq.scale);
             const float2 magic2 = make_float2(12582912.0f, 12582912.0f);
@@ -333,7 +392,7 @@ rms_norm_quant_walk_kernel(const T *__restrict__ x, int64_t rows, int cols, int6
                     b[2 * j] = __float_as_uint(r.x);
                     b[2 * j + 1] = __float_as_uint(r.y);
                 }
-                if (row_ok && has(i)) dst[t + i * tpr] = dq::gather_low_bytes(b);
+                if (row_ok && has(i)) store(i, dq::gather_low_bytes(b));
             }
         } else if (row_ok) {
 #pragma unroll
@@ -344,7 +403,7 @@ rms_norm_quant_walk_kernel(const T *__restrict__ x, int64_t rows, int cols, int6
                     e[2 * j] = f[i][j].x;
                     e[2 * j + 1] = f[i][j].y;
                 }
-                if (has(i)) dst[t + i * tpr] = dq::quantize8(e, rq, false);
+                if (has(i)) store(i, dq::quantize8(e, rq, false));
             }
         }
     }
@@ -410,8 +469,14 @@ int launch_rms_norm(const T *x, int64_t rows, int64_t cols, int64_t ld_x, const 
                               : ((ld_y % E == 0) && (reinterpret_cast<uintptr_t>(y) & 15) == 0);
     const bool vec_ok = (cols % E == 0) && (ld_x % E == 0) && out_ok && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
                         (reinterpret_cast<uintptr_t>(gamma) & 15) == 0 && cols / E <= 512 * 8;
-    if (vec_ok) {
-        const int nvec = static_cast<int>(cols / E);
+    // off the vector grid, but input and output by as much (16-bit types)
+    bool shifted = false;
+    if constexpr (E == 8) {
+        shifted = !vec_ok && (reinterpret_cast<uintptr_t>(gamma) & 15) == 0 && cols + 7 <= 512 * 8 * E &&
+                  (QUANT ? dq::same_shift(x, ld_x, 2, q, ld_q, 1) : dq::same_shift(x, ld_x, 2, y, ld_y, 2));
+    }
+    if (vec_ok || shifted) {
+        const int nvec = static_cast<int>((shifted ? cols + 2 * E - 2 : cols) / E);
         int tpr = 32;
         // eight vectors per thread where the row is long enough: the kernels are bound by instruction issue, and
         // the per-thread fixed cost (row scale, reductions, index arithmetic) is then spread over more elements
@@ -426,7 +491,8 @@ int launch_rms_norm(const T *x, int64_t rows, int64_t cols, int64_t ld_x, const 
                 const bool full = nvec == tpr * need;
                 auto pick = [&](auto v) {
                     constexpr int V = decltype(v)::value;
-                    return full ? rms_norm_quant_walk_kernel<T, V, true> : rms_norm_quant_walk_kernel<T, V, false>;
+                    return shifted ? rms_norm_quant_walk_kernel<T, V, false, true>
+                           : full  ? rms_norm_quant_walk_kernel<T, V, true> : rms_norm_quant_walk_kernel<T, V, false>;
                 };
                 using Kernel = decltype(&rms_norm_quant_walk_kernel<T, 1, true>);
                 const Kernel kernels[8] = {pick(std::integral_constant<int, 1>()), pick(std::integral_constant<int, 2>()),
@@ -445,6 +511,17 @@ int launch_rms_norm(const T *x, int64_t rows, int64_t cols, int64_t ld_x, const 
             if (need <= 1) kern = rms_norm_vec_kernel<T, 1, QUANT>;
             else if (need <= 2) kern = rms_norm_vec_kernel<T, 2, QUANT>;
             else if (need <= 4) kern = rms_norm_vec_kernel<T, 4, QUANT>;
+        }
+        if constexpr (E == 8 && QUANT) {
+            if (shifted) kern = rms_norm_vec_kernel<T, 8, QUANT, true>;
+        } else if constexpr (E == 8) {
+            if (shifted) {
+                const decltype(kern) kernels[8] = {rms_norm_vec_kernel<T, 1, QUANT, true>, rms_norm_vec_kernel<T, 2, QUANT, true>,
+                                                   rms_norm_vec_kernel<T, 3, QUANT, true>, rms_norm_vec_kernel<T, 4, QUANT, true>,
+                                                   rms_norm_vec_kernel<T, 5, QUANT, true>, rms_norm_vec_kernel<T, 6, QUANT, true>,
+                                                   rms_norm_vec_kernel<T, 7, QUANT, true>, rms_norm_vec_kernel<T, 8, QUANT, true>};
+                kern = kernels[need - 1];
+            }
         }
         QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(static_cast<unsigned>(threads)), 0, stream, x, rows,
                                icols, ld_x, gamma, eps, y, ld_y, q, ld_q, scale, rstd, tpr));

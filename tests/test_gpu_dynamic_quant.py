@@ -146,3 +146,24 @@ def test_non_finite_rows(capi, oracle, dev, dtype, cols):
     keep = [0, 1, 2, 4, 5]
     assert torch.equal(s[keep], s_ref[keep]) and torch.isinf(s[1]) and torch.isinf(s[4])
     assert not q[1].any() and not q[3].any() and not q[4].any()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [1, 7, 9, 255, 257, 2041, 2047, 4099, 16383, 32761, 32763])
+def test_rows_off_the_vector_grid(capi, oracle, dev, cols, dtype):
+    """Odd widths at every shift of a row against the 16-byte grid (nine rows), one vector to the widest row that is held in
+    registers and one past it; dense, a view that starts inside a vector, and rows of a wider tensor."""
+    g = torch.Generator().manual_seed(cols)
+    x = (torch.randn((9, cols), generator=g) * 3).to(dtype)
+    x[4] = 0
+    x[5, cols // 2] = float("inf")
+    _check(capi, oracle, x, dev)
+    q_ref, s_ref = oracle.dynamic_quant(x)
+    flat = torch.zeros(9 * cols + 3, dtype=dtype, device=dev)
+    flat[3:] = x.to(dev).flatten()
+    q, s = capi.dynamic_quant(flat[3:].view(9, cols))
+    assert torch.equal(q.cpu(), q_ref) and torch.equal(s.cpu(), s_ref)
+    wide = torch.full((9, cols + 5), 1e4, dtype=dtype, device=dev)  # neighbours that would win every maximum
+    wide[:, :cols] = x.to(dev)
+    q, s = capi.dynamic_quant(wide[:, :cols])
+    assert torch.equal(q.cpu(), q_ref) and torch.equal(s.cpu(), s_ref)

@@ -136,3 +136,31 @@ def test_torch_ops(pkg, oracle, dev):
         torch_npu.npu_rms_norm(x.to(dev), gamma.float().to(dev))
     with pytest.raises(RuntimeError, match="trailing dimensions"):
         torch_npu.npu_rms_norm(x.to(dev), gamma[:256].to(dev))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [1, 7, 9, 255, 257, 2041, 2047, 4099, 16383, 32761, 32763])
+def test_rows_off_the_vector_grid(capi, oracle, dev, cols, dtype):
+    """Odd widths at every shift of a row (and of gamma against it), one vector to the widest row that is held in registers
+    and one past it: y against the oracle, nothing written beside the rows, fused equal to the two operators."""
+    g = torch.Generator().manual_seed(cols)
+    x = (torch.randn((9, cols), generator=g) * 3).to(dtype)
+    gamma = (torch.rand(cols, generator=g) + 0.5).to(dtype)
+    y_ref, rstd_ref = oracle.rms_norm(x, gamma, 1e-6)
+    xd, gd = x.to(dev), gamma.to(dev)
+    y, rstd = capi.rms_norm(xd, gd, 1e-6)
+    np.testing.assert_allclose(rstd.cpu().numpy(), rstd_ref.numpy(), rtol=1e-5)
+    _check_y(y, y_ref, oracle)
+    q, scale, rstd_f = capi.rms_norm_dynamic_quant(xd, gd, 1e-6)
+    q_u, scale_u = capi.dynamic_quant(y)
+    assert torch.equal(rstd_f, rstd) and torch.equal(q, q_u) and torch.equal(scale, scale_u)
+    # the same rows inside wider ones: equal shifts (pitch cols + 8) and unequal ones (pitch cols + 5), guarded by marks
+    for pad in (8, 5):
+        xw = torch.full((9, cols + pad), 1e4, dtype=dtype, device=dev)
+        xw[:, :cols] = xd
+        yw = torch.full((9, cols + 8), 77.0, dtype=dtype, device=dev)
+        r = torch.empty(9, device=dev)
+        capi.check(capi.lib().qmm_rms_norm(capi._ptr(xw), capi.dtype_code(dtype), 9, cols, cols + pad, capi._ptr(gd), 1e-6,
+                                           capi._ptr(yw), cols + 8, capi._ptr(r), capi._stream()), "qmm_rms_norm")
+        assert torch.all(yw[:, cols:] == 77.0)
+        _check_y(yw[:, :cols], y_ref, oracle)
