@@ -14,6 +14,9 @@ namespace qmm {
 int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
                           const EpilogueParams &ep, int out_dtype, int64_t K, int algo, void *workspace,
                           size_t workspace_bytes, cudaStream_t stream, LaunchOptions *opts);
+// whether the kernel that QMM_ALGO_AUTO takes shares sums through scratch
+bool quant_matmul_wants_scratch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn, int64_t M,
+                                int64_t N, int64_t K);
 int validate_quant_matmul(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
                           const float *scale, int64_t scale_len, const void *bias, int bias_dtype, void *out,
                           int out_dtype, int64_t ld_out, int64_t M, int64_t N, int64_t K);
@@ -58,9 +61,9 @@ extern "C" int qmm_quant_matmul_int8(const int8_t *x1, int64_t ld_x1, const int8
     int rc = validate_quant_matmul(x1, ld_x1, x2, x2_stride_k, x2_stride_n, nullptr, 0, bias, bias ? QMM_DTYPE_I32 : QMM_DTYPE_NONE,
                                    out, QMM_DTYPE_I32, ld_out, M, N, K);
     if (rc != QMM_OK) return rc;
-    // the matmul kernels want their scratch zeroed; callers need not prepare it (decode shapes only: 0 for M > 128)
+    // the kernels that share sums through scratch want it zeroed; callers need not prepare it
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (inner > 0) QMM_CUDA_OK(cudaMemsetAsync(workspace, 0, inner, s));
+    if (inner > 0 && quant_matmul_wants_scratch(x1, ld_x1, x2, x2_stride_k, x2_stride_n, M, N, K)) QMM_CUDA_OK(cudaMemsetAsync(workspace, 0, inner, s));
     EpilogueParams ep;
     ep.scale = scale;
     ep.pertoken_scale = pertoken_scale;

@@ -1,6 +1,6 @@
 // W8A8 matmul with fused dequantization (npu_quant_matmul) for sm_100a.
 //
-// Three kernels:
+// The kernels of this file (w8a8_cluster.cu takes most shapes whose tiles are few):
 //  * w8a8_tile_kernel   — prefill shapes.  Persistent CTAs, one 128x256 output
 //    tile at a time: TMA -> 4-stage shared-memory ring -> tcgen05.mma kind::i8
 //    (128x256x32 per instruction) -> int32 accumulator in TMEM (two buffers, so
@@ -532,14 +532,13 @@ int launch_simt(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk
     return QMM_OK;
 }
 
-// Decode shapes (M <= 128): stream-K keeps every SM streaming weights whatever N is, but its split
+// Decode shapes (M <= 128) that the cluster kernel does not take - more than 148 x 256 columns, or beside a collective, where
+// its CTAs could not choose the SMs that are left free: stream-K keeps every SM streaming weights whatever N is, but its split
 // tiles pay for the int32 scratch traffic, which grows with M.  Measured on B200 (graph replay, bf16):
 // K x N = 8192 x 28672: M = 1 stream-K 45.8 us, tile kernel 62.8 us; M = 8 48.0 / 56.3 us; M = 16
 // 50.7 / 42.7 us; M = 32 59.6 / 43.1 us; M = 128 99.6 / 45.0 us.  Shapes with few tiles and a long K
 // (28672 x 8192) go to the tile kernel over K slices before this function is asked (M = 32 43.2 us,
-// M = 128 51.7 us against 52.3 / 82.0 us for the better of the other two).  Known to be on the wrong side of
-// these lines: M = 16, and short K, where nearly every tile is shared (M x K x N = 16 x 1024 x 8192 stream-K
-// 13.7 us, tile kernel 8.4 us; 64 x 1024 x 8192 42.2 / 8.6 us; 64 x 1024 x 1024 23.3 / 8.2 us).
+// M = 128 51.7 us against 52.3 / 82.0 us for the better of the other two).
 bool prefer_streamk(int64_t M, int64_t N) {
     if (M <= 16) return true;
     const int64_t tiles = (N + kBN - 1) / kBN;
@@ -563,6 +562,15 @@ int launch_streamk(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2
                    bool overlap, cudaStream_t stream);
 size_t streamk_workspace_bytes(int64_t M, int64_t N, int64_t K);
 bool streamk_supported(int64_t M, int64_t N, int64_t K, int64_t x2_sn);
+// Implemented in w8a8_cluster.cu
+int launch_cluster(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn, const EpilogueParams &ep,
+                   int out_dtype, int64_t K, cudaStream_t stream);
+bool prefer_cluster(int64_t M, int64_t N, int64_t K);  // of operands that TMA can address, with every SM to itself
+
+bool quant_matmul_wants_scratch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn, int64_t M,
+                                int64_t N, int64_t K) {
+    return M <= 128 && tma_compatible(x1, ld_x1, x2, x2_sk, x2_sn) && !prefer_cluster(M, N, K);
+}
 
 int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int64_t x2_sk, int64_t x2_sn,
                           const EpilogueParams &ep, int out_dtype, int64_t K, int algo, void *workspace,
@@ -575,6 +583,8 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
     if (algo == QMM_ALGO_AUTO) {
         if (!tma_ok)
             algo = QMM_ALGO_SIMT;
+        else if (opts == nullptr && prefer_cluster(ep.M, ep.N, K))
+            algo = QMM_ALGO_TCGEN05_CLUSTER;  // few tiles: one wave of clusters
         else if (ep.M > 16 && ep.M <= 128 && workspace != nullptr && splitk_scratch_bytes(ep.M, ep.N, K) > 0 &&
                  workspace_bytes >= splitk_scratch_bytes(ep.M, ep.N, K) &&
                  (reinterpret_cast<uintptr_t>(workspace) & 15) == 0)
@@ -588,7 +598,7 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
             algo = QMM_ALGO_TCGEN05_TILE;
     }
     if ((algo == QMM_ALGO_TCGEN05_TILE || algo == QMM_ALGO_TCGEN05_STREAMK || algo == QMM_ALGO_TCGEN05_PAIR ||
-         algo == QMM_ALGO_TCGEN05_SPLITK) && !tma_ok)
+         algo == QMM_ALGO_TCGEN05_SPLITK || algo == QMM_ALGO_TCGEN05_CLUSTER) && !tma_ok)
         return fail(QMM_ERR_UNSUPPORTED,
                     "qmm_quant_matmul: tcgen05 kernels need 16-byte aligned operands and row pitches");
     switch (algo) {
@@ -624,6 +634,8 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
             }
         case QMM_ALGO_TCGEN05_STREAMK:
             return launch_streamk(x1, ld_x1, x2, x2_sk, x2_sn, ep, out_dtype, K, workspace, workspace_bytes, overlap, stream);
+        case QMM_ALGO_TCGEN05_CLUSTER:
+            return launch_cluster(x1, ld_x1, x2, x2_sk, x2_sn, ep, out_dtype, K, stream);
         case QMM_ALGO_SIMT:
             switch (out_dtype) {
                 case QMM_DTYPE_BF16:
