@@ -21,3 +21,10 @@ def load_ops():
     from .ops_loader import load
 
     return load()
+
+
+def load_calls():
+    """The operator library's short-cut calls (see ops_loader.calls)."""
+    from .ops_loader import calls
+
+    return calls()

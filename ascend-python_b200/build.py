@@ -14,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -111,7 +112,8 @@ def build_plugin(force=False, verbose=False) -> Path:
         [OPP / "OpInterface.cpp", OPP / "TorchLibrary.cpp"]
     headers = list(OPP.rglob("*.h")) + [ROOT / "include" / "qmm_b200.h"]
     incs = [f"-I{p}" for p in cpp_extension.include_paths()] + [f"-I{ROOT / 'include'}", f"-I{PKG}",
-                                                                  "-I/usr/local/cuda/include"]
+                                                                  "-I/usr/local/cuda/include",
+                                                                  f"-I{sysconfig.get_paths()['include']}"]
     cxx = os.environ.get("CXX", "g++")
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
@@ -127,7 +129,7 @@ def build_plugin(force=False, verbose=False) -> Path:
     if force or jobs or _newer(PLUGIN_LIB, objs + [KERNEL_LIB]):
         tlib = Path(torch.__file__).parent / "lib"
         _run([cxx, "-shared", "-o", PLUGIN_LIB, *objs, f"-L{LIB}", "-lqmm_b200", f"-L{tlib}", "-ltorch", "-ltorch_cpu",
-              "-lc10", "-ltorch_cuda", "-lc10_cuda", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}"], verbose)
+              "-lc10", "-ltorch_cuda", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}"], verbose)
     return PLUGIN_LIB
 
 

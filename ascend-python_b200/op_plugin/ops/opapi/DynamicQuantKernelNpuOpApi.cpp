@@ -26,8 +26,8 @@ namespace op_api {
     const int64_t cols = input.size(-1);
     const int64_t rows = cols == 0 ? 0 : input.numel() / cols;
     at::Tensor x = input.contiguous();
-    at::Tensor y = at::empty(input.sizes(), input.options().dtype(at::kChar));
-    at::Tensor scale = at::empty(input.sizes().slice(0, input.dim() - 1), input.options().dtype(at::kFloat));
+    at::Tensor y = op_plugin_utils::empty_output(input.sizes(), input, at::kChar);
+    at::Tensor scale = op_plugin_utils::empty_output(input.sizes().slice(0, input.dim() - 1), input, at::kFloat);
     if (input.numel() == 0) {
         scale.zero_();
         return ::std::tuple<at::Tensor, at::Tensor>(y, scale);

@@ -65,7 +65,7 @@ at::Tensor npu_quant_matmul(const at::Tensor &x1, const at::Tensor &x2, const at
 
     auto output_size = x1.sizes().vec();
     output_size.back() = N;
-    at::Tensor result = at::empty(output_size, x1.options().dtype(out_type));
+    at::Tensor result = op_plugin_utils::empty_output(output_size, x1, out_type);
     if (result.numel() == 0) {
         return result;
     }

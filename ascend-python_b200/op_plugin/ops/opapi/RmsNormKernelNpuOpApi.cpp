@@ -49,8 +49,8 @@ std::vector<int64_t> rstd_sizes(const at::Tensor &self, const at::Tensor &gamma)
 {
     check_rms_norm_inputs("npu_rms_norm", self, gamma, /*allow_float=*/true);
     c10::cuda::CUDAGuard guard(self.device());
-    at::Tensor y = at::empty(self.sizes(), self.options());
-    at::Tensor rstd = at::empty(rstd_sizes(self, gamma), self.options().dtype(at::kFloat));
+    at::Tensor y = op_plugin_utils::empty_output(self.sizes(), self, self.scalar_type());
+    at::Tensor rstd = op_plugin_utils::empty_output(rstd_sizes(self, gamma), self, at::kFloat);
     if (self.numel() == 0) {
         return ::std::tuple<at::Tensor, at::Tensor>(y, rstd);
     }
@@ -71,9 +71,9 @@ std::vector<int64_t> rstd_sizes(const at::Tensor &self, const at::Tensor &gamma)
     TORCH_CHECK(gamma.dim() == 1, "npu_rms_norm_dynamic_quant: gamma should be 1D (the token dimension is the last "
                 "one), but it has ", gamma.dim(), " dimensions");
     c10::cuda::CUDAGuard guard(self.device());
-    at::Tensor q = at::empty(self.sizes(), self.options().dtype(at::kChar));
-    at::Tensor scale = at::empty(self.sizes().slice(0, self.dim() - 1), self.options().dtype(at::kFloat));
-    at::Tensor rstd = at::empty(rstd_sizes(self, gamma), self.options().dtype(at::kFloat));
+    at::Tensor q = op_plugin_utils::empty_output(self.sizes(), self, at::kChar);
+    at::Tensor scale = op_plugin_utils::empty_output(self.sizes().slice(0, self.dim() - 1), self, at::kFloat);
+    at::Tensor rstd = op_plugin_utils::empty_output(rstd_sizes(self, gamma), self, at::kFloat);
     if (self.numel() == 0) {
         scale.zero_();
         return ::std::tuple<at::Tensor, at::Tensor, at::Tensor>(q, scale, rstd);

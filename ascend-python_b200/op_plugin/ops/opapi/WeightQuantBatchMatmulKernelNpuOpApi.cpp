@@ -176,7 +176,7 @@ at::Tensor npu_weight_quant_batchmatmul(const at::Tensor &x, const at::Tensor &w
 
     auto output_size = x.sizes().vec();
     output_size.back() = N;
-    at::Tensor result = at::empty(output_size, x.options());
+    at::Tensor result = op_plugin_utils::empty_output(output_size, x, x.scalar_type());
     if (result.numel() == 0) {
         return result;
     }

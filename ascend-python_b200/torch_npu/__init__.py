@@ -36,29 +36,54 @@ def _load_pkg():
 
 _pkg = _load_pkg()
 _ops = _pkg.load_ops()
+_calls = _pkg.load_calls()
 _capi = _pkg.capi
+# While a compiler traces, the operators are torch.ops calls, which it knows; so they are where the short-cut calls decline
+# (tensor subclasses, __torch_function__ modes, arguments of other types).
+_compiling = torch.compiler.is_compiling
 
 
 def npu_dynamic_quant(input, *, smooth_scales=None):
+    if not _compiling():
+        out = _calls.dynamic_quant(input, smooth_scales)
+        if out is not NotImplemented:
+            return out
     return _ops.npu_dynamic_quant(input, smooth_scales=smooth_scales)
 
 
 def npu_rms_norm(self, gamma, epsilon=1e-06):
+    if not _compiling():
+        out = _calls.rms_norm(self, gamma, epsilon)
+        if out is not NotImplemented:
+            return out
     return _ops.npu_rms_norm(self, gamma, epsilon)
 
 
 def npu_rms_norm_dynamic_quant(self, gamma, epsilon=1e-06):
     """npu_rms_norm fused with npu_dynamic_quant: (int8 values, per-token scale, rstd)."""
+    if not _compiling():
+        out = _calls.rms_norm_dynamic_quant(self, gamma, epsilon)
+        if out is not NotImplemented:
+            return out
     return _ops.npu_rms_norm_dynamic_quant(self, gamma, epsilon)
 
 
 def npu_quant_matmul(x1, x2, scale, *, offset=None, pertoken_scale=None, bias=None, output_dtype=None):
+    if not _compiling():
+        out = _calls.quant_matmul(x1, x2, scale, offset, pertoken_scale, bias, output_dtype)
+        if out is not NotImplemented:
+            return out
     return _ops.npu_quant_matmul(x1, x2, scale, offset=offset, pertoken_scale=pertoken_scale, bias=bias,
                                  output_dtype=output_dtype)
 
 
 def npu_weight_quant_batchmatmul(x, weight, antiquant_scale, antiquant_offset=None, quant_scale=None,
                                  quant_offset=None, bias=None, antiquant_group_size=0):
+    if not _compiling():
+        out = _calls.weight_quant_batchmatmul(x, weight, antiquant_scale, antiquant_offset, quant_scale, quant_offset, bias,
+                                              antiquant_group_size)
+        if out is not NotImplemented:
+            return out
     return _ops.npu_weight_quant_batchmatmul(x, weight, antiquant_scale, antiquant_offset, quant_scale, quant_offset,
                                              bias, antiquant_group_size)
 
