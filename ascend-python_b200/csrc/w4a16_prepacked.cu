@@ -691,23 +691,39 @@ PPlan p_make_plan(int64_t M, int64_t N, int64_t K) {
         if (pl.nstages > kPMaxStages) pl.nstages = kPMaxStages;
         pl.smem = 2048 + static_cast<size_t>(pl.nxstages) * pl.mpad * 512 + static_cast<size_t>(pl.nstages) * kPStageWBytes;
     } else {
-        // As few row tiles as 256 columns of accumulator allow: every further one unpacks the weight again (1000 rows,
-        // K=4096, N=28672, short runs at the full clock: 201 us with four row tiles, 205, 209, 214, 226 us with five to eight,
-        // although seven fill the last wave best; under the power cap 231 us with four, 244 with seven).  Then the cheaper way of sharing tiles out by this model (clocks): a stage costs what its MMAs
-        // take (8 a row) or what unpacking it takes (about 1150), a tile some 12 a row more to leave tensor memory.
-        // Whole tiles leave the last wave uneven; equal shares of the stages do not, but every CTA then writes up to two
-        // tiles' sums and someone adds them (16 a row each).
-        const int64_t nblk = (M + kPMaxWide - 1) / kPMaxWide;
-        pl.mpad = static_cast<int>(((M + nblk - 1) / nblk + 15) / 16 * 16);
-        pl.nblk = static_cast<int>((M + pl.mpad - 1) / pl.mpad);
-        const int64_t tiles = static_cast<int64_t>(pl.tiles_n) * pl.nblk;
-        const int64_t stage = pl.mpad * 8 > 1150 ? pl.mpad * 8 : 1150, tile = pl.nchunks * stage + 12 * pl.mpad;
-        const int64_t whole = (tiles + sms - 1) / sms * tile, shared = tiles * tile / sms + stage + 2 * 16 * pl.mpad + 4000;
-        pl.grain = whole <= shared || tiles > static_cast<int64_t>(kPCounterBytes / 4) ? pl.nchunks : 1;  // (a counter a tile)
+        // Row tiles and the way of sharing them out by a model of the time (ns, fitted to 88 shapes of 65 .. 1500 rows, K of
+        // 1024 .. 15232 and N of 1024 .. 28672, 4 to 20 plans each).  A stage takes what unpacking it takes (790) or its MMAs
+        // (5 a row), a tile 61 a row more to leave tensor memory.  Whole tiles leave the last wave uneven; equal shares of the
+        // stages do not, but every CTA then writes the sums of up to two tiles, and the one that arrives last at a tile adds
+        // its slots one after the other: with few tiles that costs more than unpacking the weight again for lower row tiles
+        // does (256 x 8192 x 1024: one row tile 42.0 us, four 14.9; 321 x 3584 x 1096: 18.8 / 11.7).  With many, as few row
+        // tiles as the accumulator allows (1000 x 4096 x 28672: 201 us with four, 205 .. 226 with five to eight); a plan with
+        // more has to be 6 % ahead.
+        const int64_t fewest = (M + kPMaxWide - 1) / kPMaxWide;
+        int64_t best = 0;
+        for (int64_t want = fewest; want == fewest || want <= M / 32; ++want) {
+            const int64_t mpad = ((M + want - 1) / want + 15) / 16 * 16, nblk = (M + mpad - 1) / mpad;
+            const int64_t tiles = pl.tiles_n * nblk, items = tiles * pl.nchunks, ctas = items < sms ? items : sms;
+            const int64_t most = (items + ctas - 1) / ctas;
+            const int64_t stage = 47 + mpad * 5 > 790 ? 47 + mpad * 5 : 790, drain = 61 * mpad;
+            const int64_t whole = 99 + (tiles + sms - 1) / sms * (pl.nchunks * stage + drain);
+            const int64_t slots = tiles < ctas ? 16 * ctas / tiles + 16 : 32;  // of a tile, in sixteenths
+            const int64_t shared = 2187 + most * stage + drain * most / pl.nchunks + 35 * mpad + (mpad * 14 / 5 + 96) * slots / 16;
+            const bool grain = whole <= shared || tiles > static_cast<int64_t>(kPCounterBytes / 4);  // (a counter a tile)
+            const int64_t cost = (grain ? whole : shared) * (want == fewest ? 100 : 106);
+            if (best == 0 || cost < best) {
+                best = cost;
+                pl.mpad = static_cast<int>(mpad);
+                pl.nblk = static_cast<int>(nblk);
+                pl.grain = grain ? pl.nchunks : 1;
+            }
+        }
         pl.nstages = kPWideStages;
         pl.nxstages = static_cast<int>((kPSmemBudgetWide - 2048 - kPWideStages * kPStageWBytes) / (static_cast<size_t>(pl.mpad) * 128));
         if (pl.nxstages > kPMaxXStages) pl.nxstages = kPMaxXStages;
         pl.smem = 2048 + static_cast<size_t>(pl.nxstages) * pl.mpad * 128 + static_cast<size_t>(pl.nstages) * kPStageWBytes;
+        // more than half of an SM's: no other kernel that uses tensor memory fits beside a CTA, which holds all of it
+        if (pl.smem < 120 * 1024) pl.smem = 120 * 1024;
     }
     const int64_t out_tiles = static_cast<int64_t>(pl.tiles_n) * pl.nblk;
     const int64_t grains = out_tiles * (pl.nchunks / pl.grain);
