@@ -49,6 +49,7 @@
 // 75 clocks on each (45 / 51 us).  Wide: the tensor pipe and the power cap: 256 tokens 100 us, 2048
 // tokens 733 us = 1.31 PFLOP/s of a measured 1.41 sustained.
 #include "qmm_common.cuh"
+#include "w4a16_gemv.cuh"
 #include "w4a16_simt.cuh"
 
 namespace qmm {
@@ -748,32 +749,17 @@ size_t p_packed_bytes(int64_t N, int64_t K) {
     return static_cast<size_t>((N + kPTileN - 1) / kPTileN) * static_cast<size_t>(p_blocks_k(K)) * kPBlockBytes;
 }
 
-// ---- one or two tokens: integer dot products on the CUDA cores --------------------------------------------
+// ---- one or two tokens of a large weight: integer dot products on the CUDA cores -------------------------
 //
-// For a handful of tokens the tensor cores have nothing to add: a thread owns one output column, reads its
-// 64 bytes of a block straight from global memory (a warp's loads are 512 contiguous bytes), splits each
-// packed word into two words of four unsigned bytes - `w ^ 0x88888888` turns the two's complement nibbles into
-// w + 8, `& 0x0f0f0f0f` and `>> 4 & 0x0f0f0f0f` are bytes (k, k+4, k+1, k+5) and (k+2, k+6, k+3, k+7) of a
-// group of eight k - and multiplies them with dp4a by the activations, which a small kernel in front has
-// turned into two int8 digits of a block floating-point form, in that byte order: per token and block of
-// 128 k, with e the exponent of the block's absmax,
-//     X = rint(x * 2^(14 - e))  (|X| <= 2^14),   X = 128 * d1 + d2,  d1 in [-128, 127], d2 in [0, 127].
-// An activation within 2^-6 of its block's absmax is represented exactly (16-bit floats carry 8 or 11
-// significant bits); smaller ones are rounded to 2^-14 of the absmax, far below the 2^-9 / 2^-12 of the
-// output's own rounding.  Per block the exact integers D1 = sum u*d1 and D2 = sum u*d2 (u = w + 8) give
-//     y[m, n] += scale * esc[m] * (128 D1 + D2) + (offset*scale - 8 scale) * xs[m],
-// esc = 2^(e - 14), xs = esc * sum X; the weight itself is never rounded.  About 1.3 instructions per weight
-// for one token; every further token adds 64 dp4a per block and thread, which at the rate dp4a issues here costs
-// 7-8 us per token, so beyond two tokens the tensor-core kernels are faster.  A form with four columns per lane, which needs a quarter of the broadcast loads of digits, was
-// measured slower still (37 us against 33 us at two tokens): the loads are not the limit.  Making the digits inside this kernel (every
-// CTA for its own blocks) instead of in a kernel in front was measured slower: 30 us against 26 us for one token;
-// so was pulling lines of later blocks into L2 with prefetch instructions (29.6 us).
-// mma.sync forms of the same idea (the split words as register operands of m16n8k32 on these digits, pairs (k, k+1)
-// as 16-bit operands of m16n8k16, the nibbles as e4m3) were built and measured: correct, and the 16-bit and int8 MMAs
-// take 2.0 clocks an SM, but issue bounds them: 28 us at one token, 30 at eight, 42 at sixteen for the int8 form with
-// its digits made in the kernel, 35 / 45 us with 16-bit operands; the e4m3 MMA is emulated (43 / 71 us).  Work is cut into equal contiguous
-// runs of blocks, many CTAs per SM; a tile's partial sums go to per-CTA slots that the last arriver adds in
-// slot order, as in the tensor-core kernel.
+// The arithmetic of w4a16_gemv.cu (see there), which takes smaller weights.  Here the digits come from a small kernel in front
+// and a thread reads its 64 bytes of a block straight from global memory (a warp's loads are 512 contiguous bytes); work is cut
+// into equal contiguous runs of blocks, many CTAs per SM, and a tile's partial sums go to per-CTA slots that the last arriver
+// adds in slot order, as in the tensor-core kernel.  Every further token adds 64 dp4a per block and thread, 7-8 us at 8192 x 28672,
+// so beyond two tokens the tensor-core kernels are faster.  Measured slower: four columns per lane, which needs a quarter of the
+// broadcast loads of digits (37 us against 33 us at two tokens); digits made by every CTA of 128 threads for its own blocks (30 us
+// against 26 us); pulling lines of later blocks into L2 with prefetch instructions (29.6 us); mma.sync forms of the same idea
+// (28 us at one token, 30 at eight, 42 at sixteen for int8 digits, 35 / 45 us with 16-bit operands, 43 / 71 us with e4m3, whose
+// MMA is emulated).
 constexpr int kGvMaxM = 2;            // measured (K=8192, N=28672): 26 / 33 us for 1 / 2 tokens, 41 / 51 us for 3 / 4
 constexpr int kGvThreads = kPTileN;  // one output column per thread
 constexpr int kGvCtasPerSm = 5;       // resident CTAs per SM (three blocks of weights in flight per thread; best of 4..8)
@@ -1226,6 +1212,7 @@ extern "C" int qmm_weight_quant_batchmatmul_prepacked(const void *x, int x_dtype
         return fail(QMM_ERR_WORKSPACE,
                     "qmm_weight_quant_batchmatmul_prepacked: workspace missing, not 256-byte aligned or too small");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (prefer_gemv_tile(M, N, K)) return launch_gemv_tile(packed, x, x_dtype, ld_x, bias, out, ld_out, M, N, K, s);
     if (M <= kGvMaxM)  // a handful of tokens: dp4a on the CUDA cores, at the speed of the weight stream
         return (x_dtype == QMM_DTYPE_BF16)
                    ? launch_gemv_t<__nv_bfloat16>(static_cast<const uint8_t *>(packed), x, ld_x, bias, out, ld_out, M, N, K,

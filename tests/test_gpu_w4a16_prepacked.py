@@ -87,7 +87,12 @@ def test_against_oracle(capi, oracle, dev, shape, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("shape", [(1, 256, 64, 128), (2, 384, 200, 128), (2, 8192, 1024, 256), (1, 4096, 7168, 128),
-                                   (2, 1024, 4096, 1024)])
+                                   (2, 1024, 4096, 1024),
+                                   # one block and its padding; slices of K: eight up to 30 tiles, four up to 66, two up to 148;
+                                   # a long K whose digits leave a short ring; more tiles than SMs; beyond the tile kernel's range
+                                   (1, 128, 8, 128), (2, 4096, 30 * 128, 128), (1, 4096, 30 * 128 + 8, 128),
+                                   (2, 2176, 66 * 128, 128), (1, 2048, 66 * 128 + 16, 2048), (1, 1152, 148 * 128, 128),
+                                   (2, 1024, 148 * 128 + 8, 128), (2, 65536, 136, 128), (2, 8192, 9280, 128)])
 def test_one_or_two_tokens_meet_the_stock_tolerance(capi, oracle, dev, shape, dtype):
     """One or two tokens take the integer dot-product kernel, which never rounds a weight: it meets the bound of
     the stock-layout kernels, |y - y_ref| <= 2 u |y_ref| + 2^-7 (u / 2^-9) rms(row), not only the rss bound."""
@@ -232,3 +237,16 @@ def test_row_pitches_and_unaligned_output(capi, dev, shape):
         rows = flat[1:].view(M, N + 5)
         assert torch.equal(rows[:, :N], want)
         assert (rows[:, N:] == 7.0).all() and flat[0] == 7.0
+
+
+def test_slots_of_the_ring_belong_to_one_group(capi, oracle, dev):
+    """Rings of three to fifteen blocks, many calls back to back: every call the same bits, no wait that ran out."""
+    for M, K, N in ((2, 28672, 2048), (1, 384, 4096), (2, 8192, 4096), (1, 14336, 1024), (2, 57344, 256)):
+        x, packed_w, scale, offset = oracle.make_w4a16_inputs(M, K, N, seed=K, group=128)
+        buf = capi.w4a16_prepack(packed_w.to(dev), scale.to(dev), offset.to(dev), group_size=128)
+        xd = x.to(dev)
+        first = capi.weight_quant_batchmatmul_prepacked(xd, buf, N)
+        for _ in range(200):
+            last = capi.weight_quant_batchmatmul_prepacked(xd, buf, N)
+        assert torch.equal(first, last)
+    assert capi.device_status() == 0
