@@ -613,39 +613,107 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
 
 // ---- layout pass and its inverse ----------------------------------------------------------------------
 
-// one CTA per block (tile, chunk): 512 threads write the 512 vectors, the first 128 also scale and offset*scale
-template <typename T>
-__global__ void __launch_bounds__(512)
-w4a16_prepack_kernel(const int32_t *__restrict__ w, int64_t ld_w, const T *__restrict__ scale,
+// Eight words of one word column, of rows k .. k + 7, to the eight columns' words: nibble j of row e becomes the nibble of row e
+// in word j, in the block's order of rows (0, 2, 4, 6, 1, 3, 5, 7).  A transposition by halves, bytes and nibbles.
+__device__ __forceinline__ void p_transpose8(uint32_t (&w)[8]) {
+    const uint32_t b[8] = {w[0], w[2], w[4], w[6], w[1], w[3], w[5], w[7]};
+    uint32_t x[8], y[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        x[i] = __byte_perm(b[i], b[i + 4], 0x5410);
+        x[i + 4] = __byte_perm(b[i], b[i + 4], 0x7632);
+    }
+#pragma unroll
+    for (int h = 0; h < 8; h += 4)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            y[h + i] = __byte_perm(x[h + i], x[h + i + 2], 0x6240);      // columns h, h + 1
+            y[h + i + 2] = __byte_perm(x[h + i], x[h + i + 2], 0x7351);  // columns h + 2, h + 3
+        }
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+        w[j] = (y[j] & 0x0f0f0f0fu) | ((y[j + 1] & 0x0f0f0f0fu) << 4);
+        w[j + 1] = ((y[j] >> 4) & 0x0f0f0f0fu) | (y[j + 1] & 0xf0f0f0f0u);
+    }
+}
+
+// One CTA per chunk of 128 k and TILES tiles: rows of 256 (64) bytes come in, are transposed in registers and leave as four (one)
+// blocks, through one buffer in shared memory both ways.  With a load from global memory for every nibble (a thread a 16-byte
+// vector, 32 strided loads each) 8192 x 28672 took 128 us, 4096 x 4096 7.2 and 1024 x 1024 2.7; now 65, 5.7 and 2.0.  One tile a CTA
+// where four leave SMs without work (1024 x 1024: 3.9 with four).  A weight's first call pays for this pass.
+constexpr int kPPackThreads = 256;
+template <typename T, int TILES>
+__global__ void __launch_bounds__(kPPackThreads)
+w4a16_prepack_kernel(const int32_t *__restrict__ w, int64_t ld_w, int aligned, const T *__restrict__ scale,
                      const T *__restrict__ offset, int64_t group, int64_t N, int64_t K, int nchunks,
                      uint8_t *__restrict__ out) {
-    const int tile = blockIdx.y, c = blockIdx.x;  // c runs over the padded (even) number of blocks
-    uint8_t *blk = out + (static_cast<int64_t>(tile) * nchunks + c) * kPBlockBytes;
-    const int s = threadIdx.x >> 7, r = threadIdx.x & 127;
-    const int64_t n = static_cast<int64_t>(tile) * kPTileN + r;
-    const int64_t k0 = static_cast<int64_t>(c) * kPChunkK + s * kPSubK;
-    const bool real = n < N && k0 < K;  // the padding block and the padding columns are zeros
-    uint32_t words[4] = {0, 0, 0, 0};
-    if (real) {
-        const int64_t word_col = n >> 3;
-        const int sh = static_cast<int>(n & 7) * 4;
+    constexpr int kWords = TILES * kPTileN / 8;  // packed words of a row
+    constexpr int kSwap = TILES > 1 ? 3 : 1;
+    __shared__ __align__(16) uint32_t buf[kPChunkK * kWords];
+    const int c = blockIdx.x;  // runs over the padded (even) number of blocks
+    const int64_t tile0 = static_cast<int64_t>(blockIdx.y) * TILES, word0 = tile0 * (kPTileN / 8), words = N / 8;
+    const int64_t k0 = static_cast<int64_t>(c) * kPChunkK;
+    const bool real = k0 < K;  // the padding block and the padding columns are zeros
+    pdl_launch_dependents();
+    pdl_wait();
+    // word i of row k lies at i ^ 8 (k / 8 % 4): lanes that read four groups of eight rows find them in different banks (in rows
+    // of one tile, whose 16 words allow only % 2, in pairs of banks)
+    for (int v = threadIdx.x; v < kPChunkK * kWords / 4; v += kPPackThreads) {
+        const int k = v / (kWords / 4), i = v % (kWords / 4) * 4;
+        const int32_t *src = w + (k0 + k) * ld_w + word0 + i;
+        uint4 q = make_uint4(0, 0, 0, 0);
+        if (real && aligned && word0 + i + 4 <= words) {
+            q = __ldg(reinterpret_cast<const uint4 *>(src));
+        } else if (real) {
+            if (word0 + i < words) q.x = static_cast<uint32_t>(src[0]);
+            if (word0 + i + 1 < words) q.y = static_cast<uint32_t>(src[1]);
+            if (word0 + i + 2 < words) q.z = static_cast<uint32_t>(src[2]);
+            if (word0 + i + 3 < words) q.w = static_cast<uint32_t>(src[3]);
+        }
+        *reinterpret_cast<uint4 *>(buf + k * kWords + (i ^ ((k >> 3 & kSwap) << 3))) = q;
+    }
+    __syncthreads();
+    // a lane: word i of the 16-byte vectors (eight rows) and one of eight word columns; a warp: TILES of their 8 TILES places
+    const int lane = threadIdx.x & 31, i = lane & 3;
+    uint32_t t[TILES][8];
 #pragma unroll
-        for (int kk = 0; kk < kPSubK; ++kk) {
-            const uint32_t nib = (static_cast<uint32_t>(w[(k0 + kk) * ld_w + word_col]) >> sh) & 15u;
-            const int e = kk & 7;
-            words[kk >> 3] |= nib << (4 * ((e >> 1) + (e & 1) * 4));
+    for (int q = 0; q < TILES; ++q) {
+        const int place = (threadIdx.x >> 5) * TILES + q, s = place & 3, col = (place >> 2) * 8 + (lane >> 2);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) t[q][e] = buf[((s * 4 + i) * 8 + e) * kWords + (col ^ ((i & kSwap) << 3))];
+        p_transpose8(t[q]);
+    }
+    __syncthreads();
+    // vector v of a block lies at v ^ (v / 8 % 8)
+#pragma unroll
+    for (int q = 0; q < TILES; ++q) {
+        const int place = (threadIdx.x >> 5) * TILES + q, s = place & 3, col = (place >> 2) * 8 + (lane >> 2);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int v = s * kPTileN + (col & 15) * 8 + j;
+            buf[((col >> 4) * (kPWBytes / 16) + (v ^ (v >> 3 & 7))) * 4 + i] = t[q][j];
         }
     }
-    *reinterpret_cast<uint4 *>(blk + (s * kPTileN + r) * 16) = make_uint4(words[0], words[1], words[2], words[3]);
-    if (threadIdx.x < kPTileN) {
-        const int64_t g = (static_cast<int64_t>(c) * kPChunkK) / group;
+    __syncthreads();
+    const int64_t tiles = (N + kPTileN - 1) / kPTileN;
+    for (int v = threadIdx.x; v < TILES * (kPWBytes / 16); v += kPPackThreads) {
+        const int b = v / (kPWBytes / 16), x = v % (kPWBytes / 16);
+        if (tile0 + b >= tiles) break;
+        *reinterpret_cast<uint4 *>(out + ((tile0 + b) * nchunks + c) * kPBlockBytes + x * 16) =
+            *reinterpret_cast<const uint4 *>(buf + (b * (kPWBytes / 16) + (x ^ (x >> 3 & 7))) * 4);
+    }
+    const int64_t g = k0 / group;
+    for (int x = threadIdx.x; x < TILES * kPTileN; x += kPPackThreads) {
+        const int64_t n = tile0 * kPTileN + x;
+        if (tile0 + x / kPTileN >= tiles) break;
         T sv = from_float<T>(0.0f), tv = from_float<T>(0.0f);
-        if (real) {
+        if (real && n < N) {
             sv = scale[g * N + n];
             if (offset != nullptr) tv = from_float<T>(to_float(offset[g * N + n]) * to_float(sv));
         }
-        reinterpret_cast<T *>(blk + kPWBytes)[r] = sv;
-        reinterpret_cast<T *>(blk + kPWBytes + kPTileN * 2)[r] = tv;
+        T *so = reinterpret_cast<T *>(out + ((tile0 + x / kPTileN) * nchunks + c) * kPBlockBytes + kPWBytes);
+        so[x % kPTileN] = sv;
+        so[kPTileN + x % kPTileN] = tv;
     }
 }
 
@@ -1149,17 +1217,20 @@ extern "C" int qmm_w4a16_prepack(const int32_t *weight, int64_t ld_w, const void
     const int nchunks = p_blocks_k(K);
     const int64_t tiles = (N + kPTileN - 1) / kPTileN;
     QMM_REQUIRE(tiles <= 65535, "qmm_w4a16_prepack: N too large");
-    const dim3 grid(static_cast<unsigned>(nchunks), static_cast<unsigned>(tiles));
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int aligned = (reinterpret_cast<uintptr_t>(weight) & 15) == 0 && (ld_w & 3) == 0;
+    const int per_cta = (tiles + 3) / 4 * nchunks >= sm_count() ? 4 : 1;
+    const dim3 grid(static_cast<unsigned>(nchunks), static_cast<unsigned>((tiles + per_cta - 1) / per_cta));
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    auto launch = [&](auto kern, auto type) {
+        using T = decltype(type);
+        return launch_pdl(kern, grid, dim3(kPPackThreads), 0, s, weight, ld_w, aligned, static_cast<const T *>(antiquant_scale),
+                          static_cast<const T *>(antiquant_offset), group, N, K, nchunks, static_cast<uint8_t *>(packed));
+    };
     if (sdtype == QMM_DTYPE_BF16)
-        w4a16_prepack_kernel<__nv_bfloat16><<<grid, 512, 0, s>>>(
-            weight, ld_w, static_cast<const __nv_bfloat16 *>(antiquant_scale),
-            static_cast<const __nv_bfloat16 *>(antiquant_offset), group, N, K, nchunks, static_cast<uint8_t *>(packed));
+        QMM_CUDA_OK(launch(per_cta == 1 ? w4a16_prepack_kernel<__nv_bfloat16, 1> : w4a16_prepack_kernel<__nv_bfloat16, 4>,
+                           __nv_bfloat16()));
     else
-        w4a16_prepack_kernel<__half><<<grid, 512, 0, s>>>(weight, ld_w, static_cast<const __half *>(antiquant_scale),
-                                                          static_cast<const __half *>(antiquant_offset), group, N, K,
-                                                          nchunks, static_cast<uint8_t *>(packed));
-    QMM_CUDA_OK(cudaGetLastError());
+        QMM_CUDA_OK(launch(per_cta == 1 ? w4a16_prepack_kernel<__half, 1> : w4a16_prepack_kernel<__half, 4>, __half()));
     return QMM_OK;
 }
 

@@ -92,7 +92,8 @@ def test_against_oracle(capi, oracle, dev, shape, dtype):
                                    # a long K whose digits leave a short ring; more tiles than SMs; beyond the tile kernel's range
                                    (1, 128, 8, 128), (2, 4096, 30 * 128, 128), (1, 4096, 30 * 128 + 8, 128),
                                    (2, 2176, 66 * 128, 128), (1, 2048, 66 * 128 + 16, 2048), (1, 1152, 148 * 128, 128),
-                                   (2, 1024, 148 * 128 + 8, 128), (2, 65536, 136, 128), (2, 8192, 9280, 128)])
+                                   (2, 1024, 148 * 128 + 8, 128), (2, 65536, 136, 128), (2, 8192, 9280, 128),
+                                   (1, 2176, 37 * 128 - 8, 128), (2, 4096, 18 * 128, 128)])  # clusters that need two CTAs an SM
 def test_one_or_two_tokens_meet_the_stock_tolerance(capi, oracle, dev, shape, dtype):
     """One or two tokens take the integer dot-product kernel, which never rounds a weight: it meets the bound of
     the stock-layout kernels, |y - y_ref| <= 2 u |y_ref| + 2^-7 (u / 2^-9) rms(row), not only the rss bound."""
@@ -250,3 +251,21 @@ def test_slots_of_the_ring_belong_to_one_group(capi, oracle, dev):
             last = capi.weight_quant_batchmatmul_prepacked(xd, buf, N)
         assert torch.equal(first, last)
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("N", [8, 120, 128, 520, 1032])
+def test_prepack_of_a_pitched_or_unaligned_weight(capi, oracle, dev, N):
+    """Rows of the packed weight that do not start on 16 bytes, or have columns of another tensor behind them, pack the same."""
+    K = 384
+    _, packed_w, scale, offset = oracle.make_w4a16_inputs(1, K, N, seed=N, group=128)
+    w, sc, of = packed_w.to(dev), scale.to(dev), offset.to(dev)
+    want = capi.w4a16_prepack(w, sc, of, group_size=128)
+    assert torch.equal(capi.w4a16_unpack_weight(want, N, K).cpu(), packed_w)
+    for pitch, start in ((N // 8 + 3, 1), (N // 8 + 4, 0), (N // 8 + 4 - N // 8 % 4, 4)):
+        flat = torch.full((K * pitch + 8,), -1, dtype=torch.int32, device=dev)
+        rows = flat[start:start + K * pitch].view(K, pitch)[:, :N // 8]
+        rows.copy_(w)
+        got = torch.empty_like(want)
+        capi.check(capi.lib().qmm_w4a16_prepack(ctypes.c_void_p(rows.data_ptr()), pitch, capi._ptr(sc), capi._ptr(of), capi.DTYPE_BF16,
+                                                128, N, K, capi._ptr(got), got.numel(), capi._stream()), "prepack")
+        assert torch.equal(got, want)
