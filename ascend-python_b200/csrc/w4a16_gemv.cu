@@ -17,6 +17,8 @@
 // the slice's blocks, which are contiguous, into a ring in shared memory by bulk copies; meanwhile the others make the digits of
 // the slice; then three groups of 128 threads take the blocks in turn.  Their sums meet in shared memory, the slices' in the
 // first CTA's, in their order: results do not depend on timing, and there is no scratch, no counter and no second kernel.
+#include <algorithm>
+
 #include "qmm_common.cuh"
 #include "w4a16_gemv.cuh"
 
@@ -301,33 +303,84 @@ size_t v_fixed_bytes(int m, int max_blocks, int slices) {
            sizeof(VSmemTail);
 }
 
-// Slices of K: as many as leave every cluster resident, two CTAs an SM (cudaOccupancyMaxActiveClusters for 148 SMs: 74 clusters of
-// two CTAs, 33 of four, 15 of eight, with one CTA an SM).  The ring: as many blocks as fit beside the digits.
+constexpr int kVMaxSlices = 8;
+
+cudaLaunchConfig_t v_launch_config(int64_t ctas, int slices, size_t smem, cudaStream_t stream, cudaLaunchAttribute (&attr)[2]) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+    cfg.blockDim = dim3(kVThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(slices);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cfg;
+}
+
+// Clusters of each size that are resident at once, with one CTA an SM and with two (a cluster lies within a GPC, so this is less
+// than the SMs divided by the size).
+struct VResident {
+    int one[kVMaxSlices + 1], two[kVMaxSlices + 1];
+};
+const VResident &v_resident() {
+    static const VResident r = [] {
+        VResident v;
+        const auto kern = w4a16_gemv_tile_kernel<__half, 1>;
+        const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kVMaxSmem) == cudaSuccess;
+        for (int s = 0; s <= kVMaxSlices; ++s) {
+            v.one[s] = v.two[s] = 0;
+            if (s < 2 || !ok) continue;  // one CTA a tile: no cluster
+            cudaLaunchAttribute attr[2];
+            cudaLaunchConfig_t cfg = v_launch_config(s, s, kVMaxSmem, nullptr, attr);
+            cfg.numAttrs = 1;
+            if (cudaOccupancyMaxActiveClusters(&v.one[s], kern, &cfg) != cudaSuccess) v.one[s] = 0;
+            cfg.dynamicSmemBytes = kVMaxSmem / 2;
+            if (cudaOccupancyMaxActiveClusters(&v.two[s], kern, &cfg) != cudaSuccess) v.two[s] = 0;
+        }
+        (void)cudaGetLastError();
+        return v;
+    }();
+    return r;
+}
+
+// Slices of K by a model of the time, in clocks: a block takes an SM 256 for each token (dp4a), and all SMs together get a block
+// every 2.6 from memory; a CTA alone on an SM takes 1.3 times that.  Clusters that are not resident at once are not considered
+// (37 tiles: four slices, of which 33 clusters fit with one CTA an SM, 9.7 us for one token of 10624 x 4680, three slices 7.1).
+// The ring: as many blocks as fit beside the digits.
 bool v_make_plan(int m, int64_t N, int64_t K, VPlan *pl) {
     const int64_t tiles = (N + kVTileN - 1) / kVTileN, blocks = (K + 2 * kVBlockK - 1) / (2 * kVBlockK) * 2;
     const int sms = sm_count();
-    for (int slices = 8; slices >= 1; slices /= 2) {
-        const int64_t resident = slices == 1 ? tiles : slices == 2 ? sms : slices == 4 ? sms * 66 / 148 : sms * 30 / 148;
-        if (tiles > resident || (slices > 1 && blocks < 4 * slices)) continue;
+    if (blocks > (1 << 20)) return false;
+    float best = 0.0f;
+    pl->slices = 0;
+    for (int slices = 1; slices <= kVMaxSlices; ++slices) {
+        if (slices > 1 && (blocks < 4 * slices || tiles > v_resident().two[slices])) continue;
         const int64_t most = (blocks + slices - 1) / slices;
-        if (most > (1 << 20)) continue;
-        const bool twice = tiles * slices > sms;
+        const int64_t one = slices == 1 ? sms : v_resident().one[slices], an_sm = slices == 1 ? (tiles + sms - 1) / sms : tiles > one ? 2 : 1;
         const size_t fixed = v_fixed_bytes(m, static_cast<int>(most), slices);
-        size_t budget = twice ? kVMaxSmem / 2 : kVMaxSmem;
-        if (fixed + 2 * kVGroups * kVBlockBytes > budget) budget = kVMaxSmem;
+        size_t budget = an_sm > 1 ? kVMaxSmem / 2 : kVMaxSmem;
+        if (slices == 1 && fixed + 2 * kVGroups * kVBlockBytes > budget) budget = kVMaxSmem;
         if (fixed + 2 * kVGroups * kVBlockBytes > budget) continue;
+        const float busy = std::min(1.0f, static_cast<float>(tiles * slices) / static_cast<float>(sms));
+        const float cost = static_cast<float>(most * an_sm) * std::max(256.0f * m, 390.0f * busy) * (an_sm > 1 ? 1.0f : 1.3f) +
+                           (slices > 1 ? 600.0f + 60.0f * slices : 0.0f);
+        if (pl->slices != 0 && cost >= best) continue;
+        best = cost;
         pl->slices = slices;
         pl->max_blocks = static_cast<int>(most);
         // A multiple of the groups.  Otherwise blocks of different groups follow one another in a slot, and a group that is ahead
         // could test its phase of the slot's barrier before the phase in front has completed, which parity cannot tell apart.
         const int fit = static_cast<int>((budget - fixed) / kVBlockBytes) / kVGroups * kVGroups;
         const int need = static_cast<int>((most + kVGroups - 1) / kVGroups * kVGroups);
-        pl->ring = need < kVMaxRing ? need : kVMaxRing;
-        if (pl->ring > fit) pl->ring = fit;
+        pl->ring = std::min({need, kVMaxRing, fit});
         pl->smem = fixed + static_cast<size_t>(pl->ring) * kVBlockBytes;
-        return true;
     }
-    return false;
+    return pl->slices != 0;
 }
 
 template <typename T>
@@ -335,20 +388,12 @@ int launch_gemv_tile_t(VParams &p, const VPlan &pl, int64_t tiles, cudaStream_t 
     using Kernel = void (*)(VParams);
     const Kernel kern = p.M == 1 ? w4a16_gemv_tile_kernel<T, 1> : w4a16_gemv_tile_kernel<T, 2>;  // kGemvMaxM
     QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kVMaxSmem));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(tiles * pl.slices));
-    cfg.blockDim = dim3(kVThreads);
-    cfg.dynamicSmemBytes = pl.smem;
-    cfg.stream = stream;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = static_cast<unsigned>(pl.slices);
-    attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pl.slices > 1 ? 2 : 1;
+    cudaLaunchConfig_t cfg = v_launch_config(tiles * pl.slices, pl.slices, pl.smem, stream, attr);
+    if (pl.slices == 1) {  // no cluster
+        cfg.attrs = attr + 1;
+        cfg.numAttrs = 1;
+    }
     QMM_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, p));
     return QMM_OK;
 }
@@ -359,11 +404,14 @@ int launch_gemv_tile_t(VParams &p, const VPlan &pl, int64_t tiles, cudaStream_t 
 // weight has more tiles than there are SMs those with two take twice that.  The kernel of w4a16_prepacked.cu deals out the
 // blocks evenly, but pays for a kernel in front, scratch, counters and a last arrival.  us, there / here (K x N): one token
 // 1024 x 1024 5.1 / 3.0, 4096 x 4096 9.2 / 5.1, 8192 x 8192 13.4 / 8.7, 4096 x 28672 16.7 / 13.4, 28672 x 8192 25.4 / 23.2,
-// 8192 x 28672 25.5 / 24.9, 28672 x 28672 72 / 84; two tokens 4096 x 4096 10.6 / 7.1, 8192 x 8192 16.1 / 12.1, 4096 x 28672
+// 8192 x 28672 25.4 / 24.8
+// (25.9 / 26.5 with other launches between), 28672 x 28672 72 / 84; two tokens 4096 x 4096 10.6 / 7.1, 8192 x 8192 16.1 / 12.1, 4096 x 28672
 // 20.0 / 20.9, 8192 x 28672 31.9 / 38.9.
 bool prefer_gemv_tile(int64_t M, int64_t N, int64_t K) {
     VPlan pl;
-    return M >= 1 && M <= kGemvMaxM && K <= (M == 1 ? 300000000 : 75000000) / N && v_make_plan(static_cast<int>(M), N, K, &pl);
+    const bool one_wave = N <= static_cast<int64_t>(sm_count()) * kVTileN;
+    return M >= 1 && M <= kGemvMaxM && K <= (M == 2 ? 75000000 : one_wave ? 300000000 : 150000000) / N &&
+           v_make_plan(static_cast<int>(M), N, K, &pl);
 }
 
 int launch_gemv_tile(const void *packed, const void *x, int x_dtype, int64_t ld_x, const void *bias, void *out, int64_t ld_out,
