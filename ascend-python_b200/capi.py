@@ -31,6 +31,7 @@ EXPORTED_SYMBOLS = (
     "qmm_comm_attach_peer_memory",
     "qmm_w4a16_prepack_size", "qmm_w4a16_prepack", "qmm_w4a16_unpack_weight",
     "qmm_weight_quant_batchmatmul_prepacked_workspace_size", "qmm_weight_quant_batchmatmul_prepacked",
+    "qmm_weight_quant_batchmatmul_prepacked_tables",
     "qmm_rms_norm", "qmm_rms_norm_dynamic_quant", "qmm_comm_stats", "qmm_int8_mma_peak", "qmm_noalloc_status",
     "qmm_mm_reduce_scatter_workspace_size", "qmm_mm_reduce_scatter", "qmm_all_gather_mm_workspace_size",
     "qmm_all_gather_mm", "qmm_quant_matmul_int8_workspace_size", "qmm_quant_matmul_int8",
@@ -104,6 +105,10 @@ def lib() -> ctypes.CDLL:
         L.qmm_weight_quant_batchmatmul_prepacked.argtypes = [c.c_void_p, c.c_int, c.c_int64, c.c_void_p, c.c_size_t,
                                                              c.c_void_p, c.c_void_p, c.c_int64, c.c_int64, c.c_int64,
                                                              c.c_int64, c.c_void_p, c.c_size_t, c.c_void_p]
+        L.qmm_weight_quant_batchmatmul_prepacked_tables.argtypes = [
+            c.c_void_p, c.c_int, c.c_int64, c.c_void_p, c.c_size_t, c.c_void_p, c.c_void_p, c.c_int64, c.c_void_p, c.c_void_p,
+            c.c_int64, c.c_int64, c.c_int64, c.c_int64, c.c_void_p, c.c_size_t, c.c_void_p]
+        L.qmm_weight_quant_batchmatmul_prepacked_tables.restype = c.c_int
         for name in ("qmm_w4a16_prepack_size", "qmm_w4a16_prepack", "qmm_w4a16_unpack_weight",
                      "qmm_weight_quant_batchmatmul_prepacked_workspace_size",
                      "qmm_weight_quant_batchmatmul_prepacked"):
@@ -309,8 +314,9 @@ def w4a16_unpack_weight(packed, N: int, K: int):
     return w
 
 
-def weight_quant_batchmatmul_prepacked(x, packed, N: int, bias=None):
-    """x [M,K] bf16/f16 (the dtype the weights were prepacked with); packed from w4a16_prepack."""
+def weight_quant_batchmatmul_prepacked(x, packed, N: int, bias=None, tables=None):
+    """x [M,K] bf16/f16 (the dtype the weights were prepacked with); packed from w4a16_prepack.  tables: (scale, offset or
+    None, group size) the weight was packed with."""
     assert x.is_cuda and packed.dtype == torch.uint8
     M, K = x.shape
     x = x.contiguous()
@@ -320,10 +326,15 @@ def weight_quant_batchmatmul_prepacked(x, packed, N: int, bias=None):
           "qmm_weight_quant_batchmatmul_prepacked_workspace_size")
     ws_bytes = int(n.value)
     ws = get_workspace(x.device, ws_bytes, kind="w4a16_prepacked")
+    bias = None if bias is None else bias.contiguous()
+    weight = (_ptr(x), dtype_code(x.dtype), K, _ptr(packed), packed.numel())
+    rest = (_ptr(bias), _ptr(out), N, M, N, K, _ptr(ws), ws_bytes)
     with torch.cuda.device(x.device):
-        check(lib().qmm_weight_quant_batchmatmul_prepacked(
-            _ptr(x), dtype_code(x.dtype), K, _ptr(packed), packed.numel(), _ptr(None if bias is None else bias.contiguous()),
-            _ptr(out), N, M, N, K, _ptr(ws), ws_bytes, _stream()), "qmm_weight_quant_batchmatmul_prepacked")
+        if tables is None:
+            check(lib().qmm_weight_quant_batchmatmul_prepacked(*weight, *rest, _stream()), "qmm_weight_quant_batchmatmul_prepacked")
+        else:
+            check(lib().qmm_weight_quant_batchmatmul_prepacked_tables(*weight, _ptr(tables[0]), _ptr(tables[1]), tables[2], *rest,
+                                                                      _stream()), "qmm_weight_quant_batchmatmul_prepacked_tables")
     return out
 
 

@@ -226,9 +226,11 @@ __device__ __forceinline__ int p_slot(const PParams &p, int cta, int q) {
     return cta + min(q, cta + (p_first_item<WIDE>(p, cta) < q * p.nchunks ? 1 : 0));
 }
 
-// Adds the sums of tile q by its `nslots` CTAs in their order and stores the tile; thread `tid` of `threads`.
-template <typename T, bool WIDE>
-__device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots, int tid, int threads) {
+// Adds the sums of tile q by its `nslots` CTAs in their order and stores the tile; thread `tid` of `threads`.  plain(column, row):
+// what an output is that came to no number (PNoPlain: that).
+struct PNoPlain {};
+template <typename T, bool WIDE, typename Plain>
+__device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots, int tid, int threads, const Plain &plain) {
     const T *bias = static_cast<const T *>(p.bias);
     const int m0 = (q % p.nblk) * p.mpad, ncol0 = (q / p.nblk) * kPTileN;
     const int vecs = min(p.mpad, p.M - m0) * (kPTileN / 4);
@@ -277,6 +279,15 @@ __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots,
 #pragma unroll
                 for (int k = 0; k < 4; ++k) o[k] = from_float<T>(f[k]);
             }
+            if constexpr (!std::is_same<Plain, PNoPlain>::value) {
+                uint32_t again = 0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) again |= isnan(f[k]) ? 1u << k : 0u;
+                for (; again != 0; again &= again - 1) {
+                    const int k = __ffs(static_cast<int>(again)) - 1;
+                    o[k] = from_float<T>(plain(n + k, m0 + idx / (kPTileN / 4)) + (bias != nullptr ? to_float(bias[n + k]) : 0.0f));
+                }
+            }
         }
     }
 }
@@ -284,8 +295,9 @@ __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots,
 // The calling threads have stored this CTA's sums of tile q: reports that, and if it completes the tile adds the slots
 // and stores the tile.  EPILOGUE: the four epilogue warps call, otherwise the whole CTA.  Inlined: as a call with the
 // parameters' address it slows the whole kernel down (34 -> 43 us for 16 tokens).
-template <typename T, bool WIDE, bool EPILOGUE>
-__device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatile uint32_t *abort_flag, uint32_t *flag) {
+template <typename T, bool WIDE, bool EPILOGUE, typename Plain = PNoPlain>
+__device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatile uint32_t *abort_flag, uint32_t *flag,
+                                                const Plain &plain = Plain()) {
     auto barrier = [] {
         if (EPILOGUE)
             pepi_bar_sync();
@@ -308,7 +320,7 @@ __device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatil
         *flag = last;
     }
     barrier();
-    if (*reinterpret_cast<volatile uint32_t *>(flag) != 0) p_add_slots<T, WIDE>(p, q, nslots, tid, EPILOGUE ? kPEpiWarps * 32 : kPThreads);
+    if (*reinterpret_cast<volatile uint32_t *>(flag) != 0) p_add_slots<T, WIDE>(p, q, nslots, tid, EPILOGUE ? kPEpiWarps * 32 : kPThreads, plain);
     barrier();  // the flag is written again for the next tile
 }
 
@@ -611,6 +623,430 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
     if (p.grain == 1 && u_begin < u_end) p_finish_shared<T, WIDE, false>(p, (u_end - 1) / p.nchunks, abort_flag, &tail->is_last);
 }
 
+// ---- 3 to 16 token rows with the tables at hand: the weight as a whole number, scale and offset on the sums of a block ----
+//
+// The narrow form's unpack warps spend 15 instructions on a word, half of them on the subtraction and the multiply-add that
+// make a finished weight, which is then rounded to 16 bits.  With few token rows both can be left to the sums: the operand is
+// w + 24, which is a shift and one logic instruction from the nibbles (16 + (w + 8): the nibble in the mantissa of a 16-bit
+// float of exponent 16) and exact in both types, every block of 128 k has an accumulator of its own, and the epilogue warps fold
+// it into fp32 running outputs:
+//     y[m, n] += scale * acc[m, n] + scale * (offset - 24) * xs[m],    xs[m] = the block's sum of x[m, :].
+// The weight is never rounded, and scale and offset come from the caller's tables in full.  Carrying 24 along costs about two
+// bits of the 24 of the fp32 sums.  Infinite activations make infinite sums of both signs: an output that is not a number is
+// computed again, plainly (b_plain).
+//
+// A stage holds the nibbles of two blocks (not the stream's own tables) and their rows of scale and offset.  The epilogue warps
+// also make xs, from the activation tile in shared memory: warp e takes block e / 2 and eight tokens, a lane a quarter of the
+// block's k.  Everything else (roles, rings, cuts, slots) is as in the kernel above.
+//
+// us, this / the narrow form above / the stock layout (M x K x N): 8 x 1024 x 1024 5.8 / 5.5 / 17.2, 8 x 8192 x 1024 9.0 / 8.1 / 92,
+// 8 x 4096 x 4096 10.4 / 8.9 / 33.4, 8 x 8192 x 8192 18.4 / 15.4 / 30.9, 8 x 8192 x 28672 46.0 / 33.5 / 38.8.  A stage takes about
+// 1800 clocks, of which the epilogue warps' chain of instructions takes nearly all (waits are short, the issue slots 52 % used).
+// Measured without gain: two sets of epilogue warps in turn (44-48 us for the last), sums of x by warps of their own with a ring for
+// the tables (48-52), and sums of x from a kernel in front, without which the chain is half as long (42.8, but 6.5 for the first).
+constexpr int kBTok = 16;
+constexpr uint32_t kBAccBufs = 4;              // accumulators of a stage: two blocks x 16 columns
+constexpr uint32_t kBAccCols = kPPair * kBTok;
+constexpr uint32_t kBACol0 = kBAccBufs * kBAccCols;
+constexpr int kBRing = 3;
+static_assert(kBACol0 + kBRing * kPRingCols <= 512, "tensor memory");
+constexpr int kBTableBytes = kPTileN * 2;                                     // a block's row of scale, or of offset
+constexpr int kBStageBytes = kPPair * (kPWBytes + 2 * kBTableBytes);          // 17408: nibbles, nibbles, scales, offsets
+static_assert(kBStageBytes == kPStageWBytes, "the plan's stages");
+
+struct BSmemTail {
+    uint64_t w_full[kPMaxStages];
+    uint64_t w_empty[kPMaxStages];   // the unpack and the epilogue warps
+    uint64_t x_full[kPMaxXStages];
+    uint64_t x_empty[kPMaxXStages];  // the MMAs and the four epilogue warps
+    uint64_t a_full[kBRing];
+    uint64_t mma_done[kBRing];
+    uint64_t acc_full[kBAccBufs];
+    uint64_t acc_empty[kBAccBufs];
+    uint32_t tmem_base;
+    uint32_t abort_flag;
+    uint32_t is_last;
+    uint32_t epi_abort[2];           // [stage parity]: an epilogue warp gave up at that stage
+    __align__(16) float xs[2][kPPair][kBTok];  // [stage parity][block][token], read four at a time
+};
+
+struct BTables {
+    const void *scale, *offset;      // [groups][N]; offset may be null
+    int group_blocks;                // blocks of 128 k in a group
+    int nblocks;                     // blocks of 128 k along K
+    const void *x;
+    int64_t ld_x;
+};
+
+// 24 + w as a 16-bit float from the nibble of two neighbouring k; nibble p of each half word
+template <typename T>
+struct BMagic;
+template <>
+struct BMagic<__nv_bfloat16> {
+    static constexpr uint32_t kMask = 0x00780078u, kFlip = 0x41c041c0u;
+    static __device__ __forceinline__ uint32_t shifted(uint32_t w, int p) { return p == 0 ? w << 3 : w >> (4 * p - 3); }
+};
+template <>
+struct BMagic<__half> {
+    static constexpr uint32_t kMask = 0x03c003c0u, kFlip = 0x4e004e00u;
+    static __device__ __forceinline__ uint32_t shifted(uint32_t w, int p) { return p < 2 ? w << (6 - 4 * p) : w >> (4 * p - 6); }
+};
+
+// One output by the definition, for those that the sums above leave without a number.
+template <typename T>
+__device__ __noinline__ float b_plain_loop(const uint8_t *packed, const T *x, const T *scale, const T *offset, int group_blocks,
+                                           int nblocks, int nchunks, int N, int64_t n) {
+    const int r = static_cast<int>(n % kPTileN);
+    float y = 0.0f;
+    for (int blk = 0; blk < nblocks; ++blk) {
+        const uint8_t *src = packed + (n / kPTileN * nchunks * kPPair + blk) * kPBlockBytes;
+        const int64_t at = static_cast<int64_t>(blk / group_blocks) * N + n;
+        const float s = to_float(scale[at]), o = offset != nullptr ? to_float(offset[at]) : 0.0f;
+        for (int i = 0; i < kPChunkK / 8; ++i) {
+            const uint32_t word = reinterpret_cast<const uint32_t *>(src + ((i >> 2) * kPTileN + r) * 16)[i & 3];
+            for (int e = 0; e < 8; ++e) {
+                const int w = static_cast<int>(word << (28 - 4 * ((e >> 1) + (e & 1) * 4))) >> 28;
+                y = fmaf(to_float(x[blk * kPChunkK + i * 8 + e]), (static_cast<float>(w) + o) * s, y);
+            }
+        }
+    }
+    return y;
+}
+// (by value: a parameter block whose address is taken is copied to local memory, and every use of it in the kernel goes there)
+template <typename T>
+__device__ __forceinline__ float b_plain(const PParams &p, const BTables &t, int64_t n, int m) {
+    return b_plain_loop<T>(p.packed, static_cast<const T *>(t.x) + m * t.ld_x, static_cast<const T *>(t.scale),
+                           static_cast<const T *>(t.offset), t.group_blocks, t.nblocks, p.nchunks, p.N, n);
+}
+
+template <typename T>
+__device__ __forceinline__ void b_add_words(float &s, const uint4 &v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const T *h = reinterpret_cast<const T *>(&w[i]);
+        s += to_float(h[0]) + to_float(h[1]);
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kPThreads, 1)
+w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTables t) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *smem_aligned = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t nstages = static_cast<uint32_t>(p.nstages), nxstages = static_cast<uint32_t>(p.nxstages);
+    constexpr uint32_t kXBox = kBTok * 128, kXSlot = 4 * kXBox;  // an activation stage: four boxes of [16 tokens][64 k]
+    const uint32_t w_off = nxstages * kXSlot;
+    BSmemTail *tail = reinterpret_cast<BSmemTail *>(smem_aligned + w_off + nstages * kPStageWBytes);
+    volatile uint32_t *abort_flag = &tail->abort_flag;
+
+    const auto plain = [&](int64_t n, int m) { return b_plain<T>(p, t, n, m); };
+
+    const int warp = warp_id_uniform();
+    const int lane = threadIdx.x & 31;
+    const int cta = static_cast<int>(blockIdx.x);
+    const int u_begin = p_first_item<false>(p, cta), u_end = p_first_item<false>(p, cta + 1);
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < nstages; ++s) {
+            mbar_init(smem_u32(&tail->w_full[s]), 1);
+            mbar_init(smem_u32(&tail->w_empty[s]), kPUnpackWarps + kPEpiWarps);
+        }
+        for (uint32_t a = 0; a < nxstages; ++a) {
+            mbar_init(smem_u32(&tail->x_full[a]), 1);
+            mbar_init(smem_u32(&tail->x_empty[a]), 1 + kPEpiWarps);
+        }
+        for (int a = 0; a < kBRing; ++a) {
+            mbar_init(smem_u32(&tail->a_full[a]), kPUnpackWarps);
+            mbar_init(smem_u32(&tail->mma_done[a]), 1);
+        }
+        for (uint32_t b = 0; b < kBAccBufs; ++b) {
+            mbar_init(smem_u32(&tail->acc_full[b]), 1);
+            mbar_init(smem_u32(&tail->acc_empty[b]), kPEpiWarps);
+        }
+        tail->abort_flag = 0;
+        tail->epi_abort[0] = tail->epi_abort[1] = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&tmap_x);
+    }
+    if (warp == kPMmaWarp) {
+        tmem_alloc(smem_u32(&tail->tmem_base), kPTmemCols);
+        tmem_relinquish();
+        pdl_launch_dependents();
+    }
+    pdl_wait();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = warp_uniform(tail->tmem_base);
+
+    if (warp == 0) {
+        // ---------------- weight producer ----------------
+        int q = u_begin / p.nchunks, c = u_begin - q * p.nchunks;
+        uint32_t st = 0, ph = 0;
+        const uint32_t full0 = smem_u32(&tail->w_full[0]), empty0 = smem_u32(&tail->w_empty[0]);
+        for (int it = u_begin; it < u_end; ++it) {
+            if (!mbar_wait(empty0 + st * 8, ph ^ 1, abort_flag, 0x70)) break;
+            if (lane == 0) {
+                const uint32_t dst = smem_base + w_off + st * kBStageBytes, bar = full0 + st * 8;
+                // columns of this tile that exist: a multiple of eight, so the rows' copies are of whole 16 bytes
+                const uint32_t cols = static_cast<uint32_t>(min(kPTileN, p.N - q * kPTileN)) * 2;
+                const int blocks = min(kPPair, t.nblocks - c * kPPair);  // the last stage's second block may be padding
+                mbar_expect_tx(bar, kPPair * kPWBytes + blocks * cols * (t.offset != nullptr ? 2 : 1));
+                const uint8_t *src = p.packed + (static_cast<int64_t>(q) * p.nchunks + c) * kPStageWBytes;
+                for (int b = 0; b < kPPair; ++b) bulk_load_1d(dst + b * kPWBytes, src + b * kPBlockBytes, kPWBytes, bar);
+                for (int b = 0; b < blocks; ++b) {
+                    const int64_t at = (static_cast<int64_t>((c * kPPair + b) / t.group_blocks) * p.N + static_cast<int64_t>(q) * kPTileN) * 2;
+                    const uint32_t to = dst + kPPair * kPWBytes + b * kBTableBytes;
+                    bulk_load_1d(to, static_cast<const uint8_t *>(t.scale) + at, cols, bar);
+                    if (t.offset != nullptr) bulk_load_1d(to + kPPair * kBTableBytes, static_cast<const uint8_t *>(t.offset) + at, cols, bar);
+                }
+            }
+            __syncwarp();
+            if (++st == nstages) {
+                st = 0;
+                ph ^= 1;
+            }
+            if (++c == p.nchunks) {
+                c = 0;
+                ++q;
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- activation producer ----------------
+        int c = u_begin % p.nchunks;
+        uint32_t rs = 0, rph = 0;
+        for (int it = u_begin; it < u_end; ++it) {
+            if (!mbar_wait(smem_u32(&tail->x_empty[rs]), rph ^ 1, abort_flag, 0x77)) break;
+            if (lane == 0) {
+                const uint32_t bar = smem_u32(&tail->x_full[rs]);
+                mbar_expect_tx(bar, kXSlot);
+#pragma unroll
+                for (int b = 0; b < 4; ++b)  // rows beyond M and k beyond K arrive as zeros
+                    tma_load_2d(smem_base + rs * kXSlot + b * kXBox, &tmap_x, c * kPStageK + b * 64, 0, bar);
+            }
+            __syncwarp();
+            if (++rs == nxstages) {
+                rs = 0;
+                rph ^= 1;
+            }
+            if (++c == p.nchunks) c = 0;
+        }
+    } else if (warp == kPMmaWarp) {
+        // ---------------- MMA issuer: two accumulators a stage ----------------
+        const uint32_t idesc = make_idesc(/*c=f32*/ 1, PMagic<T>::kFmt, PMagic<T>::kFmt, /*a*/ 0, /*b K-major*/ 0, kPTileN, kBTok);
+        constexpr uint32_t kDescHi = smem_desc_hi_sw128(1024);
+        constexpr uint32_t kBox = kXBox >> 4;
+        uint32_t rs = 0, rph = 0, xs = 0, xph = 0, ab = 0, aph = 0;
+        for (int it = u_begin; it < u_end; ++it) {
+            if (!mbar_wait(smem_u32(&tail->acc_empty[ab]), aph ^ 1, abort_flag, 0x71)) break;
+            if (!mbar_wait(smem_u32(&tail->x_full[xs]), xph, abort_flag, 0x72)) break;
+            if (!mbar_wait(smem_u32(&tail->a_full[rs]), rph, abort_flag, 0x73)) break;
+            tc_fence_after();
+            const uint32_t d = tmem_base + ab * kBAccCols;
+            const uint32_t a = tmem_base + kBACol0 + rs * kPRingCols;
+            const uint32_t x_lo = smem_desc_lo(smem_base + xs * kXSlot, 16);
+            mma_f16_ts_warp_x8(d, a, x_lo, x_lo + kBox, kDescHi, idesc, 0);
+            mma_f16_ts_warp_x8(d + kBTok, a + 64, x_lo + 2 * kBox, x_lo + 3 * kBox, kDescHi, idesc, 0);
+            tc_commit_warp(smem_u32(&tail->acc_full[ab]));
+            tc_commit_warp(smem_u32(&tail->x_empty[xs]));
+            tc_commit_warp(smem_u32(&tail->mma_done[rs]));
+            if (++xs == nxstages) {
+                xs = 0;
+                xph ^= 1;
+            }
+            if (++rs == kBRing) {
+                rs = 0;
+                rph ^= 1;
+            }
+            if (++ab == kBAccBufs) {
+                ab = 0;
+                aph ^= 1;
+            }
+        }
+    } else if (warp < kPFirstEpiWarp) {
+        // ---------------- unpack warps ----------------
+        const int team = (warp - kPFirstUnpackWarp) >> 2;
+        const int quarter = warp & 3;
+        const int r = quarter * 32 + lane;
+        const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kBACol0 + team * 16;
+        uint32_t st = 0, ph = 0, rs = 0, rph = 0;
+        int pending = -1;  // ring slot whose stores are in flight
+        for (int it = u_begin; it < u_end; ++it) {
+            if (!mbar_wait(smem_u32(&tail->w_full[st]), ph, abort_flag, 0x74)) break;
+            const uint8_t *blk = smem_aligned + w_off + st * kBStageBytes;
+            uint4 wv[kPPair];
+#pragma unroll
+            for (int b = 0; b < kPPair; ++b) wv[b] = *reinterpret_cast<const uint4 *>(blk + b * kPWBytes + (team * kPTileN + r) * 16);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&tail->w_empty[st]));
+            uint32_t v[kPPair][16];
+#pragma unroll
+            for (int b = 0; b < kPPair; ++b) {
+                const uint32_t words[4] = {wv[b].x, wv[b].y, wv[b].z, wv[b].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        v[b][4 * i + j] = p_and_xor(BMagic<T>::shifted(words[i], j), BMagic<T>::kMask, BMagic<T>::kFlip);
+            }
+            // the previous stage's stores have had this stage's arithmetic to complete: announce them
+            if (pending >= 0) {
+                tmem_st_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&tail->a_full[pending]));
+            }
+            if (!mbar_wait(smem_u32(&tail->mma_done[rs]), rph ^ 1, abort_flag, 0x75)) break;
+            tc_fence_after();
+            tmem_st_32x16(lane_taddr + rs * kPRingCols, v[0]);
+            tmem_st_32x16(lane_taddr + rs * kPRingCols + 64, v[1]);
+            pending = static_cast<int>(rs);
+            if (++rs == kBRing) {
+                rs = 0;
+                rph ^= 1;
+            }
+            if (++st == nstages) {
+                st = 0;
+                ph ^= 1;
+            }
+        }
+        if (pending >= 0) {
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&tail->a_full[pending]));
+        }
+    } else {
+        // ---------------- epilogue warps: thread = tensor-memory lane = one output column ----------------
+        const int quarter = warp & 3;
+        const int row = quarter * 32 + lane;
+        const int ew = warp - kPFirstEpiWarp;
+        const T *bias = static_cast<const T *>(p.bias);
+        T *out = static_cast<T *>(p.out);
+        const int M = p.M;
+        // its share of xs: block ew / 2 of a stage, token 8 * (ew % 2) + lane % 8, k quarter lane / 8
+        const int xb = ew >> 1, xtok = 8 * (ew & 1) + (lane & 7), xq = lane >> 3;
+        const uint32_t x_row = (2 * xb + (xq >> 1)) * kXBox + xtok * 128;
+        int u = u_begin;
+        uint32_t ab = 0, aph = 0, xst = 0, xph = 0, wst = 0, wph = 0, parity = 0;
+        bool ok = true;
+        while (u < u_end && ok) {
+            const int q = u / p.nchunks;
+            const int tile_begin = q * p.nchunks, tile_end = tile_begin + p.nchunks;
+            const int seg_end = min(tile_end, u_end);
+            const bool whole = (u == tile_begin && seg_end == tile_end);
+            const int64_t n = static_cast<int64_t>(q) * kPTileN + row;
+            const bool n_ok = n < p.N;
+            const float b = (n_ok && bias != nullptr) ? to_float(bias[n]) : 0.0f;
+            float y[kBTok];
+#pragma unroll
+            for (int j = 0; j < kBTok; ++j) y[j] = 0.0f;
+            for (int it = u; it < seg_end; ++it) {
+                ok = mbar_wait(smem_u32(&tail->x_full[xst]), xph, abort_flag, 0x78);
+                float sum = 0.0f;
+                const uint8_t *xr = smem_aligned + xst * kXSlot + x_row;
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    b_add_words<T>(sum, *reinterpret_cast<const uint4 *>(xr + (((4 * (xq & 1) + c) ^ (xtok & 7)) << 4)));
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&tail->x_empty[xst]));
+                sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+                if (lane < 8) tail->xs[parity][xb][xtok] = sum;
+                // scale and scale * (offset - 24) of the stage's two blocks
+                ok = ok && mbar_wait(smem_u32(&tail->w_full[wst]), wph, abort_flag, 0x79);
+                float sc[kPPair], tc[kPPair];
+                const T *table = reinterpret_cast<const T *>(smem_aligned + w_off + wst * kBStageBytes + kPPair * kPWBytes) + row;
+#pragma unroll
+                for (int k = 0; k < kPPair; ++k) {
+                    const bool real = n_ok && (it - tile_begin) * kPPair + k < t.nblocks;
+                    sc[k] = real ? to_float(table[k * kPTileN]) : 0.0f;
+                    tc[k] = sc[k] * ((real && t.offset != nullptr ? to_float(table[(kPPair + k) * kPTileN]) : 0.0f) - 24.0f);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&tail->w_empty[wst]));
+                ok = ok && mbar_wait(smem_u32(&tail->acc_full[ab]), aph, abort_flag, 0x76);
+                // the four warps meet at named barriers, so they leave together or not at all
+                volatile uint32_t *gave_up = &tail->epi_abort[parity];
+                if (!ok) *gave_up = 1;
+                pepi_bar_sync();
+                if (*gave_up != 0) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + ab * kBAccCols;
+                uint32_t v[kPPair][16];
+                tmem_ld_32x16(taddr, v[0]);
+                tmem_ld_32x16(taddr + kBTok, v[1]);
+                tmem_ld_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&tail->acc_empty[ab]));
+#pragma unroll
+                for (int k = 0; k < kPPair; ++k)
+#pragma unroll
+                    for (int j = 0; j < kBTok; j += 4) {
+                        if (j >= M) break;
+                        const float4 x4 = *reinterpret_cast<const float4 *>(&tail->xs[parity][k][j]);
+                        y[j] = fmaf(tc[k], x4.x, fmaf(sc[k], __uint_as_float(v[k][j]), y[j]));
+                        y[j + 1] = fmaf(tc[k], x4.y, fmaf(sc[k], __uint_as_float(v[k][j + 1]), y[j + 1]));
+                        y[j + 2] = fmaf(tc[k], x4.z, fmaf(sc[k], __uint_as_float(v[k][j + 2]), y[j + 2]));
+                        y[j + 3] = fmaf(tc[k], x4.w, fmaf(sc[k], __uint_as_float(v[k][j + 3]), y[j + 3]));
+                    }
+                parity ^= 1;
+                if (++wst == nstages) {
+                    wst = 0;
+                    wph ^= 1;
+                }
+                if (++xst == nxstages) {
+                    xst = 0;
+                    xph ^= 1;
+                }
+                if (++ab == kBAccBufs) {
+                    ab = 0;
+                    aph ^= 1;
+                }
+            }
+            if (!ok) break;
+            if (whole) {
+                if (n_ok) {
+                    uint32_t again = 0;
+#pragma unroll
+                    for (int j = 0; j < kBTok; ++j) {
+                        if (j >= M) break;
+                        again |= isnan(y[j]) ? 1u << j : 0u;
+                        out[static_cast<int64_t>(j) * p.ld_out + n] = from_float<T>(y[j] + b);
+                    }
+                    for (; again != 0; again &= again - 1) {
+                        const int j = __ffs(static_cast<int>(again)) - 1;
+                        out[static_cast<int64_t>(j) * p.ld_out + n] = from_float<T>(b_plain<T>(p, t, n, j) + b);
+                    }
+                }
+            } else {
+                float *mine = p.slots + p_slot<false>(p, cta, q) * (static_cast<int64_t>(p.mpad) * kPTileN) + row;
+#pragma unroll
+                for (int j = 0; j < kBTok; ++j)
+                    if (j < M) __stcg(mine + j * kPTileN, y[j]);
+                if (seg_end < u_end) p_finish_shared<T, false, true>(p, q, abort_flag, &tail->is_last, plain);
+            }
+            u = seg_end;
+        }
+    }
+
+    // ---------------- teardown ----------------
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && tail->abort_flag != 0 && p.status != nullptr) atomicMax(p.status, tail->abort_flag);
+    if (warp == kPMmaWarp) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, kPTmemCols);
+    }
+    if (u_begin < u_end) p_finish_shared<T, false, false>(p, (u_end - 1) / p.nchunks, abort_flag, &tail->is_last, plain);
+}
+
 // ---- layout pass and its inverse ----------------------------------------------------------------------
 
 // Eight words of one word column, of rows k .. k + 7, to the eight columns' words: nibble j of row e becomes the nibble of row e
@@ -640,7 +1076,8 @@ __device__ __forceinline__ void p_transpose8(uint32_t (&w)[8]) {
 // One CTA per chunk of 128 k and TILES tiles: rows of 256 (64) bytes come in, are transposed in registers and leave as four (one)
 // blocks, through one buffer in shared memory both ways.  With a load from global memory for every nibble (a thread a 16-byte
 // vector, 32 strided loads each) 8192 x 28672 took 128 us, 4096 x 4096 7.2 and 1024 x 1024 2.7; now 65, 5.7 and 2.0.  One tile a CTA
-// where four leave SMs without work (1024 x 1024: 3.9 with four).  A weight's first call pays for this pass.
+// where four leave SMs without work (1024 x 1024: 3.9 with four).  A weight's first call pays for this pass, and every call of three to eight rows that
+// the operator sends here.
 constexpr int kPPackThreads = 256;
 template <typename T, int TILES>
 __global__ void __launch_bounds__(kPPackThreads)
@@ -1154,7 +1591,7 @@ int launch_gemv_t(const uint8_t *packed, const void *x, int64_t ld_x, const void
 
 template <typename T>
 int launch_prepacked_t(const uint8_t *packed, const void *x, int64_t ld_x, const void *bias, void *out, int64_t ld_out,
-                       int64_t M, int64_t N, int64_t K, void *workspace, cudaStream_t stream) {
+                       int64_t M, int64_t N, int64_t K, const BTables *tables, void *workspace, cudaStream_t stream) {
     const PPlan pl = p_make_plan(M, N, K);
     PParams p;
     p.packed = packed;
@@ -1183,7 +1620,13 @@ int launch_prepacked_t(const uint8_t *packed, const void *x, int64_t ld_x, const
     int rc = make_tmap_2d(&tx, x, 2, static_cast<uint64_t>(K), static_cast<uint64_t>(M), static_cast<uint64_t>(ld_x), 64,
                           static_cast<uint32_t>(pl.mpad), true);
     if (rc != QMM_OK) return rc;
-    static_assert(sizeof(PSmemTail) <= 1024, "the tail has 1 KiB");
+    static_assert(sizeof(PSmemTail) <= 1024 && sizeof(BSmemTail) <= 1024, "the tail has 1 KiB");
+    if (tables != nullptr && M <= kBTok) {
+        auto kern = w4a16_block_kernel<T>;
+        QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pl.smem)));
+        QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(pl.grid)), dim3(kPThreads), pl.smem, stream, tx, p, *tables));
+        return QMM_OK;
+    }
     auto kern = M <= kPMaxM ? w4a16_prepacked_kernel<T, false> : w4a16_prepacked_kernel<T, true>;
     QMM_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(pl.smem)));
     QMM_CUDA_OK(launch_pdl(kern, dim3(static_cast<unsigned>(pl.grid)), dim3(kPThreads), pl.smem, stream, tx, p));
@@ -1259,11 +1702,11 @@ extern "C" int qmm_weight_quant_batchmatmul_prepacked_workspace_size(int64_t M, 
     return QMM_OK;
 }
 
-extern "C" int qmm_weight_quant_batchmatmul_prepacked(const void *x, int x_dtype, int64_t ld_x, const void *packed,
-                                                      size_t packed_bytes, const void *bias, void *out,
-                                                      int64_t ld_out, int64_t M, int64_t N, int64_t K,
-                                                      void *workspace, size_t workspace_bytes, void *stream) {
-    using namespace qmm;
+namespace qmm {
+namespace {
+int prepacked_matmul(const void *x, int x_dtype, int64_t ld_x, const void *packed, size_t packed_bytes, const BTables *tables,
+                     const void *bias, void *out, int64_t ld_out, int64_t M, int64_t N, int64_t K, void *workspace,
+                     size_t workspace_bytes, void *stream) {
     QMM_REQUIRE(M >= 0, "qmm_weight_quant_batchmatmul_prepacked: negative M");
     QMM_REQUIRE(x_dtype == QMM_DTYPE_BF16 || x_dtype == QMM_DTYPE_F16,
                 "qmm_weight_quant_batchmatmul_prepacked: x must be bf16 or f16");
@@ -1292,7 +1735,41 @@ extern "C" int qmm_weight_quant_batchmatmul_prepacked(const void *x, int x_dtype
                                            workspace, s);
     return (x_dtype == QMM_DTYPE_BF16)
                ? launch_prepacked_t<__nv_bfloat16>(static_cast<const uint8_t *>(packed), x, ld_x, bias, out, ld_out, M, N, K,
-                                                   workspace, s)
+                                                   tables, workspace, s)
                : launch_prepacked_t<__half>(static_cast<const uint8_t *>(packed), x, ld_x, bias, out, ld_out, M, N, K,
-                                            workspace, s);
+                                            tables, workspace, s);
+}
+}  // namespace
+}  // namespace qmm
+
+extern "C" int qmm_weight_quant_batchmatmul_prepacked(const void *x, int x_dtype, int64_t ld_x, const void *packed,
+                                                      size_t packed_bytes, const void *bias, void *out,
+                                                      int64_t ld_out, int64_t M, int64_t N, int64_t K,
+                                                      void *workspace, size_t workspace_bytes, void *stream) {
+    return qmm::prepacked_matmul(x, x_dtype, ld_x, packed, packed_bytes, nullptr, bias, out, ld_out, M, N, K, workspace,
+                                 workspace_bytes, stream);
+}
+
+extern "C" int qmm_weight_quant_batchmatmul_prepacked_tables(const void *x, int x_dtype, int64_t ld_x, const void *packed,
+                                                             size_t packed_bytes, const void *antiquant_scale,
+                                                             const void *antiquant_offset, int64_t group, const void *bias,
+                                                             void *out, int64_t ld_out, int64_t M, int64_t N, int64_t K,
+                                                             void *workspace, size_t workspace_bytes, void *stream) {
+    using namespace qmm;
+    if (group <= 0) group = K;
+    if (!p_shape_ok(N, K, group))
+        return fail(QMM_ERR_UNSUPPORTED, "qmm_weight_quant_batchmatmul_prepacked_tables: needs N % 8 == 0, K % 128 == 0 and a "
+                                         "group that is a multiple of 128 dividing K");
+    QMM_REQUIRE(antiquant_scale != nullptr, "qmm_weight_quant_batchmatmul_prepacked_tables: NULL scale");
+    BTables t;
+    t.scale = antiquant_scale;
+    t.offset = antiquant_offset;
+    t.group_blocks = static_cast<int>(group / kPChunkK);
+    t.nblocks = static_cast<int>(K / kPChunkK);
+    t.x = x;
+    t.ld_x = ld_x;
+    // the tables' rows are fetched by copies of whole 16 bytes
+    const bool aligned = ((reinterpret_cast<uintptr_t>(antiquant_scale) | reinterpret_cast<uintptr_t>(antiquant_offset)) & 15) == 0;
+    return prepacked_matmul(x, x_dtype, ld_x, packed, packed_bytes, aligned ? &t : nullptr, bias, out, ld_out, M, N, K, workspace,
+                            workspace_bytes, stream);
 }

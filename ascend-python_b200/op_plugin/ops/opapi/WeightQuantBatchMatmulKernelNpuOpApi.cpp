@@ -15,11 +15,14 @@
 // storages are alive and their version counters are unchanged (an in-place update re-packs); the cache holds
 // a second copy of the weights, bounded by QMM_W4_PREPACK_MAX_MB (default 16384; QMM_W4_PREPACK=0 switches
 // the format off).  Callers that want a single copy prepack explicitly through the C ABI and drop the original.
+#include <algorithm>
 #include <cstdlib>
 #include <map>
 #include <mutex>
 #include <optional>
 #include <tuple>
+
+#include <ATen/cuda/CUDAContext.h>
 
 #include "op_plugin/OpApiInterface.h"
 #include "op_plugin/utils/qmm_api_common.h"
@@ -121,6 +124,33 @@ at::Tensor prepacked_weight(const at::Tensor &w, const at::Tensor &scale, const 
     return packed;
 }
 
+// Three to eight rows: whether to rewrite the weight as the stream, for this call alone, and to multiply over that.  Both ways
+// keep the weight unrounded.  The stock layout's kernel is short of parallel work unless the weight is large and has many
+// groups: it cuts K at groups only, and its last CTA of 512 columns adds a share of every CTA before it.  Its time (us, 3 rows; up
+// to 20 % more for 8) is close to 4 + 1.25 shares + 1.25 for every 128 k of a CTA, that of packing and the kernel over the
+// stream to 8 + 0.45 for every 2^20 weights; measured, stock / this: 1024 x 1024 14.3 / 7.7, 8192 x 1024 88 / 13, 4096 x 4096
+// 28.7 / 16.7, 5120 x 4608 28.6 / 17.7, 28672 x 768 in one group 269 / 19, 2048 x 12288 17.1 / 18.5, 8192 x 8192 26.8 / 37.
+// Stock rows that TMA cannot address leave only a CUDA-core kernel there (4480 x 4712 154 / 17.5, 128 x 72 32.3 / 6.6,
+// 8192 x 28680 533 / 113).  Small weights of addressable rows keep the stock kernel, and with it its bits (1024 x 512).
+bool few_rows_repack(const at::Tensor &x, const at::Tensor &w, const at::Tensor &scale, const at::Tensor &offset, int64_t group,
+                     int64_t N, int64_t K)
+{
+    auto aligned16 = [](const at::Tensor &t) { return !t.defined() || (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15) == 0; };
+    if (K <= 0 || K * N > (256ll << 20) || !aligned16(x) || !aligned16(scale) || !aligned16(offset)) {
+        return false;
+    }
+    if (N % 32 != 0 || group % 64 != 0 || !aligned16(w)) {
+        return true;
+    }
+    if (K * N < (1ll << 20)) {
+        return false;
+    }
+    const float groups = static_cast<float>(K / group), items = groups * static_cast<float>((N + 511) / 512);
+    const float per_cta = std::max(1.0f, items / at::cuda::getCurrentDeviceProperties()->multiProcessorCount);
+    const float stock = 4.0f + 1.25f * (groups / per_cta + 1.0f) + 1.25f / 128 * per_cta * static_cast<float>(group);
+    return 8.0f + 0.45f / (1 << 20) * static_cast<float>(K * N) < stock;
+}
+
 }  // namespace
 
 at::Tensor npu_weight_quant_batchmatmul(const at::Tensor &x, const at::Tensor &weight,
@@ -186,10 +216,26 @@ at::Tensor npu_weight_quant_batchmatmul(const at::Tensor &x, const at::Tensor &w
     at::Tensor oc = offset_real.defined() ? offset_real.contiguous() : offset_real;
     at::Tensor bc = bias_real.defined() ? bias_real.contiguous() : bias_real;
     // One or two token rows (integer dot products) and more than eight (operand unpacked into tensor memory) go to the
-    // kernels over the prepacked stream.  Three to eight stay on the stock layout, whose kernel does not round the weight
-    // to 16 bits, although it is slower by now (8 tokens, stock / prepacked: 8192 x 28672 39.3 / 34.0 us, 4096 x 4096
-    // 33.7 / 9.0 us; 9 tokens 47.8 / 34.0 and 33.0 / 9.2 us).
-    if (prepack_enabled() && (M <= 2 || M > 8) && K > 0) {
+    // kernels over the prepacked stream; three to eight go to the two below, neither of which rounds the weight to 16 bits.
+    const bool few = M > 2 && M <= 8;
+    if (few && prepack_enabled() && few_rows_repack(xc, wc, sc, oc, group, N, K)) {
+        size_t bytes = 0, ws_size = 0;
+        EXEC_QMM_CMD(qmm_w4a16_prepack_size, N, K, group, &bytes);
+        if (bytes != 0) {
+            at::Tensor packed = op_plugin_utils::empty_output({static_cast<int64_t>(bytes)}, xc, at::kByte);
+            EXEC_QMM_CMD(qmm_w4a16_prepack, static_cast<const int32_t *>(wc.const_data_ptr()), N / 8, sc.const_data_ptr(),
+                         op_plugin_utils::opt_ptr(oc), op_plugin_utils::qmm_dtype(sc.scalar_type()), group, N, K,
+                         packed.data_ptr(), bytes, op_plugin_utils::current_stream(xc));
+            EXEC_QMM_CMD(qmm_weight_quant_batchmatmul_prepacked_workspace_size, M, N, K, &ws_size);
+            at::Tensor ws = op_plugin_utils::qmm_workspace(xc, ws_size, /*family=*/2);
+            EXEC_QMM_CMD(qmm_weight_quant_batchmatmul_prepacked_tables, xc.const_data_ptr(),
+                         op_plugin_utils::qmm_dtype(xc.scalar_type()), K, packed.const_data_ptr(), bytes, sc.const_data_ptr(),
+                         op_plugin_utils::opt_ptr(oc), group, op_plugin_utils::opt_ptr(bc), result.data_ptr(), N, M, N, K,
+                         ws.defined() ? ws.data_ptr() : nullptr, ws_size, op_plugin_utils::current_stream(xc));
+            return result;
+        }
+    }
+    if (prepack_enabled() && !few && K > 0) {
         at::Tensor packed = prepacked_weight(wc, sc, oc, group, N, K);
         if (packed.defined()) {
             size_t ws_size = 0;

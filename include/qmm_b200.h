@@ -255,6 +255,14 @@ QMM_API int qmm_weight_quant_batchmatmul_prepacked(const void *x, int x_dtype, i
                                                    size_t packed_bytes, const void *bias, void *out,
                                                    int64_t ld_out, int64_t M, int64_t N, int64_t K,
                                                    void *workspace, size_t workspace_bytes, void *stream);
+/* The same with the tables the weight was packed with, [K / group, N] in x's type (antiquant_offset may be NULL): 3 to 16 rows
+ * then apply scale and offset to the sums of 128 k, from these tables in full, and do not round the weight.  (Tables that are
+ * not 16-byte aligned are not used.) */
+QMM_API int qmm_weight_quant_batchmatmul_prepacked_tables(const void *x, int x_dtype, int64_t ld_x, const void *packed,
+                                                          size_t packed_bytes, const void *antiquant_scale,
+                                                          const void *antiquant_offset, int64_t group, const void *bias,
+                                                          void *out, int64_t ld_out, int64_t M, int64_t N, int64_t K,
+                                                          void *workspace, size_t workspace_bytes, void *stream);
 
 /*
  * Communicator registry.  The reference passes a communicator NAME into its

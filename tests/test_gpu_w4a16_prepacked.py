@@ -269,3 +269,73 @@ def test_prepack_of_a_pitched_or_unaligned_weight(capi, oracle, dev, N):
         capi.check(capi.lib().qmm_w4a16_prepack(ctypes.c_void_p(rows.data_ptr()), pitch, capi._ptr(sc), capi._ptr(of), capi.DTYPE_BF16,
                                                 128, N, K, capi._ptr(got), got.numel(), capi._stream()), "prepack")
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(3, 128, 8, 128), (8, 384, 200, 128), (5, 1152, 4104, 384), (4, 8192, 1024, 256), (7, 2048, 136, 2048),
+                                   (16, 1024, 1032, 128), (9, 640, 20008, 128)])
+def test_few_tokens_with_tables_meet_the_stock_tolerance(capi, oracle, dev, shape, dtype):
+    """Three to sixteen rows with the tables at hand: the weight is never rounded, so the stock layout's bound holds (see above);
+    with and without offset and bias; tables at odd addresses are not used, which leaves the bound of the rounded weight."""
+    M, K, N, group = shape
+    x, packed_w, scale, offset = oracle.make_w4a16_inputs(M, K, N, seed=M + K + N, group=group, dtype=dtype)
+    bias = torch.randn(N, generator=torch.Generator().manual_seed(N)).to(dtype)
+    u = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
+    for off, b in ((offset, None), (None, bias)):
+        y_ref = oracle.weight_quant_batchmatmul(x, packed_w, scale, off, bias=b, antiquant_group_size=group)
+        sd, od = scale.to(dev), None if off is None else off.to(dev)
+        buf = capi.w4a16_prepack(packed_w.to(dev), sd, od, group_size=group)
+        got = [capi.weight_quant_batchmatmul_prepacked(x.to(dev), buf, N, bias=None if b is None else b.to(dev), tables=(sd, od, group))
+               for _ in range(20)]
+        assert all(torch.equal(got[0], g) for g in got)
+        y = got[0].float().cpu().numpy()
+        rms = np.sqrt(np.mean(y_ref ** 2, axis=1, keepdims=True))
+        assert np.all(np.abs(y - y_ref) <= 2 * u * np.abs(y_ref) + 2.0 ** -7 * (u / 2.0 ** -9) * rms + 1e-30)
+        shifted = torch.empty(sd.numel() + 1, dtype=dtype, device=dev)
+        shifted[1:] = sd.flatten()
+        y1 = capi.weight_quant_batchmatmul_prepacked(x.to(dev), buf, N, bias=None if b is None else b.to(dev), tables=(shifted[1:], od, group))
+        _assert_close(y1, y_ref, _rss(oracle, x, packed_w, scale, off, group), dtype)
+    assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(4, 256, 136), (6, 4096, 1032), (8, 640, 2056)])
+def test_few_tokens_infinities_and_nans(capi, oracle, dev, shape):
+    """An infinity in a row makes its outputs infinite with the weight's sign, two of them or a NaN what plain arithmetic makes
+    of it, and leaves the other rows alone: whole tiles and tiles that CTAs share."""
+    M, K, N = shape
+    x, packed_w, scale, offset = oracle.make_w4a16_inputs(M, K, N, seed=K, group=128)
+    clean = x.clone()
+    x[0, 3], x[1, K - 1] = float("inf"), float("-inf")
+    x[2, 5], x[2, 9] = float("inf"), float("-inf")
+    x[3, 7] = float("nan")
+    sd, od = scale.to(dev), offset.to(dev)
+    buf = capi.w4a16_prepack(packed_w.to(dev), sd, od, group_size=128)
+    W = torch.from_numpy(np.asarray(oracle.antiquant_weight(packed_w, scale, offset, 128), dtype=np.float32))
+    want = (x.float()[:4, :, None] * W[None]).sum(dim=1)
+    y = capi.weight_quant_batchmatmul_prepacked(x.to(dev), buf, N, tables=(sd, od, 128)).float().cpu()
+    assert torch.equal(torch.isnan(y[:4]), torch.isnan(want)) and torch.equal(torch.isinf(y[:4]), torch.isinf(want))
+    assert torch.equal(torch.sign(y[:2]), torch.sign(want[:2]))
+    y_clean = capi.weight_quant_batchmatmul_prepacked(clean.to(dev), buf, N, tables=(sd, od, 128)).float().cpu()
+    assert torch.equal(y[4:], y_clean[4:])
+
+
+def test_operator_takes_few_rows_of_any_width(oracle, dev):
+    """npu_weight_quant_batchmatmul with 3 to 8 rows: widths whose packed rows TMA cannot address, small and large, x at an odd
+    address; never further from 64 bits than the stock layout's bound."""
+    import sys
+    from pathlib import Path
+
+    sys.path.insert(0, str(Path(__file__).resolve().parent.parent / "ascend-python_b200"))
+    try:
+        import torch_npu
+    finally:
+        sys.path.pop(0)
+    for M, K, N, group in ((3, 1024, 1024, 128), (8, 4096, 6144, 128), (5, 4096, 6176, 128), (3, 384, 1000, 0), (8, 2048, 13528, 128), (4, 192, 72, 64)):
+        x, packed_w, scale, offset = oracle.make_w4a16_inputs(M, K, N, seed=M + N, group=group or K)
+        y_ref = oracle.weight_quant_batchmatmul(x, packed_w, scale, offset, antiquant_group_size=group or K)
+        rms = np.sqrt(np.mean(y_ref ** 2, axis=1, keepdims=True))
+        flat = torch.empty(M * K + 1, dtype=x.dtype, device=dev)
+        flat[1:] = x.to(dev).flatten()
+        for xd in (x.to(dev), flat[1:].view(M, K)):
+            y = torch_npu.npu_weight_quant_batchmatmul(xd, packed_w.to(dev), scale.to(dev), offset.to(dev), antiquant_group_size=group)
+            assert np.all(np.abs(y.float().cpu().numpy() - y_ref) <= 2.0 ** -8 * np.abs(y_ref) + 2.0 ** -7 * rms)
