@@ -93,7 +93,14 @@ __device__ __forceinline__ int requant_one(int32_t acc, float scale_n, float per
 // staging row by row, a warp's lanes on consecutive columns: with every lane on a
 // row of its own they took 2.9 ms at 8170 x 1952 x 23465.
 // Per-column scale and bias of a chunk are fetched once per warp (coalesced)
-// into a small shared array and read back as broadcasts.
+// into a small shared array and read back as broadcasts.  Loads run one step
+// ahead of their use - the next 32 columns of the accumulator and the next
+// chunk's constants are under way while these columns are computed: one warp
+// per scheduler has nothing else to cover them with.
+// us before / now, CTA-pair kernel, M x K x N: 272 x 1024 x 28672 32.6 / 22.3,
+// 2048 x 1024 x 28672 90.1 / 64.8 (int8 out 93.7 / 72.9), 2048 x 2048 x 8192 35.0 /
+// 28.4; at K = 4096, where only the last tile's epilogue shows, 512 x 4096 x 28672
+// 49.9 / 47.5; one-CTA kernel, 100 x 8192 x 28672 44.1 / 40.7.
 //
 // `stage` points to this warp's 8 KiB staging area (1024-byte aligned),
 // `colbuf` to its 2*64 floats.  `chunk_counter` persists across tiles: it
@@ -141,6 +148,35 @@ __device__ __forceinline__ void epilogue_warp_tile(const EpilogueParams &p, cons
     const uint32_t stage_u32 = smem_u32(stage);
     if (m_warp0 >= p.M) return;  // the warp's rows are all padding
 
+    // constants of 32 columns a word: of a chunk (16- and 32-bit outputs), or of the next 32 columns (int8)
+    constexpr int kAhead = is_i8 ? 1 : CC / 32;
+    float next_sc[kAhead], next_add[kAhead];  // add: bias (16-bit), int32 bias as bits (int32), offset (int8)
+    int32_t next_bias = 0;                    // int8
+    auto fetch = [&](int64_t first) {
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            const int64_t n = first + q * 32 + lane;
+            next_sc[q] = is_i8 ? 0.0f : 1.0f;
+            next_add[q] = 0.0f;
+            if (is_i8) next_bias = 0;
+            if (n >= p.N) continue;
+            if constexpr (is_int) {
+                if (has_bias) next_add[q] = __int_as_float(__ldg(static_cast<const int32_t *>(p.bias) + n));
+            } else {
+                next_sc[q] = p.scale_is_scalar ? __ldg(p.scale) : __ldg(p.scale + n);
+                if constexpr (is_i8) {
+                    if (p.offset != nullptr) next_add[q] = p.offset_is_scalar ? __ldg(p.offset) : __ldg(p.offset + n);
+                    if (has_bias) next_bias = __ldg(static_cast<const int32_t *>(p.bias) + n);
+                } else if (has_bias) {
+                    next_add[q] = load_bias_f32(p, n);
+                }
+            }
+        }
+    };
+    fetch(n_tile0);
+    uint32_t ahead[32];
+    tmem_ld_32x32(taddr_warp, ahead);
+
 #pragma unroll 1
     for (int c = 0; c < TILE_N / CC; ++c) {
         const int64_t n0 = n_tile0 + static_cast<int64_t>(c) * CC;
@@ -151,22 +187,13 @@ __device__ __forceinline__ void epilogue_warp_tile(const EpilogueParams &p, cons
         __syncwarp();
 
         if constexpr (!is_i8) {
-            // per-column constants of this chunk -> shared (coalesced), as fp32 bit patterns
+            // per-column constants of this chunk -> shared, as fp32 bit patterns
 #pragma unroll
-            for (int i = lane; i < CC; i += 32) {
-                const int64_t n = n0 + i;
-                float sc = 1.0f, bi = 0.0f;
-                if (n < p.N) {
-                    if (is_int) {
-                        if (has_bias) bi = __int_as_float(__ldg(static_cast<const int32_t *>(p.bias) + n));
-                    } else {
-                        sc = p.scale_is_scalar ? __ldg(p.scale) : __ldg(p.scale + n);
-                        if (has_bias) bi = load_bias_f32(p, n);
-                    }
-                }
-                colbuf[i] = sc;
-                colbuf[64 + i] = bi;
+            for (int q = 0; q < kAhead; ++q) {
+                colbuf[q * 32 + lane] = next_sc[q];
+                colbuf[64 + q * 32 + lane] = next_add[q];
             }
+            if (c + 1 < TILE_N / CC) fetch(n0 + CC);
             __syncwarp();
         }
 
@@ -174,23 +201,21 @@ __device__ __forceinline__ void epilogue_warp_tile(const EpilogueParams &p, cons
 #pragma unroll
         for (int h = 0; h < CC / 32; ++h) {
             if constexpr (is_i8) {  // scale, offset and int32 bias of 32 columns at a time
-                const int64_t n = n0 + h * 32 + lane;
-                float sc = 0.0f, off = 0.0f;
-                int32_t bi = 0;
-                if (n < p.N) {
-                    sc = p.scale_is_scalar ? __ldg(p.scale) : __ldg(p.scale + n);
-                    if (p.offset != nullptr) off = p.offset_is_scalar ? __ldg(p.offset) : __ldg(p.offset + n);
-                    if (has_bias) bi = __ldg(static_cast<const int32_t *>(p.bias) + n);
-                }
                 __syncwarp();  // the previous columns' constants have been read
-                colbuf[lane] = sc;
-                colbuf[32 + lane] = off;
-                colbuf[64 + lane] = __int_as_float(bi);
+                colbuf[lane] = next_sc[0];
+                colbuf[32 + lane] = next_add[0];
+                colbuf[64 + lane] = __int_as_float(next_bias);
+                if (h + 1 < CC / 32 || c + 1 < TILE_N / CC) fetch(n0 + h * 32 + 32);
                 __syncwarp();
             }
             uint32_t acc[32];
-            tmem_ld_32x32(taddr_warp + c * CC + h * 32, acc);
             tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                acc[j] = ahead[j];
+                asm volatile("" : "+r"(acc[j]));  // read behind the wait
+            }
+            if (h + 1 < CC / 32 || c + 1 < TILE_N / CC) tmem_ld_32x32(taddr_warp + c * CC + (h + 1) * 32, ahead);
             if constexpr (is_i8) {
                 const bool has_off = p.offset != nullptr;
 #pragma unroll
@@ -261,6 +286,7 @@ __device__ __forceinline__ void epilogue_warp_tile(const EpilogueParams &p, cons
         }
         ++chunk_counter;
     }
+    tmem_ld_wait();  // of a tile that ends inside the output's last columns, one load is still under way
 }
 
 // One element (used by kernels whose threads own a column of the accumulator).

@@ -103,3 +103,20 @@ def test_int8_stream_k_time(dev):
     whole = us(lambda: torch_npu.npu_quant_matmul(a, w, scale, bias=bias, output_dtype=torch.int32))
     narrow = us(lambda: torch_npu.npu_quant_matmul(a, w, scale, offset=scale, pertoken_scale=pt, bias=bias, output_dtype=torch.int8))
     assert narrow < 1.45 * whole, f"int8 {narrow:.1f} us, int32 {whole:.1f} us"
+
+
+@pytest.mark.parametrize("N", [16, 32, 48, 96, 112, 160, 208, 240, 272, 400, 496])
+def test_tiles_that_end_inside_a_chunk(capi, dev, N):
+    """Loads run one step ahead of their use: outputs whose last columns end in any 32 or 64 of a tile, in both kernels that share
+    the epilogue, equal the dp4a kernel's (the same fp32 operations in the same order), bias and per-token scale included."""
+    M, K = 300, 272
+    g = torch.Generator(device=dev).manual_seed(N)
+    a = torch.randint(-128, 128, (M, K), generator=g, device=dev, dtype=torch.int8)
+    w = torch.randint(-128, 128, (K, N), generator=g, device=dev, dtype=torch.int8)
+    scale, pt = torch.rand(N, generator=g, device=dev) * 1e-2, torch.rand(M, generator=g, device=dev)
+    bias, ibias = torch.randn(N, generator=g, device=dev), torch.arange(N, device=dev, dtype=torch.int32) - 7
+    for algo in (capi.ALGO_PAIR, capi.ALGO_TILE):
+        for dtype, sc, p, b in ((torch.bfloat16, scale, pt, bias), (torch.float16, scale, None, bias.half()), (torch.int32, None, None, ibias)):
+            got = capi.quant_matmul(a, w, sc, pertoken_scale=p, bias=b, output_dtype=dtype, algo=algo)
+            assert torch.equal(got, capi.quant_matmul(a, w, sc, pertoken_scale=p, bias=b, output_dtype=dtype, algo=capi.ALGO_SIMT))
+    assert capi.device_status() == 0
