@@ -451,6 +451,10 @@ bool prefer_cluster(int64_t M, int64_t N, int64_t K) {
     // so few columns and so long a K that four slices leave a CTA a long chain: stream-K (M x K x N = 1 x 28672 x 512 9.0 us,
     // here 10.9; 8 x 28672 x 1024 10.8 / 11.6; 16 x 28672 x 1024 12.2 / 11.6; 8 x 16384 x 1024 10.0 / 8.0)
     if (M <= 8 && N <= 4 * kCUnitN && num_kb > 176) return false;
+    // tiles of 256 x 256 either way: the persistent kernel computes one while it stores the one before (us, here / there:
+    // 512 x 4096 x 14336 29.0 / 26.9, 2048 x 4096 x 4096 28.6 / 26.7, 1024 x 1024 x 4096 9.9 / 9.4, 2048 x 14336 x 4096 77.9 / 77.2;
+    // 640 x 4096 x 8192, three lower tiles here, 19.8 / 25.9)
+    if (M > 128 && pl.T == kCMaxT && pl.slices == 1) return false;
     // some SMs with two high tiles, others with one, over a long K (145 x 22544 x 25264 int32 172 us with the CTA-pair kernel,
     // 176 here; 192 x 14336 x 25264 97 / 76)
     if (pl.T > 128 && num_kb > 160 && pl.slices == 1 && pl.clusters > sm_count() / 2 && pl.clusters < sm_count() * 4 / 5) return false;
