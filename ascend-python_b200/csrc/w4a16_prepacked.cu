@@ -587,13 +587,18 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
             if (whole) {
                 // The next 16 tokens' sums are under way while these are stored, and the accumulator is free once the last are in
                 // registers: with one accumulator the tensor pipe waits for this loop.  Loading and storing in turn, 1000 x 4096 x
-                // 28672 took 195 us and 1000 x 1024 x 28672 97; now 190 and 85.
+                // 28672 took 191-195 us and 1000 x 1024 x 28672 97; now 178-180 and 60-80.
                 auto store = [&](const uint32_t(&v)[16], int c0) {
                     if (!n_ok) return;
                     T *at = o + static_cast<int64_t>(c0) * p.ld_out;
+                    if (c0 + 16 <= rows) {  // (without this form the two take 190 and 85)
 #pragma unroll
-                    for (int j = 0; j < 16; ++j, at += p.ld_out)
-                        if (c0 + j < rows) *at = from_float<T>(__uint_as_float(v[j]) + b);
+                        for (int j = 0; j < 16; ++j, at += p.ld_out) *at = from_float<T>(__uint_as_float(v[j]) + b);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j, at += p.ld_out)
+                            if (c0 + j < rows) *at = from_float<T>(__uint_as_float(v[j]) + b);
+                    }
                 };
                 auto arrived = [&](uint32_t(&v)[16], bool last) {
                     tmem_ld_wait();
