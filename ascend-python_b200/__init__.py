@@ -24,7 +24,7 @@ def load_ops():
 
 
 def load_calls():
-    """The operator library's short-cut calls (see ops_loader.calls)."""
+    """The operators' short-cut calls (see ops_loader.calls)."""
     from .ops_loader import calls
 
     return calls()

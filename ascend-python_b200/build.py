@@ -1,9 +1,12 @@
-"""In-tree build of the two native libraries.
+"""In-tree build of the native libraries.
 
 * ``lib/libqmm_b200.so``  — the CUDA kernels behind the C ABI of
   ``include/qmm_b200.h`` (nvcc, sm_100a only).
 * ``lib/libop_plugin_b200.so`` — the C++ operator host code (``op_plugin/``)
-  with its generated torch-library registration, linked against the first.
+  with its generated torch-library registration, linked against the first.  It
+  needs no Python: a C++ program loads it as it is.
+* ``lib/_op_plugin_calls.so`` — the operators' short-cut calls, a Python
+  extension module beside it (``op_plugin/utils/python_calls.cpp``).
 
 Objects are rebuilt only when a source or header is newer than the object.
 Run ``python build.py`` (add ``--force`` to rebuild everything).
@@ -31,6 +34,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-fvisibilit
 
 KERNEL_LIB = LIB / "libqmm_b200.so"
 PLUGIN_LIB = LIB / "libop_plugin_b200.so"
+CALLS_LIB = LIB / "_op_plugin_calls.so"
 
 
 def _nvcc() -> str:
@@ -108,6 +112,7 @@ def build_plugin(force=False, verbose=False) -> Path:
 
     BUILD.mkdir(exist_ok=True)
     LIB.mkdir(exist_ok=True)
+    calls_source = OPP / "utils" / "python_calls.cpp"
     sources = sorted((OPP / "ops" / "opapi").glob("*.cpp")) + sorted((OPP / "utils").glob("*.cpp")) + \
         [OPP / "OpInterface.cpp", OPP / "TorchLibrary.cpp"]
     headers = list(OPP.rglob("*.h")) + [ROOT / "include" / "qmm_b200.h"]
@@ -119,17 +124,24 @@ def build_plugin(force=False, verbose=False) -> Path:
     flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={abi}",
              "-DTORCH_API_INCLUDE_EXTENSION_H", "-Wno-deprecated-declarations", *incs]
     jobs, objs = [], []
+    calls_obj = None
     for src in sources:
         obj = BUILD / ("opp_" + src.stem + ".o")
-        objs.append(obj)
+        if src == calls_source:
+            calls_obj = obj
+        else:
+            objs.append(obj)
         if force or _newer(obj, [src, *headers]):
             jobs.append([cxx, *flags, "-c", src, "-o", obj])
     with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
         list(ex.map(lambda c: _run(c, verbose), jobs))
+    tlib = Path(torch.__file__).parent / "lib"
+    torch_libs = [f"-L{tlib}", "-ltorch", "-ltorch_cpu", "-lc10", f"-Wl,-rpath,{tlib}"]
     if force or jobs or _newer(PLUGIN_LIB, objs + [KERNEL_LIB]):
-        tlib = Path(torch.__file__).parent / "lib"
-        _run([cxx, "-shared", "-o", PLUGIN_LIB, *objs, f"-L{LIB}", "-lqmm_b200", f"-L{tlib}", "-ltorch", "-ltorch_cpu",
-              "-lc10", "-ltorch_cuda", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}"], verbose)
+        _run([cxx, "-shared", "-o", PLUGIN_LIB, *objs, f"-L{LIB}", "-lqmm_b200", *torch_libs, "-ltorch_cuda", "-lc10_cuda",
+              "-Wl,-rpath,$ORIGIN"], verbose)
+    if force or jobs or _newer(CALLS_LIB, [calls_obj]):
+        _run([cxx, "-shared", "-o", CALLS_LIB, calls_obj, *torch_libs, "-ltorch_python"], verbose)
     return PLUGIN_LIB
 
 

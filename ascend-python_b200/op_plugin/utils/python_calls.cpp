@@ -6,7 +6,8 @@
 // tracing, functorch and dispatch modes see what they saw before.  What it does not know - subclasses of Tensor, an active
 // __torch_function__ mode, arguments of other types - it leaves to torch.ops: it returns NotImplemented.
 //
-// The library is a Python extension module for this (ops_loader.py); importing it adds nothing to the registrations.
+// A Python extension module of its own (ops_loader.py): the operators are looked up by name in the dispatcher, so the library that
+// registers them needs no Python and a C++ program can load it.
 #include <torch/csrc/python_headers.h>
 
 #include <ATen/PythonTorchFunctionTLS.h>
@@ -168,8 +169,8 @@ PyMethodDef methods[] = {method<dynamic_quant>("dynamic_quant"),
                          method<weight_quant_batchmatmul>("weight_quant_batchmatmul"),
                          {nullptr, nullptr, 0, nullptr}};
 
-PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "libop_plugin_b200", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_op_plugin_calls", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 
-extern "C" OP_PLUGIN_EXPORT PyObject *PyInit_libop_plugin_b200() { return PyModule_Create(&module_def); }
+extern "C" OP_PLUGIN_EXPORT PyObject *PyInit__op_plugin_calls() { return PyModule_Create(&module_def); }

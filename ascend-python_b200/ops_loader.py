@@ -1,6 +1,6 @@
 """Loads the operator library so that ``torch.ops.npu.npu_*`` resolve, and its short-cut calls (``calls()``).
 
-No fallback exists: if ``lib/libop_plugin_b200.so`` is missing this raises and
+No fallback exists: if a library under ``lib/`` is missing this raises and
 tells how to build it.
 """
 from __future__ import annotations
@@ -13,16 +13,21 @@ import torch
 
 _PKG = Path(__file__).resolve().parent
 PLUGIN_PATH = _PKG / "lib" / "libop_plugin_b200.so"
+CALLS_PATH = _PKG / "lib" / "_op_plugin_calls.so"
 _loaded = False
 _calls = None
+
+
+def _require(path):
+    if not path.exists():
+        raise RuntimeError(f"{path} is not built; run `python {_PKG / 'build.py'}` "
+                           "(there is no fallback implementation)")
 
 
 def load():
     global _loaded
     if not _loaded:
-        if not PLUGIN_PATH.exists():
-            raise RuntimeError(f"{PLUGIN_PATH} is not built; run `python {_PKG / 'build.py'}` "
-                               "(there is no fallback implementation)")
+        _require(PLUGIN_PATH)
         from . import capi
 
         capi.lib()  # RTLD_GLOBAL: the plugin resolves qmm_* from it
@@ -32,13 +37,14 @@ def load():
 
 
 def calls():
-    """The library as a Python module: operators called by position, without schema matching.  A call that it leaves to
+    """A Python module beside the library: operators called by position, without schema matching.  A call that it leaves to
     ``torch.ops`` returns ``NotImplemented``."""
     global _calls
     if _calls is None:
         load()
-        loader = ExtensionFileLoader("libop_plugin_b200", str(PLUGIN_PATH))
-        spec = importlib.util.spec_from_file_location("libop_plugin_b200", PLUGIN_PATH, loader=loader)
+        _require(CALLS_PATH)
+        loader = ExtensionFileLoader("_op_plugin_calls", str(CALLS_PATH))
+        spec = importlib.util.spec_from_file_location("_op_plugin_calls", CALLS_PATH, loader=loader)
         module = importlib.util.module_from_spec(spec)
         loader.exec_module(module)
         _calls = module

@@ -4,6 +4,8 @@ torch-library registration carries the operator schemas, and the codegen reprodu
 reference's declaration style."""
 import ctypes
 import re
+import shutil
+import subprocess
 import sys
 from pathlib import Path
 
@@ -158,3 +160,21 @@ def test_codegen_declarations(tmp_path):
     bad.write_text("official:\ncustom:\n")
     with pytest.raises(AssertionError, match="symint"):
         gen.parse_native_yaml(bad)
+
+
+def test_operator_library_loads_without_python(tmp_path):
+    """A host program without an interpreter (libtorch from C++) can load the operators: nothing in the library needs Python."""
+    lib = PKG_DIR / "lib"
+    compiler = shutil.which("gcc") or shutil.which("cc")
+    if compiler is None:
+        pytest.skip("no C compiler")
+    source = tmp_path / "host.c"
+    source.write_text("#include <dlfcn.h>\n#include <stdio.h>\n"
+                      "int main(int argc, char **argv) {\n"
+                      "    for (int i = 1; i < argc; ++i)\n"
+                      "        if (!dlopen(argv[i], RTLD_NOW | RTLD_GLOBAL)) { printf(\"%s\\n\", dlerror()); return 1; }\n"
+                      "    return 0;\n}\n")
+    subprocess.run([compiler, str(source), "-o", str(tmp_path / "host"), "-ldl"], check=True)
+    r = subprocess.run([str(tmp_path / "host"), str(lib / "libqmm_b200.so"), str(lib / "libop_plugin_b200.so")],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout
