@@ -15,6 +15,8 @@
 // storages are alive and their version counters are unchanged (an in-place update re-packs); the cache holds
 // a second copy of the weights, bounded by QMM_W4_PREPACK_MAX_MB (default 16384; QMM_W4_PREPACK=0 switches
 // the format off).  Callers that want a single copy prepack explicitly through the C ABI and drop the original.
+// Packing is asynchronous: a call on another stream than the one that packs waits for it on the device.  What is packed
+// while a graph is captured exists when that graph runs: it serves the calls of that capture and no others.
 #include <algorithm>
 #include <cstdlib>
 #include <map>
@@ -23,6 +25,9 @@
 #include <tuple>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 
 #include "op_plugin/OpApiInterface.h"
 #include "op_plugin/utils/qmm_api_common.h"
@@ -35,7 +40,42 @@ struct PrepackEntry {
     at::Tensor packed;
     std::optional<c10::weak_intrusive_ptr<c10::StorageImpl>> storages[3];
     uint32_t versions[3] = {0, 0, 0};
+    at::cuda::CUDAEvent packed_event{cudaEventDisableTiming};  // behind the packing, on `stream`
+    c10::cuda::CUDAStream stream;
+    bool complete = false;           // the host has seen the event: nobody waits for it any more
+    unsigned long long capture = 0;  // the graph capture that packs it, 0: none
+    explicit PrepackEntry(c10::cuda::CUDAStream s) : stream(s) {}
 };
+
+// The capture that `stream` is part of, 0: none.
+unsigned long long capture_id(c10::cuda::CUDAStream stream)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream.stream(), &status, &id));
+    return status == cudaStreamCaptureStatusNone ? 0 : id;
+}
+
+// Orders `stream` behind the packing of `e`, and keeps the buffer for what `stream` does with it.
+void use_entry(PrepackEntry &e, c10::cuda::CUDAStream stream, unsigned long long capture)
+{
+    if (!e.complete) {
+        c10::cuda::CUDAStreamCaptureModeGuard relaxed{cudaStreamCaptureModeRelaxed};  // any thread may be capturing
+        if (e.capture != 0) {
+            e.packed_event.block(stream);  // the same capture: an edge of its graph
+        } else if (capture != 0) {
+            e.packed_event.synchronize();  // a graph may run on any stream, and cannot wait for what is not part of it
+            e.complete = true;
+        } else if (e.packed_event.query()) {
+            e.complete = true;
+        } else {
+            e.packed_event.block(stream);
+        }
+    }
+    if (stream != e.stream) {
+        c10::cuda::CUDACachingAllocator::recordStream(e.packed.storage().data_ptr(), stream);
+    }
+}
 
 using PrepackKey = std::tuple<const void *, const void *, const void *, int64_t, int64_t, int64_t, int>;
 
@@ -80,10 +120,12 @@ at::Tensor prepacked_weight(const at::Tensor &w, const at::Tensor &scale, const 
     const at::Tensor *parts[3] = {&w, &scale, &offset};
     const PrepackKey key{w.const_data_ptr(), scale.const_data_ptr(), op_plugin_utils::opt_ptr(offset), K, N, group,
                          static_cast<int>(scale.scalar_type())};
+    const c10::cuda::CUDAStream stream = at::cuda::getCurrentCUDAStream(w.device().index());
+    const unsigned long long capture = capture_id(stream);
     std::lock_guard<std::mutex> lock(mutex);
     auto it = cache.find(key);
     if (it != cache.end()) {
-        bool valid = true;
+        bool valid = it->second.capture == 0 || it->second.capture == capture;
         for (int i = 0; i < 3 && valid; ++i) {
             if (!it->second.storages[i].has_value()) {
                 valid = !parts[i]->defined();
@@ -94,6 +136,7 @@ at::Tensor prepacked_weight(const at::Tensor &w, const at::Tensor &scale, const 
                     it->second.versions[i] == version_of(*parts[i]);
         }
         if (valid) {
+            use_entry(it->second, stream, capture);
             return it->second.packed;
         }
         cached_bytes -= static_cast<size_t>(it->second.packed.numel());
@@ -106,11 +149,13 @@ at::Tensor prepacked_weight(const at::Tensor &w, const at::Tensor &scale, const 
         cache.clear();
         cached_bytes = 0;
     }
-    PrepackEntry e;
+    PrepackEntry e(stream);
+    e.capture = capture;
     e.packed = at::empty({static_cast<int64_t>(bytes)}, w.options().dtype(at::kByte));
     EXEC_QMM_CMD(qmm_w4a16_prepack, static_cast<const int32_t *>(w.const_data_ptr()), N / 8, scale.const_data_ptr(),
                  op_plugin_utils::opt_ptr(offset), op_plugin_utils::qmm_dtype(scale.scalar_type()), group, N, K,
                  e.packed.data_ptr(), bytes, op_plugin_utils::current_stream(w));
+    e.packed_event.record(stream);
     for (int i = 0; i < 3; ++i) {
         if (parts[i]->defined()) {
             e.storages[i].emplace(
