@@ -214,32 +214,6 @@ rms_norm_vec_kernel(const T *__restrict__ x, int64_t rows, int cols, int64_t ld_
     }
 }
 
-// two fp32 operations an instruction, each rounded as the scalar one
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("{.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-        "mul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
-        "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("{.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-        "add.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-
 // The fused kernel for rows of up to 256 threads: a CTA walks rows.  FULL: the row fills all vectors (cols == tpr * VPT *
 // 8), no guards.  With one row per CTA and scalar arithmetic (the kernel above) it was bound by instruction issue: 20
 // instructions an element, 30.8 us at 8192 x 4096 where the memory needs 15.  So the fp32 arithmetic is two

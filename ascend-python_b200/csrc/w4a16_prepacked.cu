@@ -655,22 +655,21 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
 
 // ---- 3 to 16 token rows with the tables at hand: the weight as a whole number, scale and offset on the sums of a block ----
 //
-// The narrow form's unpack warps spend 15 instructions on a word, half of them on the subtraction and the multiply-add that
-// make a finished weight, which is then rounded to 16 bits.  With few token rows both can be left to the sums: the operand is
-// w + 24, which is a shift and one logic instruction from the nibbles (16 + (w + 8): the nibble in the mantissa of a 16-bit
-// float of exponent 16) and exact in both types, every block of 128 k has an accumulator of its own, and the epilogue warps fold
+// The narrow form's unpack warps finish a weight with a multiply-add, which rounds it to 16 bits.  With few token rows that can be
+// left to the sums: the operand is w itself, every block of 128 k has an accumulator of its own, and the epilogue warps fold
 // it into fp32 running outputs:
-//     y[m, n] += scale * acc[m, n] + scale * (offset - 24) * xs[m],    xs[m] = the block's sum of x[m, :].
-// The weight is never rounded, and scale and offset come from the caller's tables in full.  Carrying 24 along costs about two
-// bits of the 24 of the fp32 sums.  Infinite activations make infinite sums of both signs: an output that is not a number is
-// computed again, plainly (b_plain).
+//     y[m, n] += scale * acc[m, n] + scale * offset * xs[m],    xs[m] = the block's sum of x[m, :].
+// The weight is never rounded, and scale and offset come from the caller's tables in full.  (An operand of w + 24 saves the
+// subtraction, but its sums hold 24 times the sum of x as well: a block with one large activation loses the small ones.)
+// Infinite activations make sums that are no numbers: such an output is computed again, plainly (b_plain).
 //
 // A stage holds the nibbles of two blocks (not the stream's own tables) and their rows of scale and offset.  The epilogue warps
 // also make xs, from the activation tile in shared memory: warp e takes block e / 2 and eight tokens, a lane a quarter of the
 // block's k.  Everything else (roles, rings, cuts, slots) is as in the kernel above.
 //
-// us, this / the narrow form above / the stock layout (M x K x N): 8 x 1024 x 1024 5.8 / 5.5 / 17.2, 8 x 8192 x 1024 9.0 / 8.1 / 92,
-// 8 x 4096 x 4096 10.4 / 8.9 / 33.4, 8 x 8192 x 8192 18.4 / 15.4 / 30.9, 8 x 8192 x 28672 46.0 / 33.5 / 38.8.  A stage takes about
+// us, this / the narrow form above / the stock layout (M x K x N): 8 x 1024 x 1024 6.0 / 5.5 / 17.2, 8 x 8192 x 1024 9.4 / 8.1 / 92,
+// 8 x 4096 x 4096 11.1 / 8.9 / 33.4, 8 x 8192 x 8192 19.5 / 15.4 / 30.9, 8 x 8192 x 28672 50.2 / 33.5 / 38.8 (with w + 24 as the operand
+// 6.0, 9.3, 10.7, 18.6 and 46.7; with one fp32 operation an instruction in the epilogue 6.1, 9.6, 11.1, 20.0 and 51.2).  A stage takes about
 // 1800 clocks, of which the epilogue warps' chain of instructions takes nearly all (waits are short, the issue slots 52 % used).
 // Measured without gain: two sets of epilogue warps in turn (44-48 us for the last), sums of x by warps of their own with a ring for
 // the tables (48-52), and sums of x from a kernel in front, without which the chain is half as long (42.8, but 6.5 for the first).
@@ -708,20 +707,6 @@ struct BTables {
     int64_t ld_x;
 };
 
-// 24 + w as a 16-bit float from the nibble of two neighbouring k; nibble p of each half word
-template <typename T>
-struct BMagic;
-template <>
-struct BMagic<__nv_bfloat16> {
-    static constexpr uint32_t kMask = 0x00780078u, kFlip = 0x41c041c0u;
-    static __device__ __forceinline__ uint32_t shifted(uint32_t w, int p) { return p == 0 ? w << 3 : w >> (4 * p - 3); }
-};
-template <>
-struct BMagic<__half> {
-    static constexpr uint32_t kMask = 0x03c003c0u, kFlip = 0x4e004e00u;
-    static __device__ __forceinline__ uint32_t shifted(uint32_t w, int p) { return p < 2 ? w << (6 - 4 * p) : w >> (4 * p - 6); }
-};
-
 // One output by the definition, for those that the sums above leave without a number.
 template <typename T>
 __device__ __noinline__ float b_plain_loop(const uint8_t *packed, const T *x, const T *scale, const T *offset, int group_blocks,
@@ -750,12 +735,12 @@ __device__ __forceinline__ float b_plain(const PParams &p, const BTables &t, int
 }
 
 template <typename T>
-__device__ __forceinline__ void b_add_words(float &s, const uint4 &v) {
+__device__ __forceinline__ void b_add_words(float2 &s, const uint4 &v) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const T *h = reinterpret_cast<const T *>(&w[i]);
-        s += to_float(h[0]) + to_float(h[1]);
+        s = add2(s, make_float2(to_float(h[0]), to_float(h[1])));
     }
 }
 
@@ -900,6 +885,8 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
         const int team = (warp - kPFirstUnpackWarp) >> 2;
         const int quarter = warp & 3;
         const int r = quarter * 32 + lane;
+        using T2 = typename PMagic<T>::T2;
+        const T2 bias2 = PMagic<T>::bias2();
         const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kBACol0 + team * 16;
         uint32_t st = 0, ph = 0, rs = 0, rph = 0;
         int pending = -1;  // ring slot whose stores are in flight
@@ -918,8 +905,11 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        v[b][4 * i + j] = p_and_xor(BMagic<T>::shifted(words[i], j), BMagic<T>::kMask, BMagic<T>::kFlip);
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t raw = p_and_xor(words[i] >> (4 * j), 0x000f000fu, PMagic<T>::kFlip);
+                        const T2 wq = __hsub2(*reinterpret_cast<const T2 *>(&raw), bias2);  // exact: w itself
+                        v[b][4 * i + j] = *reinterpret_cast<const uint32_t *>(&wq);
+                    }
             }
             // the previous stage's stores have had this stage's arithmetic to complete: announce them
             if (pending >= 0) {
@@ -970,22 +960,24 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
             const int64_t n = static_cast<int64_t>(q) * kPTileN + row;
             const bool n_ok = n < p.N;
             const float b = (n_ok && bias != nullptr) ? to_float(bias[n]) : 0.0f;
-            float y[kBTok];
+            float2 y[kBTok / 2];  // of two tokens
 #pragma unroll
-            for (int j = 0; j < kBTok; ++j) y[j] = 0.0f;
+            for (int j = 0; j < kBTok / 2; ++j) y[j] = make_float2(0.0f, 0.0f);
+            auto output = [&](int j) { return j & 1 ? y[j >> 1].y : y[j >> 1].x; };
             for (int it = u; it < seg_end; ++it) {
                 ok = mbar_wait(smem_u32(&tail->x_full[xst]), xph, abort_flag, 0x78);
-                float sum = 0.0f;
+                float2 sums = make_float2(0.0f, 0.0f);
                 const uint8_t *xr = smem_aligned + xst * kXSlot + x_row;
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
-                    b_add_words<T>(sum, *reinterpret_cast<const uint4 *>(xr + (((4 * (xq & 1) + c) ^ (xtok & 7)) << 4)));
+                    b_add_words<T>(sums, *reinterpret_cast<const uint4 *>(xr + (((4 * (xq & 1) + c) ^ (xtok & 7)) << 4)));
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&tail->x_empty[xst]));
+                float sum = sums.x + sums.y;
                 sum += __shfl_xor_sync(0xffffffffu, sum, 8);
                 sum += __shfl_xor_sync(0xffffffffu, sum, 16);
                 if (lane < 8) tail->xs[parity][xb][xtok] = sum;
-                // scale and scale * (offset - 24) of the stage's two blocks
+                // scale and scale * offset of the stage's two blocks
                 ok = ok && mbar_wait(smem_u32(&tail->w_full[wst]), wph, abort_flag, 0x79);
                 float sc[kPPair], tc[kPPair];
                 const T *table = reinterpret_cast<const T *>(smem_aligned + w_off + wst * kBStageBytes + kPPair * kPWBytes) + row;
@@ -993,7 +985,7 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
                 for (int k = 0; k < kPPair; ++k) {
                     const bool real = n_ok && (it - tile_begin) * kPPair + k < t.nblocks;
                     sc[k] = real ? to_float(table[k * kPTileN]) : 0.0f;
-                    tc[k] = sc[k] * ((real && t.offset != nullptr ? to_float(table[(kPPair + k) * kPTileN]) : 0.0f) - 24.0f);
+                    tc[k] = real && t.offset != nullptr ? sc[k] * to_float(table[(kPPair + k) * kPTileN]) : 0.0f;
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&tail->w_empty[wst]));
@@ -1021,10 +1013,12 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
                     for (int j = 0; j < kBTok; j += 4) {
                         if (j >= M) break;
                         const float4 x4 = *reinterpret_cast<const float4 *>(&tail->xs[parity][k][j]);
-                        y[j] = fmaf(tc[k], x4.x, fmaf(sc[k], __uint_as_float(v[k][j]), y[j]));
-                        y[j + 1] = fmaf(tc[k], x4.y, fmaf(sc[k], __uint_as_float(v[k][j + 1]), y[j + 1]));
-                        y[j + 2] = fmaf(tc[k], x4.z, fmaf(sc[k], __uint_as_float(v[k][j + 2]), y[j + 2]));
-                        y[j + 3] = fmaf(tc[k], x4.w, fmaf(sc[k], __uint_as_float(v[k][j + 3]), y[j + 3]));
+                        const float2 sc2 = make_float2(sc[k], sc[k]), tc2 = make_float2(tc[k], tc[k]);
+                        auto fold = [&](float2 &to, float2 xs, uint32_t a0, uint32_t a1) {
+                            to = fma2(tc2, xs, fma2(sc2, make_float2(__uint_as_float(a0), __uint_as_float(a1)), to));
+                        };
+                        fold(y[j / 2], make_float2(x4.x, x4.y), v[k][j], v[k][j + 1]);
+                        fold(y[j / 2 + 1], make_float2(x4.z, x4.w), v[k][j + 2], v[k][j + 3]);
                     }
                 parity ^= 1;
                 if (++wst == nstages) {
@@ -1047,8 +1041,8 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
 #pragma unroll
                     for (int j = 0; j < kBTok; ++j) {
                         if (j >= M) break;
-                        again |= isnan(y[j]) ? 1u << j : 0u;
-                        out[static_cast<int64_t>(j) * p.ld_out + n] = from_float<T>(y[j] + b);
+                        again |= isnan(output(j)) ? 1u << j : 0u;
+                        out[static_cast<int64_t>(j) * p.ld_out + n] = from_float<T>(output(j) + b);
                     }
                     for (; again != 0; again &= again - 1) {
                         const int j = __ffs(static_cast<int>(again)) - 1;
@@ -1059,7 +1053,7 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
                 float *mine = p.slots + p_slot<false>(p, cta, q) * (static_cast<int64_t>(p.mpad) * kPTileN) + row;
 #pragma unroll
                 for (int j = 0; j < kBTok; ++j)
-                    if (j < M) __stcg(mine + j * kPTileN, y[j]);
+                    if (j < M) __stcg(mine + j * kPTileN, output(j));
                 if (seg_end < u_end) p_finish_shared<T, false, true>(p, q, abort_flag, &tail->is_last, plain);
             }
             u = seg_end;

@@ -339,3 +339,24 @@ def test_operator_takes_few_rows_of_any_width(oracle, dev):
         for xd in (x.to(dev), flat[1:].view(M, K)):
             y = torch_npu.npu_weight_quant_batchmatmul(xd, packed_w.to(dev), scale.to(dev), offset.to(dev), antiquant_group_size=group)
             assert np.all(np.abs(y.float().cpu().numpy() - y_ref) <= 2.0 ** -8 * np.abs(y_ref) + 2.0 ** -7 * rms)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(3, 512, 136), (8, 4096, 1032)])
+def test_few_tokens_one_large_activation_a_block(capi, oracle, dev, shape, dtype):
+    """Every 128th activation is 16384 and meets weights of zero, the others are near 1/64: the sum of the others is left as it is.
+    Bound: the output's rounding, and K roundings of fp32 sums of what is summed (a zero times 16384 counts as 1 at most, the
+    smallest exponent of an f16)."""
+    M, K, N = shape
+    x, packed_w, scale, _ = oracle.make_w4a16_inputs(M, K, N, seed=K + N, group=128, dtype=dtype)
+    x = (x.float() / 64).to(dtype)
+    x[:, ::128] = 16384
+    packed_w[::128] = 0
+    y_ref = oracle.weight_quant_batchmatmul(x, packed_w, scale, None, antiquant_group_size=128)
+    sums = np.abs(x.double().numpy()) @ np.abs(np.asarray(oracle.antiquant_weight(packed_w, scale, None, 128), dtype=np.float64))
+    sd = scale.to(dev)
+    buf = capi.w4a16_prepack(packed_w.to(dev), sd, None, group_size=128)
+    y = capi.weight_quant_batchmatmul_prepacked(x.to(dev), buf, N, tables=(sd, None, 128)).float().cpu().numpy()
+    u = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
+    bound = 2 * u * np.abs(y_ref) + K * 2.0 ** -23 * (sums + scale.float().max().item())
+    assert np.all(np.abs(y - y_ref) <= bound), f"error is {np.max(np.abs(y - y_ref) / bound):.1f}x the bound"
