@@ -227,7 +227,7 @@ __device__ __forceinline__ int p_slot(const PParams &p, int cta, int q) {
 }
 
 // Adds the sums of tile q by its `nslots` CTAs in their order and stores the tile; thread `tid` of `threads`.  plain(column, row):
-// what an output is that came to no number (PNoPlain: that).
+// what an output is whose sums are not finite (PNoPlain: that).
 struct PNoPlain {};
 template <typename T, bool WIDE, typename Plain>
 __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots, int tid, int threads, const Plain &plain) {
@@ -282,7 +282,7 @@ __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots,
             if constexpr (!std::is_same<Plain, PNoPlain>::value) {
                 uint32_t again = 0;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) again |= isnan(f[k]) ? 1u << k : 0u;
+                for (int k = 0; k < 4; ++k) again |= !isfinite(f[k]) ? 1u << k : 0u;
                 for (; again != 0; again &= again - 1) {
                     const int k = __ffs(static_cast<int>(again)) - 1;
                     o[k] = from_float<T>(plain(n + k, m0 + idx / (kPTileN / 4)) + (bias != nullptr ? to_float(bias[n + k]) : 0.0f));
@@ -661,7 +661,8 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
 //     y[m, n] += scale * acc[m, n] + scale * offset * xs[m],    xs[m] = the block's sum of x[m, :].
 // The weight is never rounded, and scale and offset come from the caller's tables in full.  (An operand of w + 24 saves the
 // subtraction, but its sums hold 24 times the sum of x as well: a block with one large activation loses the small ones.)
-// Infinite activations make sums that are no numbers: such an output is computed again, plainly (b_plain).
+// Infinite activations make sums that are no numbers, and very large ones sums that leave fp32 where the output, which is scaled,
+// would not: what is not finite is computed again, plainly (b_plain).
 //
 // A stage holds the nibbles of two blocks (not the stream's own tables) and their rows of scale and offset.  The epilogue warps
 // also make xs, from the activation tile in shared memory: warp e takes block e / 2 and eight tokens, a lane a quarter of the
@@ -707,7 +708,7 @@ struct BTables {
     int64_t ld_x;
 };
 
-// One output by the definition, for those that the sums above leave without a number.
+// One output by the definition, for those whose sums above are not finite.
 template <typename T>
 __device__ __noinline__ float b_plain_loop(const uint8_t *packed, const T *x, const T *scale, const T *offset, int group_blocks,
                                            int nblocks, int nchunks, int N, int64_t n) {
@@ -1041,7 +1042,7 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
 #pragma unroll
                     for (int j = 0; j < kBTok; ++j) {
                         if (j >= M) break;
-                        again |= isnan(output(j)) ? 1u << j : 0u;
+                        again |= !isfinite(output(j)) ? 1u << j : 0u;
                         out[static_cast<int64_t>(j) * p.ld_out + n] = from_float<T>(output(j) + b);
                     }
                     for (; again != 0; again &= again - 1) {

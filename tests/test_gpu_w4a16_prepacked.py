@@ -360,3 +360,24 @@ def test_few_tokens_one_large_activation_a_block(capi, oracle, dev, shape, dtype
     u = 2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12
     bound = 2 * u * np.abs(y_ref) + K * 2.0 ** -23 * (sums + scale.float().max().item())
     assert np.all(np.abs(y - y_ref) <= bound), f"error is {np.max(np.abs(y - y_ref) / bound):.1f}x the bound"
+
+
+@pytest.mark.parametrize("shape", [(4, 256, 136), (6, 4096, 1032)])
+def test_few_tokens_sums_beyond_fp32(capi, oracle, dev, shape):
+    """Activations of up to 2^124 in one row: sums of products with whole-number weights leave the range of fp32, the outputs (the
+    scales are near 2^-7) do not.  Bound: the output's rounding and K roundings of the fp32 sums.  The other rows stay as they are."""
+    M, K, N = shape
+    x, packed_w, scale, offset = oracle.make_w4a16_inputs(M, K, N, seed=K + 1, group=128)
+    clean = x.clone()
+    x[1] = (x[1].float().clamp(-4, 4) * 2.0 ** 122).to(torch.bfloat16)
+    y_ref = oracle.weight_quant_batchmatmul(x, packed_w, scale, offset, antiquant_group_size=128)
+    assert np.abs(y_ref).max() < 2.0 ** 127
+    sums = np.abs(x.double().numpy()) @ np.abs(np.asarray(oracle.antiquant_weight(packed_w, scale, offset, 128), dtype=np.float64))
+    sd, od = scale.to(dev), offset.to(dev)
+    buf = capi.w4a16_prepack(packed_w.to(dev), sd, od, group_size=128)
+    y = capi.weight_quant_batchmatmul_prepacked(x.to(dev), buf, N, tables=(sd, od, 128)).cpu()
+    y_clean = capi.weight_quant_batchmatmul_prepacked(clean.to(dev), buf, N, tables=(sd, od, 128)).cpu()
+    others = [m for m in range(M) if m != 1]
+    assert torch.equal(y[others], y_clean[others])
+    error = np.abs(y[1].double().numpy() - y_ref[1])
+    assert np.all(error <= 2.0 ** -8 * np.abs(y_ref[1]) + K * 2.0 ** -23 * sums[1])
