@@ -1230,10 +1230,14 @@ PPlan p_make_plan(int64_t M, int64_t N, int64_t K) {
         // does (256 x 8192 x 1024: one row tile 42.0 us, four 14.9; 321 x 3584 x 1096: 18.8 / 11.7).  With many, as few row
         // tiles as the accumulator allows (1000 x 4096 x 28672: 201 us with four, 205 .. 226 with five to eight); a plan with
         // more has to be 6 % ahead.
+        // A height of a multiple of 16 gives a number of row tiles, so there are sixteen candidates at most, whatever M is (a
+        // search over the numbers took the host 31 us for 65536 rows, on each of a call's three visits here; 0.3 so).
         const int64_t fewest = (M + kPMaxWide - 1) / kPMaxWide;
         int64_t best = 0;
-        for (int64_t want = fewest; want == fewest || want <= M / 32; ++want) {
-            const int64_t mpad = ((M + want - 1) / want + 15) / 16 * 16, nblk = (M + mpad - 1) / mpad;
+        for (int64_t mpad = kPMaxWide; mpad >= 16; mpad -= 16) {
+            const int64_t nblk = (M + mpad - 1) / mpad;
+            if (((M + nblk - 1) / nblk + 15) / 16 * 16 != mpad) continue;  // a lower tile gives as many
+            if (nblk != fewest && nblk > M / 32) break;
             const int64_t tiles = pl.tiles_n * nblk, items = tiles * pl.nchunks, ctas = items < sms ? items : sms;
             const int64_t most = (items + ctas - 1) / ctas;
             const int64_t stage = 47 + mpad * 5 > 790 ? 47 + mpad * 5 : 790, drain = 61 * mpad;
@@ -1241,7 +1245,7 @@ PPlan p_make_plan(int64_t M, int64_t N, int64_t K) {
             const int64_t slots = tiles < ctas ? 16 * ctas / tiles + 16 : 32;  // of a tile, in sixteenths
             const int64_t shared = 2187 + most * stage + drain * most / pl.nchunks + 35 * mpad + (mpad * 14 / 5 + 96) * slots / 16;
             const bool grain = whole <= shared || tiles > static_cast<int64_t>(kPCounterBytes / 4);  // (a counter a tile)
-            const int64_t cost = (grain ? whole : shared) * (want == fewest ? 100 : 106);
+            const int64_t cost = (grain ? whole : shared) * (nblk == fewest ? 100 : 106);
             if (best == 0 || cost < best) {
                 best = cost;
                 pl.mpad = static_cast<int>(mpad);

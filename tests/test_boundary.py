@@ -7,6 +7,7 @@ import re
 import shutil
 import subprocess
 import sys
+import time
 from pathlib import Path
 
 import pytest
@@ -178,3 +179,53 @@ def test_operator_library_loads_without_python(tmp_path):
     r = subprocess.run([str(tmp_path / "host"), str(lib / "libqmm_b200.so"), str(lib / "libop_plugin_b200.so")],
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout
+
+
+def _w4a16_scratch(M, N, K, sms=148):
+    """The prepacked W4A16 scratch for more than 64 rows, with the row tiles searched by their number."""
+    tiles_n, nchunks = -(-N // 128), -(-K // 256)
+    fewest, best = -(-M // 256), None
+    for want in range(fewest, max(fewest, M // 32) + 1):
+        mpad = -(-(-(-M // want)) // 16) * 16
+        nblk = -(-M // mpad)
+        tiles = tiles_n * nblk
+        ctas = min(tiles * nchunks, sms)
+        most = -(-tiles * nchunks // ctas)
+        stage, drain = max(47 + mpad * 5, 790), 61 * mpad
+        whole = 99 + -(-tiles // sms) * (nchunks * stage + drain)
+        slots = 16 * ctas // tiles + 16 if tiles < ctas else 32
+        shared = 2187 + most * stage + drain * most // nchunks + 35 * mpad + (mpad * 14 // 5 + 96) * slots // 16
+        grain = whole <= shared or tiles > 16384
+        cost = (whole if grain else shared) * (100 if want == fewest else 106)
+        if best is None or cost < best[0]:
+            best = cost, mpad, nblk, grain
+    _, mpad, nblk, grain = best
+    grid = min(tiles_n * nblk * (1 if grain or nchunks == 1 else nchunks), sms)
+    slots = 0 if grain or nchunks == 1 else grid + min(tiles_n * nblk, grid)
+    return slots * mpad * 128 * 4
+
+
+def test_w4a16_row_tiles(capi):
+    """The row tiles of more than 64 rows: the choice of the model, without a search that grows with the number of rows."""
+    lib, n = capi.lib(), ctypes.c_size_t(0)
+
+    def size(M, N, K):
+        assert lib.qmm_weight_quant_batchmatmul_prepacked_workspace_size(M, N, K, ctypes.byref(n)) == 0
+        return n.value
+
+    if not torch.cuda.is_available():  # 148 SMs are assumed
+        base = size(65, 128, 128)  # one block pair along K: the counters alone
+        shapes = [(M, N, K) for M in (65, 100, 256, 257, 321, 1000, 1500, 2049, 5000, 8192)
+                  for N in (8, 1096, 4096, 28672) for K in (256, 1024, 3584, 14336)]
+        for shape in shapes:
+            assert size(*shape) == base + _w4a16_scratch(*shape), shape
+
+    def best_time(M):
+        times = []
+        for _ in range(10):
+            begin = time.perf_counter()
+            size(M, 1024, 1024)
+            times.append(time.perf_counter() - begin)
+        return min(times)
+
+    assert best_time(1 << 26) < 2 * best_time(256) + 2e-3
