@@ -226,11 +226,11 @@ __device__ __forceinline__ int p_slot(const PParams &p, int cta, int q) {
     return cta + min(q, cta + (p_first_item<WIDE>(p, cta) < q * p.nchunks ? 1 : 0));
 }
 
-// Adds the sums of tile q by its `nslots` CTAs in their order and stores the tile; thread `tid` of `threads`.  plain(column, row):
-// what an output is whose sums are not finite (PNoPlain: that).
-struct PNoPlain {};
-template <typename T, bool WIDE, typename Plain>
-__device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots, int tid, int threads, const Plain &plain) {
+// Adds the sums of tile q by its `nslots` CTAs in their order and stores the tile; thread `tid` of `threads`.  report(row): called
+// for a row of the tile with a sum that is not finite (PNoReport: nothing is).
+struct PNoReport {};
+template <typename T, bool WIDE, typename Report>
+__device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots, int tid, int threads, const Report &report) {
     const T *bias = static_cast<const T *>(p.bias);
     const int m0 = (q % p.nblk) * p.mpad, ncol0 = (q / p.nblk) * kPTileN;
     const int vecs = min(p.mpad, p.M - m0) * (kPTileN / 4);
@@ -270,6 +270,9 @@ __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots,
             const int n = ncol0 + (idx % (kPTileN / 4)) * 4;
             if (idx >= vecs || n >= p.N) continue;  // N is a multiple of eight
             float f[4] = {v[e].x, v[e].y, v[e].z, v[e].w};
+            if constexpr (!std::is_same<Report, PNoReport>::value) {
+                if (!(isfinite(f[0]) && isfinite(f[1]) && isfinite(f[2]) && isfinite(f[3]))) report(idx / (kPTileN / 4));
+            }
 #pragma unroll
             for (int k = 0; k < 4; ++k) f[k] += bias != nullptr ? to_float(bias[n + k]) : 0.0f;
             T *o = static_cast<T *>(p.out) + static_cast<int64_t>(m0 + idx / (kPTileN / 4)) * p.ld_out + n;
@@ -279,15 +282,6 @@ __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots,
 #pragma unroll
                 for (int k = 0; k < 4; ++k) o[k] = from_float<T>(f[k]);
             }
-            if constexpr (!std::is_same<Plain, PNoPlain>::value) {
-                uint32_t again = 0;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) again |= !isfinite(f[k]) ? 1u << k : 0u;
-                for (; again != 0; again &= again - 1) {
-                    const int k = __ffs(static_cast<int>(again)) - 1;
-                    o[k] = from_float<T>(plain(n + k, m0 + idx / (kPTileN / 4)) + (bias != nullptr ? to_float(bias[n + k]) : 0.0f));
-                }
-            }
         }
     }
 }
@@ -295,9 +289,9 @@ __device__ __forceinline__ void p_add_slots(const PParams &p, int q, int nslots,
 // The calling threads have stored this CTA's sums of tile q: reports that, and if it completes the tile adds the slots
 // and stores the tile.  EPILOGUE: the four epilogue warps call, otherwise the whole CTA.  Inlined: as a call with the
 // parameters' address it slows the whole kernel down (34 -> 43 us for 16 tokens).
-template <typename T, bool WIDE, bool EPILOGUE, typename Plain = PNoPlain>
+template <typename T, bool WIDE, bool EPILOGUE, typename Report = PNoReport>
 __device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatile uint32_t *abort_flag, uint32_t *flag,
-                                                const Plain &plain = Plain()) {
+                                                const Report &report = Report()) {
     auto barrier = [] {
         if (EPILOGUE)
             pepi_bar_sync();
@@ -320,7 +314,7 @@ __device__ __forceinline__ void p_finish_shared(const PParams &p, int q, volatil
         *flag = last;
     }
     barrier();
-    if (*reinterpret_cast<volatile uint32_t *>(flag) != 0) p_add_slots<T, WIDE>(p, q, nslots, tid, EPILOGUE ? kPEpiWarps * 32 : kPThreads, plain);
+    if (*reinterpret_cast<volatile uint32_t *>(flag) != 0) p_add_slots<T, WIDE>(p, q, nslots, tid, EPILOGUE ? kPEpiWarps * 32 : kPThreads, report);
     barrier();  // the flag is written again for the next tile
 }
 
@@ -662,15 +656,15 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
 // The weight is never rounded, and scale and offset come from the caller's tables in full.  (An operand of w + 24 saves the
 // subtraction, but its sums hold 24 times the sum of x as well: a block with one large activation loses the small ones.)
 // Infinite activations make sums that are no numbers, and very large ones sums that leave fp32 where the output, which is scaled,
-// would not: what is not finite is computed again, plainly (b_plain).
+// would not: what is not finite is computed again, plainly (b_plain_tiles).
 //
 // A stage holds the nibbles of two blocks (not the stream's own tables) and their rows of scale and offset.  The epilogue warps
 // also make xs, from the activation tile in shared memory: warp e takes block e / 2 and eight tokens, a lane a quarter of the
 // block's k.  Everything else (roles, rings, cuts, slots) is as in the kernel above.
 //
-// us, this / the narrow form above / the stock layout (M x K x N): 8 x 1024 x 1024 6.0 / 5.5 / 17.2, 8 x 8192 x 1024 9.4 / 8.1 / 92,
-// 8 x 4096 x 4096 11.1 / 8.9 / 33.4, 8 x 8192 x 8192 19.5 / 15.4 / 30.9, 8 x 8192 x 28672 50.2 / 33.5 / 38.8 (with w + 24 as the operand
-// 6.0, 9.3, 10.7, 18.6 and 46.7; with one fp32 operation an instruction in the epilogue 6.1, 9.6, 11.1, 20.0 and 51.2).  A stage takes about
+// us, this / the narrow form above / the stock layout (M x K x N): 8 x 1024 x 1024 5.7 / 5.5 / 17.2, 8 x 8192 x 1024 9.1 / 8.1 / 92,
+// 8 x 4096 x 4096 10.7 / 8.9 / 33.4, 8 x 8192 x 8192 19.0 / 15.4 / 30.9, 8 x 8192 x 28672 48.4 / 33.5 / 38.8 (with w + 24 as the operand
+// 5.8, 9.3, 10.4, 18.5 and 46.3; two fp32 operations an instruction in the epilogue save 1 to 3 %).  A stage takes about
 // 1800 clocks, of which the epilogue warps' chain of instructions takes nearly all (waits are short, the issue slots 52 % used).
 // Measured without gain: two sets of epilogue warps in turn (44-48 us for the last), sums of x by warps of their own with a ring for
 // the tables (48-52), and sums of x from a kernel in front, without which the chain is half as long (42.8, but 6.5 for the first).
@@ -697,6 +691,7 @@ struct BSmemTail {
     uint32_t abort_flag;
     uint32_t is_last;
     uint32_t epi_abort[2];           // [stage parity]: an epilogue warp gave up at that stage
+    uint32_t bad_rows, bad_tiles;    // with sums that are not finite, see b_plain_tiles
     __align__(16) float xs[2][kPPair][kBTok];  // [stage parity][block][token], read four at a time
 };
 
@@ -708,31 +703,110 @@ struct BTables {
     int64_t ld_x;
 };
 
-// One output by the definition, for those whose sums above are not finite.
-template <typename T>
-__device__ __noinline__ float b_plain_loop(const uint8_t *packed, const T *x, const T *scale, const T *offset, int group_blocks,
-                                           int nblocks, int nchunks, int N, int64_t n) {
-    const int r = static_cast<int>(n % kPTileN);
-    float y = 0.0f;
-    for (int blk = 0; blk < nblocks; ++blk) {
-        const uint8_t *src = packed + (n / kPTileN * nchunks * kPPair + blk) * kPBlockBytes;
-        const int64_t at = static_cast<int64_t>(blk / group_blocks) * N + n;
-        const float s = to_float(scale[at]), o = offset != nullptr ? to_float(offset[at]) : 0.0f;
-        for (int i = 0; i < kPChunkK / 8; ++i) {
-            const uint32_t word = reinterpret_cast<const uint32_t *>(src + ((i >> 2) * kPTileN + r) * 16)[i & 3];
-            for (int e = 0; e < 8; ++e) {
-                const int w = static_cast<int>(word << (28 - 4 * ((e >> 1) + (e & 1) * 4))) >> 28;
-                y = fmaf(to_float(x[blk * kPChunkK + i * 8 + e]), (static_cast<float>(w) + o) * s, y);
-            }
-        }
+// The products of eight k, a word of a column and their activations, added to y.  NONFINITE: those of the activations that are not
+// finite alone.
+template <typename T, bool NONFINITE>
+__device__ __forceinline__ float b_plain_step(float y, const uint4 &x, uint32_t word, float s, float o) {
+    const uint32_t xw[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const int w = static_cast<int>(word << (28 - 4 * ((e >> 1) + (e & 1) * 4))) >> 28;
+        const unsigned short bits = static_cast<unsigned short>(xw[e >> 1] >> (16 * (e & 1)));
+        const float v = to_float(*reinterpret_cast<const T *>(&bits));
+        if (!NONFINITE || !isfinite(v)) y = fmaf(v, (static_cast<float>(w) + o) * s, y);
     }
     return y;
 }
-// (by value: a parameter block whose address is taken is copied to local memory, and every use of it in the kernel goes there)
+// whether any (NAN_ONLY: any NaN) of eight activations is not finite
+template <typename T, bool NAN_ONLY>
+__device__ __forceinline__ bool b_any_not_finite(const uint4 &x) {
+    constexpr uint32_t kInf = std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u;
+    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+    bool any = false;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t lo = w[j] & 0x7fffu, hi = w[j] >> 16 & 0x7fffu;
+        any = any || (NAN_ONLY ? lo > kInf || hi > kInf : lo >= kInf || hi >= kInf);
+    }
+    return any;
+}
+
+// Outputs whose sums are not finite, by the definition: rows (a bit each) of the tiles q0 + i of bit i (the last bit: and beyond),
+// as the CTA has stored them.  By the whole CTA, behind its work: in the epilogue this code costs the main loop registers
+// (8 x 8192 x 8192: 19.0 us, 19.5 with a call there, 22.0 with a longer function), and a thread with all of K for itself is slow.  us, operator,
+// 8 x 4096 x 4096, finite 18: a NaN in every row 440 -> 23, an infinity in one 347 -> 20, 43 in every row 440 -> 70, sums of one row that leave
+// fp32 347 -> 41; 8 x 28672 x 768, finite 21: 2952 -> 36, 2308 -> 30, 2953 -> 94, 2309 -> 168.  A NaN among the activations is one among the sums already; infinite activations decide alone, so only their
+// products are added; where all are finite, sums left fp32, and five groups of 128 threads share K.  The scratch: 5 x 128 floats.
 template <typename T>
-__device__ __forceinline__ float b_plain(const PParams &p, const BTables &t, int64_t n, int m) {
-    return b_plain_loop<T>(p.packed, static_cast<const T *>(t.x) + m * t.ld_x, static_cast<const T *>(t.scale),
-                           static_cast<const T *>(t.offset), t.group_blocks, t.nblocks, p.nchunks, p.N, n);
+__device__ __forceinline__ void b_plain_tiles(const PParams &p, const BTables &t, uint32_t rows, uint32_t tiles, int q0, int q1, float *part) {
+    constexpr int kGroups = kPThreads / kPTileN, kVecs = kPChunkK / 8;  // vectors of eight k of a block
+    const int r = threadIdx.x % kPTileN, group = threadIdx.x / kPTileN, lane = threadIdx.x & 31;
+    const int vecs = t.nblocks * kVecs;
+    for (; rows != 0; rows &= rows - 1) {
+        const int m = __ffs(static_cast<int>(rows)) - 1;
+        const uint4 *xv = reinterpret_cast<const uint4 *>(static_cast<const T *>(t.x) + m * t.ld_x);
+        bool nan = false, inf = false;
+        for (int v = threadIdx.x; v < vecs; v += kPThreads) {
+            const uint4 x = __ldg(xv + v);
+            nan = nan || b_any_not_finite<T, true>(x);
+            inf = inf || b_any_not_finite<T, false>(x);
+        }
+        if (__syncthreads_or(nan)) continue;
+        const bool infinite = __syncthreads_or(inf);
+        for (int q = q0; q <= q1; ++q) {
+            if ((tiles >> min(q - q0, 31) & 1) == 0) continue;
+            const int64_t n = static_cast<int64_t>(q) * kPTileN + r;
+            T *out = static_cast<T *>(p.out) + m * p.ld_out + n;
+            unsigned short stored = 0;
+            if (group < kGroups && n < p.N) stored = __ldcg(reinterpret_cast<const unsigned short *>(out));
+            const bool wanted = group < kGroups && n < p.N && !isfinite(to_float(*reinterpret_cast<const T *>(&stored)));
+            if (!__syncthreads_or(wanted)) continue;
+            float y = 0.0f, s = 0.0f, o = 0.0f;
+            auto load_tables = [&](int blk) {
+                const int64_t at = static_cast<int64_t>(blk / t.group_blocks) * p.N + min(n, static_cast<int64_t>(p.N) - 1);
+                s = to_float(static_cast<const T *>(t.scale)[at]);
+                o = t.offset != nullptr ? to_float(static_cast<const T *>(t.offset)[at]) : 0.0f;
+            };
+            const uint8_t *stream = p.packed + static_cast<int64_t>(q) * p.nchunks * kPStageWBytes + r * 16;
+            if (group < kGroups) {
+                const int first = t.nblocks * group / kGroups, end = t.nblocks * (group + 1) / kGroups;
+                if (infinite) {
+                    bool decided = false;  // every output of the warp is a NaN already
+                    for (int v0 = first * kVecs; v0 < end * kVecs && !decided; v0 += 32) {
+                        const bool hit = v0 + lane < end * kVecs && b_any_not_finite<T, false>(__ldg(xv + v0 + lane));
+                        for (unsigned hits = __ballot_sync(0xffffffffu, hit); hits != 0; hits &= hits - 1) {
+                            const int v = v0 + __ffs(static_cast<int>(hits)) - 1, blk = v / kVecs, i = v % kVecs;
+                            load_tables(blk);
+                            const uint8_t *words = stream + static_cast<int64_t>(blk) * kPBlockBytes + (i >> 2) * kPTileN * 16;
+                            y = b_plain_step<T, true>(y, __ldg(xv + v), __ldg(reinterpret_cast<const uint32_t *>(words) + (i & 3)), s, o);
+                            decided = __all_sync(0xffffffffu, !wanted || isnan(y));
+                            if (decided) break;
+                        }
+                    }
+                } else {
+                    for (int blk = first; blk < end; ++blk) {
+                        load_tables(blk);
+#pragma unroll 1
+                        for (int sub = 0; sub < kPChunkK / kPSubK; ++sub) {
+                            const uint4 w = __ldg(reinterpret_cast<const uint4 *>(stream + static_cast<int64_t>(blk) * kPBlockBytes) + sub * kPTileN);
+                            const uint4 *at = xv + blk * kVecs + sub * 4;
+                            y = b_plain_step<T, false>(y, __ldg(at), w.x, s, o);
+                            y = b_plain_step<T, false>(y, __ldg(at + 1), w.y, s, o);
+                            y = b_plain_step<T, false>(y, __ldg(at + 2), w.z, s, o);
+                            y = b_plain_step<T, false>(y, __ldg(at + 3), w.w, s, o);
+                        }
+                    }
+                }
+                part[group * kPTileN + r] = y;
+            }
+            __syncthreads();
+            if (group == 0 && wanted) {
+                for (int g = 1; g < kGroups; ++g) y += part[g * kPTileN + r];
+                *out = from_float<T>(y + (p.bias != nullptr ? to_float(static_cast<const T *>(p.bias)[n]) : 0.0f));
+            }
+            __syncthreads();
+        }
+    }
 }
 
 template <typename T>
@@ -757,12 +831,14 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
     BSmemTail *tail = reinterpret_cast<BSmemTail *>(smem_aligned + w_off + nstages * kPStageWBytes);
     volatile uint32_t *abort_flag = &tail->abort_flag;
 
-    const auto plain = [&](int64_t n, int m) { return b_plain<T>(p, t, n, m); };
-
     const int warp = warp_id_uniform();
     const int lane = threadIdx.x & 31;
     const int cta = static_cast<int>(blockIdx.x);
     const int u_begin = p_first_item<false>(p, cta), u_end = p_first_item<false>(p, cta + 1);
+    const auto report = [&](int q, uint32_t rows) {
+        atomicOr(&tail->bad_rows, rows);
+        atomicOr(&tail->bad_tiles, 1u << min(q - u_begin / p.nchunks, 31));
+    };
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < nstages; ++s) {
@@ -783,6 +859,7 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
         }
         tail->abort_flag = 0;
         tail->epi_abort[0] = tail->epi_abort[1] = 0;
+        tail->bad_rows = tail->bad_tiles = 0;
         mbar_fence_init();
         tma_prefetch_desc(&tmap_x);
     }
@@ -1045,17 +1122,14 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
                         again |= !isfinite(output(j)) ? 1u << j : 0u;
                         out[static_cast<int64_t>(j) * p.ld_out + n] = from_float<T>(output(j) + b);
                     }
-                    for (; again != 0; again &= again - 1) {
-                        const int j = __ffs(static_cast<int>(again)) - 1;
-                        out[static_cast<int64_t>(j) * p.ld_out + n] = from_float<T>(b_plain<T>(p, t, n, j) + b);
-                    }
+                    if (again != 0) report(q, again);
                 }
             } else {
                 float *mine = p.slots + p_slot<false>(p, cta, q) * (static_cast<int64_t>(p.mpad) * kPTileN) + row;
 #pragma unroll
                 for (int j = 0; j < kBTok; ++j)
                     if (j < M) __stcg(mine + j * kPTileN, output(j));
-                if (seg_end < u_end) p_finish_shared<T, false, true>(p, q, abort_flag, &tail->is_last, plain);
+                if (seg_end < u_end) p_finish_shared<T, false, true>(p, q, abort_flag, &tail->is_last, [&](int j) { report(q, 1u << j); });
             }
             u = seg_end;
         }
@@ -1069,7 +1143,12 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
         tc_fence_after();
         tmem_dealloc(tmem_base, kPTmemCols);
     }
-    if (u_begin < u_end) p_finish_shared<T, false, false>(p, (u_end - 1) / p.nchunks, abort_flag, &tail->is_last, plain);
+    if (u_begin < u_end) {
+        const int q1 = (u_end - 1) / p.nchunks;
+        p_finish_shared<T, false, false>(p, q1, abort_flag, &tail->is_last, [&](int j) { report(q1, 1u << j); });
+        const uint32_t rows = *static_cast<volatile uint32_t *>(&tail->bad_rows), tiles = *static_cast<volatile uint32_t *>(&tail->bad_tiles);
+        if (rows != 0 && *abort_flag == 0) b_plain_tiles<T>(p, t, rows, tiles, u_begin / p.nchunks, q1, reinterpret_cast<float *>(smem_aligned));
+    }
 }
 
 // ---- layout pass and its inverse ----------------------------------------------------------------------

@@ -381,3 +381,51 @@ def test_few_tokens_sums_beyond_fp32(capi, oracle, dev, shape):
     assert torch.equal(y[others], y_clean[others])
     error = np.abs(y[1].double().numpy() - y_ref[1])
     assert np.all(error <= 2.0 ** -8 * np.abs(y_ref[1]) + K * 2.0 ** -23 * sums[1])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("shape", [(8, 512, 136), (8, 4096, 4096)])
+def test_few_tokens_not_finite_rows_and_bias(capi, oracle, dev, shape, dtype):
+    """Rows with activations or columns with a bias that is not finite: infinities, their signs and NaN as plain arithmetic has them,
+    everything else as without them, and in little more than the time of finite ones (twice, and 10 us)."""
+    M, K, N = shape
+    x, packed_w, scale, offset = oracle.make_w4a16_inputs(M, K, N, seed=K + N, group=128, dtype=dtype)
+    w = torch.from_numpy(np.asarray(oracle.antiquant_weight(packed_w, scale, offset, 128), dtype=np.float64))
+    sd, od = scale.to(dev), offset.to(dev)
+    buf = capi.w4a16_prepack(packed_w.to(dev), sd, od, group_size=128)
+
+    def call(xd, b):
+        return capi.weight_quant_batchmatmul_prepacked(xd, buf, N, bias=b, tables=(sd, od, 128))
+
+    def us(xd, b):
+        call(xd, b)
+        best = float("inf")
+        for _ in range(7):
+            s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda._sleep(4_000_000)
+            s.record()
+            for _ in range(20):
+                call(xd, b)
+            e.record()
+            torch.cuda.synchronize()
+            best = min(best, s.elapsed_time(e) * 1e3 / 20)
+        return best
+
+    bias = torch.zeros(N, dtype=dtype)
+    bias[::2] = float("-inf")
+    bad = x.clone()
+    bad[0, K // 2 + 5] = float("nan")
+    bad[1, ::131] = float("inf")
+    bad[2, K - 1] = float("-inf")
+    bad[4, 0], bad[4, K - 1] = float("inf"), float("nan")
+    bad[6, :] = float("nan")
+    clean = call(x.to(dev), None)
+    for xs, b in ((bad, None), (x, bias), (bad, bias)):
+        xd, bd = xs.to(dev), None if b is None else b.to(dev)
+        y = call(xd, bd).cpu()
+        want = xs.double() @ w + (0 if b is None else b.double())
+        special = ~torch.isfinite(want)
+        assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isfinite(y), ~special)
+        assert torch.equal(torch.sign(y[torch.isinf(want)]).double(), torch.sign(want[torch.isinf(want)]))
+        assert torch.equal(y[~special], clean.cpu()[~special])
+        assert us(xd, bd) < 2 * us(x.to(dev), None if b is None else torch.zeros_like(bd)) + 10
