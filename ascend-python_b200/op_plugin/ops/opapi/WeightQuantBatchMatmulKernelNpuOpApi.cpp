@@ -266,13 +266,20 @@ at::Tensor npu_weight_quant_batchmatmul(const at::Tensor &x, const at::Tensor &w
     if (few && prepack_enabled() && few_rows_repack(xc, wc, sc, oc, group, N, K)) {
         size_t bytes = 0, ws_size = 0;
         EXEC_QMM_CMD(qmm_w4a16_prepack_size, N, K, group, &bytes);
+        EXEC_QMM_CMD(qmm_weight_quant_batchmatmul_prepacked_workspace_size, M, N, K, &ws_size);
+        at::Tensor packed, ws;
         if (bytes != 0) {
-            at::Tensor packed = op_plugin_utils::empty_output({static_cast<int64_t>(bytes)}, xc, at::kByte);
+            try {
+                ws = op_plugin_utils::qmm_workspace(xc, ws_size, /*family=*/2);
+                packed = op_plugin_utils::empty_output({static_cast<int64_t>(bytes)}, xc, at::kByte);
+            } catch (const c10::OutOfMemoryError &) {
+                // the kernel below needs neither
+            }
+        }
+        if (packed.defined()) {
             EXEC_QMM_CMD(qmm_w4a16_prepack, static_cast<const int32_t *>(wc.const_data_ptr()), N / 8, sc.const_data_ptr(),
                          op_plugin_utils::opt_ptr(oc), op_plugin_utils::qmm_dtype(sc.scalar_type()), group, N, K,
                          packed.data_ptr(), bytes, op_plugin_utils::current_stream(xc));
-            EXEC_QMM_CMD(qmm_weight_quant_batchmatmul_prepacked_workspace_size, M, N, K, &ws_size);
-            at::Tensor ws = op_plugin_utils::qmm_workspace(xc, ws_size, /*family=*/2);
             EXEC_QMM_CMD(qmm_weight_quant_batchmatmul_prepacked_tables, xc.const_data_ptr(),
                          op_plugin_utils::qmm_dtype(xc.scalar_type()), K, packed.const_data_ptr(), bytes, sc.const_data_ptr(),
                          op_plugin_utils::opt_ptr(oc), group, op_plugin_utils::opt_ptr(bc), result.data_ptr(), N, M, N, K,

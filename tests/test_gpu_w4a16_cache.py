@@ -79,3 +79,26 @@ def test_what_a_capture_packs_serves_that_capture(npu, oracle, dev, M):
         torch.cuda.synchronize()
         assert torch.equal(a, want) and torch.equal(b, want)
         assert torch.equal(call(), want)
+
+
+def test_few_rows_without_memory_for_the_packing(npu, oracle, dev):
+    """Three to eight rows pack the weight for the call; where there is no memory for that, the call needs none of it."""
+    M, K, N = 5, 28672, 768
+    x, w, s, o = oracle.make_w4a16_inputs(M, K, N, seed=11, group=K)
+    y_ref = oracle.weight_quant_batchmatmul(x, w, s, o, antiquant_group_size=K)
+    rms = ((y_ref ** 2).mean(axis=1, keepdims=True)) ** 0.5
+    xd, wd, sd, od = (t.to(dev) for t in (x, w, s, o))
+    odd = torch.empty(M * K + 1, dtype=x.dtype, device=dev)[1:].view(M, K)
+    odd.copy_(xd)
+    npu.npu_weight_quant_batchmatmul(odd, wd, sd, od, antiquant_group_size=K)  # the scratch of the stock layout's kernels
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(dev).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved(dev) + (6 << 20)) / total, dev)
+        with pytest.raises(torch.OutOfMemoryError):
+            torch.empty(K * N // 2, dtype=torch.uint8, device=dev)
+        y = npu.npu_weight_quant_batchmatmul(xd, wd, sd, od, antiquant_group_size=K).double().cpu().numpy()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, dev)
+    assert (abs(y - y_ref) <= 2.0 ** -8 * abs(y_ref) + 2.0 ** -7 * rms).all()
