@@ -120,3 +120,29 @@ def test_tiles_that_end_inside_a_chunk(capi, dev, N):
             got = capi.quant_matmul(a, w, sc, pertoken_scale=p, bias=b, output_dtype=dtype, algo=algo)
             assert torch.equal(got, capi.quant_matmul(a, w, sc, pertoken_scale=p, bias=b, output_dtype=dtype, algo=capi.ALGO_SIMT))
     assert capi.device_status() == 0
+
+
+# More columns than the cluster kernel takes (148 x 256), so that the kernels which share the epilogue serve the call: stream-K
+# (up to 16 rows), the one-CTA tile kernel (up to 128) and the CTA-pair kernel.  Ragged rows, one and several k blocks, columns that
+# end 16, 112 and 128 into a tile, and (weight stored [N, K]) at odd ones, where output rows start at odd addresses.
+@pytest.mark.parametrize("N,trans", [(37904, False), (38000, False), (38016, True), (37891, True)])
+@pytest.mark.parametrize("M,K", [(1, 272), (16, 1040), (70, 272), (128, 128), (129, 272), (300, 400)])
+def test_int8_output_of_the_kernels_beside_the_cluster_kernel(capi, dev, M, K, N, trans):
+    """clamp(rint(float(acc + bias) * scale[n] * pertoken[m] + offset[n])), each operation rounded to fp32, over the exact sums of
+    the dp4a kernel; with and without bias, offset and per-token scale."""
+    g = torch.Generator(device=dev).manual_seed(M + K + N)
+    a = torch.randint(-128, 128, (M, K), generator=g, device=dev, dtype=torch.int8)
+    w = torch.randint(-128, 128, (N, K) if trans else (K, N), generator=g, device=dev, dtype=torch.int8)
+    w = w.t() if trans else w
+    acc = capi.quant_matmul(a, w, None, output_dtype=torch.int32, algo=capi.ALGO_SIMT)
+    pt = torch.rand(M, generator=g, device=dev) + 0.5
+    scale = (torch.rand(N, generator=g, device=dev) + 0.5) * (40.0 / (5400.0 * K ** 0.5))
+    offset = torch.linspace(-30, 30, N, device=dev)
+    bias = torch.randint(-4096, 4096, (N,), generator=g, device=dev, dtype=torch.int32)
+    for p, o, b in ((pt, offset, bias), (None, None, None), (pt, None, bias), (None, offset, None)):
+        want = (acc if b is None else acc + b).float() * scale
+        want = want if p is None else want * p[:, None]
+        want = want if o is None else want + o
+        got = capi.quant_matmul_int8(a, w, scale, offset=o, pertoken_scale=p, bias=b)
+        assert torch.equal(got, want.round().clamp(-128, 127).to(torch.int8))
+    assert capi.device_status() == 0
