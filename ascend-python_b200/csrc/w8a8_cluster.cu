@@ -344,6 +344,13 @@ struct ClusterPlan {
     uint32_t tmem_cols = 32;
 };
 
+// Stages of the operand ring.  Two CTAs of an SM never want more tensor memory (T <= 256 columns each) or shared memory than it
+// has; three do not fit.
+int cluster_stages(int stage_bytes, bool two) {
+    const int budget = (two ? kCMaxSmem / 2 : kCMaxSmem) - static_cast<int>(sizeof(ClusterSmemTail));
+    return std::min(kCMaxStages, budget / stage_bytes);
+}
+
 // Token height and number of K slices by a model of the time (ns, fitted to about 190 shapes of 1 .. 2048 tokens, K and N of
 // 1024 .. 28672, every T and S each; its choice takes 0.5 % more than the best one on average, 10 % at most):
 //   a k block of a CTA takes what its loads take at 105 B/ns or what its MMAs take, 1.4 ns a token;
@@ -371,6 +378,9 @@ bool cluster_make_plan(int64_t M, int64_t N, int64_t K, ClusterPlan *out) {
             const int64_t clusters = static_cast<int64_t>(tiles_n) * tiles;
             if (clusters > 2 * resident) continue;
             const bool twice = clusters > resident;
+            // the ring receives the other slices' sums (256 tokens over four slices with two CTAs an SM fill all of it)
+            const int stage_bytes = kCWBytes + T / 2 * kCBK;
+            if ((slices - 1) * (T / slices) * (kCUnitN / 2) * 4 > cluster_stages(stage_bytes, twice) * stage_bytes) continue;
             const int blocks = (num_kb + slices - 1) / slices;
             const float loop = blocks * block * (twice ? 2 : 1), l2 = clusters * 2.0f * slices * blocks * bytes / 14000.0f;
             const float exchange = slices == 1 ? 0.0f : (slices == 2 ? 1200.0f : 2400.0f) + 12.0f * T;
@@ -386,9 +396,7 @@ bool cluster_make_plan(int64_t M, int64_t N, int64_t K, ClusterPlan *out) {
     }
     if (out->T == 0) return false;
     out->stage_bytes = kCWBytes + out->T / 2 * kCBK;
-    // two CTAs of an SM never want more tensor memory (T <= 256 columns each) or shared memory than it has; three do not fit
-    const int budget = (two ? kCMaxSmem / 2 : kCMaxSmem) - static_cast<int>(sizeof(ClusterSmemTail));
-    out->stages = std::min(kCMaxStages, budget / out->stage_bytes);
+    out->stages = cluster_stages(out->stage_bytes, two);
     out->smem = static_cast<size_t>(out->stages) * out->stage_bytes + sizeof(ClusterSmemTail);
     while (out->tmem_cols < static_cast<uint32_t>(out->T)) out->tmem_cols *= 2;
     return true;

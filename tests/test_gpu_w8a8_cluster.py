@@ -70,3 +70,28 @@ def test_shapes_beyond_one_wave_are_refused(capi, dev):
         capi.quant_matmul(a, w, None, output_dtype=torch.int32, algo=capi.ALGO_CLUSTER)
     got = capi.quant_matmul(a, w, None, output_dtype=torch.int32)
     assert torch.equal(got, capi.quant_matmul(a, w, None, output_dtype=torch.int32, algo=capi.ALGO_SIMT))
+
+
+# What the plan makes of these on 148 SMs, token height / slices: 64 / 4, 64 / 2, 96 / 4 (three groups of tokens an owner), 96 / 2, 128 / 4,
+# 128 / 2, 160 / 4, 160 / 2, 192 / 4, 192 / 2, 224 / 4, 256 / 2, and 256 / 4, whose received sums fill the operand ring
+SLICED = [(250, 6144, 272), (100, 4096, 2064), (500, 8192, 272), (250, 4096, 2064), (100, 8192, 2064), (300, 6144, 2064),
+          (130, 12288, 2000), (300, 6144, 4096), (500, 8192, 1040), (500, 8192, 2064), (200, 12288, 2064), (500, 12288, 4096),
+          (250, 28672, 2064)]
+
+
+@pytest.mark.parametrize("shape", SLICED)
+def test_high_tiles_of_several_slices(capi, dev, shape):
+    """The exchange of sums with several groups of tokens an owner, all four output types."""
+    M, K, N = shape
+    a, w, scale, pt, bias = _inputs(dev, M, K, N, M + K + N, M % 20 == 0)
+    acc = capi.quant_matmul(a, w, None, output_dtype=torch.int32, algo=capi.ALGO_SIMT)
+    assert torch.equal(capi.quant_matmul(a, w, None, output_dtype=torch.int32, algo=capi.ALGO_CLUSTER), acc)
+    for dtype, p, b in ((torch.bfloat16, pt, bias.bfloat16()), (torch.float16, pt, None)):
+        got = capi.quant_matmul(a, w, scale, pertoken_scale=p, bias=b, output_dtype=dtype, algo=capi.ALGO_CLUSTER)
+        assert torch.equal(got, capi.quant_matmul(a, w, scale, pertoken_scale=p, bias=b, output_dtype=dtype, algo=capi.ALGO_SIMT))
+    s8, off = scale * (8000.0 / (5400.0 * K ** 0.5)), torch.linspace(-20, 20, N, device=dev)
+    ib = torch.arange(N, device=dev, dtype=torch.int32) - 7
+    got = capi.quant_matmul_int8(a, w, s8, offset=off, pertoken_scale=pt * 10, bias=ib)
+    want = (acc + ib).float() * s8 * (pt * 10)[:, None] + off
+    assert torch.equal(got, want.round().clamp(-128, 127).to(torch.int8))
+    assert capi.device_status() == 0
