@@ -588,7 +588,7 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
         else if (ep.M > 16 && ep.M <= 128 && workspace != nullptr && splitk_scratch_bytes(ep.M, ep.N, K) > 0 &&
                  workspace_bytes >= splitk_scratch_bytes(ep.M, ep.N, K) &&
                  (reinterpret_cast<uintptr_t>(workspace) & 15) == 0)
-            algo = QMM_ALGO_TCGEN05_SPLITK;  // few tiles, long K: the slices fill the SMs
+            algo = QMM_ALGO_TCGEN05_SPLITK;  // beside a collective: few tiles, long K, the slices fill the SMs
         else if (streamk_supported(ep.M, ep.N, K, x2_sn) && workspace != nullptr &&
                  workspace_bytes >= streamk_workspace_bytes(ep.M, ep.N, K) && prefer_streamk(ep.M, ep.N))
             algo = QMM_ALGO_TCGEN05_STREAMK;
@@ -627,8 +627,8 @@ int quant_matmul_dispatch(const int8_t *x1, int64_t ld_x1, const int8_t *x2, int
                     return launch_tile_splitk<__nv_bfloat16>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, overlap, stream);
                 case QMM_DTYPE_F16:
                     return launch_tile_splitk<__half>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, overlap, stream);
-                case kOutI8:
-                    return launch_tile_splitk<int8_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, overlap, stream);
+                case kOutI8:  // has no launch options and no choice of kernel: the cluster kernel takes what could be split
+                    return fail(QMM_ERR_UNSUPPORTED, "qmm_quant_matmul: split-K has no int8 output");
                 default:
                     return launch_tile_splitk<int32_t>(x1, ld_x1, x2, x2_sk, x2_sn, ep, K, workspace, sm_reserve, overlap, stream);
             }
