@@ -12,11 +12,11 @@
 // with one tile a CTA nothing else hides those loads (the tile kernel fetches them for every 64 columns, between two loads
 // from tensor memory).
 //
-// What bounds it and what it measured (us, M x K x N, bf16, repeated calls; before: the better of the tile, split-K, stream-K and
-// CTA-pair kernels as they were chosen).  Small: launch, first data and the hand-offs, 4 us: 128 x 1024 x 1024 9.3 -> 4.2,
-// 64 x 1024 x 8192 42.4 -> 4.6, 1 x 4096 x 4096 11.3 -> 6.0.  Decode: HBM: 1 x 8192 x 28672 46.1 -> 38.8 (35.9 at the copy
-// rate), 32 x 28672 x 8192 43.8 -> 36.7 (36.1).  A prompt of some hundred tokens: shared memory's fill from L2, about 105 B/ns
-// an SM, then the MMA rate: 333 x 4096 x 6144 20.4 -> 10.9, 512 x 14336 x 4096 42.4 -> 24.1, 2048 x 14336 x 4096 83 -> 80.
+// What bounds it and what it measured (us, M x K x N, bf16, the kernel replayed in a CUDA graph, operands rotated past L2; this / the best
+// of the tile, split-K, stream-K and CTA-pair kernels; a call through the operator takes up to 1 us more).  Small: launch, first data and the
+// hand-offs: 128 x 1024 x 1024 3.9 / 7.5, 64 x 1024 x 8192 4.7 / 7.8 (stream-K, which used to take it, 38.7), 1 x 4096 x 4096 7.2 / 12.1.
+// Decode: HBM: 1 x 8192 x 28672 39.2 / 46.2 (36.4 at the copy rate), 32 x 28672 x 8192 38.9 / 46.1 (36.6).  A prompt of some hundred tokens:
+// shared memory's fill from L2, about 105 B/ns an SM, then the MMA rate: 333 x 4096 x 6144 11.3 / 16.5, 512 x 14336 x 4096 25.9 / 38.3.
 //
 // Synchronisation of a pair (s = stage): full[s] on the pair's leader counts the bytes of both CTAs' loads; empty[s] and done,
 // one per CTA, are arrived on by the leader's tcgen05.commit.  Cluster barriers separate the end of all main loops (the
@@ -461,11 +461,11 @@ bool prefer_cluster(int64_t M, int64_t N, int64_t K) {
     if (M <= 8 && N <= 4 * kCUnitN && num_kb > 176) return false;
     // tiles of 256 x 256 either way: the persistent kernel computes one while it stores the one before (us, here / there:
     // 512 x 4096 x 14336 29.0 / 26.9, 2048 x 4096 x 4096 28.6 / 26.7, 1024 x 1024 x 4096 9.9 / 9.4, 2048 x 14336 x 4096 77.9 / 77.2;
-    // 640 x 4096 x 8192, three lower tiles here, 19.8 / 25.9)
+    // 640 x 4096 x 8192, three lower tiles here, 19.8 / 25.9).  Lower tiles stay here, also those with two an SM on some SMs and one on
+    // others.  Time here over there, least, median and most of 75 to 148 clusters of one slice, K of 1024 to 28672, 16-bit and int32
+    // outputs, both weight layouts: 160 tokens a tile 0.64 0.82 1.00, 192 0.72 0.92 1.03, 224 0.80 0.94 1.10 (about even with 16-bit outputs
+    // for K up to 3072, and for a long K where a row of the operands is no multiple of 128 bytes).
     if (M > 128 && pl.T == kCMaxT && pl.slices == 1) return false;
-    // some SMs with two high tiles, others with one, over a long K (145 x 22544 x 25264 int32 172 us with the CTA-pair kernel,
-    // 176 here; 192 x 14336 x 25264 97 / 76)
-    if (pl.T > 128 && num_kb > 160 && pl.slices == 1 && pl.clusters > sm_count() / 2 && pl.clusters < sm_count() * 4 / 5) return false;
     return true;
 }
 

@@ -95,3 +95,27 @@ def test_high_tiles_of_several_slices(capi, dev, shape):
     want = (acc + ib).float() * s8 * (pt * 10)[:, None] + off
     assert torch.equal(got, want.round().clamp(-128, 127).to(torch.int8))
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(145, 20608, 19440), (300, 24576, 14064)])
+def test_time_of_lower_tiles_over_a_long_k(capi, dev, shape):
+    """Tiles of 160 tokens, two on some SMs and one on others, K of more than 160 blocks: the kernel that is chosen is the faster one of
+    the cluster and CTA-pair kernels (0.65 to 0.72 of the other's time), with a tenth for noise."""
+    M, K, N = shape
+    a, w, scale, pt, _ = _inputs(dev, M, K, N, 1, True)
+
+    def us(algo):
+        best = float("inf")
+        for _ in range(7):
+            s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            capi.quant_matmul(a, w, scale, pertoken_scale=pt, output_dtype=torch.bfloat16, algo=algo)
+            s.record()
+            for _ in range(5):
+                capi.quant_matmul(a, w, scale, pertoken_scale=pt, output_dtype=torch.bfloat16, algo=algo)
+            e.record()
+            torch.cuda.synchronize()
+            best = min(best, s.elapsed_time(e) * 1e3 / 5)
+        return best
+
+    chosen, cluster, pair = (us(algo) for algo in (capi.ALGO_AUTO, capi.ALGO_CLUSTER, capi.ALGO_PAIR))
+    assert chosen < 1.1 * min(cluster, pair), f"chosen {chosen:.1f} us, cluster {cluster:.1f}, pair {pair:.1f}"
