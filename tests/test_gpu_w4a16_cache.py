@@ -96,8 +96,10 @@ def test_few_rows_without_memory_for_the_packing(npu, oracle, dev):
     total = torch.cuda.get_device_properties(dev).total_memory
     try:
         torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved(dev) + (6 << 20)) / total, dev)
-        with pytest.raises(torch.OutOfMemoryError):
-            torch.empty(K * N // 2, dtype=torch.uint8, device=dev)
+        held = []
+        with pytest.raises(torch.OutOfMemoryError):  # what is left, of the allocator's blocks as well
+            while True:
+                held.append(torch.empty(K * N // 2, dtype=torch.uint8, device=dev))
         y = npu.npu_weight_quant_batchmatmul(xd, wd, sd, od, antiquant_group_size=K).double().cpu().numpy()
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0, dev)
