@@ -183,7 +183,7 @@ w4a16_gemv_tile_kernel(VParams p) {
             }
         }
     } else {
-        // six loads under way at a time: 1 x 8192 x 28672 has six a warp
+        // six loads under way at a time (1 x 7680 x 19200, whose tiles are one slice each, has five a warp)
         for (int i0 = warp; i0 < nb * M; i0 += 6 * kVWarps) {
             uint2 raw[6];
 #pragma unroll

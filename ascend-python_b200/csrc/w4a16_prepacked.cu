@@ -581,7 +581,7 @@ w4a16_prepacked_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p) {
             if (whole) {
                 // The next 16 tokens' sums are under way while these are stored, and the accumulator is free once the last are in
                 // registers: with one accumulator the tensor pipe waits for this loop.  Loading and storing in turn, 1000 x 4096 x
-                // 28672 took 191-195 us and 1000 x 1024 x 28672 97; now 178-180 and 60-80.
+                // 28672 took 191-195 us and 1000 x 1024 x 28672 97; now 174 and 59 at the full clock (201 and 65 under the power cap).
                 auto store = [&](const uint32_t(&v)[16], int c0) {
                     if (!n_ok) return;
                     T *at = o + static_cast<int64_t>(c0) * p.ld_out;
@@ -1308,7 +1308,10 @@ PPlan p_make_plan(int64_t M, int64_t N, int64_t K) {
         // its slots one after the other: with few tiles that costs more than unpacking the weight again for lower row tiles
         // does (256 x 8192 x 1024: one row tile 42.0 us, four 14.9; 321 x 3584 x 1096: 18.8 / 11.7).  With many, as few row
         // tiles as the accumulator allows (1000 x 4096 x 28672: 201 us with four, 205 .. 226 with five to eight); a plan with
-        // more has to be 6 % ahead.
+        // more has to be 6 % ahead.  The fit and these figures are older than the epilogue that loads one step ahead, which leaves
+        // tensor memory in about half the time: where tiles are high and K is short the model is now above the measured
+        // time (us, model / measured at the full clock: 1000 x 1024 x 28672 139 / 59, 1000 x 4096 x 28672 236 / 174,
+        // 2048 x 4096 x 11008 184 / 140, 512 x 1024 x 8192 21 / 15).  With 30 for the 61, 6 % of the plans would differ; not measured.
         // A height of a multiple of 16 gives a number of row tiles, so there are sixteen candidates at most, whatever M is (a
         // search over the numbers took the host 31 us for 65536 rows, on each of a call's three visits here; 0.3 so).
         const int64_t fewest = (M + kPMaxWide - 1) / kPMaxWide;
@@ -1336,7 +1339,8 @@ PPlan p_make_plan(int64_t M, int64_t N, int64_t K) {
         pl.nxstages = static_cast<int>((kPSmemBudgetWide - 2048 - kPWideStages * kPStageWBytes) / (static_cast<size_t>(pl.mpad) * 128));
         if (pl.nxstages > kPMaxXStages) pl.nxstages = kPMaxXStages;
         pl.smem = 2048 + static_cast<size_t>(pl.nxstages) * pl.mpad * 128 + static_cast<size_t>(pl.nstages) * kPStageWBytes;
-        // more than half of an SM's: no other kernel that uses tensor memory fits beside a CTA, which holds all of it
+        // more than half of an SM's: the next call's CTA is not placed beside this one, which holds all of the tensor memory (one of
+        // the W8A8 cluster kernel with two an SM is, and waits for it)
         if (pl.smem < 120 * 1024) pl.smem = 120 * 1024;
     }
     const int64_t out_tiles = static_cast<int64_t>(pl.tiles_n) * pl.nblk;

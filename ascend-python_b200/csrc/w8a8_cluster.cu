@@ -463,7 +463,7 @@ bool prefer_cluster(int64_t M, int64_t N, int64_t K) {
     // 512 x 4096 x 14336 29.0 / 26.9, 2048 x 4096 x 4096 28.6 / 26.7, 1024 x 1024 x 4096 9.9 / 9.4, 2048 x 14336 x 4096 77.9 / 77.2;
     // 640 x 4096 x 8192, three lower tiles here, 19.8 / 25.9).  Lower tiles stay here, also those with two an SM on some SMs and one on
     // others.  Time here over there, least, median and most of 75 to 148 clusters of one slice, K of 1024 to 28672, 16-bit and int32
-    // outputs, both weight layouts: 160 tokens a tile 0.64 0.82 1.00, 192 0.72 0.92 1.03, 224 0.80 0.94 1.10 (about even with 16-bit outputs
+    // outputs, both weight layouts: 160 tokens a tile 0.64 0.83 1.00, 192 0.72 0.88 1.03, 224 0.80 0.94 1.10 (about even with 16-bit outputs
     // for K up to 3072, and for a long K where a row of the operands is no multiple of 128 bytes).
     if (M > 128 && pl.T == kCMaxT && pl.slices == 1) return false;
     return true;

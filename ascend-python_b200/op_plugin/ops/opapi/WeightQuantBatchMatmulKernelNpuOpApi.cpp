@@ -173,10 +173,10 @@ at::Tensor prepacked_weight(const at::Tensor &w, const at::Tensor &scale, const 
 // keep the weight unrounded.  The stock layout's kernel is short of parallel work unless the weight is large and has many
 // groups: it cuts K at groups only, and its last CTA of 512 columns adds a share of every CTA before it.  Its time (us, 3 rows; up
 // to 20 % more for 8) is close to 4 + 1.25 shares + 1.25 for every 128 k of a CTA, that of packing and the kernel over the
-// stream to 8 + 0.45 for every 2^20 weights; measured, stock / this: 1024 x 1024 14.3 / 7.7, 8192 x 1024 88 / 13, 4096 x 4096
-// 28.7 / 16.7, 5120 x 4608 28.6 / 17.7, 28672 x 768 in one group 269 / 19, 2048 x 12288 17.1 / 18.5, 8192 x 8192 26.8 / 37.
-// Stock rows that TMA cannot address leave only a CUDA-core kernel there (4480 x 4712 154 / 17.5, 128 x 72 32.3 / 6.6,
-// 8192 x 28680 533 / 113).  Small weights of addressable rows keep the stock kernel, and with it its bits (1024 x 512).
+// stream to 8 + 0.45 for every 2^20 weights; measured, stock / this: 1024 x 1024 14.6 / 8.3, 8192 x 1024 88 / 13.5, 4096 x 4096
+// 28.6 / 17.8, 5120 x 4608 27.4 / 18.9, 28672 x 768 in one group 269 / 20.5, 2048 x 12288 17.7 / 18.5, 8192 x 8192 25.8 / 37.
+// Stock rows that TMA cannot address leave only a CUDA-core kernel there (4480 x 4712 156 / 18.5, 128 x 72 32.9 / 5.5,
+// 8192 x 28680 530 / 116).  Small weights of addressable rows keep the stock kernel, and with it its bits (1024 x 512).
 bool few_rows_repack(const at::Tensor &x, const at::Tensor &w, const at::Tensor &scale, const at::Tensor &offset, int64_t group,
                      int64_t N, int64_t K)
 {

@@ -384,7 +384,7 @@ def test_few_tokens_sums_beyond_fp32(capi, oracle, dev, shape):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("shape", [(8, 512, 136), (8, 4096, 4096)])
+@pytest.mark.parametrize("shape", [(8, 512, 136), (8, 4096, 4096), (7, 256, 40008)])  # the last: several tiles a CTA
 def test_few_tokens_not_finite_rows_and_bias(capi, oracle, dev, shape, dtype):
     """Rows with activations or columns with a bias that is not finite: infinities, their signs and NaN as plain arithmetic has them,
     everything else as without them, and in little more than the time of finite ones (twice, and 10 us)."""
