@@ -731,8 +731,10 @@ __device__ __forceinline__ bool b_any_not_finite(const uint4 &x) {
     return any;
 }
 
-// Outputs whose sums are not finite, by the definition: rows (a bit each) of the tiles q0 + i of bit i (the last bit: and beyond),
-// as the CTA has stored them.  By the whole CTA, behind its work: in the epilogue this code costs the main loop registers
+// The bit of tile q of a CTA whose tiles are q0 .. q1: the last one, which another CTA may finish, has one of its own.
+__device__ __forceinline__ uint32_t b_tile_bit(int q, int q0, int q1) { return 1u << (q == q1 ? 31 : min(q - q0, 30)); }
+
+// Outputs whose sums are not finite, by the definition: rows (a bit each) of tiles (b_tile_bit), as the CTA has stored them.  By the whole CTA, behind its work: in the epilogue this code costs the main loop registers
 // (8 x 8192 x 8192: 19.0 us, 19.5 with a call there, 22.0 with a longer function), and a thread with all of K for itself is slow.  us, operator,
 // 8 x 4096 x 4096, finite 18: a NaN in every row 440 -> 23, an infinity in one 347 -> 20, 43 in every row 440 -> 70, sums of one row that leave
 // fp32 347 -> 41; 8 x 28672 x 768, finite 21: 2952 -> 36, 2308 -> 30, 2953 -> 94, 2309 -> 168.  A NaN among the activations is one among the sums already; infinite activations decide alone, so only their
@@ -754,7 +756,7 @@ __device__ __forceinline__ void b_plain_tiles(const PParams &p, const BTables &t
         if (__syncthreads_or(nan)) continue;
         const bool infinite = __syncthreads_or(inf);
         for (int q = q0; q <= q1; ++q) {
-            if ((tiles >> min(q - q0, 31) & 1) == 0) continue;
+            if ((tiles & b_tile_bit(q, q0, q1)) == 0) continue;
             const int64_t n = static_cast<int64_t>(q) * kPTileN + r;
             T *out = static_cast<T *>(p.out) + m * p.ld_out + n;
             unsigned short stored = 0;
@@ -837,7 +839,7 @@ w4a16_block_kernel(const __grid_constant__ CUtensorMap tmap_x, PParams p, BTable
     const int u_begin = p_first_item<false>(p, cta), u_end = p_first_item<false>(p, cta + 1);
     const auto report = [&](int q, uint32_t rows) {
         atomicOr(&tail->bad_rows, rows);
-        atomicOr(&tail->bad_tiles, 1u << min(q - u_begin / p.nchunks, 31));
+        atomicOr(&tail->bad_tiles, b_tile_bit(q, u_begin / p.nchunks, (u_end - 1) / p.nchunks));
     };
 
     if (threadIdx.x == 0) {

@@ -429,3 +429,27 @@ def test_few_tokens_not_finite_rows_and_bias(capi, oracle, dev, shape, dtype):
         assert torch.equal(torch.sign(y[torch.isinf(want)]).double(), torch.sign(want[torch.isinf(want)]))
         assert torch.equal(y[~special], clean.cpu()[~special])
         assert us(xd, bd) < 2 * us(x.to(dev), None if b is None else torch.zeros_like(bd)) + 10
+
+
+def test_few_tokens_not_finite_many_tiles_a_cta(capi, dev):
+    """More tiles a CTA than it notes one by one (33 of whole K): as calls over 148 tiles each, a tile a CTA, have it."""
+    M, K, part = 4, 256, 148 * 128
+    N = 33 * part - 40
+    g = torch.Generator(device=dev).manual_seed(9)
+    w = torch.randint(-2 ** 31, 2 ** 31 - 1, (K, N // 8), generator=g, device=dev, dtype=torch.int64).to(torch.int32)
+    scale = (torch.rand((K // 128, N), generator=g, device=dev) * 1e-2 + 1e-3).bfloat16()
+    x = torch.randn((M, K), generator=g, device=dev).bfloat16()
+    x[0, 5], x[1, 200], x[1, 3] = float("inf"), float("inf"), float("-inf")
+    x[2] = (x[2].float().clamp(-4, 4) * 2.0 ** 122).bfloat16()
+
+    def call(lo, hi):
+        s = scale[:, lo:hi].contiguous()
+        buf = capi.w4a16_prepack(w[:, lo // 8:hi // 8].contiguous(), s, None, group_size=128)
+        return capi.weight_quant_batchmatmul_prepacked(x, buf, hi - lo, tables=(s, None, 128))
+
+    whole, again = call(0, N), call(0, N)
+    parts = torch.cat([call(lo, min(lo + part, N)) for lo in range(0, N, part)], dim=1)
+    for y in (whole, again):
+        assert torch.equal(torch.isnan(y), torch.isnan(parts))
+        assert torch.equal(torch.nan_to_num(y), torch.nan_to_num(parts))
+    assert torch.isfinite(parts[2:]).all()
