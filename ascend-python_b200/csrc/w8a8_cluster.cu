@@ -378,20 +378,19 @@ bool cluster_make_plan(int64_t M, int64_t N, int64_t K, ClusterPlan *out) {
             const int64_t clusters = static_cast<int64_t>(tiles_n) * tiles;
             if (clusters > 2 * resident) continue;
             const bool twice = clusters > resident;
-            // the ring receives the other slices' sums (256 tokens over four slices with two CTAs an SM fill all of it)
-            const int stage_bytes = kCWBytes + T / 2 * kCBK;
-            if ((slices - 1) * (T / slices) * (kCUnitN / 2) * 4 > cluster_stages(stage_bytes, twice) * stage_bytes) continue;
             const int blocks = (num_kb + slices - 1) / slices;
             const float loop = blocks * block * (twice ? 2 : 1), l2 = clusters * 2.0f * slices * blocks * bytes / 14000.0f;
             const float exchange = slices == 1 ? 0.0f : (slices == 2 ? 1200.0f : 2400.0f) + 12.0f * T;
             const float cost = std::max(std::max(loop, l2), memory) + exchange + 4.0f * T / slices * (twice ? 2 : 1);
-            if (out->T == 0 || cost < best) {
-                best = cost;
-                two = twice;
-                out->T = T;
-                out->slices = slices;
-                out->clusters = clusters;
-            }
+            if (out->T != 0 && cost >= best) continue;
+            // the ring receives the other slices' sums (256 tokens over four slices with two CTAs an SM fill all of it)
+            const int stage_bytes = kCWBytes + T / 2 * kCBK;
+            if ((slices - 1) * (T / slices) * (kCUnitN / 2) * 4 > cluster_stages(stage_bytes, twice) * stage_bytes) continue;
+            best = cost;
+            two = twice;
+            out->T = T;
+            out->slices = slices;
+            out->clusters = clusters;
         }
     }
     if (out->T == 0) return false;
